@@ -190,3 +190,40 @@ def test_markov_step_matches_torch():
     tok = int(block[step + 1]) - vbase
     assert 0 <= tok < vlocal
     assert score[tok].item() >= score.max().item() - 1e-3
+
+
+@pytest.mark.parametrize("vlocal", [65, 1500, 37888, 37889, 76288, 152571])
+def test_markov_chain_equals_its_steps(vlocal):
+    """The one-launch forms (factor in registers up to 37,888 tokens, partly in shared memory beyond) draw what seven single
+    steps draw: logits and proposals bit for bit."""
+    K = _K()
+    g = torch.Generator(device="cuda").manual_seed(vlocal)
+    vocab, steps = vlocal + 100, 7
+    w1 = (torch.randn(vocab, 256, device="cuda", generator=g) * 0.3).bfloat16()
+    w2 = (torch.randn(vlocal, 256, device="cuda", generator=g) * 0.3).bfloat16()
+    logits = torch.randn(16, vlocal, device="cuda", generator=g) * 2
+    params = torch.tensor([1, 0.95, 1, 0, 0, -1, 1.25, 0], dtype=torch.float32, device="cuda")
+    seed = torch.tensor([99], dtype=torch.int64, device="cuda")
+    ctrl = torch.full((16,), 3, dtype=torch.int32, device="cuda")
+    sync = torch.zeros(2, dtype=torch.int64, device="cuda")
+    st, epoch = torch.zeros(4, dtype=torch.int32, device="cuda"), torch.ones(1, dtype=torch.int32, device="cuda")
+    got = []
+    for chain in (False, True, True):
+        zq, block = torch.zeros(8, vlocal, device="cuda"), torch.tensor([5] + [0] * 7, dtype=torch.int32, device="cuda")
+        best, ticket = torch.zeros(8, dtype=torch.int64, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        m = K.MarkovArgs()
+        m.logits, m.ld, m.w1, m.w2, m.rank_dim = logits.data_ptr(), vlocal, w1.data_ptr(), w2.data_ptr(), 256
+        m.vlocal, m.vbase, m.vocab = vlocal, 100, vocab
+        m.block_ids, m.zq, m.params, m.seed, m.ctrl = block.data_ptr(), zq.data_ptr(), params.data_ptr(), seed.data_ptr(), ctrl.data_ptr()
+        m.best, m.ticket = best.data_ptr(), ticket.data_ptr()
+        m.x.epoch, m.x.status, m.x.tp, m.x.rank, m.x.timeout_ns = epoch.data_ptr(), st.data_ptr(), 1, 0, 10 ** 9
+        if chain:
+            assert K.markov_chain(m, steps, sync, pdl=False) == 0
+        else:
+            for i in range(steps):
+                K.markov_step(m, i, pdl=False)
+        torch.cuda.synchronize()
+        assert int(st[0]) == 0 and not best.any()
+        got.append((zq, block))
+    for zq, block in got[1:]:
+        assert torch.equal(zq, got[0][0]) and torch.equal(block, got[0][1])
