@@ -270,70 +270,132 @@ int launch(const CUtensorMap& w, const CUtensorMap& w2, const CUtensorMap& x, co
 }
 
 // ------------------------------------------------------------------------------------ float form
-constexpr int kFT = 64, kFK = 16;             // 64 features x 64 rows per CTA, 4 x 4 per thread
+// T x T tiles (features x rows), a thread has T / 16 rows x 4 features; inner steps of 32 through four stages of asynchronous
+// copies, weights still bf16 in shared memory.  A product of a small model is a chain of a few steps on a few CTAs, so what counts
+// is that no step waits for memory and that tiles are small enough to occupy the SMs: the products of 301 rows of a width of 320 take
+// 7.3 us on average, 26 us with 64 x 64 tiles loaded element by element between two barriers.  Every output is one chain of fused multiply-adds in ascending k.
+constexpr int kFK = 32, kFStages = 4;
 
-template <int EPI>
-__global__ void __launch_bounds__(256) stack_gemm_f32_kernel(const StackGemmArgs p, const int row_tiles) {
+__device__ __forceinline__ void copy16(void* dst, const void* src, int bytes) {     // the rest of the 16 bytes becomes zero
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+
+template <int T, bool DUAL>
+struct F32Stage {
+  float x[T][kFK + 4];                        // odd strides in 16-byte words: rows fall into different banks
+  __nv_bfloat16 w[DUAL ? 2 : 1][T][kFK + 8];
+};
+
+template <int T, int EPI>
+__global__ void __launch_bounds__(T * 4) stack_gemm_f32_kernel(const StackGemmArgs p, const int row_tiles) {
   constexpr bool DUAL = EPI == kSEpiClampedGlu || EPI == kSEpiSiluGlu;
-  __shared__ float sw[kFK][kFT + 4], sw2[DUAL ? kFK : 1][kFT + 4], sx[kFK][kFT + 4];
+  constexpr int THREADS = T * 4, TX = T / 4, RT = T / 16;                // threads over features, rows per thread
+  extern __shared__ __align__(16) uint8_t f32_smem[];
+  using Stage = F32Stage<T, DUAL>;
+  Stage* stages = reinterpret_cast<Stage*>(f32_smem);
   griddep_wait();
   griddep_launch();
   Item it;
   int row_lim;
   if (p.n_items) {
-    // a segment may be taller than a tile: segments are cut into 64-row pieces
-    const int per = (p.item_rows + kFT - 1) / kFT;
+    // a segment may be taller than a tile: segments are cut into pieces of T rows
+    const int per = (p.item_rows + T - 1) / T;
     const int item = blockIdx.y / per, part = blockIdx.y % per;
     it.live = item < min(*p.n_items, p.max_items);
     if (!it.live) return;
     it.z = p.item_z[item];
     row_lim = p.item_row[item] + p.item_rows;
-    it.row0 = p.item_row[item] + part * kFT;
+    it.row0 = p.item_row[item] + part * T;
   } else {
-    it = item_of(p, blockIdx.y, row_tiles, kFT, 0);
+    it = item_of(p, blockIdx.y, row_tiles, T, 0);
     row_lim = p.rows;
   }
-  const int n0 = blockIdx.x * kFT;
+  const int n0 = blockIdx.x * T;
   const float* X = reinterpret_cast<const float*>(p.act) + (p.n_items ? 0 : it.z * p.act_zstride);
-  const __nv_bfloat16* W = p.w + it.z * p.w_zstride;
-  const __nv_bfloat16* W2 = DUAL ? p.w2 + it.z * p.w_zstride : nullptr;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  float acc[4][4] = {}, acc2[4][4] = {};
-  for (int k0 = 0; k0 < p.k; k0 += kFK) {
-    for (int i = threadIdx.x; i < kFT * kFK; i += 256) {
-      const int r = i / kFK, k = i % kFK;
-      const bool kin = k0 + k < p.k;
-      sw[k][r] = kin && n0 + r < p.n ? bf(W + (long long)(n0 + r) * p.w_ld + k0 + k) : 0.f;
-      if (DUAL) sw2[k][r] = kin && n0 + r < p.n ? bf(W2 + (long long)(n0 + r) * p.w_ld + k0 + k) : 0.f;
-      sx[k][r] = kin && it.row0 + r < row_lim ? X[(long long)(it.row0 + r) * p.act_ld + k0 + k] : 0.f;
+  const __nv_bfloat16* W[2] = {p.w + it.z * p.w_zstride, DUAL ? p.w2 + it.z * p.w_zstride : nullptr};
+  const bool vec_x = (reinterpret_cast<uintptr_t>(X) & 15) == 0 && (p.act_ld & 3) == 0;
+  const bool vec_w = ((reinterpret_cast<uintptr_t>(W[0]) | (DUAL ? reinterpret_cast<uintptr_t>(W[1]) : 0)) & 15) == 0 && (p.w_ld & 7) == 0;
+  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
+  const int steps = (p.k + kFK - 1) / kFK;
+
+  auto load = [&](int step) {
+    Stage& st = stages[step % kFStages];
+    const int k0 = step * kFK;
+    if (vec_x) {
+#pragma unroll
+      for (int i = threadIdx.x; i < T * (kFK / 4); i += THREADS) {
+        const int r = i / (kFK / 4), k = i % (kFK / 4) * 4;
+        const int n = it.row0 + r < row_lim ? max(0, min(4, p.k - k0 - k)) : 0;
+        copy16(&st.x[r][k], n ? X + (long long)(it.row0 + r) * p.act_ld + k0 + k : X, n * 4);
+      }
+    } else {
+      for (int i = threadIdx.x; i < T * kFK; i += THREADS) {
+        const int r = i / kFK, k = i % kFK;
+        st.x[r][k] = it.row0 + r < row_lim && k0 + k < p.k ? X[(long long)(it.row0 + r) * p.act_ld + k0 + k] : 0.f;
+      }
     }
-    __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kFK; ++k) {
-      float xv[4], wv[4], w2v[4];
+    for (int d = 0; d < (DUAL ? 2 : 1); ++d) {
+      if (vec_w) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        xv[i] = sx[k][ty * 4 + i];
-        wv[i] = sw[k][tx + 16 * i];
-        w2v[i] = DUAL ? sw2[DUAL ? k : 0][tx + 16 * i] : 0.f;
+        for (int i = threadIdx.x; i < T * (kFK / 8); i += THREADS) {
+          const int r = i / (kFK / 8), k = i % (kFK / 8) * 8;
+          const int n = n0 + r < p.n ? max(0, min(8, p.k - k0 - k)) : 0;
+          copy16(&st.w[d][r][k], n ? W[d] + (long long)(n0 + r) * p.w_ld + k0 + k : W[d], n * 2);
+        }
+      } else {
+        for (int i = threadIdx.x; i < T * kFK; i += THREADS) {
+          const int r = i / kFK, k = i % kFK;
+          st.w[d][r][k] = n0 + r < p.n && k0 + k < p.k ? W[d][(long long)(n0 + r) * p.w_ld + k0 + k] : __float2bfloat16_rn(0.f);
+        }
+      }
+    }
+  };
+  float acc[RT][4] = {}, acc2[RT][4] = {};
+#pragma unroll 1
+  for (int i = 0; i < kFStages - 1; ++i) {
+    if (i < steps) load(i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+#pragma unroll 1
+  for (int i = 0; i < steps; ++i) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kFStages - 2) : "memory");
+    __syncthreads();                                                     // step i has landed; everybody is done with step i - 1
+    if (i + kFStages - 1 < steps) load(i + kFStages - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const Stage& st = stages[i % kFStages];
+#pragma unroll
+    for (int k = 0; k < kFK; k += 8) {
+      float xv[RT][8];
+#pragma unroll
+      for (int r = 0; r < RT; ++r) {
+        *reinterpret_cast<float4*>(&xv[r][0]) = *reinterpret_cast<const float4*>(&st.x[ty * RT + r][k]);
+        *reinterpret_cast<float4*>(&xv[r][4]) = *reinterpret_cast<const float4*>(&st.x[ty * RT + r][k + 4]);
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 4; ++j) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[i][j] = fmaf(xv[i], wv[j], acc[i][j]);
-          if (DUAL) acc2[i][j] = fmaf(xv[i], w2v[j], acc2[i][j]);
+        for (int d = 0; d < (DUAL ? 2 : 1); ++d) {
+          const uint4 w = *reinterpret_cast<const uint4*>(&st.w[d][tx + TX * j][k]);
+          const float wv[8] = {bf16_lo(w.x), bf16_hi(w.x), bf16_lo(w.y), bf16_hi(w.y), bf16_lo(w.z), bf16_hi(w.z), bf16_lo(w.w), bf16_hi(w.w)};
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+#pragma unroll
+            for (int r = 0; r < RT; ++r) {
+              if (d == 0) acc[r][j] = fmaf(xv[r][q], wv[q], acc[r][j]);
+              else acc2[r][j] = fmaf(xv[r][q], wv[q], acc2[r][j]);
+            }
         }
+      }
     }
-    __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int row = it.row0 + ty * 4 + i;
+  for (int i = 0; i < RT; ++i) {
+    const int row = it.row0 + ty * RT + i;
     if (row >= row_lim) continue;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx + 16 * j;
+      const int n = n0 + tx + TX * j;
       if (n >= p.n) continue;
       const float bias = epi_has_bias<EPI>() ? bf(p.bias + (size_t)it.z * p.n + n) : 0.f;
       const float rate = EPI == kSEpiDecaySoft ? p.rate[n] : 0.f;
@@ -343,12 +405,28 @@ __global__ void __launch_bounds__(256) stack_gemm_f32_kernel(const StackGemmArgs
   }
 }
 
+template <int T, int EPI>
+int launch_f32_tile(const StackGemmArgs& a, cudaStream_t stream) {
+  constexpr bool DUAL = EPI == kSEpiClampedGlu || EPI == kSEpiSiluGlu;
+  constexpr int smem = kFStages * (int)sizeof(F32Stage<T, DUAL>);
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(stack_gemm_f32_kernel<T, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  const int row_tiles = (a.rows + T - 1) / T;
+  const long long items = a.n_items ? (long long)a.max_items * ((a.item_rows + T - 1) / T) : (long long)a.zcount * row_tiles;
+  if (items < 1 || items > 65535) return -3;
+  return launch_pdl(stack_gemm_f32_kernel<T, EPI>, dim3((a.n + T - 1) / T, (unsigned)items), dim3(T * 4), smem, stream, false, a, row_tiles);
+}
+
+// Tiles of 32 until tiles of 64 fill the SMs twice: below that the longest CTA is the time of the launch.
 template <int EPI>
 int launch_f32(const StackGemmArgs& a, cudaStream_t stream) {
-  const int row_tiles = (a.rows + kFT - 1) / kFT;
-  const int items = a.n_items ? a.max_items * ((a.item_rows + kFT - 1) / kFT) : a.zcount * row_tiles;
-  if (items < 1 || items > 65535) return -3;
-  return launch_pdl(stack_gemm_f32_kernel<EPI>, dim3((a.n + kFT - 1) / kFT, items), dim3(256), 0, stream, false, a, row_tiles);
+  const long long rows = a.n_items ? (long long)a.max_items * a.item_rows : (long long)a.zcount * a.rows;
+  const long long big = ((a.n + 63) / 64) * ((rows + 63) / 64);
+  return big >= 2 * sm_count() || (rows + 31) / 32 > 32767 ? launch_f32_tile<64, EPI>(a, stream) : launch_f32_tile<32, EPI>(a, stream);
 }
 
 }  // namespace
