@@ -15,75 +15,177 @@ using namespace nrt;
 namespace {
 
 // ------------------------------------------------------------------------------------ chunk path, plain form
-// One warp per (row, head); keys 32 at a time.  Used by the float form; also carries state over key blocks.
-__global__ void __launch_bounds__(128) latent_attn_rows_kernel(const LatentAttnArgs a) {
-  __shared__ float sq[4][512];
+// Used by the float form and by heads wider than the tensor-core form takes; also carries state over key blocks.  A CTA has eight
+// rows of one head, two per warp; keys and values pass through shared memory in tiles of 32, read once per CTA and coalesced.
+// A lane scores one key of the tile and accumulates every 32nd channel of the values; each sum runs in ascending order.
+// A chunk of a small model is bound by the chain of tiles of its last rows: the next tile is copied while one is worked on (301 rows,
+// 6 heads of 48: 33 us; 258 us when every warp read the keys of its row from global memory, a line per lane).
+constexpr int kRowWarps = 4, kRowsWarp = 2, kRowTile = 32;
+
+__host__ __device__ inline int rows_ld(int dim) { return ((dim + 3) / 4 | 1) * 4; }      // an odd number of 16-byte words: no bank conflicts
+__host__ __device__ inline int rows_tile(int dim, int vdim) { return kRowTile * (rows_ld(dim) + (vdim + 3) / 4 * 4); }      // floats
+__host__ __device__ inline int rows_stages(int dim, int vdim) { return rows_tile(dim, vdim) <= 24 * 1024 ? 2 : 1; }
+__host__ __device__ inline int rows_smem(int dim, int vdim) {
+  return (rows_stages(dim, vdim) * rows_tile(dim, vdim) + kRowWarps * kRowsWarp * rows_ld(dim)) * 4;
+}
+// `bytes` of 4 or 16, both addresses multiples of it
+template <int BYTES>
+__device__ __forceinline__ void row_copy(void* dst, const void* src) {
+  if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+// rows [0, live) x `width` floats or bf16 values -> shared memory, rows `ld` floats apart; the other rows of the tile become zero
+__device__ __forceinline__ void row_tile(float* dst, int ld, const void* src, long long at, long long stride, int width, int live, int f32) {
+  if (f32) {
+    const float* s = reinterpret_cast<const float*>(src) + at;
+    if (((reinterpret_cast<uintptr_t>(s) & 15) | (stride & 3) | (width & 3)) == 0) {
+      const int w4 = width / 4;
+#pragma unroll 2
+      for (int i = threadIdx.x; i < live * w4; i += kRowWarps * 32) row_copy<16>(dst + i / w4 * ld + i % w4 * 4, s + i / w4 * stride + i % w4 * 4);
+    } else {
+      for (int i = threadIdx.x; i < live * width; i += kRowWarps * 32) row_copy<4>(dst + i / width * ld + i % width, s + i / width * stride + i % width);
+    }
+  } else {
+    const __nv_bfloat16* s = reinterpret_cast<const __nv_bfloat16*>(src) + at;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < live * width; i += kRowWarps * 32) dst[i / width * ld + i % width] = bf(s + i / width * stride + i % width);
+  }
+  for (int i = live * width + (int)threadIdx.x; i < kRowTile * width; i += kRowWarps * 32) dst[i / width * ld + i % width] = 0.f;
+}
+
+// NC: channels per lane
+template <int NC>
+__global__ void __launch_bounds__(kRowWarps * 32) latent_attn_rows_kernel(const LatentAttnArgs a) {
+  extern __shared__ __align__(16) float rows_mem[];
+  const int ld = rows_ld(a.dim);
+  float* sq = rows_mem;                                          // [8][ld]
+  float* tile0 = sq + kRowWarps * kRowsWarp * ld;                // stages of keys [32][ld] and values [32][vs]
+  const int vs = (a.vdim + 3) / 4 * 4, tile = rows_tile(a.dim, a.vdim), stages = rows_stages(a.dim, a.vdim);
   griddep_wait();
   griddep_launch();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int unit = blockIdx.x * 4 + warp;
-  if (unit >= a.rows * a.heads) return;
-  const int r = unit / a.heads, h = unit % a.heads;
-  const int pos = *a.pos0 + r;
-  const int n = min(a.kv_rows, pos + 1 - a.kv0);            // visible keys of this block: [first_key, n)
-  const int first_key = max(0, (a.window > 0 ? pos / a.window * a.window : 0) - a.kv0);
-  const int hk = h / a.group, kv_heads = a.heads / a.group;
+  // row groups of one head run side by side, those with the most keys first
+  const int h = blockIdx.y, row0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kRowWarps * kRowsWarp;
+  const int pos0 = *a.pos0, hk = h / a.group, kv_heads = a.heads / a.group;
   const long long kld = (long long)kv_heads * a.dim, vld = (long long)kv_heads * a.vdim;
-  for (int d = lane; d < a.dim; d += 32) sq[warp][d] = load_act(a.q, ((long long)r * a.heads + h) * a.dim + d, a.f32);
-  __syncwarp();
-  float o[16];
+  const int last = min(row0 + kRowWarps * kRowsWarp, a.rows) - 1;
+  auto low_of = [&](int r) { return max(0, (a.window > 0 ? (pos0 + r) / a.window * a.window : 0) - a.kv0); };
+  const int end = min(a.kv_rows, pos0 + last + 1 - a.kv0), begin = low_of(row0);      // keys that any row of the CTA sees
+  const int d4 = (a.dim + 3) / 4;
+  int n[kRowsWarp], low[kRowsWarp];                              // visible keys of a row: [low, n)
+  float o[kRowsWarp][NC], m[kRowsWarp], l[kRowsWarp];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) o[i] = 0.f;
-  float m = -FLT_MAX, l = 0.f;
-  float* st = a.state ? a.state + ((size_t)r * a.heads + h) * (a.vdim + 2) : nullptr;
-  if (!a.first) {
-    m = st[0];
-    l = st[1];
+  for (int i = 0; i < kRowsWarp; ++i) {
+    const int r = row0 + warp * kRowsWarp + i;
+    const bool live = r < a.rows;
+    n[i] = live ? min(a.kv_rows, pos0 + r + 1 - a.kv0) : 0;
+    low[i] = live ? low_of(r) : 0;
+    for (int d = lane; d < ld; d += 32)
+      sq[(warp * kRowsWarp + i) * ld + d] = live && d < a.dim ? load_act(a.q, ((long long)r * a.heads + h) * a.dim + d, a.f32) : 0.f;
+    m[i] = -FLT_MAX;
+    l[i] = 0.f;
 #pragma unroll
-    for (int i = 0; i < 16; ++i)
-      if (lane + 32 * i < a.vdim) o[i] = st[2 + lane + 32 * i];
+    for (int c = 0; c < NC; ++c) o[i][c] = 0.f;
+    if (!a.first && live) {
+      const float* st = a.state + ((size_t)r * a.heads + h) * (a.vdim + 2);
+      m[i] = st[0];
+      l[i] = st[1];
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+        if (lane + 32 * c < a.vdim) o[i][c] = st[2 + lane + 32 * c];
+    }
   }
-  for (int j0 = first_key; j0 < n; j0 += 32) {
+  auto request = [&](int j0, int stage) {
+    const int live = min(kRowTile, end - j0);
+    float* t = tile0 + stage * tile;
+    if (live > 0) {
+      row_tile(t, ld, a.k, j0 * kld + hk * a.dim, kld, a.dim, live, a.f32);
+      row_tile(t + kRowTile * ld, vs, a.v, j0 * vld + hk * a.vdim, vld, a.vdim, live, a.f32);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // the padding of a row of keys is read as well
+  for (int i = threadIdx.x; i < stages * kRowTile * (d4 * 4 - a.dim); i += kRowWarps * 32) {
+    const int w = d4 * 4 - a.dim, row = i / w;
+    tile0[row / kRowTile * tile + row % kRowTile * ld + a.dim + i % w] = 0.f;
+  }
+  const int first = begin / kRowTile * kRowTile;
+  if (stages == 2) request(first, 0);
+  for (int j0 = first, stage = 0; j0 < end; j0 += kRowTile) {
+    if (stages == 2) {
+      request(j0 + kRowTile, stage ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      request(j0, 0);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const float* sk = tile0 + stage * tile;
+    const float* sv = sk + kRowTile * ld;
     const int j = j0 + lane;
-    float s = -FLT_MAX;
-    if (j < n) {
-      s = 0.f;
-      const long long base = (long long)j * kld + hk * a.dim;
-      for (int d = 0; d < a.dim; ++d) s = fmaf(sq[warp][d], load_act(a.k, base + d, a.f32), s);
-      s *= a.scale;
+    float p[kRowsWarp], s[kRowsWarp];
+#pragma unroll
+    for (int i = 0; i < kRowsWarp; ++i) s[i] = 0.f;
+    const float4* kr = reinterpret_cast<const float4*>(sk + lane * ld);
+#pragma unroll 4
+    for (int d = 0; d < d4; ++d) {
+      const float4 k = kr[d];
+#pragma unroll
+      for (int i = 0; i < kRowsWarp; ++i) {
+        const float4 q = reinterpret_cast<const float4*>(sq + (warp * kRowsWarp + i) * ld)[d];
+        s[i] = fmaf(q.w, k.w, fmaf(q.z, k.z, fmaf(q.y, k.y, fmaf(q.x, k.x, s[i]))));
+      }
     }
-    float mt = s;
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, off));
-    const float mn = fmaxf(m, mt), corr = expf(m - mn);
-    const float p = j < n ? expf(s - mn) : 0.f;
-    l = l * corr + lane_sum(p);
-    m = mn;
+    for (int i = 0; i < kRowsWarp; ++i) {
+      const bool in = j >= low[i] && j < n[i];
+      s[i] = in ? s[i] * a.scale : -FLT_MAX;
+      float mt = s[i];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) o[i] *= corr;
-    const int live = min(32, n - j0);
-    for (int t = 0; t < live; ++t) {
-      const float pt = __shfl_sync(0xffffffffu, p, t);
-      const long long base = (long long)(j0 + t) * vld + hk * a.vdim;
+      for (int off = 16; off > 0; off >>= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, off));
+      const float mn = fmaxf(m[i], mt), corr = expf(m[i] - mn);
+      p[i] = in ? expf(s[i] - mn) : 0.f;
+      l[i] = l[i] * corr + lane_sum(p[i]);
+      m[i] = mn;
 #pragma unroll
-      for (int i = 0; i < 16; ++i)
-        if (lane + 32 * i < a.vdim) o[i] = fmaf(pt, load_act(a.v, base + lane + 32 * i, a.f32), o[i]);
+      for (int c = 0; c < NC; ++c) o[i][c] *= corr;
     }
-  }
-  if (!a.last) {
-    if (lane == 0) { st[0] = m; st[1] = l; }
+    const int used = min(kRowTile, end - j0);
+    int at[NC];                                                  // channels beyond the head's read (and drop) its first one
 #pragma unroll
-    for (int i = 0; i < 16; ++i)
-      if (lane + 32 * i < a.vdim) st[2 + lane + 32 * i] = o[i];
-    return;
-  }
-  const float inv = 1.0f / l;
+    for (int c = 0; c < NC; ++c) at[c] = lane + 32 * c < a.vdim ? lane + 32 * c : 0;
+#pragma unroll 8
+    for (int t = 0; t < used; ++t) {
+      float pt[kRowsWarp];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const int c = lane + 32 * i;
-    if (c < a.vdim) {
-      const float g = a.gate ? sigmoid_f(a.gate[(long long)r * a.gate_ld + h * a.vdim + c]) : 1.f;
-      store_act(a.out, ((long long)r * a.heads + h) * a.vdim + c, o[i] * inv * g, a.f32);
+      for (int i = 0; i < kRowsWarp; ++i) pt[i] = __shfl_sync(0xffffffffu, p[i], t);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const float v = sv[t * vs + at[c]];
+#pragma unroll
+        for (int i = 0; i < kRowsWarp; ++i) o[i][c] = fmaf(pt[i], v, o[i][c]);
+      }
+    }
+    __syncthreads();                                             // everybody is done with this tile
+    if (stages == 2) stage ^= 1;
+  }
+#pragma unroll
+  for (int i = 0; i < kRowsWarp; ++i) {
+    const int r = row0 + warp * kRowsWarp + i;
+    if (r >= a.rows) continue;
+    float* st = a.last ? nullptr : a.state + ((size_t)r * a.heads + h) * (a.vdim + 2);
+    if (st && lane == 0) { st[0] = m[i]; st[1] = l[i]; }
+    const float inv = 1.0f / l[i];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int at = lane + 32 * c;
+      if (at >= a.vdim) continue;
+      if (st) {
+        st[2 + at] = o[i][c];
+      } else {
+        const float g = a.gate ? sigmoid_f(a.gate[(long long)r * a.gate_ld + h * a.vdim + at]) : 1.f;
+        store_act(a.out, ((long long)r * a.heads + h) * a.vdim + at, o[i][c] * inv * g, a.f32);
+      }
     }
   }
 }
@@ -576,6 +678,19 @@ int launch_decode_tc(const LatentDecodeArgs& a, cudaStream_t stream, bool pdl) {
   return launch_pdl(latent_decode_tc_kernel<MT>, dim3((a.heads + MT * 16 - 1) / (MT * 16), a.splits), dim3(256), dec_smem(a.rank, MT), stream, pdl, a);
 }
 
+template <int NC>
+int launch_rows(const LatentAttnArgs& a, cudaStream_t stream) {
+  static bool configured = false;
+  if (!configured) {
+    // (the largest of the sizes on both sides of the change from two stages to one)
+    const cudaError_t e = cudaFuncSetAttribute(latent_attn_rows_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 24 * 1024 * 4 + 8 * rows_ld(512) * 4);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  const int per = kRowWarps * kRowsWarp;
+  return launch_pdl(latent_attn_rows_kernel<NC>, dim3((a.rows + per - 1) / per, a.heads), dim3(kRowWarps * 32), rows_smem(a.dim, a.vdim), stream, false, a);
+}
+
 }  // namespace
 
 extern "C" int nrt_latent_attn_args_size() { return (int)sizeof(LatentAttnArgs); }
@@ -585,7 +700,8 @@ extern "C" int nrt_latent_attn_rows(const void* args, void* stream) {
   LatentAttnArgs a;
   memcpy(&a, args, sizeof(a));
   if (a.rows < 1 || a.group < 1 || a.heads % a.group || a.window < 0 || a.dim > 512 || a.vdim > 512 || ((!a.first || !a.last) && !a.state)) return -3;
-  return launch_pdl(latent_attn_rows_kernel, dim3((a.rows * a.heads + 3) / 4), dim3(128), 0, reinterpret_cast<cudaStream_t>(stream), false, a);
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  return a.vdim <= 64 ? launch_rows<2>(a, s) : a.vdim <= 128 ? launch_rows<4>(a, s) : a.vdim <= 256 ? launch_rows<8>(a, s) : launch_rows<16>(a, s);
 }
 
 // bf16; a.dim and a.vdim multiples of 8 up to 256.  tmQ / tmK: (dim, heads, rows) boxes of 64 x 1 x 128 / 64; tmV: feature-major

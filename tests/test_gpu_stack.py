@@ -277,6 +277,66 @@ def test_slow_decay_keeps_the_first_token():
 
 
 # --------------------------------------------------------------------------- products
+@pytest.mark.parametrize("rows,n,k,z,off", [(1, 1, 1, 1, 0), (31, 33, 31, 1, 0), (32, 32, 32, 1, 1), (33, 64, 96, 1, 4), (65, 129, 97, 3, 2),
+                                            (700, 1700, 130, 1, 0), (2048, 640, 33, 1, 3)])
+def test_float_products_against_torch(rows, n, k, z, off):
+    """Both tile sizes of the float form, one and two matrices; activations on and off 16-byte boundaries.  A sum of k products in fp32 is
+    off by at most k 2^-24 of the sum of their magnitudes."""
+    from naivert_b200.ops import stack_kernels as S
+    from naivert_b200.runtime.packing import pack
+    cfg = CASES["mixed"]
+    eng = engine(cfg, weights(cfg), "fp32", capacity=64, chunk=64)
+    g = torch.Generator(device="cuda").manual_seed(rows + n)
+    try:
+        ld = z * k + (0 if off == 4 else off)
+        mem = torch.randn(off + rows * ld, generator=g, device="cuda")
+        x = mem[off:].view(rows, ld)[:, : z * k].reshape(rows, z, k)
+        w, w2 = (torch.randn(z, n, k, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+        a, b = (torch.einsum("rzk,znk->rzn", x.double(), m.double()) for m in (w, w2))
+        bound = [k * 2.0 ** -24 * torch.einsum("rzk,znk->rzn", x.double().abs(), m.double().abs()) + 1e-12 for m in (w, w2)]
+        p, p2 = pack(w, "cuda"), pack(w2, "cuda")
+        kw = dict(z=z, x_z=k, out_z=n, x_off=off)
+        out = torch.full((rows, z, n), float("nan"), device="cuda")
+        eng.prefill.gemm(S.EPI_STORE, p, mem, ld, rows, out, z * n, **kw)
+        assert ((out.double() - a).abs() <= bound[0]).all()
+        out.fill_(float("nan"))
+        eng.prefill.gemm(S.EPI_SILU_GLU, p, mem, ld, rows, out, z * n, w2=p2, **kw)
+        want = a * torch.sigmoid(a) * b
+        slack = 1.2 * (bound[0] * b.abs() + bound[1] * a.abs()) + 1e-5 * want.abs() + 1e-9       # |silu'| < 1.1; expf and a division
+        assert ((out.double() - want).abs() <= slack).all()
+    finally:
+        eng.close()
+
+
+@pytest.mark.parametrize("f32", [1, 0])
+@pytest.mark.parametrize("rows,heads,group,dim,vdim,pos0,window", [
+    (1, 2, 1, 4, 4, 0, 0), (8, 2, 2, 48, 40, 31, 0), (9, 3, 1, 7, 33, 24, 0), (33, 4, 2, 60, 65, 5, 16), (17, 2, 1, 130, 129, 70, 48), (5, 2, 1, 512, 510, 40, 0)])
+def test_plain_chunk_attention_against_torch(rows, heads, group, dim, vdim, pos0, window, f32):
+    """Head widths around the lanes' channels and the copies' 16 bytes, one and two stages, masks by chunk, two blocks of keys with the
+    state carried over; scores and sums of a few hundred terms in fp32."""
+    from naivert_b200.ops import stack_kernels as S
+    S.lib()
+    g = torch.Generator(device="cuda").manual_seed(rows * 7 + dim)
+    t, n, kv = torch.float32 if f32 else torch.bfloat16, pos0 + rows, heads // group
+    q, k, v = (torch.randn(*s, generator=g, device="cuda").to(t) for s in ((rows, heads, dim), (n, kv, dim), (n, kv, vdim)))
+    out = torch.full((rows, heads, vdim), float("nan"), dtype=t, device="cuda")
+    state = torch.zeros(rows * heads * (vdim + 2), device="cuda")
+    pos = torch.tensor([pos0], dtype=torch.int32, device="cuda")
+    cut = n // 2
+    for lo, hi in ((0, cut), (cut, n)) if cut else ((0, n),):
+        a = S.LatentAttnArgs()
+        a.q, a.k, a.v, a.out, a.f32 = q.data_ptr(), k[lo:].data_ptr(), v[lo:].data_ptr(), out.data_ptr(), f32
+        a.rows, a.heads, a.dim, a.vdim, a.scale, a.pos0, a.group, a.window = rows, heads, dim, vdim, dim ** -0.5, pos.data_ptr(), group, window
+        a.state, a.kv0, a.kv_rows, a.first, a.last = state.data_ptr(), lo, hi - lo, int(lo == 0), int(hi == n)
+        S.latent_attn_rows(a)
+    torch.cuda.synchronize()
+    at, key = pos0 + torch.arange(rows, device="cuda")[:, None], torch.arange(n, device="cuda")[None, :]
+    seen = (key <= at) & ((key >= at // window * window) if window else (key >= 0))
+    sc = torch.einsum("rhd,khd->hrk", q.double(), k.double().repeat_interleave(group, 1)) * dim ** -0.5
+    want = torch.einsum("hrk,khd->rhd", torch.softmax(sc.masked_fill(~seen, float("-inf")), -1), v.double().repeat_interleave(group, 1))
+    assert float((out.double() - want).abs().max() / want.abs().max()) < (5e-6 if f32 else 2.0 ** -8)
+
+
 @pytest.mark.parametrize("rows", [1, 63, 200, 700])
 def test_products_against_torch(rows):
     """Every epilogue and tile width of the chunk product, sizes off every multiple."""
