@@ -130,7 +130,7 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 LAUNCHES = {"count": 0}          # kernels launched through this module (sampler chain counts as 9)

@@ -68,7 +68,7 @@ def lib() -> C.CDLL:
 
 
 def _stream() -> VP:
-    return VP(torch.cuda.current_stream().cuda_stream)
+    return VP(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def weight_map(w: torch.Tensor, k: int) -> K.TensorMap:
