@@ -1,14 +1,17 @@
 // Row attention for prefill chunks with the query heads of one KV head handled together.
 //
-// One CTA (8 warps) per (KV head, query row): the up to 16 query heads that share the KV head form the
-// M = 16 side of bf16 tensor-core tiles, so every gathered key/value row is read once per KV head instead of
-// once per query head (grouped-query attention: 16 heads per KV head in the sparse layers at tp = 1, 8 at
-// tp = 8).  Keys come in chunks of 64 (the row's sliding window, its dense prefix, or its top-k selection
-// list), are staged in shared memory with cp.async (two buffers: the next chunk's gather overlaps the current
-// chunk's math), scored with m16n8k16 MMAs (S = Q K^T, 16 heads x 64 keys), soft-maxed online per head, and accumulated with a second set of MMAs
-// (O += P V, V fragments through ldmatrix.trans).  The work per CTA is a gather of ~1.3 MB at top-k 2048, so
-// the kernel is bound by L2/HBM gather bandwidth, not by tensor throughput; with M = 16 live rows there is no
-// 128-lane UMMA shape to fill, which is why this kernel uses warp-level MMAs rather than tcgen05.
+// The up to 16 query heads that share a KV head are rows of the M = 16 side of m16n8k16 tiles.  A warp keeps everything of its tile in
+// registers: scores of a key tile, their exponentials (a score fragment is the A fragment of P V as it stands), the
+// running maximum and sum of its rows, 16 x 128 outputs.  Two forms:
+//   selection list / dense prefix   one CTA per (KV head, row); each of the four warps walks every fourth tile of 16 keys
+//       through a ring of its own (no barrier inside the walk) and the four partial results are merged at the end.
+//       Bound by the gather, 1.3 MB per CTA at 2048 keys: 2048 rows x 4 KV heads in 1.51 ms, 7.1 TB/s out of the L2.
+//   sliding window   one CTA per (KV head, 4 warps x 16 / heads rows): neighbouring rows share all but one key of their
+//       window, so the rows' keys are staged once, 32 at a time, and every warp masks what its rows do not see.  Window 128,
+//       2048 rows x 64 heads: 114 us.
+// A 16,001-token document of two sparse and four window layers spends 27.8 ms in them; 61.2 ms when every row gathered its keys for
+// itself into tiles that eight warps shared between four barriers.
+// With M = 16 live rows there is no 128-lane UMMA shape to fill, which is why this uses warp-level MMAs rather than tcgen05.
 //
 // Output: bf16-rounded o, written as bf16 and/or as the e4m3 packet (one power-of-two scale per head) that
 // the o_proj GEMM consumes.  Probabilities are rounded to bf16 before P V (and summed as rounded), so results
@@ -52,26 +55,21 @@ struct AttnArgs {               // must match target_kernels.cu
   unsigned long long* stamps;   // opt-in phase stamps of the tensor-core decode kernel (%globaltimer, ns), [CTA][8]; null: none
 };
 
-constexpr int kHd = 192, kVd = 128, kChunk = 64, kM = 16, kStagesKV = 2;
-constexpr int kQStride = kHd + 8;        // bf16 elements; 400-byte rows: fragment loads hit 32 distinct banks
-constexpr int kVStride = kVd + 8;        // 272-byte rows: ldmatrix rows fall into distinct 16-byte bank groups
-constexpr int kSStride = kVd + 4;        // fp32; also carries the 128 output channels at the end
-constexpr int kPStride = kChunk + 8;     // bf16
-
-struct Smem {
-  __nv_bfloat16 q[kM][kQStride];
-  __nv_bfloat16 k[kStagesKV][kChunk][kQStride];
-  __nv_bfloat16 v[kStagesKV][kChunk][kVStride];
-  float s[kM][kSStride];
-  __nv_bfloat16 p[kM][kPStride];
-  float m[kM], l[kM], corr[kM];
-};
+constexpr int kHd = 192, kVd = 128, kM = 16;
+constexpr int kKRow = kHd * 2 + 16, kVRow = kVd * 2 + 16;      // bytes of a staged row: odd in 16-byte words, so ldmatrix rows miss one another's banks
+constexpr int kListWarps = 4, kListKeys = 16, kListStages = 2;
+constexpr int kListStage = kListKeys * (kKRow + kVRow);
+constexpr int kPartRow = kVd + 4;                                // fp32
+constexpr int kListSmem = kListWarps * kListStages * kListStage;
+static_assert(kListWarps * (kM * kPartRow + 2 * kM) * 4 <= kListSmem, "the merge reuses the rings");
+constexpr int kWinWarps = 4, kWinKeys = 32, kWinStages = 3;
+constexpr int kWinStage = kWinKeys * (kKRow + kVRow);
+constexpr int kWinSmem = kWinStages * kWinStage;
 
 // 16-byte asynchronous copy global -> shared; `valid` false writes zeros (nothing is read)
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
   const int bytes = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -82,205 +80,329 @@ __device__ __forceinline__ void mma16816(float c[4], const uint32_t a[4], uint32
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void ldmatrix_x2_trans(uint32_t& r0, uint32_t& r1, const void* p) {
-  const uint32_t addr = (uint32_t)__cvta_generic_to_shared(p);
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
+__device__ __forceinline__ void ldmatrix_x4(uint32_t r[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t r[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ float quad_max(float v) {
+  v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+  return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+}
+__device__ __forceinline__ float quad_sum(float v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 __device__ __forceinline__ float wmax(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
-__device__ __forceinline__ float wsum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 __device__ __forceinline__ float rbf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-__global__ void __launch_bounds__(256, 2) attn_group_kernel(const AttnArgs a) {
-  extern __shared__ uint4 smem_raw[];
-  Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
-  const int g = blockIdx.x, r = blockIdx.y;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int hpg = a.heads / a.kv_heads;                      // live query heads (<= 16)
-  const int h0 = g * hpg;
-  const int pos = *a.pos0 + r;
-  const int qr = lane >> 2, qc = (lane & 3) * 2;             // fragment row / column pair of this lane
+__device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
 
-  // ---- stage Q (dead rows zero) and reset the running statistics
-  for (int i = tid; i < kM * (kHd / 8); i += 256) {
-    const int h = i / (kHd / 8), c = i - h * (kHd / 8);
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (h < hpg) v = reinterpret_cast<const uint4*>(a.q + ((size_t)r * a.heads + h0 + h) * kHd)[c];
-    *reinterpret_cast<uint4*>(&sm.q[h][c * 8]) = v;
-  }
-  if (tid < kM) { sm.m[tid] = -FLT_MAX; sm.l[tid] = 0.f; }
-  __syncthreads();
-  uint32_t qa[kHd / 16][4];
+// What a warp carries over the keys: fragment rows `lane / 4` ("lo") and `lane / 4 + 8` ("hi") of its sixteen.
+struct Walk {
+  uint32_t q[kHd / 16][4];
+  float o[kVd / 8][4];
+  float m[2], l[2];                                    // l: this thread's share of the sum
+
+  // q_lo / q_hi: the rows' queries, null: a dead row
+  __device__ __forceinline__ void open(const __nv_bfloat16* q_lo, const __nv_bfloat16* q_hi, int qc) {
 #pragma unroll
-  for (int ks = 0; ks < kHd / 16; ++ks) {
-    qa[ks][0] = *reinterpret_cast<const uint32_t*>(&sm.q[qr][ks * 16 + qc]);
-    qa[ks][1] = *reinterpret_cast<const uint32_t*>(&sm.q[qr + 8][ks * 16 + qc]);
-    qa[ks][2] = *reinterpret_cast<const uint32_t*>(&sm.q[qr][ks * 16 + qc + 8]);
-    qa[ks][3] = *reinterpret_cast<const uint32_t*>(&sm.q[qr + 8][ks * 16 + qc + 8]);
-  }
-
-  int lo = 0, count = 0;
-  bool use_sel = false;
-  if (a.mode == 0) { lo = max(0, pos - a.window + 1); count = pos - lo + 1; }
-  else { use_sel = pos + 1 > a.top_k; count = use_sel ? a.top_k : pos + 1; }
-
-  float oc[2][4];
-#pragma unroll
-  for (int t = 0; t < 2; ++t)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) oc[t][j] = 0.f;
-
-  // Key chunks of 64 are staged with cp.async into two buffers: the gather of chunk c + 1 is in flight while
-  // chunk c is scored, so a CTA covers its own gather latency (two CTAs per SM cover the rest).
-  auto issue = [&](int c0, int stage) {
-    for (int i = tid; i < kChunk * (kHd / 8); i += 256) {
-      const int t = i / (kHd / 8), c = i - t * (kHd / 8);
-      const int j = c0 + t;
-      const bool valid = j < count;
-      const int id = !valid ? 0 : (a.mode == 1 ? (use_sel ? a.sel[(size_t)r * a.top_k + j] : j) : lo + j);
-      const size_t slot = a.ring > 0 ? (size_t)(id % a.ring) : (size_t)id;
-      cp_async16(&sm.k[stage][t][c * 8], a.k_cache + (slot * a.kv_heads + g) * kHd + c * 8, valid);
+    for (int ks = 0; ks < kHd / 16; ++ks) {
+      q[ks][0] = q_lo ? *reinterpret_cast<const uint32_t*>(q_lo + ks * 16 + qc) : 0u;
+      q[ks][1] = q_hi ? *reinterpret_cast<const uint32_t*>(q_hi + ks * 16 + qc) : 0u;
+      q[ks][2] = q_lo ? *reinterpret_cast<const uint32_t*>(q_lo + ks * 16 + qc + 8) : 0u;
+      q[ks][3] = q_hi ? *reinterpret_cast<const uint32_t*>(q_hi + ks * 16 + qc + 8) : 0u;
     }
-    for (int i = tid; i < kChunk * (kVd / 8); i += 256) {
-      const int t = i / (kVd / 8), c = i - t * (kVd / 8);
-      const int j = c0 + t;
-      const bool valid = j < count;
-      const int id = !valid ? 0 : (a.mode == 1 ? (use_sel ? a.sel[(size_t)r * a.top_k + j] : j) : lo + j);
-      const size_t slot = a.ring > 0 ? (size_t)(id % a.ring) : (size_t)id;
-      cp_async16(&sm.v[stage][t][c * 8], a.v_cache + (slot * a.kv_heads + g) * kVd + c * 8, valid);
-    }
-  };
-  const int nchunks = (count + kChunk - 1) / kChunk;
-  issue(0, 0);
-  cp_async_commit();
-  for (int ci = 0; ci < nchunks; ++ci) {
-    const int c0 = ci * kChunk, st = ci & 1;
-    const int n = min(kChunk, count - c0);
-    if (ci + 1 < nchunks) issue(c0 + kChunk, st ^ 1);
-    cp_async_commit();                                        // (possibly empty) group of chunk ci + 1
-    cp_async_wait<1>();                                       // this thread's copies of chunk ci have landed
-    __syncthreads();                                          // ... and everybody else's
-    // ---- S = Q K^T: warp w scores keys [8w, 8w + 8) for all heads
-    {
-      const int key0 = warp * 8;
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int ks = 0; ks < kHd / 16; ++ks) {
-        const uint32_t b0 = *reinterpret_cast<const uint32_t*>(&sm.k[st][key0 + qr][ks * 16 + qc]);
-        const uint32_t b1 = *reinterpret_cast<const uint32_t*>(&sm.k[st][key0 + qr][ks * 16 + qc + 8]);
-        mma16816(c, qa[ks], b0, b1);
+    for (int t = 0; t < kVd / 8; ++t)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[t][j] = 0.f;
+    m[0] = m[1] = -FLT_MAX;
+    l[0] = l[1] = 0.f;
+  }
+
+  // One tile of KEYS staged keys; seen(hi, key of the tile) says whether a row sees a key.
+  template <int KEYS, typename Seen>
+  __device__ __forceinline__ void tile(uint32_t sk, uint32_t sv, int lane, float scale, Seen&& seen) {
+    float s[KEYS / 8][4];
+#pragma unroll
+    for (int t = 0; t < KEYS / 8; ++t)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[t][j] = 0.f;
+    const uint32_t ka = sk + ((lane & 7) + ((lane >> 4) << 3)) * kKRow + ((lane >> 3) & 1) * 16;
+#pragma unroll
+    for (int ks = 0; ks < kHd / 16; ++ks)
+#pragma unroll
+      for (int t = 0; t < KEYS / 16; ++t) {
+        uint32_t b[4];
+        ldmatrix_x4(b, ka + t * 16 * kKRow + ks * 32);
+        mma16816(s[2 * t], q[ks], b[0], b[1]);
+        mma16816(s[2 * t + 1], q[ks], b[2], b[3]);
       }
-      const int kc = key0 + qc;
-      sm.s[qr][kc] = kc < n ? c[0] * a.scale : -FLT_MAX;
-      sm.s[qr][kc + 1] = kc + 1 < n ? c[1] * a.scale : -FLT_MAX;
-      sm.s[qr + 8][kc] = kc < n ? c[2] * a.scale : -FLT_MAX;
-      sm.s[qr + 8][kc + 1] = kc + 1 < n ? c[3] * a.scale : -FLT_MAX;
-    }
-    __syncthreads();
-    // ---- online softmax: warp w owns heads 2w and 2w + 1
+    const int qc = (lane & 3) * 2;
+    float corr[2];
+    uint32_t p[KEYS / 8][2];
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      const int h = warp * 2 + t;
-      float v[kChunk / 32];
+    for (int hi = 0; hi < 2; ++hi) {
       float mx = -FLT_MAX;
 #pragma unroll
-      for (int j = 0; j < kChunk / 32; ++j) { v[j] = sm.s[h][lane + 32 * j]; mx = fmaxf(mx, v[j]); }
-      mx = wmax(mx);
-      const float m_old = sm.m[h];
-      const float m_new = fmaxf(m_old, mx);
+      for (int t = 0; t < KEYS / 8; ++t)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float& v = s[t][2 * hi + j];
+          v = seen(hi, t * 8 + qc + j) ? v * scale : -FLT_MAX;
+          mx = fmaxf(mx, v);
+        }
+      const float mn = fmaxf(m[hi], quad_max(mx));
+      corr[hi] = __expf(m[hi] - mn);
+      m[hi] = mn;
       float sum = 0.f;
 #pragma unroll
-      for (int j = 0; j < kChunk / 32; ++j) {
-        const int kc = lane + 32 * j;
-        const float p = kc < n ? rbf16(__expf(v[j] - m_new)) : 0.f;
-        sm.p[h][kc] = __float2bfloat16_rn(p);
-        sum += p;
+      for (int t = 0; t < KEYS / 8; ++t) {
+        const float p0 = seen(hi, t * 8 + qc) ? rbf16(__expf(s[t][2 * hi] - mn)) : 0.f;
+        const float p1 = seen(hi, t * 8 + qc + 1) ? rbf16(__expf(s[t][2 * hi + 1] - mn)) : 0.f;
+        sum += p0 + p1;
+        p[t][hi] = bf16_pair(p0, p1);
       }
-      sum = wsum(sum);
-      if (lane == 0) {
-        const float corr = __expf(m_old - m_new);
-        sm.corr[h] = corr;
-        sm.l[h] = sm.l[h] * corr + sum;
-        sm.m[h] = m_new;
+      l[hi] = l[hi] * corr[hi] + sum;
+    }
+    if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {
+#pragma unroll
+      for (int t = 0; t < kVd / 8; ++t) { o[t][0] *= corr[0]; o[t][1] *= corr[0]; o[t][2] *= corr[1]; o[t][3] *= corr[1]; }
+    }
+    const uint32_t va = sv + ((lane & 7) + ((lane >> 3) & 1) * 8) * kVRow + (lane >> 4) * 16;
+#pragma unroll
+    for (int t = 0; t < KEYS / 16; ++t) {
+      const uint32_t pa[4] = {p[2 * t][0], p[2 * t][1], p[2 * t + 1][0], p[2 * t + 1][1]};
+#pragma unroll
+      for (int c = 0; c < kVd / 16; ++c) {
+        uint32_t b[4];
+        ldmatrix_x4_trans(b, va + t * 16 * kVRow + c * 32);
+        mma16816(o[2 * c], pa, b[0], b[1]);
+        mma16816(o[2 * c + 1], pa, b[2], b[3]);
       }
     }
-    __syncthreads();
-    // ---- O = O * corr + P V: warp w owns channels [16w, 16w + 16)
-    {
-      const float c_lo = sm.corr[qr], c_hi = sm.corr[qr + 8];
+  }
+};
+
+// factor of a row's output: the sink column (no value) joins the sum, then normalisation
+__device__ __forceinline__ float row_factor(float m, float l, const __nv_bfloat16* sink, int head) {
+  float corr = 1.f;
+  if (sink) {
+    const float sv = __bfloat162float(sink[head]);
+    const float mn = fmaxf(m, sv);
+    corr = __expf(m - mn);
+    l = l * corr + __expf(sv - mn);
+  }
+  return l > 0.f ? corr / l : 0.f;
+}
+
+// ------------------------------------------------------------------------------------ selection list or dense prefix
+__global__ void __launch_bounds__(kListWarps * 32, 2) attn_list_kernel(const AttnArgs a) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  griddep_wait();
+  griddep_launch();
+  const int g = blockIdx.x, r = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int hpg = a.heads / a.kv_heads, h0 = g * hpg;               // live query heads (<= 16)
+  const int pos = *a.pos0 + r;
+  const bool use_sel = pos + 1 > a.top_k;
+  const int count = use_sel ? a.top_k : pos + 1, tiles = (count + kListKeys - 1) / kListKeys;
+  const int* sel = use_sel ? a.sel + (size_t)r * a.top_k : nullptr;
+  const uint32_t ring = smem_u32(smem) + warp * kListStages * kListStage;
+  const uint8_t* kc = reinterpret_cast<const uint8_t*>(a.k_cache + (size_t)g * kHd) + (lane & 7) * 16;
+  const uint8_t* vc = reinterpret_cast<const uint8_t*>(a.v_cache + (size_t)g * kVd) + (lane & 7) * 16;
+  const size_t k_pitch = (size_t)a.kv_heads * kHd * 2, v_pitch = (size_t)a.kv_heads * kVd * 2;
+
+  auto ids_of = [&](int t) {                                        // lane i < 16: key i of the tile (-1: none)
+    const int j = t * kListKeys + lane;
+    return lane < kListKeys && t < tiles && j < count ? (sel ? __ldg(sel + j) : j) : -1;
+  };
+  // eight lanes copy one key, 128 bytes at a time
+  auto request = [&](int stage, int ids) {
+    const uint32_t sk = ring + stage * kListStage + (lane & 7) * 16, sv = sk + kListKeys * kKRow;
 #pragma unroll
-      for (int t = 0; t < 2; ++t) { oc[t][0] *= c_lo; oc[t][1] *= c_lo; oc[t][2] *= c_hi; oc[t][3] *= c_hi; }
+    for (int i = 0; i < kListKeys / 4; ++i) {
+      const int key = i * 4 + (lane >> 3), id = __shfl_sync(0xffffffffu, ids, key);
+      const bool valid = id >= 0;
+      const size_t slot = !valid ? 0 : a.ring > 0 ? (size_t)(id % a.ring) : (size_t)id;
 #pragma unroll
-      for (int kk = 0; kk < kChunk / 16; ++kk) {
-        uint32_t pa[4];
-        pa[0] = *reinterpret_cast<const uint32_t*>(&sm.p[qr][kk * 16 + qc]);
-        pa[1] = *reinterpret_cast<const uint32_t*>(&sm.p[qr + 8][kk * 16 + qc]);
-        pa[2] = *reinterpret_cast<const uint32_t*>(&sm.p[qr][kk * 16 + qc + 8]);
-        pa[3] = *reinterpret_cast<const uint32_t*>(&sm.p[qr + 8][kk * 16 + qc + 8]);
+      for (int c = 0; c < 3; ++c) cp_async16(sk + key * kKRow + c * 128, kc + slot * k_pitch + c * 128, valid);
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          uint32_t b0, b1;
-          ldmatrix_x2_trans(b0, b1, &sm.v[st][kk * 16 + (lane & 15)][warp * 16 + t * 8]);
-          mma16816(oc[t], pa, b0, b1);
-        }
-      }
+      for (int c = 0; c < 2; ++c) cp_async16(sv + key * kVRow + c * 128, vc + slot * v_pitch + c * 128, valid);
     }
-    __syncthreads();                                          // stage st is free for chunk ci + 2
+  };
+  int ids = ids_of(warp);
+  request(0, ids);
+  cp_async_commit();
+  ids = ids_of(warp + kListWarps);
+  Walk w;
+  {
+    const int qr = lane >> 2;
+    const __nv_bfloat16* q = a.q + ((size_t)r * a.heads + h0) * kHd;
+    w.open(qr < hpg ? q + qr * kHd : nullptr, qr + 8 < hpg ? q + (qr + 8) * kHd : nullptr, (lane & 3) * 2);
+  }
+  int stage = 0;
+#pragma unroll 1
+  for (int t = warp; t < tiles; t += kListWarps) {
+    if (t + kListWarps < tiles) request(stage ^ 1, ids);
+    cp_async_commit();
+    ids = ids_of(t + 2 * kListWarps);
+    cp_async_wait<1>();
+    __syncwarp();
+    const uint32_t sk = ring + stage * kListStage;
+    const int live = count - t * kListKeys;
+    w.tile<kListKeys>(sk, sk + kListKeys * kKRow, lane, a.scale, [&](int, int key) { return key < live; });
+    __syncwarp();                                                   // every lane has read the stage before it is filled anew
+    stage ^= 1;
   }
   cp_async_wait<0>();
   __syncthreads();
-  // ---- sink column (no value), normalisation, bf16 rounding; o goes through shared memory for the packet
-  if (tid < kM) {
-    float m = sm.m[tid], l = sm.l[tid], corr = 1.f;
-    if (a.sink && tid < hpg) {
-      const float sv = __bfloat162float(a.sink[h0 + tid]);
-      const float m_new = fmaxf(m, sv);
-      corr = __expf(m - m_new);
-      l = l * corr + __expf(sv - m_new);
-    }
-    sm.corr[tid] = l > 0.f ? corr / l : 0.f;
-  }
-  __syncthreads();
+  // merge: the warps' results side by side in shared memory, then a warp per head
+  float* part = reinterpret_cast<float*>(smem);                     // [warp][16][kPartRow]
+  float* ml = part + kListWarps * kM * kPartRow;                    // [warp][16][2]
   {
-    const float c_lo = sm.corr[qr], c_hi = sm.corr[qr + 8];
+    const int qr = lane >> 2, qc = (lane & 3) * 2;
+    const float l_lo = quad_sum(w.l[0]), l_hi = quad_sum(w.l[1]);
+    float* o = part + (warp * kM + qr) * kPartRow + qc;
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      const int ch = warp * 16 + t * 8 + qc;
-      sm.s[qr][ch] = rbf16(oc[t][0] * c_lo);
-      sm.s[qr][ch + 1] = rbf16(oc[t][1] * c_lo);
-      sm.s[qr + 8][ch] = rbf16(oc[t][2] * c_hi);
-      sm.s[qr + 8][ch + 1] = rbf16(oc[t][3] * c_hi);
+    for (int t = 0; t < kVd / 8; ++t) {
+      *reinterpret_cast<float2*>(o + t * 8) = make_float2(w.o[t][0], w.o[t][1]);
+      *reinterpret_cast<float2*>(o + 8 * kPartRow + t * 8) = make_float2(w.o[t][2], w.o[t][3]);
+    }
+    if ((lane & 3) == 0) {
+      ml[(warp * kM + qr) * 2] = w.m[0];
+      ml[(warp * kM + qr) * 2 + 1] = l_lo;
+      ml[(warp * kM + qr + 8) * 2] = w.m[1];
+      ml[(warp * kM + qr + 8) * 2 + 1] = l_hi;
     }
   }
   __syncthreads();
   const size_t ldo = (size_t)a.heads * kVd;
+#pragma unroll 1
+  for (int h = warp; h < hpg; h += kListWarps) {
+    float m = -FLT_MAX, l = 0.f;
 #pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const int h = warp * 2 + t;
-    if (h >= hpg) continue;
-    float v[4];
+    for (int i = 0; i < kListWarps; ++i) m = fmaxf(m, ml[(i * kM + h) * 2]);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < kListWarps; ++i) {
+      const float f = __expf(ml[(i * kM + h) * 2] - m);
+      l = fmaf(ml[(i * kM + h) * 2 + 1], f, l);
+      const float4 p = *reinterpret_cast<const float4*>(part + (i * kM + h) * kPartRow + lane * 4);
+      v = make_float4(fmaf(p.x, f, v.x), fmaf(p.y, f, v.y), fmaf(p.z, f, v.z), fmaf(p.w, f, v.w));
+    }
+    const float f = row_factor(m, l, a.sink, h0 + h);
+    v = make_float4(rbf16(v.x * f), rbf16(v.y * f), rbf16(v.z * f), rbf16(v.w * f));
+    const size_t base = (size_t)r * ldo + (size_t)(h0 + h) * kVd + lane * 4;
+    if (a.o_bf16) *reinterpret_cast<uint2*>(a.o_bf16 + base) = make_uint2(bf16_pair(v.x, v.y), bf16_pair(v.z, v.w));
+    if (a.o8) {
+      const float sc = pow2_scale(wmax(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)))));
+      const __nv_fp8_e4m3 c[4] = {__nv_fp8_e4m3(v.x / sc), __nv_fp8_e4m3(v.y / sc), __nv_fp8_e4m3(v.z / sc), __nv_fp8_e4m3(v.w / sc)};
+      uint32_t word = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) word |= (uint32_t)c[i].__x << (8 * i);
+      *reinterpret_cast<uint32_t*>(a.o8 + base) = word;
+      if (lane == 0) a.o_scale[(size_t)r * (ldo / 128) + h0 + h] = sc;
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------ sliding window
+__global__ void __launch_bounds__(kWinWarps * 32, 2) attn_window_kernel(const AttnArgs a) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  griddep_wait();
+  griddep_launch();
+  const int g = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int hpg = a.heads / a.kv_heads, h0 = g * hpg, rpw = kM / hpg;     // rows per warp
+  const int r0 = blockIdx.y * kWinWarps * rpw, pos0 = *a.pos0;
+  const int r_last = min(r0 + kWinWarps * rpw, a.rows) - 1;
+  const int key0 = max(0, pos0 + r0 - a.window + 1), key_end = pos0 + r_last + 1;       // keys of the CTA's rows
+  const int tiles = (key_end - key0 + kWinKeys - 1) / kWinKeys;
+  const uint32_t base = smem_u32(smem);
+  const int chunk = (threadIdx.x & 7) * 16;                                             // eight threads copy one key
+  const uint8_t* kc = reinterpret_cast<const uint8_t*>(a.k_cache + (size_t)g * kHd) + chunk;
+  const uint8_t* vc = reinterpret_cast<const uint8_t*>(a.v_cache + (size_t)g * kVd) + chunk;
+  const size_t k_pitch = (size_t)a.kv_heads * kHd * 2, v_pitch = (size_t)a.kv_heads * kVd * 2;
+  auto request = [&](int t) {
+    const uint32_t st = base + (t % kWinStages) * kWinStage + chunk;
+#pragma unroll
+    for (int key = threadIdx.x >> 3; key < kWinKeys; key += kWinWarps * 4) {
+      const int id = key0 + t * kWinKeys + key;
+      const bool valid = id < key_end;
+      const size_t slot = !valid ? 0 : a.ring > 0 ? (size_t)(id % a.ring) : (size_t)id;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) cp_async16(st + key * kKRow + c * 128, kc + slot * k_pitch + c * 128, valid);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) cp_async16(st + kWinKeys * kKRow + key * kVRow + c * 128, vc + slot * v_pitch + c * 128, valid);
+    }
+  };
+#pragma unroll
+  for (int t = 0; t < kWinStages - 1; ++t) {
+    if (t < tiles) request(t);
+    cp_async_commit();
+  }
+  // fragment row -> (token row, head); rows beyond the chunk see no key
+  int row[2], head[2], low[2], high[2];
+#pragma unroll
+  for (int hi = 0; hi < 2; ++hi) {
+    const int at = (lane >> 2) + 8 * hi, slot = at / hpg;
+    row[hi] = slot < rpw ? min(r0 + warp * rpw + slot, a.rows) : a.rows;
+    head[hi] = h0 + at - slot * hpg;
+    const int pos = pos0 + row[hi];
+    low[hi] = row[hi] < a.rows ? max(0, pos - a.window + 1) : 0;
+    high[hi] = row[hi] < a.rows ? pos : -1;
+  }
+  Walk w;
+  w.open(row[0] < a.rows ? a.q + ((size_t)row[0] * a.heads + head[0]) * kHd : nullptr,
+         row[1] < a.rows ? a.q + ((size_t)row[1] * a.heads + head[1]) * kHd : nullptr, (lane & 3) * 2);
+  const int w_low = pos0 + r0 + warp * rpw - a.window + 1, w_high = pos0 + min(r0 + (warp + 1) * rpw, a.rows) - 1;   // keys any row of the warp sees
+#pragma unroll 1
+  for (int t = 0; t < tiles; ++t) {
+    cp_async_wait<kWinStages - 2>();
+    __syncthreads();                                                  // tile t has landed; everybody is done with tile t - 1
+    if (t + kWinStages - 1 < tiles) request(t + kWinStages - 1);
+    cp_async_commit();
+    const int k0 = key0 + t * kWinKeys;
+    if (k0 > w_high || k0 + kWinKeys <= w_low || r0 + warp * rpw >= a.rows) continue;
+    const uint32_t sk = base + (t % kWinStages) * kWinStage;
+    w.tile<kWinKeys>(sk, sk + kWinKeys * kKRow, lane, a.scale, [&](int hi, int i) { return k0 + i >= low[hi] && k0 + i <= high[hi]; });
+  }
+  cp_async_wait<0>();
+  const size_t ldo = (size_t)a.heads * kVd;
+#pragma unroll
+  for (int hi = 0; hi < 2; ++hi) {
+    const float l = quad_sum(w.l[hi]);
+    const bool live = row[hi] < a.rows;
+    const float f = live ? row_factor(w.m[hi], l, a.sink, head[hi]) : 0.f;
     float am = 0.f;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) { v[j] = sm.s[h][lane + 32 * j]; am = fmaxf(am, fabsf(v[j])); }
-    am = wmax(am);
-    const size_t base = (size_t)r * ldo + (size_t)(h0 + h) * kVd;
+    for (int t = 0; t < kVd / 8; ++t)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        float& v = w.o[t][2 * hi + j];
+        v = rbf16(v * f);
+        am = fmaxf(am, fabsf(v));
+      }
+    const float sc = pow2_scale(quad_max(am));
+    if (!live) continue;
+    const size_t at = (size_t)row[hi] * ldo + (size_t)head[hi] * kVd + (lane & 3) * 2;
     if (a.o_bf16)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) a.o_bf16[base + lane + 32 * j] = __float2bfloat16_rn(v[j]);
+      for (int t = 0; t < kVd / 8; ++t) *reinterpret_cast<uint32_t*>(a.o_bf16 + at + t * 8) = bf16_pair(w.o[t][2 * hi], w.o[t][2 * hi + 1]);
     if (a.o8) {
-      const float sc = pow2_scale(am);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const __nv_fp8_e4m3 q8(v[j] / sc);
-        a.o8[base + lane + 32 * j] = *reinterpret_cast<const uint8_t*>(&q8);
+      for (int t = 0; t < kVd / 8; ++t) {
+        const __nv_fp8_e4m3 c0(w.o[t][2 * hi] / sc), c1(w.o[t][2 * hi + 1] / sc);
+        *reinterpret_cast<uint16_t*>(a.o8 + at + t * 8) = (uint16_t)(c0.__x | (uint32_t)c1.__x << 8);
       }
-      if (lane == 0) a.o_scale[(size_t)r * (ldo / 128) + h0 + h] = sc;
+      if ((lane & 3) == 0) a.o_scale[(size_t)row[hi] * (ldo / 128) + head[hi]] = sc;
     }
   }
 }
@@ -299,10 +421,13 @@ extern "C" int nrt_attn_group(const void* args, void* stream, int pdl) {
   if (a.rows > 65535) return -3;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem));
+    cudaError_t e = cudaFuncSetAttribute(attn_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kListSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_window_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWinSmem);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  return launch_pdl(attn_group_kernel, dim3(a.kv_heads, a.rows), dim3(256), sizeof(Smem), reinterpret_cast<cudaStream_t>(stream),
-                    pdl != 0, a);
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (a.mode == 1) return launch_pdl(attn_list_kernel, dim3(a.kv_heads, a.rows), dim3(kListWarps * 32), kListSmem, s, pdl != 0, a);
+  const int rows = kWinWarps * (kM / (a.heads / a.kv_heads));
+  return launch_pdl(attn_window_kernel, dim3(a.kv_heads, (a.rows + rows - 1) / rows), dim3(kWinWarps * 32), kWinSmem, s, pdl != 0, a);
 }

@@ -182,6 +182,55 @@ def test_grouped_head_attention_matches_row_attention():
             assert (got8 - ref8).abs().max().item() <= 0.08 * ref.abs().max().item(), (heads, kvh, mode, pos0)
 
 
+@pytest.mark.parametrize("heads,kvh,rows,window,pos0,top_k", [
+    (8, 8, 1, 1, 0, 1), (24, 8, 7, 33, 5, 4), (64, 8, 17, 128, 0, 16), (64, 8, 131, 128, 999, 17), (64, 4, 9, 31, 63, 64), (16, 1, 3, 160, 200, 63)])
+def test_grouped_head_attention_at_the_edges_of_its_tiles(heads, kvh, rows, window, pos0, top_k):
+    """Windows and selection lists around the sizes of key tiles (16, 32) and row tiles (16 / heads of a group), against fp64.  Outputs
+    are rounded to bf16 once and probabilities before P V: 2^-8 of the largest value each."""
+    from naivert_b200.ops import kernels as K
+    K.lib()
+    g = torch.Generator(device="cuda").manual_seed(rows * 131 + window)
+    hd, vd, cap = 192, 128, pos0 + rows
+    ring = min(cap, window + rows)
+    q = torch.randn(rows, heads, hd, device="cuda", generator=g).bfloat16()
+    kc = torch.randn(cap, kvh, hd, device="cuda", generator=g).bfloat16()
+    vc = torch.randn(cap, kvh, vd, device="cuda", generator=g).bfloat16()
+    sink = torch.randn(heads, device="cuda", generator=g).bfloat16()
+    p = torch.tensor([pos0], dtype=torch.int32, device="cuda")
+    sel = torch.zeros(rows, top_k, dtype=torch.int32, device="cuda")
+    for r in range(rows):
+        if pos0 + r + 1 > top_k:
+            sel[r] = torch.sort(torch.randperm(pos0 + r + 1, device="cuda", generator=g)[:top_k])[0].int()
+    last = torch.arange(max(0, cap - ring), cap, device="cuda")
+    kr, vr = torch.zeros(ring, kvh, hd, device="cuda", dtype=torch.bfloat16), torch.zeros(ring, kvh, vd, device="cuda", dtype=torch.bfloat16)
+    kr[last % ring], vr[last % ring] = kc[last], vc[last]
+    for mode in (0, 1):
+        o = torch.full((rows, heads * vd), float("nan"), device="cuda", dtype=torch.bfloat16)
+        o8, osc = torch.zeros(rows, heads * vd, device="cuda", dtype=torch.uint8), torch.zeros(rows, heads, device="cuda")
+        a = K.AttnArgs()
+        a.q, a.pos0, a.rows, a.heads, a.kv_heads, a.head_dim, a.v_dim = q.data_ptr(), p.data_ptr(), rows, heads, kvh, hd, vd
+        a.scale, a.mode, a.o_bf16, a.o8, a.o_scale = hd ** -0.5, mode, o.data_ptr(), o8.data_ptr(), osc.data_ptr()
+        if mode == 0:
+            a.k_cache, a.v_cache, a.window, a.ring, a.sink = kr.data_ptr(), vr.data_ptr(), window, ring, sink.data_ptr()
+        else:
+            a.k_cache, a.v_cache, a.top_k, a.sel = kc.data_ptr(), vc.data_ptr(), top_k, sel.data_ptr()
+        K.attn_group(a, pdl=False)
+        torch.cuda.synchronize()
+        packet = o8.view(torch.float8_e4m3fn).double() * osc.repeat_interleave(vd, 1).double()
+        for r in range(rows):
+            pos = pos0 + r
+            keys = (torch.arange(max(0, pos - window + 1), pos + 1, device="cuda") if mode == 0 else
+                    sel[r].long() if pos + 1 > top_k else torch.arange(pos + 1, device="cuda"))
+            kk, vv = (t[keys].double().repeat_interleave(heads // kvh, 1) for t in (kc, vc))
+            sc = torch.einsum("khd,hd->hk", kk, q[r].double()) * hd ** -0.5
+            pr = torch.softmax(torch.cat((sc, sink.double()[:, None]), 1) if mode == 0 else sc, 1)[:, : len(keys)]
+            want = torch.einsum("hk,khd->hd", pr, vv)
+            have = o[r].view(heads, vd).double()
+            top = want.abs().amax(1, keepdim=True)
+            assert ((have - want).abs() <= 2 * 2.0 ** -8 * vv.abs().amax((0, 2))[:, None] + 1e-6).all(), (mode, r)
+            assert ((packet[r].view(heads, vd) - have).abs() <= 2.0 ** -4 * top + 1e-2 * top).all(), (mode, r)
+
+
 def test_tcgen05_index_sweep_matches_cuda_core_form():
     from naivert_b200.ops import kernels as K
     spec, rt, _ = _build(layers=1, capacity=2048)
