@@ -6,7 +6,8 @@
                        expert -> grouped products -> weighted sum inside the next row kernel
 
 A chunk may start and end anywhere and has any length up to ``chunk`` rows; the caches and states it leaves are those
-the step continues from.
+the step continues from.  Where the chunks are too short to fill the routed experts, several go through the layers side by side
+(a span): mixers and dense feed-forwards take them one after the other with the scratch of one, the experts' products all at once.
 """
 from __future__ import annotations
 
@@ -22,6 +23,10 @@ from ..runtime.stack import StackRuntime
 from .stack_mixers import MIXERS
 
 SMS = 148
+# Pairs (token, choice) per expert that a span is filled up to, and its most rows.  Below, an expert's product is bound by the read of its
+# weights (12.9 GB a layer at 256 experts of 4096 x 2048), which a span does once: with three such layers, 8192 rows in chunks of 2048 take
+# 30.1 ms, 47.0 ms when every chunk went through the experts by itself (their products: 28.3 -> 11.0 ms).  A span's rows cost 2 GB there.
+SPAN_PAIRS, SPAN_ROWS = 256, 8192
 
 
 class StackPrefill:
@@ -37,6 +42,9 @@ class StackPrefill:
         ffs = [d["spec"].mlp for d in L if d["spec"].mlp is not None]
         moe = [f for f in ffs if f.kind == "moe"]
         self.h_ld = pad(s.hidden, 8)
+        filled = min([-(-SPAN_PAIRS * f.routing.expert_count // f.routing.top_k) for f in moe], default=0)
+        self.span = max(C, min(SPAN_ROWS, filled, runtime.capacity) // C * C)
+        P = self.span
 
         def z(n: int, t=f32) -> torch.Tensor:
             return torch.zeros(max(8, n), dtype=t, device=dev)
@@ -44,12 +52,12 @@ class StackPrefill:
         def most(it) -> int:
             return max(list(it), default=0)
 
-        self.pos = torch.zeros(1, dtype=i32, device=dev)
-        self.tokens = torch.zeros(C, dtype=i32, device=dev)
-        self.x = torch.zeros(C, s.hidden, dtype=f32, device=dev)
-        self.h = torch.zeros(C, self.h_ld, dtype=self.act, device=dev)
-        self.y = torch.zeros(C, s.hidden, dtype=f32, device=dev)
-        self.y2 = torch.zeros(C, s.hidden, dtype=f32, device=dev) if any(d["kind"] == "parallel" for d in L) else None
+        self.tokens = torch.zeros(P, dtype=i32, device=dev)
+        # per span: position of each chunk, stream, input and output rows of the sublayers
+        self.rows_of = {"pos": torch.zeros(P // C, dtype=i32, device=dev), "x": torch.zeros(P, s.hidden, dtype=f32, device=dev),
+                        "h": torch.zeros(P, self.h_ld, dtype=self.act, device=dev), "y": torch.zeros(P, s.hidden, dtype=f32, device=dev),
+                        "y2": torch.zeros(P, s.hidden, dtype=f32, device=dev) if any(d["kind"] == "parallel" for d in L) else None}
+        self._window()
         # buffers of the mixers, one per role, shared by the layers (sizes differ from layer to layer)
         sizes: Dict[tuple, int] = {}
         for d in L:
@@ -59,11 +67,11 @@ class StackPrefill:
         self.ff = z(C * most(pad(f.ff, 8) for f in ffs if f.kind != "moe"), self.act)
         if moe:
             E, T = most(f.routing.expert_count for f in moe), most(f.routing.top_k for f in moe)
-            self.scores, self.ids, self.probs = z(C * E), z(C * T, i32), z(C * T)
-            self.slot_of, self.n_items, self.seg_rows = z(C * T, i32), z(1, i32), z(E, i32)
-            self.max_items = -(-C * T // 64) + E
+            self.scores, self.ids, self.probs = z(P * E), z(P * T, i32), z(P * T)
+            self.slot_of, self.n_items, self.seg_rows = z(P * T, i32), z(1, i32), z(E, i32)
+            self.max_items = -(-P * T // 64) + E
             self.item_z, self.item_row = z(self.max_items, i32), z(self.max_items, i32)
-            self.cap = most(self._segment_rows(C, f.routing) for f in moe)
+            self.cap = most(self._segment_rows(P, f.routing) for f in moe)
             self.sorted = z(self.cap * self.h_ld, self.act)
             self.ea = z(self.cap * most(pad(f.ff, 8) for f in moe), self.act)
             self.ey = z(self.cap * s.hidden)
@@ -151,7 +159,21 @@ class StackPrefill:
         wbytes = w.nbytes * (2 if dual else 1)
         S.gemm(epi, ntok, self._wmap(w), self._wmap(w2) if dual else None, xm, a, items is None and wbytes > (96 << 20))
 
-    # ------------------------------------------------------------------ one chunk
+    # ------------------------------------------------------------------ one span
+    def _window(self, chunk: Optional[int] = None) -> None:
+        """``pos``, ``x``, ``h``, ``y`` and ``y2`` become those of one chunk of the span, or of the whole of it."""
+        for name, t in self.rows_of.items():
+            if chunk is not None and t is not None:
+                t = t[chunk:chunk + 1] if name == "pos" else t[chunk * self.C:(chunk + 1) * self.C]
+            setattr(self, name, t)
+
+    def _chunks(self, R: int, pos0: int):
+        """(rows, first position) of the chunks of a span of R rows, each with its own rows in place."""
+        for i in range(-(-R // self.C)):
+            self._window(i)
+            yield min(self.C, R - i * self.C), pos0 + i * self.C
+        self._window()
+
     def _rows(self, R: int, *, embed: bool = False, y: Optional[torch.Tensor] = None, post=None, y2: Optional[torch.Tensor] = None, join=None,
               moe=None, add=None, pre=None, copy: bool = False) -> None:
         """Stream update; then the input rows ``h`` of the next sublayer: normed by ``pre``, or the stream itself (``copy``)."""
@@ -177,16 +199,18 @@ class StackPrefill:
         f, W = d["spec"].mlp, self.spec.hidden
         fp = pad(f.ff, 8)
         if f.kind == "relu2":
-            with self.stage("ff_up"):
-                self.gemm(S.EPI_RELU2, d["up"], self.h, self.h_ld, R, self.ff, fp)
-            with self.stage("ff_down"):
-                self.gemm(S.EPI_STORE, d["down"], self.ff, fp, R, self.y, W)
+            for n, _ in self._chunks(R, 0):
+                with self.stage("ff_up"):
+                    self.gemm(S.EPI_RELU2, d["up"], self.h, self.h_ld, n, self.ff, fp)
+                with self.stage("ff_down"):
+                    self.gemm(S.EPI_STORE, d["down"], self.ff, fp, n, self.y, W)
             return self.y
         if f.kind == "dense":
-            with self.stage("dense_gate_up"):
-                self.gemm(S.EPI_CLAMPED_GLU, d["gate"], self.h, self.h_ld, R, self.ff, fp, w2=d["up"], limit=f.limit, alpha=f.alpha)
-            with self.stage("dense_down"):
-                self.gemm(S.EPI_STORE, d["down"], self.ff, fp, R, self.y, W)
+            for n, _ in self._chunks(R, 0):
+                with self.stage("dense_gate_up"):
+                    self.gemm(S.EPI_CLAMPED_GLU, d["gate"], self.h, self.h_ld, n, self.ff, fp, w2=d["up"], limit=f.limit, alpha=f.alpha)
+                with self.stage("dense_down"):
+                    self.gemm(S.EPI_STORE, d["down"], self.ff, fp, n, self.y, W)
             return self.y
         rt = f.routing
         with self.stage("router"):
@@ -224,13 +248,16 @@ class StackPrefill:
         """Rows [0, R) of ``tokens`` at positions pos0 ..: fills caches and states; logits of the rows in ``want``.
         ``trace`` collects the stream after every layer run."""
         t, s = self.t, self.spec
-        self.pos.fill_(pos0)
+        self._window()
+        for i in range(-(-R // self.C)):
+            self.pos[i:i + 1].fill_(pos0 + i * self.C)
         wait = dict(embed=True)                         # what the next row kernel adds to the stream first
         for r in t.runs:
             d, run = r["layer"], r["run"]
             add = None if run.pass_start is None else t.loop_step[run.pass_start]
             self._rows(R, add=add, pre=d["norm1"], copy=d["norm1"] is None and d["kind"] != "wkv", **wait)
-            MIXERS[d["kind"]].run(self, r, R, pos0)
+            for n, p in self._chunks(R, pos0):
+                MIXERS[d["kind"]].run(self, r, n, p)
             wait = dict(y=self.y, post=d["norm1b"])
             if d["kind"] == "parallel":
                 wait.update(y2=self.y2, join=(d["out"], d["out2"]))
@@ -255,7 +282,7 @@ class StackPrefill:
 
     # ------------------------------------------------------------------ public API (that of ``NativePrefill``)
     def extend(self, tokens: torch.Tensor, pos0: int, want: Sequence[int] = (), trace: Optional[list] = None) -> torch.Tensor:
-        """Feed ``tokens`` (host or device) at positions pos0 .. in chunks; logits [len(want), vocab] of the rows in ``want``."""
+        """Feed ``tokens`` (host or device) at positions pos0 .. in spans of chunks; logits [len(want), vocab] of the rows in ``want``."""
         n = int(tokens.numel())
         if not 0 <= pos0 <= pos0 + n <= self.t.capacity:
             raise ValueError(f"rows [{pos0}, {pos0 + n}) outside the cache capacity {self.t.capacity}")
@@ -263,8 +290,8 @@ class StackPrefill:
         order = [w for w in want]
         if order != sorted(order):
             raise ValueError("wanted rows must ascend")
-        for c0 in range(0, n, self.C):
-            R = min(self.C, n - c0)
+        for c0 in range(0, n, self.span):
+            R = min(self.span, n - c0)
             self.tokens[:R].copy_(tokens[c0:c0 + R].to(torch.int32), non_blocking=True)
             got = self._chunk(pos0 + c0, R, [w - c0 for w in order if c0 <= w < c0 + R], trace)
             if got is not None:
