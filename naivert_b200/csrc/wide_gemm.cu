@@ -7,9 +7,9 @@
 // receive buffer), so a weight tile feeds four times the math.
 //   warp 0     : TMA producer (weights 128 x 128 B, tokens 64 x 128 B, 128-byte swizzle, no multicast)
 //   warp 1     : TMEM allocator + UMMA issuer (M = 128, N = 64; kind::f8f6f4 or kind::f16)
-//   warps 2..9 : epilogue; thread = output feature x one half (32) of the token columns: two warps per TMEM
-//                lane quadrant, so every scheduler has two epilogue warps to hide TMEM-load latency
-// Block-scaled e4m3: one fresh TMEM accumulator per 128-wide K block (ring of 4), scaled by weight-block x
+//   warps 2..17: epilogue; thread = output feature x a quarter (16) of the token columns: four warps per TMEM lane
+//                quadrant, so that a thread has the registers to fetch the next accumulator while it adds the last one
+// Block-scaled e4m3: one fresh TMEM accumulator per 128-wide K block (a ring of pairs), scaled by weight-block x
 // activation-block scale and promoted in fp32 registers in ascending K order (the same arithmetic as the
 // 16-column engine, so both produce identical values).  Activation scales of the item are staged in shared
 // memory once (after the first accumulator is ready, i.e. after the producer has seen the rows arrive).
@@ -35,8 +35,10 @@ struct WideCfg {
   static constexpr int kStageBytes = (DUAL ? 2 : 1) * kATileBytes + kWBTileBytes;
   static constexpr int kStages = DUAL ? 4 : 6;
   static constexpr int kAccCols = DUAL ? 2 * kWTok : kWTok;
-  static constexpr int kAccBufs = FP8 ? 4 : 2;                     // bf16: one accumulator per tile, two tiles in flight
-  static constexpr int kTmemCols = kAccCols * kAccBufs;            // 128, 256 or 512
+  // e4m3: accumulators change hands in pairs (two K blocks); bf16: one accumulator per tile, two tiles in flight
+  static constexpr int kPair = FP8 ? 2 : 1;
+  static constexpr int kAccBufs = FP8 ? 512 / (2 * kAccCols) : 2;
+  static constexpr int kTmemCols = kAccCols * kPair * kAccBufs;    // 128 or 512
   static constexpr int kMaxKBlocks = 128;                          // K <= 16384 for e4m3
   static constexpr int kScaleBytes = kMaxKBlocks * kWTok * 4;      // activation scales [K blocks][64]
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*align*/ + 2048 /*barriers + scratch*/ + kScaleBytes;
@@ -52,8 +54,34 @@ struct WideTail {
   float red[4][kWTok];
 };
 
-constexpr int kWThreads = 320;
-constexpr int kWHalf = kWTok / 2;                // token columns per epilogue thread
+constexpr int kWEpiWarps = 16, kWThreads = 64 + 32 * kWEpiWarps;
+constexpr int kWCols = kWTok / (kWEpiWarps / 4);      // token columns per epilogue thread
+static_assert(kWCols == 16, "one TMEM load per accumulator");
+
+// two fp32 values in one register pair: one instruction for both, each rounded as by its scalar form
+__device__ __forceinline__ uint64_t pack2u(uint32_t a, uint32_t b) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t pack2(float a, float b) { return pack2u(__float_as_uint(a), __float_as_uint(b)); }
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// The wait for TMEM loads names their registers, so that nothing which reads them can be moved in front of it.
+__device__ __forceinline__ void tmem_landed(uint32_t (&v)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]),
+                 "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])::"memory");
+}
 
 // Persistent CTAs (one per SM) walk the (feature tile, item) work list with a fixed stride, so the TMA producer
 // and the MMA issuer run ahead into the next tile while the epilogue warps still store the previous one; the
@@ -77,7 +105,7 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < Cfg::kStages; ++i) { mbar_init(&tail->full[i], 1); mbar_init(&tail->empty[i], 1); }
-    for (int i = 0; i < Cfg::kAccBufs; ++i) { mbar_init(&tail->acc_full[i], 1); mbar_init(&tail->acc_empty[i], 256); }
+    for (int i = 0; i < Cfg::kAccBufs; ++i) { mbar_init(&tail->acc_full[i], 1); mbar_init(&tail->acc_empty[i], kWEpiWarps); }
     mbar_fence_init();
     tma_prefetch_desc(&tmA0);
     tma_prefetch_desc(&tmB);
@@ -102,16 +130,16 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     if (elect_one()) {
       bool ready = !(p.fab.ag_call >= 0 && p.fab.tp > 1);
       bool ok = true;
-      int u = 0;                                               // stage counter over all tiles of this CTA
+      int st = 0;                                              // stage, over all tiles of this CTA
+      uint32_t phase = 1;
+      bool first = true;                                       // the ring has not been filled once
       for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
         NRT_WIDE_DECODE(w, n_tile, item)
         if (item >= na) continue;
         const int z = p.active_ids[item];
         const int brow = p.row_offsets ? p.row_offsets[item] : item * kWTok;
-        for (int kb = 0; kb < kb_total; ++kb, ++u) {
-          const int st = u % Cfg::kStages;
-          if (u >= Cfg::kStages &&
-              !mbar_wait(&tail->empty[st], ((u / Cfg::kStages) & 1) ^ 1, p.status, kSiteStageEmpty | st)) { ok = false; break; }
+        for (int kb = 0; kb < kb_total; ++kb) {
+          if (!first && !mbar_wait(&tail->empty[st], phase, p.status, kSiteStageEmpty | st)) { ok = false; break; }
           uint8_t* sa = smem + st * Cfg::kStageBytes;
           const int kx = kb * kElemsPerStage;
           mbar_expect_tx(&tail->full[st], Cfg::kStageBytes);
@@ -131,35 +159,32 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
             ready = true;
           }
           tma_load_2d(sa + (DUAL ? 2 : 1) * kATileBytes, &tmB, &tail->full[st], kx, brow);
+          if (++st == Cfg::kStages) { st = 0; phase ^= 1; first = false; }
         }
       }
     }
   } else if (warp == 1) {
     if (elect_one()) {
+      // One thread runs this loop for every K block, so it is kept short: descriptors by addition, counters instead of remainders.
       constexpr uint32_t idesc = umma_idesc(FP8 ? 0u : 1u, kTileN, kWTok);
+      const uint64_t desc = umma_desc_sw128(smem_u32(smem));
       bool ok = true;
-      int u = 0, v = 0, t = 0;                                 // stages, accumulator uses, live tiles of this CTA
+      int st = 0, buf = 0, uses = 0;                           // stage, accumulator, accumulators handed out
+      uint32_t phase = 0, acc_phase = 1;
       for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
         NRT_WIDE_DECODE(w, n_tile, item)
         (void)n_tile;
         if (item >= na) continue;
-        for (int kb = 0; kb < kb_total; ++kb, ++u) {
-          const int st = u % Cfg::kStages;
-          // e4m3: a fresh accumulator per K block; bf16: one accumulator per tile, two tiles in flight
-          const bool new_acc = FP8 || kb == 0;
-          const int buf = FP8 ? (v % Cfg::kAccBufs) : (t % Cfg::kAccBufs);
-          if (new_acc) {
-            const int uses = FP8 ? v : t;
-            if (uses >= Cfg::kAccBufs &&
-                !mbar_wait(&tail->acc_empty[buf], ((uses / Cfg::kAccBufs) & 1) ^ 1, p.status, kSiteAccEmpty | buf)) { ok = false; break; }
+        for (int kb = 0; kb < kb_total; ++kb) {
+          if (FP8 ? (kb & 1) == 0 : kb == 0) {
+            if (uses >= Cfg::kAccBufs && !mbar_wait(&tail->acc_empty[buf], acc_phase, p.status, kSiteAccEmpty | buf)) { ok = false; break; }
+            ++uses;
           }
-          if (!mbar_wait(&tail->full[st], (u / Cfg::kStages) & 1, p.status, kSiteTmaFull | st)) { ok = false; break; }
+          if (!mbar_wait(&tail->full[st], phase, p.status, kSiteTmaFull | st)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t sa = smem_u32(smem + st * Cfg::kStageBytes);
-          const uint64_t da0 = umma_desc_sw128(sa);
-          const uint64_t da1 = umma_desc_sw128(sa + kATileBytes);
-          const uint64_t db = umma_desc_sw128(sa + (DUAL ? 2 : 1) * kATileBytes);
-          const uint32_t d0 = tmem + buf * Cfg::kAccCols;
+          const uint64_t da0 = desc + (uint32_t)(st * Cfg::kStageBytes >> 4);
+          const uint64_t da1 = da0 + (kATileBytes >> 4), db = da0 + ((DUAL ? 2 : 1) * kATileBytes >> 4);
+          const uint32_t d0 = tmem + (buf * Cfg::kPair + (FP8 ? kb & 1 : 0)) * Cfg::kAccCols;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const uint32_t acc = FP8 ? (j > 0) : (kb > 0 || j > 0);
@@ -171,93 +196,142 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
             }
           }
           umma_commit(&tail->empty[st]);
-          if (FP8 || kb == kb_total - 1) umma_commit(&tail->acc_full[buf]);
-          if (FP8) ++v;
+          if (kb == kb_total - 1 || (FP8 && (kb & 1))) {
+            umma_commit(&tail->acc_full[buf]);
+            if (++buf == Cfg::kAccBufs) { buf = 0; acc_phase ^= 1; }
+          }
+          if (++st == Cfg::kStages) { st = 0; phase ^= 1; }
         }
-        ++t;
       }
     }
   } else {
+    // e4m3: every K block is promoted - commit, load from TMEM, scale, add - and these hand-overs and the two threads that drive the
+    // ring are what bounds a block, not the tensor cores (29 % busy) or the copies.  Per K block: o_proj (K 8192, 2048 rows, weights in
+    // L2) 382 ns, 500 ns with one accumulator per hand-over and eight warps that finished one block before they asked for the next; gate
+    // and up of 256 experts of ~64 rows 767 ns (4.2 TB/s of weights), 1079 ns.
     const int quad = warp & 3;                       // TMEM lane quadrant this warp may read
-    const int half = (warp - 2) >> 2;                // which 32 token columns
-    const int c0 = half * kWHalf;
+    const int c0 = ((warp - 2) >> 2) * kWCols;       // first of its token columns
     const int row = quad * 32 + lane;                // feature within the tile
-    const int e = threadIdx.x - 64;                  // 0..255 among the epilogue threads
-    const uint32_t lane_addr = tmem + (uint32_t(quad * 32) << 16);
+    const int e = threadIdx.x - 64;                  // 0..511 among the epilogue threads
+    const uint32_t lane_addr = tmem + (uint32_t(quad * 32) << 16) + c0;
     const int nt_count = p.n_total / kTileN;
     bool ok = true;
-    int v = 0, t = 0;
+    int v = 0, t = 0;                                // pairs of K blocks and tiles so far
     for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
       NRT_WIDE_DECODE(w, n_tile, item)
       if (item >= na) continue;
       const int z = p.active_ids[item];
       const int brow = p.row_offsets ? p.row_offsets[item] : item * kWTok;
       const int n = n_tile * kTileN + row;
-      float acc0[kWHalf];
-      float acc1[DUAL ? kWHalf : 1];
-#pragma unroll
-      for (int r = 0; r < kWHalf; ++r) acc0[r] = 0.f;
-      if (DUAL) {
-#pragma unroll
-        for (int r = 0; r < kWHalf; ++r) acc1[r] = 0.f;
-      }
+      float acc0[kWCols];
+      float acc1[DUAL ? kWCols : 1];
       if (FP8) {
+        uint32_t b0[16], b1[16];
+        uint64_t sum0[kWCols / 2], sum1[DUAL ? kWCols / 2 : 1];       // two columns each
+#pragma unroll
+        for (int r = 0; r < kWCols / 2; ++r) {
+          sum0[r] = 0;
+          if (DUAL) sum1[DUAL ? r : 0] = 0;
+        }
         const float* ws0 = p.w_scale0 + ((size_t)z * nt_count + n_tile) * kb_total;
         const float* ws1 = DUAL ? p.w_scale1 + ((size_t)z * nt_count + n_tile) * kb_total : nullptr;
-        for (int kb = 0; kb < kb_total; ++kb, ++v) {
-          const int buf = v % Cfg::kAccBufs;
-          const float w0 = __ldg(ws0 + kb);
-          const float w1 = DUAL ? __ldg(ws1 + kb) : 0.f;
-          if (!mbar_wait(&tail->acc_full[buf], (v / Cfg::kAccBufs) & 1, p.status, kSiteAccFull | buf)) { ok = false; break; }
-          if (kb == 0) {
-            // activation scales of the item's 64 rows, transposed to [K block][row]; read coherently after the first
-            // accumulator is ready (in the expert-parallel path peers wrote them shortly before).  The first barrier
-            // keeps a fast warp from overwriting the table while a slow one still reads the previous tile's scales.
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-            const float* as = p.a_scale + (size_t)brow * kb_total;
-            for (int i = e; i < kWTok * kb_total; i += 256) {
-              const int r = i / kb_total, k = i - r * kb_total;
-              as_s[k * kWTok + r] = __ldcv(as + i);
-            }
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-          }
+        float wl0 = 0.f, wl1 = 0.f;                                   // scales of 32 K blocks, one per lane
+        // wait for the pair of K blocks from `kb` on and request the first's accumulator
+        auto ask = [&](int kb) {
+          const int use = v + (kb >> 1), buf = use % Cfg::kAccBufs;
+          if (!__all_sync(0xffffffffu, mbar_wait(&tail->acc_full[buf], (use / Cfg::kAccBufs) & 1, p.status, kSiteAccFull | buf))) return false;
           tc_fence_after();
-          uint32_t v0[kWHalf], v1[DUAL ? kWHalf : 1];
-          const uint32_t t0 = lane_addr + buf * Cfg::kAccCols + c0;
-          tmem_ld16_nowait(t0, v0);
-          tmem_ld16_nowait(t0 + 16, v0 + 16);
-          if (DUAL) {
-            tmem_ld16_nowait(t0 + kWTok, v1);
-            tmem_ld16_nowait(t0 + kWTok + 16, v1 + 16);
-          }
-          tmem_ld_wait();
+          tmem_ld16_nowait(lane_addr + buf * 2 * Cfg::kAccCols, b0);
+          return true;
+        };
+        auto acc_of = [&](int kb) { return lane_addr + ((v + (kb >> 1)) % Cfg::kAccBufs * 2 + (kb & 1)) * Cfg::kAccCols; };
+        auto give_back = [&](int kb) {                                // the warp's values are in registers
           tc_fence_before();
-          mbar_arrive(&tail->acc_empty[buf]);            // values are in registers: the buffer can be reused
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tail->acc_empty[(v + (kb >> 1)) % Cfg::kAccBufs]);
+        };
+        auto scales = [&](int kb) {
+          if ((kb & 31) == 0) {
+            wl0 = kb + lane < kb_total ? __ldg(ws0 + kb + lane) : 0.f;
+            if (DUAL) wl1 = kb + lane < kb_total ? __ldg(ws1 + kb + lane) : 0.f;
+          }
+        };
+        auto add = [&](uint64_t* sum, const uint32_t (&b)[16], int kb, float wl) {
+          const float wv = __shfl_sync(0xffffffffu, wl, kb & 31);
+          const uint64_t ww = pack2(wv, wv);
           const float4* sc4 = reinterpret_cast<const float4*>(as_s + kb * kWTok + c0);
 #pragma unroll
-          for (int q = 0; q < kWHalf / 4; ++q) {
+          for (int q = 0; q < kWCols / 4; ++q) {
             const float4 s = sc4[q];
-            const float sv[4] = {s.x, s.y, s.z, s.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              acc0[q * 4 + j] += __uint_as_float(v0[q * 4 + j]) * (sv[j] * w0);
-              if (DUAL) acc1[q * 4 + j] += __uint_as_float(v1[DUAL ? q * 4 + j : 0]) * (sv[j] * w1);
+            sum[q * 2] = fma2(pack2u(b[q * 4], b[q * 4 + 1]), mul2(pack2(s.x, s.y), ww), sum[q * 2]);
+            sum[q * 2 + 1] = fma2(pack2u(b[q * 4 + 2], b[q * 4 + 3]), mul2(pack2(s.z, s.w), ww), sum[q * 2 + 1]);
+          }
+        };
+        ok = ask(0);
+        if (!ok) break;
+        // activation scales of the item's 64 rows, transposed to [K block][row]; read coherently after the first
+        // accumulator is ready (in the expert-parallel path peers wrote them shortly before).  The first barrier
+        // keeps a fast warp from overwriting the table while a slow one still reads the previous tile's scales.
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+        const float* as = p.a_scale + (size_t)brow * kb_total;
+        for (int i = e; i < kWTok * kb_total; i += 32 * kWEpiWarps) {
+          const int r = i / kb_total, k = i - r * kb_total;
+          as_s[k * kWTok + r] = __ldcv(as + i);
+        }
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+        // one accumulator is on its way while the one before it is added
+        for (int kb = 0; kb < kb_total; kb += 2) {
+          const bool two = kb + 1 < kb_total, more = kb + 2 < kb_total;
+          scales(kb);
+          tmem_landed(b0);
+          if (DUAL) {
+            tmem_ld16_nowait(acc_of(kb) + kWTok, b1);
+            add(sum0, b0, kb, wl0);
+            tmem_landed(b1);
+            if (two) {
+              tmem_ld16_nowait(acc_of(kb + 1), b0);
+              add(sum1, b1, kb, wl1);
+              tmem_landed(b0);
+              tmem_ld16_nowait(acc_of(kb + 1) + kWTok, b1);
+              add(sum0, b0, kb + 1, wl0);
+              tmem_landed(b1);
+            }
+            give_back(kb);
+            if (more && !(ok = ask(kb + 2))) break;
+            add(sum1, b1, two ? kb + 1 : kb, wl1);
+          } else {
+            if (two) {
+              tmem_ld16_nowait(acc_of(kb + 1), b1);
+              add(sum0, b0, kb, wl0);
+              tmem_landed(b1);
+              give_back(kb);
+              if (more && !(ok = ask(kb + 2))) break;
+              add(sum0, b1, kb + 1, wl0);
+            } else {
+              give_back(kb);
+              add(sum0, b0, kb, wl0);
             }
           }
         }
         if (!ok) break;
+        v += (kb_total + 1) / 2;
+#pragma unroll
+        for (int r = 0; r < kWCols / 2; ++r) {
+          unpack2(sum0[r], acc0[2 * r], acc0[2 * r + 1]);
+          if (DUAL) unpack2(sum1[DUAL ? r : 0], acc1[DUAL ? 2 * r : 0], acc1[DUAL ? 2 * r + 1 : 0]);
+        }
       } else {
         const int buf = t % Cfg::kAccBufs;
-        if (!mbar_wait(&tail->acc_full[buf], (t / Cfg::kAccBufs) & 1, p.status, kSiteAccFull | buf)) { ok = false; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait(&tail->acc_full[buf], (t / Cfg::kAccBufs) & 1, p.status, kSiteAccFull | buf))) { ok = false; break; }
         tc_fence_after();
-        uint32_t v0[kWHalf];
-        tmem_ld16_nowait(lane_addr + buf * Cfg::kAccCols + c0, v0);
-        tmem_ld16_nowait(lane_addr + buf * Cfg::kAccCols + c0 + 16, v0 + 16);
-        tmem_ld_wait();
+        uint32_t v0[16];
+        tmem_ld16_nowait(lane_addr + buf * Cfg::kAccCols, v0);
+        tmem_landed(v0);
         tc_fence_before();
-        mbar_arrive(&tail->acc_empty[buf]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tail->acc_empty[buf]);
 #pragma unroll
-        for (int r = 0; r < kWHalf; ++r) acc0[r] = __uint_as_float(v0[r]);
+        for (int r = 0; r < kWCols; ++r) acc0[r] = __uint_as_float(v0[r]);
       }
       ++t;
 
@@ -266,23 +340,23 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
       if (EPI == kEpiStoreF32) {
         if (live)
 #pragma unroll
-          for (int r = 0; r < kWHalf; ++r) p.out_f32[(out_row0 + r) * p.ld_out + n] = acc0[r] * p.out_scale;
+          for (int r = 0; r < kWCols; ++r) p.out_f32[(out_row0 + r) * p.ld_out + n] = acc0[r] * p.out_scale;
       } else if (EPI == kEpiStoreBF16) {
         if (live)
 #pragma unroll
-          for (int r = 0; r < kWHalf; ++r) p.out_bf16[(out_row0 + r) * p.ld_out + n] = __float2bfloat16_rn(acc0[r] * p.out_scale);
+          for (int r = 0; r < kWCols; ++r) p.out_bf16[(out_row0 + r) * p.ld_out + n] = __float2bfloat16_rn(acc0[r] * p.out_scale);
       } else if (EPI == kEpiSiluQuant) {
 #pragma unroll
-        for (int r = 0; r < kWHalf; ++r) {
+        for (int r = 0; r < kWCols; ++r) {
           acc0[r] = silu(acc0[r]) * acc1[DUAL ? r : 0];
           float m = fabsf(acc0[r]);
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
           if (lane == 0) tail->red[quad][c0 + r] = m;
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
+        asm volatile("bar.sync 1, 512;" ::: "memory");
 #pragma unroll
-        for (int r = 0; r < kWHalf; ++r) {
+        for (int r = 0; r < kWCols; ++r) {
           const int c = c0 + r;
           const float am = fmaxf(fmaxf(tail->red[0][c], tail->red[1][c]), fmaxf(tail->red[2][c], tail->red[3][c]));
           const float s = pow2_scale(am);
@@ -290,13 +364,13 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
           p.out_q[(out_row0 + r) * p.n_total + n] = *reinterpret_cast<const uint8_t*>(&q);
           if (row == 0) p.out_qscale[(out_row0 + r) * nt_count + n_tile] = s;
         }
-        asm volatile("bar.sync 1, 256;" ::: "memory");      // the amax scratch is reused by the next tile
+        asm volatile("bar.sync 1, 512;" ::: "memory");      // the amax scratch is reused by the next tile
       } else if (EPI == kEpiReturn) {
         const uint32_t dtag = (*p.fab.epoch) * 1024u + (uint32_t)p.ep_dispatch_call + 1u;
         const uint32_t rtag = (*p.fab.epoch) * 1024u + (uint32_t)p.ep_return_call + 1u;
         const int words = p.n_total / 2;
 #pragma unroll
-        for (int r = 0; r < kWHalf; ++r) {
+        for (int r = 0; r < kWCols; ++r) {
           const int4 m = p.ep_meta[out_row0 + r];
           const float other = __shfl_down_sync(0xffffffffu, acc0[r], 1);
           if ((uint32_t)m.w == dtag && (lane & 1) == 0) {

@@ -257,3 +257,37 @@ def test_chunk_gemm_fp8_gate_up_matches_torch():
     assert (got - want).abs().max().item() <= 0.07 * want.abs().max().item()
     wq, wsc = quantize_act_pow2(want)
     assert torch.equal(ys, wsc.float()) or (ys - wsc.float()).abs().max().item() <= ys.max().item()
+
+
+@pytest.mark.parametrize("k,n,rows", [(128, 128, 64), (256, 384, 64), (384, 256, 192), (1152, 128, 128), (4224, 256, 64), (640, 2048, 1024)])
+def test_chunk_gemm_fp8_pairs_of_k_blocks(k, n, rows):
+    """One, two, odd and many K blocks (accumulators change hands in pairs), more tiles than CTAs: e4m3 products against the torch
+    recipe.  fp32 sums of k products of bf16-rounded outputs: 2^-8 of the value and k 2^-24 of the magnitudes."""
+    K = _setup()
+    from naivert_b200.ops.quant import dequant_act, quantize_act_pow2, quantize_fp8_block, w8a8_linear_ref
+    g = torch.Generator(device="cuda").manual_seed(k + n)
+    ws = [quantize_fp8_block(torch.randn(n, k, device="cuda", generator=g) * 0.05) for _ in range(2)]
+    x = torch.randn(rows, k, device="cuda", generator=g).bfloat16().float()
+    xq, xs = quantize_act_pow2(x)
+    x8, xs = xq.view(torch.uint8).contiguous(), xs.float().contiguous()
+    off, ids, cnt = _items(rows // 64)
+    maps = [K.weight_tmap(w.view(torch.uint8)) for w, _ in ws]
+    for dual in (False, True):
+        out = torch.zeros(rows, n, dtype=torch.bfloat16, device="cuda")
+        y8, ys, st = torch.zeros(rows, n, dtype=torch.uint8, device="cuda"), torch.zeros(rows, n // 128, device="cuda"), _status()
+        a = K.GemmArgs()
+        a.n_total, a.k_total, a.rows, a.out_scale = n, k, 64, 1.0
+        a.n_active, a.active_ids, a.max_slots, a.row_offsets = cnt.data_ptr(), ids.data_ptr(), rows // 64, off.data_ptr()
+        a.w_scale0, a.w_scale1, a.a_scale = ws[0][1].data_ptr(), ws[1][1].data_ptr(), xs.data_ptr()
+        a.out_q, a.out_qscale, a.out_bf16, a.ld_out, a.status = y8.data_ptr(), ys.data_ptr(), out.data_ptr(), n, st.data_ptr()
+        K.wide_gemm(K.gemm_variant(True, dual, K.EPI_SILU_QUANT if dual else K.EPI_STORE_BF16, K.GROUP_ITEM), maps[0], maps[1] if dual else None,
+                    K.act_tmap(x8, 64), a, n // 128, rows // 64)
+        torch.cuda.synchronize()
+        assert int(st[0]) == 0
+        gate, up = (w8a8_linear_ref(x, w, s) for w, s in ws)
+        if dual:
+            want = torch.nn.functional.silu(gate) * up
+            assert (dequant_act(y8.view(torch.float8_e4m3fn), ys) - want).abs().max().item() <= 0.07 * want.abs().max().item()
+        else:
+            slack = k * 2.0 ** -24 * dequant_act(xq, xs).abs().max() * k ** 0.5
+            assert ((out.float() - gate).abs() <= 2.0 ** -8 * gate.abs() + slack).all()
