@@ -1,7 +1,7 @@
 // Token-chunk products of layer stacks.
 //
 // Tensor-core form (bf16): features are the M = 128 side of tcgen05.mma (weights = A operand), token rows the N side
-// (64, 128 or 256 per tile), both staged by TMA with 128-byte swizzle.  Persistent CTAs walk the (feature tile, item)
+// (64, 128, 192 or 256 per tile), both staged by TMA with 128-byte swizzle.  Persistent CTAs walk the (feature tile, item)
 // list; two accumulators in TMEM let the products of the next tile run under the stores of the previous one.
 //   warp 0    TMA producer        warp 1    UMMA issuer (and TMEM owner)
 //   warps 2-9 epilogue: thread = feature x one half of the token columns
@@ -29,10 +29,11 @@ struct Cfg {
   static constexpr int kStage = (DUAL ? 2 : 1) * kATile + NTOK * 128;
   static constexpr int kStages = (200 * 1024) / kStage > 8 ? 8 : (200 * 1024) / kStage;
   static constexpr int kAccCols = (DUAL ? 2 : 1) * NTOK;
-  static constexpr int kTmem = 2 * kAccCols;                     // two tiles in flight
+  static constexpr int kBufs = 2 * kAccCols <= 512 ? 2 : 1;      // two tiles in flight where they fit
+  static constexpr int kTmem = kBufs * kAccCols <= 128 ? 128 : kBufs * kAccCols <= 256 ? 256 : 512;
   static constexpr int kSmem = kStages * kStage + 1024 + 512;
 };
-static_assert(Cfg<256, false>::kTmem == 512 && Cfg<128, true>::kTmem == 512 && Cfg<64, false>::kTmem == 128, "TMEM columns");
+static_assert(Cfg<256, false>::kTmem == 512 && Cfg<128, true>::kTmem == 512 && Cfg<64, false>::kTmem == 128 && Cfg<192, true>::kBufs == 1, "TMEM columns");
 
 struct Tail {
   uint64_t full[8], empty[8], acc_full[2], acc_empty[2];
@@ -136,8 +137,8 @@ stack_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         NRT_TILE(w, tile, item)
         (void)tile;
         if (!item_of(p, item, row_tiles, NTOK, na).live) continue;
-        const int buf = t & 1;
-        if (t >= 2 && !mbar_wait(&tail->acc_empty[buf], ((t >> 1) & 1) ^ 1, p.status, kSiteAccEmpty | buf)) { ok = false; break; }
+        const int buf = t % C::kBufs;
+        if (t >= C::kBufs && !mbar_wait(&tail->acc_empty[buf], ((t / C::kBufs) & 1) ^ 1, p.status, kSiteAccEmpty | buf)) { ok = false; break; }
         tc_fence_after();
         for (int kb = 0; kb < kb_total; ++kb, ++u) {
           const int st = u % C::kStages;
@@ -168,8 +169,8 @@ stack_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       NRT_TILE(w, tile, item)
       const Item it = item_of(p, item, row_tiles, NTOK, na);
       if (!it.live) continue;
-      const int buf = t & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(&tail->acc_full[buf], (t >> 1) & 1, p.status, kSiteAccFull | buf));
+      const int buf = t % C::kBufs;
+      ok = __all_sync(0xffffffffu, mbar_wait(&tail->acc_full[buf], (t / C::kBufs) & 1, p.status, kSiteAccFull | buf));
       if (!ok) break;
       tc_fence_after();
       const int n = tile * kFeat + feat;
@@ -433,7 +434,7 @@ int launch_f32(const StackGemmArgs& a, cudaStream_t stream) {
 
 extern "C" int nrt_stack_gemm_args_size() { return (int)sizeof(StackGemmArgs); }
 
-// ntok: token rows per tile (64, 128, 256; two-product epilogues 64 or 128); the token map's box has that many rows.
+// ntok: token rows per tile (64 to 256; two-product epilogues up to 192); the token map's box has that many rows.
 extern "C" int nrt_stack_gemm(int epi, int ntok, const void* tmW, const void* tmW2, const void* tmX, const void* args,
                               int items_fastest, void* stream) {
   CUtensorMap w, w2, x;
@@ -448,12 +449,12 @@ extern "C" int nrt_stack_gemm(int epi, int ntok, const void* tmW, const void* tm
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
 #define NRT_CASE(N, E) \
   if (ntok == N && epi == E) return launch<N, E>(w, w2, x, a, items_fastest, s);
-  NRT_CASE(64, kSEpiStore) NRT_CASE(128, kSEpiStore) NRT_CASE(256, kSEpiStore)
-  NRT_CASE(64, kSEpiBias) NRT_CASE(256, kSEpiBias)
+  NRT_CASE(64, kSEpiStore) NRT_CASE(128, kSEpiStore) NRT_CASE(192, kSEpiStore) NRT_CASE(256, kSEpiStore)
+  NRT_CASE(64, kSEpiBias) NRT_CASE(128, kSEpiBias) NRT_CASE(192, kSEpiBias) NRT_CASE(256, kSEpiBias)
   NRT_CASE(64, kSEpiTranspose) NRT_CASE(256, kSEpiTranspose)
-  NRT_CASE(64, kSEpiClampedGlu) NRT_CASE(128, kSEpiClampedGlu)
+  NRT_CASE(64, kSEpiClampedGlu) NRT_CASE(128, kSEpiClampedGlu) NRT_CASE(192, kSEpiClampedGlu)
   NRT_CASE(64, kSEpiSiluGlu) NRT_CASE(128, kSEpiSiluGlu)
-  NRT_CASE(64, kSEpiRelu2) NRT_CASE(128, kSEpiRelu2) NRT_CASE(256, kSEpiRelu2)
+  NRT_CASE(64, kSEpiRelu2) NRT_CASE(128, kSEpiRelu2) NRT_CASE(192, kSEpiRelu2) NRT_CASE(256, kSEpiRelu2)
   NRT_CASE(64, kSEpiTanh) NRT_CASE(256, kSEpiTanh)
   NRT_CASE(64, kSEpiDecaySoft) NRT_CASE(256, kSEpiDecaySoft)
   NRT_CASE(64, kSEpiDecayExp) NRT_CASE(256, kSEpiDecayExp)

@@ -23,6 +23,9 @@ from ..runtime.stack import StackRuntime
 from .stack_mixers import MIXERS
 
 SMS = 148
+# tile sizes of the chunk products by epilogue (the others: 64 and 256)
+TILE_ROWS = {S.EPI_STORE: (64, 128, 192, 256), S.EPI_RELU2: (64, 128, 192, 256), S.EPI_BIAS: (64, 128, 192, 256), S.EPI_CLAMPED_GLU: (64, 128, 192),
+             S.EPI_SILU_GLU: (64, 128)}
 # Pairs (token, choice) per expert that a span is filled up to, and its most rows.  Below, an expert's product is bound by the read of its
 # weights (12.9 GB a layer at 256 experts of 4096 x 2048), which a span does once: with three such layers, 8192 rows in chunks of 2048 take
 # 30.1 ms, 47.0 ms when every chunk went through the experts by itself (their products: 28.3 -> 11.0 ms).  A span's rows cost 2 GB there.
@@ -122,6 +125,18 @@ class StackPrefill:
             self.maps[key] = S.weight_map(p.w, p.k)
         return self.maps[key]
 
+    @staticmethod
+    def tile_rows(epi: int, tiles: int, rows: int) -> int:
+        """Token rows per tile of a product with ``tiles`` feature tiles.  Few rows are one tile where the feature tiles occupy about
+        half of the SMs: every weight is then fetched by one CTA only, and what is in flight - which bounds a product that streams
+        its weights - is all different: 152,576 features of 4096 x 1 row 419 -> 212 us, 10,240 x 187 rows 49 -> 38 us, and 16,384 x 187
+        rows of two products 90 -> 87 us against the widest tile that fills the SMs, which larger products take."""
+        sizes = TILE_ROWS.get(epi, (64, 256))
+        whole = next((t for t in sizes if t >= rows), None)
+        if whole is not None and tiles >= 64:
+            return whole
+        return next((t for t in reversed(sizes) if t != 192 and tiles * -(-rows // t) >= SMS - 20), 64)
+
     def _xmap(self, t: torch.Tensor, k: int, zcount: int, zstride: int, rows: int, ld: int, box: int, offset: int) -> K.TensorMap:
         key = ("x", t.data_ptr(), k, zcount, zstride, rows, ld, box, offset)
         if key not in self.maps:
@@ -151,9 +166,7 @@ class StackPrefill:
         if items is not None:
             ntok = items[0]
         else:
-            tiles = -(-w.n // 128) * z
-            sizes = (128, 64) if dual else (256, 128, 64) if epi in (S.EPI_STORE, S.EPI_RELU2) else (256, 64)
-            ntok = next((t for t in sizes if tiles * -(-rows // t) >= SMS - 20), 64)
+            ntok = self.tile_rows(epi, -(-w.n // 128) * z, rows)
         live = x_rows if x_rows is not None else x.numel() // x_ld
         xm = self._xmap(x, w.k, z, x_z, live, x_ld, ntok, x_off)
         wbytes = w.nbytes * (2 if dual else 1)

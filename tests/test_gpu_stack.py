@@ -337,6 +337,33 @@ def test_plain_chunk_attention_against_torch(rows, heads, group, dim, vdim, pos0
     assert float((out.double() - want).abs().max() / want.abs().max()) < (5e-6 if f32 else 2.0 ** -8)
 
 
+@pytest.mark.parametrize("rows", [1, 64, 65, 129, 187, 192, 193, 256])
+def test_few_rows_are_one_tile(rows):
+    """Products of many features: tiles of 64 to 256 rows, one and (two products of 192 rows) a single accumulator in flight."""
+    from naivert_b200.ops import stack_kernels as S
+    from naivert_b200.runtime.packing import pack
+    cfg = CASES["mixed"]
+    eng = engine(cfg, weights(cfg), "bf16", capacity=256, chunk=256)
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    n, k = 20000, 136                                            # 157 feature tiles: some CTAs have two
+    try:
+        assert eng.prefill.tile_rows(S.EPI_STORE, 157, rows) == -(-rows // 64) * 64
+        x = torch.randn(rows, k, generator=g, device="cuda").to(torch.bfloat16)
+        w, w2 = (torch.randn(n, k, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+        a, b = x.double() @ w.double().t(), x.double() @ w2.double().t()
+        p, p2, bias = pack(w, "cuda"), pack(w2, "cuda"), torch.randn(n, generator=g, device="cuda").to(torch.bfloat16)
+        gl, u = a.clamp(max=1.2), b.clamp(-1.2, 1.2)
+        for epi, want, more in ((S.EPI_STORE, a, {}), (S.EPI_BIAS, a + bias.double(), dict(bias=bias)), (S.EPI_RELU2, a.clamp(min=0) ** 2, {}),
+                                (S.EPI_CLAMPED_GLU, gl * torch.sigmoid(1.702 * gl) * (u + 1), dict(w2=p2, limit=1.2, alpha=1.702))):
+            out = torch.full((rows, n), float("nan"), device="cuda")
+            eng.prefill.gemm(epi, p, x, k, rows, out, n, **more)
+            torch.cuda.synchronize()
+            assert float((out.double() - want).abs().max() / want.abs().max()) < 1e-4, epi
+        eng.fabric.check()
+    finally:
+        eng.close()
+
+
 @pytest.mark.parametrize("rows", [1, 63, 200, 700])
 def test_products_against_torch(rows):
     """Every epilogue and tile width of the chunk product, sizes off every multiple."""
