@@ -266,39 +266,43 @@ __global__ void __launch_bounds__(kDecThreads) group_decode_kernel(const GroupDe
   cluster_sync_all();                                                    // nobody leaves while its shared memory is read
 }
 
-// Tensor-core form: grid (splits, key heads, tiles of 16 or 32 query heads).  The query heads of a key head are the M side of bf16
-// m16n8k16 MMAs; keys and values come 64 at a time through two to four cp.async stages, the first requested before the wait for the
-// predecessor (older rows do not depend on it; the token's own row is put into its tile by hand).  tcgen05 is not used: the kernel
-// streams the cache once, and most of its M = 128 rows would idle.
-constexpr int kTcHead = 256;
+// Tensor-core form: grid (splits, key heads, tiles of 16 query heads).  The query heads of a key head are the M side of bf16 m16n8k16
+// MMAs.  A warp walks every so-many-th tile of 16 keys of the split through a ring of its own and keeps scores, probabilities (a score
+// fragment is the A fragment of P V as it stands) and outputs in registers: no barrier inside the walk, and the eight rings together keep the
+// 140 KB in flight that one SM's share of the memory's rate needs.  The warps' results are merged once, then the cluster's.  The first
+// tiles are requested before the wait for the predecessor (older rows do not depend on it; the token's own row is put into its tile by
+// hand).  tcgen05 is not used: the kernel streams the cache once, and most of its M = 128 rows would idle.
+// 12,290 keys, 8 key heads of 4 x 128: 40 us inside a step; 62 us with tiles of 64 keys that all warps worked on between four barriers.
+constexpr int kTcHead = 256, kWalkKeys = 16, kWalkM = 16, kWalkSmem = 225 * 1024;
 __host__ __device__ inline int tc_pitch(int n) { return (n + 15) / 16 * 16 + 8; }              // bf16 elements; rows fall into distinct banks
-__host__ __device__ inline int group_tc_smem(int dp, int vp, int ht, int stages) {
-  return 2 * (ht + stages * kTile) * tc_pitch(dp) + 2 * stages * kTile * tc_pitch(vp) + 4 * ht * (kTile + 4) + 2 * ht * (kTile + 8) + 4 * 3 * ht + 4 * ht * vp +
-         4 * (8 * kTcHead + kTcHead) + 2 * (dp + vp);
+struct WalkShape { int warps, stages; };               // walking warps of a CTA, ring stages of each
+__host__ __device__ inline int walk_ring(int dp, int vp, WalkShape w) { return 2 * w.warps * w.stages * kWalkKeys * (tc_pitch(dp) + tc_pitch(vp)); }
+__host__ __device__ inline int walk_smem(int dp, int vp, WalkShape w) {
+  return walk_ring(dp, vp, w) + 2 * kWalkM * tc_pitch(dp) + 4 * (2 * kWalkM * (w.warps + 1) + 8 * kTcHead + kTcHead) + 2 * (dp + vp);
 }
 
-template <int MT>
-__global__ void __launch_bounds__(kDecThreads, 1) group_decode_tc_kernel(const GroupDecodeArgs a, const int stages) {
+// DIM: most columns of keys and values (registers of the outputs).  Up to 128 the kernel keeps to half of an SM's registers, so that it starts
+// while its predecessor still runs.
+template <int DIM>
+__global__ void __launch_bounds__(kDecThreads, DIM <= 128 ? 2 : 1) group_decode_tc_kernel(const GroupDecodeArgs a, const WalkShape ws) {
   extern __shared__ __align__(16) uint8_t raw[];
-  constexpr int HT = MT * 16, kSP = kTile + 4, kPP = kTile + 8, kNT = kTcHead / 64;
   const GroupPrepArgs& p = a.p;
-  const int kp = tc_pitch(p.dp), vpitch = tc_pitch(p.vp), rp = (p.dp + 15) / 16 * 16;
-  __nv_bfloat16* sq = reinterpret_cast<__nv_bfloat16*>(raw);             // [HT][kp]
-  __nv_bfloat16* sk = sq + HT * kp;                                      // [stages][64][kp]
-  __nv_bfloat16* sv = sk + stages * kTile * kp;                          // [stages][64][vpitch]
-  __nv_bfloat16* sp = sv + stages * kTile * vpitch;                           // [HT][kPP]
-  float* ss = reinterpret_cast<float*>(sp + HT * kPP);                   // [HT][kSP]
-  float* sm = ss + HT * kSP;
-  float* sl = sm + HT;
-  float* scorr = sl + HT;
-  float* so = scorr + HT;                                                // [HT][vp]
-  float* cs = so + HT * p.vp;
+  const int kp = tc_pitch(p.dp), vpitch = tc_pitch(p.vp), rp = (p.dp + 15) / 16 * 16, stage_elems = kWalkKeys * (kp + vpitch);
+  __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(raw);           // [warps][stages][16 keys, 16 values]
+  __nv_bfloat16* sq = ring + ws.warps * ws.stages * stage_elems;         // [16][kp]
+  float* sm = reinterpret_cast<float*>(sq + kWalkM * kp);                // [16], then [warps][16]
+  float* sl = sm + kWalkM * (ws.warps + 1);
+  float* cs = sl + kWalkM * (ws.warps + 1);
   float* sn = cs + kTcHead / 2;
   float* buf = sn + kTcHead / 2;                                         // [8][256]
   __nv_bfloat16* new_k = reinterpret_cast<__nv_bfloat16*>(buf + 8 * kTcHead);
   __nv_bfloat16* new_v = new_k + p.dp;
+  // after the walk the rings hold the warps' outputs and the CTA's
+  const int part_row = p.vp + 4;
+  float* part = reinterpret_cast<float*>(raw);                           // [warps][16][part_row]
+  float* so = part + ws.warps * kWalkM * part_row;                       // [16][vp]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int split = blockIdx.x, hk = blockIdx.y, group = p.heads / p.kv_heads, h0 = blockIdx.z * HT, nh = min(HT, group - h0);
+  const int split = blockIdx.x, hk = blockIdx.y, group = p.heads / p.kv_heads, h0 = blockIdx.z * kWalkM, nh = min(kWalkM, group - h0);
   const int half = p.rot_dims / 2;
   const int pos = *reinterpret_cast<const volatile int*>(p.pos0);
   const bool inside = pos >= 0 && pos < p.capacity;
@@ -306,41 +310,40 @@ __global__ void __launch_bounds__(kDecThreads, 1) group_decode_tc_kernel(const G
   const int per = ((n + a.splits - 1) / a.splits + kTile - 1) / kTile * kTile;
   const int j_lo = min(n, split * per), j_hi = min(n, j_lo + per);
   const bool owner = j_hi == n && j_lo < j_hi;
-  {
-    uint4* z = reinterpret_cast<uint4*>(raw);                            // columns beyond a head stay zero
-    const int words = ((HT + stages * kTile) * kp + stages * kTile * vpitch) / 8;
-    for (int i = tid; i < words; i += kDecThreads) z[i] = make_uint4(0u, 0u, 0u, 0u);
-  }
-  for (int i = tid; i < HT * p.vp; i += kDecThreads) so[i] = 0.f;
-  for (int i = tid; i < HT; i += kDecThreads) { sm[i] = -FLT_MAX; sl[i] = scorr[i] = 0.f; }
-  for (int i = tid; i < HT * kPP; i += kDecThreads) sp[i] = __float2bfloat16_rn(0.f);
-  __syncthreads();
+  const int step = ws.warps * kWalkKeys;                                 // keys from one tile of a warp to its next
   const __nv_bfloat16* kc = reinterpret_cast<const __nv_bfloat16*>(p.k_cache) + (long long)hk * p.dp;
   const __nv_bfloat16* vc = reinterpret_cast<const __nv_bfloat16*>(p.v_cache) + (long long)hk * p.vp;
-  // a thread copies one 16-byte piece of every so-many-th row
+  __nv_bfloat16* mine = ring + warp * ws.stages * stage_elems;
+  // a lane copies one 16-byte piece of every so-many-th row; rows beyond the split become zero
   auto rows_in = [&](int j0, __nv_bfloat16* dst, int pitch, const __nv_bfloat16* src, int width) {
     int lanes = 1;
     while (lanes < width / 8) lanes *= 2;
-    const int c = tid & (lanes - 1), step = kDecThreads / lanes;
+    const int c = lane & (lanes - 1), rows = 32 / lanes;
     if (c >= width / 8) return;
     const long long row_step = (long long)p.kv_heads * width;
-    int t = tid / lanes;
-    const __nv_bfloat16* s0 = src + (long long)(start + j0 + t) * row_step + c * 8;
-    __nv_bfloat16* d = dst + t * pitch + c * 8;
-#pragma unroll 4
-    for (; t < kTile; t += step, s0 += step * row_step, d += step * pitch) {
+#pragma unroll 8
+    for (int t = lane / lanes; t < kWalkKeys; t += rows) {
       const bool in = j0 + t < j_hi && j0 + t != n - 1;                  // the token's own row is not in the cache yet
-      cp16(d, in ? s0 : src, in);
+      cp16(dst + t * pitch + c * 8, in ? src + (long long)(start + j0 + t) * row_step + c * 8 : src, in);
     }
   };
-  auto request = [&](int j0, int st) {         // the 64 rows from j0 on (none beyond the split: an empty group keeps the count)
+  auto request = [&](int j0, int st) {         // the 16 rows from j0 on (none beyond the split: an empty group keeps the count)
     if (j0 < j_hi) {
-      rows_in(j0, sk + st * kTile * kp, kp, kc, p.dp);
-      rows_in(j0, sv + st * kTile * vpitch, vpitch, vc, p.vp);
+      rows_in(j0, mine + st * stage_elems, kp, kc, p.dp);
+      rows_in(j0, mine + st * stage_elems + kWalkKeys * kp, vpitch, vc, p.vp);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  for (int i = 0; i + 1 < stages; ++i) request(j_lo + i * kTile, i);
+  const int j_first = j_lo + warp * kWalkKeys;
+  const bool walks = warp < ws.warps;
+  if (walks) {
+    if (rp > p.dp)                                                       // columns between the head and a whole step stay zero
+      for (int i = lane; i < ws.stages * kWalkKeys; i += 32)
+        *reinterpret_cast<uint4*>(mine + i / kWalkKeys * stage_elems + i % kWalkKeys * kp + p.dp) = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = 0; i + 1 < ws.stages; ++i) request(j_first + i * step, i);
+  }
+  for (int i = tid; i < kWalkM * kp / 8; i += kDecThreads) reinterpret_cast<uint4*>(sq)[i] = make_uint4(0u, 0u, 0u, 0u);
+  for (int i = tid; i < kWalkM * (ws.warps + 1); i += kDecThreads) { sm[i] = -FLT_MAX; sl[i] = 0.f; }
   griddep_wait();
   griddep_launch();
   if (j_lo < j_hi) {
@@ -367,113 +370,121 @@ __global__ void __launch_bounds__(kDecThreads, 1) group_decode_tc_kernel(const G
       }
       __syncwarp();
     }
-    float o[MT][kNT][4];
+    __syncthreads();
+    const int fr = lane >> 2, fc = (lane & 3) * 2;
+    float o[DIM / 8][4], m[2] = {-FLT_MAX, -FLT_MAX}, l[2] = {0.f, 0.f};    // rows fr and fr + 8 of the sixteen heads
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
+    for (int t = 0; t < DIM / 8; ++t)
 #pragma unroll
-      for (int t = 0; t < kNT; ++t)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) o[i][t][q] = 0.f;
-    const int ntiles = p.vp / 8, fr = lane >> 2, fc = (lane & 3) * 2;
-    const float c2 = 1.4426950408889634f;                                // scores in powers of two
-    int st = 0;
-    for (int j0 = j_lo; j0 < j_hi; j0 += kTile, st = st + 1 == stages ? 0 : st + 1) {
-      request(j0 + (stages - 1) * kTile, st == 0 ? stages - 1 : st - 1);
-      if (stages == 4) asm volatile("cp.async.wait_group 3;" ::: "memory");
-      else if (stages == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
-      else asm volatile("cp.async.wait_group 1;" ::: "memory");
-      __syncthreads();
-      if (owner && n - 1 < j0 + kTile) {                                 // the last tile: the token's own row
-        for (int c = tid; c < p.dp; c += kDecThreads) sk[(st * kTile + n - 1 - j0) * kp + c] = new_k[c];
-        for (int c = tid; c < p.vp; c += kDecThreads) sv[(st * kTile + n - 1 - j0) * vpitch + c] = new_v[c];
-        __syncthreads();
-      }
-      const __nv_bfloat16* kt = sk + st * kTile * kp;
-      const __nv_bfloat16* vt = sv + st * kTile * vpitch;
-      // scores: warp = 8 keys, all heads
-      float acc[MT][2][4];                                               // even and odd steps: two chains
-#pragma unroll
-      for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int q = 0; q < 8; ++q) acc[i][q >> 2][q & 3] = 0.f;
-      const __nv_bfloat16* krow = kt + (warp * 8 + (lane & 7)) * kp + ((lane >> 3) & 1) * 8;
+      for (int q = 0; q < 4; ++q) o[t][q] = 0.f;
+    if (walks) {
+      const float c2 = 1.4426950408889634f;                              // scores in powers of two
       const __nv_bfloat16* qrow = sq + (lane & 15) * kp + (lane >> 4) * 8;
-#pragma unroll 2
-      for (int k = 0; k < rp; k += 32) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          if (e && k + 16 >= rp) break;
-          uint32_t b0, b1;
-          ldsm2(b0, b1, krow + k + 16 * e);
-#pragma unroll
-          for (int i = 0; i < MT; ++i) {
-            uint32_t af[4];
-            ldsm4(af, qrow + i * 16 * kp + k + 16 * e);
-            mma16816(acc[i][e], af, b0, b1);
-          }
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < MT; ++i) {
-        float* d = ss + (i * 16 + fr) * kSP + warp * 8 + fc;
-        d[0] = (acc[i][0][0] + acc[i][1][0]) * c2;
-        d[1] = (acc[i][0][1] + acc[i][1][1]) * c2;
-        d[8 * kSP] = (acc[i][0][2] + acc[i][1][2]) * c2;
-        d[8 * kSP + 1] = (acc[i][0][3] + acc[i][1][3]) * c2;
-      }
-      __syncthreads();
-      const int live = j_hi - j0;
-#pragma unroll
-      for (int ti = 0; ti < HT / 8; ++ti) {
-        const int t = warp + 8 * ti;
-        if (t >= nh) break;                                              // (rows without a head stay zero)
-        const float s0 = lane < live ? ss[t * kSP + lane] : -FLT_MAX, s1 = lane + 32 < live ? ss[t * kSP + lane + 32] : -FLT_MAX;
-        float mt = fmaxf(s0, s1);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, off));
-        const float m_old = sm[t], mn = fmaxf(m_old, mt), corr = exp2_approx(m_old - mn);
-        const float p0 = lane < live ? exp2_approx(s0 - mn) : 0.f, p1 = lane + 32 < live ? exp2_approx(s1 - mn) : 0.f;
-        const float l = lane_sum(p0 + p1);
-        sp[t * kPP + lane] = __float2bfloat16_rn(p0);
-        sp[t * kPP + lane + 32] = __float2bfloat16_rn(p1);
+      int st = 0;
+#pragma unroll 1
+      for (int j0 = j_first; j0 < j_hi; j0 += step, st = st + 1 == ws.stages ? 0 : st + 1) {
+        request(j0 + (ws.stages - 1) * step, st == 0 ? ws.stages - 1 : st - 1);
+        if (ws.stages == 4) asm volatile("cp.async.wait_group 3;" ::: "memory");
+        else if (ws.stages == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+        else asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncwarp();
-        if (lane == 0) { sm[t] = mn; sl[t] = sl[t] * corr + l; scorr[t] = corr; }
-      }
-      __syncthreads();
-      // outputs: warp = every eighth group of 8 value columns
+        __nv_bfloat16* kt = mine + st * stage_elems;
+        __nv_bfloat16* vt = kt + kWalkKeys * kp;
+        if (owner && j0 < n && n - 1 < j0 + kWalkKeys) {                 // the token's own row
+          if (lane < p.dp / 8) reinterpret_cast<uint4*>(kt + (n - 1 - j0) * kp)[lane] = reinterpret_cast<const uint4*>(new_k)[lane];
+          if (lane < p.vp / 8) reinterpret_cast<uint4*>(vt + (n - 1 - j0) * vpitch)[lane] = reinterpret_cast<const uint4*>(new_v)[lane];
+          __syncwarp();
+        }
+        float s[2][4] = {}, s2[2][4] = {};                               // keys 0-7 and 8-15; even and odd steps: two chains
+        const __nv_bfloat16* krow = kt + ((lane & 7) + ((lane >> 4) << 3)) * kp + ((lane >> 3) & 1) * 8;
 #pragma unroll
-      for (int i = 0; i < MT; ++i) {
-        const float ca = scorr[i * 16 + fr], cb = scorr[i * 16 + fr + 8];
-        uint32_t pf[4][4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) ldsm4(pf[k], sp + (i * 16 + (lane & 15)) * kPP + k * 16 + (lane >> 4) * 8);
-#pragma unroll
-        for (int t = 0; t < kNT; ++t) {
-          const int nt = warp + 8 * t;
-          if (nt >= ntiles) continue;
-          o[i][t][0] *= ca;
-          o[i][t][1] *= ca;
-          o[i][t][2] *= cb;
-          o[i][t][3] *= cb;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            uint32_t b0, b1;
-            ldsm2t(b0, b1, vt + (k * 16 + (lane & 15)) * vpitch + nt * 8);
-            mma16816(o[i][t], pf[k], b0, b1);
+        for (int k = 0; k < DIM / 16; ++k)
+          if (k * 16 < rp) {
+            uint32_t q[4], b[4];
+            ldsm4(q, qrow + k * 16);
+            ldsm4(b, krow + k * 16);
+            mma16816(k & 1 ? s2[0] : s[0], q, b[0], b[1]);
+            mma16816(k & 1 ? s2[1] : s[1], q, b[2], b[3]);
           }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s[i >> 2][i & 3] += s2[i >> 2][i & 3];
+        const int live = j_hi - j0;
+        float corr[2];
+        uint32_t pf[4];
+#pragma unroll
+        for (int hi = 0; hi < 2; ++hi) {
+          float v[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) v[i] = (i >> 1) * 8 + fc + (i & 1) < live ? s[i >> 1][2 * hi + (i & 1)] * c2 : -FLT_MAX;
+          float mx = fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3]));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+          const float mn = fmaxf(m[hi], mx);
+          corr[hi] = exp2_approx(m[hi] - mn);
+          m[hi] = mn;
+          float e[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) e[i] = (i >> 1) * 8 + fc + (i & 1) < live ? exp2_approx(v[i] - mn) : 0.f;
+          l[hi] = fmaf(l[hi], corr[hi], (e[0] + e[1]) + (e[2] + e[3]));
+          pf[hi] = pack_bf16x2(e[0], e[1]);
+          pf[2 + hi] = pack_bf16x2(e[2], e[3]);
+        }
+        if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {
+#pragma unroll
+          for (int t = 0; t < DIM / 8; ++t) { o[t][0] *= corr[0]; o[t][1] *= corr[0]; o[t][2] *= corr[1]; o[t][3] *= corr[1]; }
+        }
+        const __nv_bfloat16* vrow = vt + ((lane & 7) + ((lane >> 3) & 1) * 8) * vpitch + (lane >> 4) * 8;
+#pragma unroll
+        for (int c = 0; c < DIM / 16; ++c)
+          if (c * 16 < p.vp) {
+            uint32_t b[4];
+            ldsm4t(b, vrow + c * 16);
+            mma16816(o[2 * c], pf, b[0], b[1]);
+            mma16816(o[2 * c + 1], pf, b[2], b[3]);
+          }
+        __syncwarp();                                                    // every lane has read the stage before it is filled anew
+      }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+      for (int hi = 0; hi < 2; ++hi) {
+        l[hi] += __shfl_xor_sync(0xffffffffu, l[hi], 1);
+        l[hi] += __shfl_xor_sync(0xffffffffu, l[hi], 2);
+        if ((lane & 3) == 0) {
+          sm[(warp + 1) * kWalkM + fr + 8 * hi] = m[hi];
+          sl[(warp + 1) * kWalkM + fr + 8 * hi] = l[hi];
         }
       }
-      __syncthreads();                                                   // the stage and the P tile are free again
     }
+    __syncthreads();                                                     // the rings are free
+    if (walks) {
+      float* d = part + (warp * kWalkM + fr) * part_row + fc;
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-      for (int t = 0; t < kNT; ++t) {
-        const int c = (warp + 8 * t) * 8 + fc;
-        if (c >= p.vp) continue;
-        *reinterpret_cast<float2*>(so + (i * 16 + fr) * p.vp + c) = make_float2(o[i][t][0], o[i][t][1]);
-        *reinterpret_cast<float2*>(so + (i * 16 + fr + 8) * p.vp + c) = make_float2(o[i][t][2], o[i][t][3]);
+      for (int t = 0; t < DIM / 8; ++t)
+        if (t * 8 < p.vp) {
+          if (fr < nh) *reinterpret_cast<float2*>(d + t * 8) = make_float2(o[t][0], o[t][1]);
+          if (fr + 8 < nh) *reinterpret_cast<float2*>(d + 8 * part_row + t * 8) = make_float2(o[t][2], o[t][3]);
+        }
+    }
+    __syncthreads();
+    const int v4 = p.vp / 4;
+    for (int i = tid; i < nh * v4; i += kDecThreads) {
+      const int h = i / v4, c = (i - h * v4) * 4;
+      float mx = -FLT_MAX, sum = 0.f;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int w = 0; w < ws.warps; ++w) mx = fmaxf(mx, sm[(w + 1) * kWalkM + h]);
+#pragma unroll 4
+      for (int w = 0; w < ws.warps; ++w) {
+        const float f = exp2_approx(sm[(w + 1) * kWalkM + h] - mx);
+        const float4 x = *reinterpret_cast<const float4*>(part + (w * kWalkM + h) * part_row + c);
+        sum = fmaf(f, sl[(w + 1) * kWalkM + h], sum);
+        v = make_float4(fmaf(f, x.x, v.x), fmaf(f, x.y, v.y), fmaf(f, x.z, v.z), fmaf(f, x.w, v.w));
       }
+      *reinterpret_cast<float4*>(so + h * p.vp + c) = v;
+      if (c == 0) { sm[h] = mx; sl[h] = sum; }
+    }
+  } else {
+    for (int i = tid; i < nh * p.vp; i += kDecThreads) so[i] = 0.f;
   }
   cluster_sync_all();
   // every CTA of the cluster finishes a share of the heads' columns
@@ -491,19 +502,25 @@ __global__ void __launch_bounds__(kDecThreads, 1) group_decode_tc_kernel(const G
   cluster_sync_all();                                                    // nobody leaves while its shared memory is read
 }
 
-template <int MT>
+template <int DIM>
 int launch_decode_tc(const GroupDecodeArgs& a, cudaStream_t stream, bool pdl) {
   static bool configured = false;
   if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(group_decode_tc_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
+    const cudaError_t e = cudaFuncSetAttribute(group_decode_tc_kernel<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
+  // eight warps with the most stages that fit, four where the rows are too wide for two stages of eight (or the merge for their rings)
+  WalkShape w = {8, 4};
+  const int dp = a.p.dp, vp = a.p.vp;
+  auto merge = [&]() { return 4 * kWalkM * (w.warps * (vp + 4) + vp); };
+  while (w.stages > 2 && walk_smem(dp, vp, w) > kWalkSmem) --w.stages;
+  if (walk_smem(dp, vp, w) > kWalkSmem || merge() > walk_ring(dp, vp, w)) w = {4, 3};
+  const int smem = walk_smem(dp, vp, w);
+  if (smem > kWalkSmem || merge() > walk_ring(dp, vp, w)) return -3;
   const int group = a.p.heads / a.p.kv_heads;
-  int stages = 4;
-  while (stages > 2 && group_tc_smem(a.p.dp, a.p.vp, MT * 16, stages) > 220 * 1024) --stages;
-  return launch_cluster(group_decode_tc_kernel<MT>, dim3(a.splits, a.p.kv_heads, (group + MT * 16 - 1) / (MT * 16)), dim3(kDecThreads), dim3(a.splits, 1, 1),
-                        group_tc_smem(a.p.dp, a.p.vp, MT * 16, stages), stream, pdl, a, stages);
+  return launch_cluster(group_decode_tc_kernel<DIM>, dim3(a.splits, a.p.kv_heads, (group + kWalkM - 1) / kWalkM), dim3(kDecThreads), dim3(a.splits, 1, 1),
+                        smem, stream, pdl, a, w);
 }
 
 template <bool F32, int VC>
@@ -553,7 +570,7 @@ extern "C" int nrt_group_decode(const void* args, void* stream, int pdl) {
   memcpy(&a, args, sizeof(a));
   if (!prep_ok(a.p) || a.p.rows != 1 || a.splits < 1 || a.splits > 8 || a.window < 0) return -3;
   const bool wide = a.p.vdim > kDecThreads, p = pdl != 0;
-  if (!a.p.f32 && a.p.dp <= kTcHead && a.p.vp <= kTcHead) return a.p.heads / a.p.kv_heads <= 16 ? launch_decode_tc<1>(a, S(stream), p) : launch_decode_tc<2>(a, S(stream), p);
+  if (!a.p.f32 && a.p.dp <= kTcHead && a.p.vp <= kTcHead) return a.p.dp <= 128 && a.p.vp <= 128 ? launch_decode_tc<128>(a, S(stream), p) : launch_decode_tc<256>(a, S(stream), p);
   if (a.p.f32) return wide ? launch_decode<true, 2>(a, S(stream), p) : launch_decode<true, 1>(a, S(stream), p);
   return wide ? launch_decode<false, 2>(a, S(stream), p) : launch_decode<false, 1>(a, S(stream), p);
 }

@@ -508,3 +508,41 @@ def test_checkpoint_and_trace_program(tmp_path):
             if rows:
                 got = torch.frombuffer(bytearray(path.read_bytes()), dtype=torch.float32).view(len(rows), cfg["vocab"])
                 check(got, torch.stack([ref[rid][p] for rid, p in rows]), short, i)
+
+
+@pytest.mark.parametrize("heads,kv,dim,vdim,pos,window,splits", [
+    (1, 1, 8, 8, 0, 0, 1), (4, 2, 56, 48, 15, 0, 1), (4, 2, 56, 48, 16, 0, 2), (32, 8, 128, 128, 700, 0, 8), (6, 2, 120, 136, 333, 256, 4),
+    (16, 1, 256, 256, 517, 0, 2), (20, 1, 64, 72, 130, 0, 1), (40, 2, 24, 256, 200, 0, 2), (8, 8, 200, 16, 300, 128, 8), (3, 1, 128, 128, 127, 128, 4)])
+def test_grouped_one_token_attention_against_its_float_form(heads, kv, dim, vdim, pos, window, splits):
+    """Tiles of 16 keys, rings of two to four stages, one and more tiles of heads, splits without keys: the tensor-core form on bf16 caches
+    against the plain form on the same values in 32 bits.  Queries, the new row and probabilities are rounded to bf16: 3 x 2^-8."""
+    from naivert_b200.ops import stack_kernels as S
+    from naivert_b200.runtime.packing import pad
+    S.lib()
+    g = torch.Generator(device="cuda").manual_seed(heads + dim + pos)
+    dp, vp, cap = pad(dim, 8), pad(vdim, 8), pos + 3
+    proj = torch.randn(heads * dim + kv * (dim + vdim), generator=g, device="cuda")
+    k = torch.zeros(cap, kv, dp, device="cuda")
+    v = torch.zeros(cap, kv, vp, device="cuda")
+    k[:pos, :, :dim] = torch.randn(pos, kv, dim, generator=g, device="cuda").bfloat16().float()
+    v[:pos, :, :vdim] = torch.randn(pos, kv, vdim, generator=g, device="cuda").bfloat16().float()
+    norms = [torch.ones(dim, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    where, status = torch.tensor([pos], dtype=torch.int32, device="cuda"), torch.zeros(4, dtype=torch.int32, device="cuda")
+    outs = []
+    for f32 in (1, 0):
+        t = torch.float32 if f32 else torch.bfloat16
+        kc, vc, out = k.to(t), v.to(t), torch.full((heads, vp), float("nan"), device="cuda")
+        a = S.GroupDecodeArgs()
+        p = a.p
+        p.proj, p.ld, p.q_off, p.k_off, p.v_off = proj.data_ptr(), proj.numel(), 0, heads * dim, heads * dim + kv * dim
+        p.rows, p.heads, p.kv_heads, p.dim, p.vdim, p.dp, p.vp = 1, heads, kv, dim, vdim, dp, vp
+        p.q_norm, p.k_norm, p.rot_dims, p.eps, p.scale = norms[0].data_ptr(), norms[1].data_ptr(), 0, 1e-6, dim ** -0.5
+        p.k_cache, p.v_cache, p.f32, p.pos0, p.capacity = kc.data_ptr(), vc.data_ptr(), f32, where.data_ptr(), cap
+        a.window, a.splits, a.out = window, splits, out.data_ptr()
+        S.group_decode(a, False)
+        torch.cuda.synchronize()
+        assert (kc[pos + 1:] == 0).all() and (vc[pos + 1:] == 0).all()
+        outs.append((out[:, :vdim], kc[pos].float(), vc[pos].float()))
+    (want, k0, v0), (got, k1, v1) = outs
+    assert float((got - want).abs().max() / want.abs().max()) < 3 * 2.0 ** -8
+    assert (k1 - k0).abs().max() <= 2.0 ** -8 * k0.abs().max() and (v1 - v0).abs().max() <= 2.0 ** -8 * v0.abs().max()
