@@ -11,6 +11,7 @@
 //       2048 rows x 64 heads: 114 us.
 // A 16,001-token document of two sparse and four window layers spends 27.8 ms in them; 61.2 ms when every row gathered its keys for
 // itself into tiles that eight warps shared between four barriers.
+// Against fp64 (bf16 outputs, windows / lists of 2048 / prefixes): 1.82e-3 / 1.81e-3 / 1.79e-3; before 1.84e-3 / 1.91e-3 / 1.88e-3.
 // With M = 16 live rows there is no 128-lane UMMA shape to fill, which is why this uses warp-level MMAs rather than tcgen05.
 //
 // Output: bf16-rounded o, written as bf16 and/or as the e4m3 packet (one power-of-two scale per head) that
