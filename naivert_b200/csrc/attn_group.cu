@@ -27,6 +27,8 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "gemm.cuh"
 #include "launch.hpp"
 
@@ -129,9 +131,10 @@ struct Walk {
     l[0] = l[1] = 0.f;
   }
 
-  // One tile of KEYS staged keys; seen(hi, key of the tile) says whether a row sees a key.
-  template <int KEYS, typename Seen>
-  __device__ __forceinline__ void tile(uint32_t sk, uint32_t sv, int lane, float scale, Seen&& seen) {
+  // One tile of KEYS staged keys; seen(hi, key of the tile) says whether a row sees a key.  ONE: the walk has one token row (queries of the
+  // others are null), and value rows that it does not see (kept(key)) are zero whatever memory holds.
+  template <int KEYS, bool ONE = false, typename Seen, typename Kept>
+  __device__ __forceinline__ void tile(uint32_t sk, uint32_t sv, int lane, float scale, Seen&& seen, Kept&& kept) {
     float s[KEYS / 8][4];
 #pragma unroll
     for (int t = 0; t < KEYS / 8; ++t)
@@ -182,10 +185,20 @@ struct Walk {
 #pragma unroll
     for (int t = 0; t < KEYS / 16; ++t) {
       const uint32_t pa[4] = {p[2 * t][0], p[2 * t][1], p[2 * t + 1][0], p[2 * t + 1][1]};
+      uint32_t keep[2] = {0xffffffffu, 0xffffffffu};                // of this thread's keys qc, qc + 1 and qc + 8, qc + 9
+      if (ONE)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int key = t * 16 + h * 8 + qc;
+          keep[h] = (kept(key) ? 0xffffu : 0u) | (kept(key + 1) ? 0xffff0000u : 0u);
+        }
 #pragma unroll
       for (int c = 0; c < kVd / 16; ++c) {
         uint32_t b[4];
         ldmatrix_x4_trans(b, va + t * 16 * kVRow + c * 32);
+        if (ONE)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) b[i] &= keep[i & 1];
         mma16816(o[2 * c], pa, b[0], b[1]);
         mma16816(o[2 * c + 1], pa, b[2], b[3]);
       }
@@ -259,7 +272,7 @@ __global__ void __launch_bounds__(kListWarps * 32, 2) attn_list_kernel(const Att
     __syncwarp();
     const uint32_t sk = ring + stage * kListStage;
     const int live = count - t * kListKeys;
-    w.tile<kListKeys>(sk, sk + kListKeys * kKRow, lane, a.scale, [&](int, int key) { return key < live; });
+    w.tile<kListKeys>(sk, sk + kListKeys * kKRow, lane, a.scale, [&](int, int key) { return key < live; }, [](int) { return true; });
     __syncwarp();                                                   // every lane has read the stage before it is filled anew
     stage ^= 1;
   }
@@ -344,11 +357,13 @@ __global__ void __launch_bounds__(kWinWarps * 32, 2) attn_window_kernel(const At
       for (int c = 0; c < 2; ++c) cp_async16(st + kWinKeys * kKRow + key * kVRow + c * 128, vc + slot * v_pitch + c * 128, valid);
     }
   };
+  auto open_ring = [&]() {
 #pragma unroll
-  for (int t = 0; t < kWinStages - 1; ++t) {
-    if (t < tiles) request(t);
-    cp_async_commit();
-  }
+    for (int t = 0; t < kWinStages - 1; ++t) {
+      if (t < tiles) request(t);
+      cp_async_commit();
+    }
+  };
   // fragment row -> (token row, head); rows beyond the chunk see no key
   int row[2], head[2], low[2], high[2];
 #pragma unroll
@@ -361,50 +376,79 @@ __global__ void __launch_bounds__(kWinWarps * 32, 2) attn_window_kernel(const At
     high[hi] = row[hi] < a.rows ? pos : -1;
   }
   Walk w;
-  w.open(row[0] < a.rows ? a.q + ((size_t)row[0] * a.heads + head[0]) * kHd : nullptr,
-         row[1] < a.rows ? a.q + ((size_t)row[1] * a.heads + head[1]) * kHd : nullptr, (lane & 3) * 2);
-  const int w_low = pos0 + r0 + warp * rpw - a.window + 1, w_high = pos0 + min(r0 + (warp + 1) * rpw, a.rows) - 1;   // keys any row of the warp sees
+  auto query = [&](int hi) { return a.q + ((size_t)row[hi] * a.heads + head[hi]) * kHd; };
+  // keys that any token row of the warp sees; `one`: only its row at `slot` is worked on
+  auto walk = [&](auto one, int slot) {
+    constexpr bool ONE = decltype(one)::value;
+    const int r_lo = r0 + warp * rpw + (ONE ? slot : 0), r_hi = ONE ? r_lo + 1 : min(r_lo + rpw, a.rows);
+    const int w_low = pos0 + r_lo - a.window + 1, w_high = pos0 + r_hi - 1;
+    const bool on[2] = {row[0] < a.rows && (!ONE || row[0] == r_lo), row[1] < a.rows && (!ONE || row[1] == r_lo)};
+    w.open(on[0] ? query(0) : nullptr, on[1] ? query(1) : nullptr, (lane & 3) * 2);
 #pragma unroll 1
-  for (int t = 0; t < tiles; ++t) {
-    cp_async_wait<kWinStages - 2>();
-    __syncthreads();                                                  // tile t has landed; everybody is done with tile t - 1
-    if (t + kWinStages - 1 < tiles) request(t + kWinStages - 1);
-    cp_async_commit();
-    const int k0 = key0 + t * kWinKeys;
-    if (k0 > w_high || k0 + kWinKeys <= w_low || r0 + warp * rpw >= a.rows) continue;
-    const uint32_t sk = base + (t % kWinStages) * kWinStage;
-    w.tile<kWinKeys>(sk, sk + kWinKeys * kKRow, lane, a.scale, [&](int hi, int i) { return k0 + i >= low[hi] && k0 + i <= high[hi]; });
-  }
-  cp_async_wait<0>();
-  const size_t ldo = (size_t)a.heads * kVd;
-#pragma unroll
-  for (int hi = 0; hi < 2; ++hi) {
-    const float l = quad_sum(w.l[hi]);
-    const bool live = row[hi] < a.rows;
-    const float f = live ? row_factor(w.m[hi], l, a.sink, head[hi]) : 0.f;
-    float am = 0.f;
-#pragma unroll
-    for (int t = 0; t < kVd / 8; ++t)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        float& v = w.o[t][2 * hi + j];
-        v = rbf16(v * f);
-        am = fmaxf(am, fabsf(v));
-      }
-    const float sc = pow2_scale(quad_max(am));
-    if (!live) continue;
-    const size_t at = (size_t)row[hi] * ldo + (size_t)head[hi] * kVd + (lane & 3) * 2;
-    if (a.o_bf16)
-#pragma unroll
-      for (int t = 0; t < kVd / 8; ++t) *reinterpret_cast<uint32_t*>(a.o_bf16 + at + t * 8) = bf16_pair(w.o[t][2 * hi], w.o[t][2 * hi + 1]);
-    if (a.o8) {
-#pragma unroll
-      for (int t = 0; t < kVd / 8; ++t) {
-        const __nv_fp8_e4m3 c0(w.o[t][2 * hi] / sc), c1(w.o[t][2 * hi + 1] / sc);
-        *reinterpret_cast<uint16_t*>(a.o8 + at + t * 8) = (uint16_t)(c0.__x | (uint32_t)c1.__x << 8);
-      }
-      if ((lane & 3) == 0) a.o_scale[(size_t)row[hi] * (ldo / 128) + head[hi]] = sc;
+    for (int t = 0; t < tiles; ++t) {
+      cp_async_wait<kWinStages - 2>();
+      __syncthreads();                                                // tile t has landed; everybody is done with tile t - 1
+      if (t + kWinStages - 1 < tiles) request(t + kWinStages - 1);
+      cp_async_commit();
+      const int k0 = key0 + t * kWinKeys;
+      if (k0 > w_high || k0 + kWinKeys <= w_low || r_lo >= a.rows) continue;
+      const uint32_t sk = base + (t % kWinStages) * kWinStage;
+      w.tile<kWinKeys, ONE>(sk, sk + kWinKeys * kKRow, lane, a.scale, [&](int hi, int i) { return on[hi] && k0 + i >= low[hi] && k0 + i <= high[hi]; },
+                            [&](int i) { return k0 + i >= w_low && k0 + i <= w_high; });
     }
+    cp_async_wait<0>();
+  };
+  const size_t ldo = (size_t)a.heads * kVd;
+  auto store = [&](int slot) {                                        // the rows of one slot, -1: all
+#pragma unroll
+    for (int hi = 0; hi < 2; ++hi) {
+      const float l = quad_sum(w.l[hi]);
+      const bool live = row[hi] < a.rows && (slot < 0 || row[hi] == r0 + warp * rpw + slot);
+      const float f = live ? row_factor(w.m[hi], l, a.sink, head[hi]) : 0.f;
+      float am = 0.f;
+#pragma unroll
+      for (int t = 0; t < kVd / 8; ++t)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float& v = w.o[t][2 * hi + j];
+          v = rbf16(v * f);
+          am = fmaxf(am, fabsf(v));
+        }
+      const float sc = pow2_scale(quad_max(am));
+      if (!live) continue;
+      const size_t at = (size_t)row[hi] * ldo + (size_t)head[hi] * kVd + (lane & 3) * 2;
+      if (a.o_bf16)
+#pragma unroll
+        for (int t = 0; t < kVd / 8; ++t) *reinterpret_cast<uint32_t*>(a.o_bf16 + at + t * 8) = bf16_pair(w.o[t][2 * hi], w.o[t][2 * hi + 1]);
+      if (a.o8) {
+#pragma unroll
+        for (int t = 0; t < kVd / 8; ++t) {
+          const __nv_fp8_e4m3 c0(w.o[t][2 * hi] / sc), c1(w.o[t][2 * hi + 1] / sc);
+          *reinterpret_cast<uint16_t*>(a.o8 + at + t * 8) = (uint16_t)(c0.__x | (uint32_t)c1.__x << 8);
+        }
+        if ((lane & 3) == 0) a.o_scale[(size_t)row[hi] * (ldo / 128) + head[hi]] = sc;
+      }
+    }
+  };
+  open_ring();
+  walk(std::false_type{}, 0);
+  // A probability of zero does not hide an infinity or NaN of a value row that only other rows of the CTA see; what it
+  // leaves in an output stays non-finite to the end.  Then every token row is walked again by itself, unseen values zeroed.
+  float top = 0.f;
+#pragma unroll
+  for (int t = 0; t < kVd / 8; ++t)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) top = fmaxf(top, fabsf(w.o[t][j] - w.o[t][j]) == 0.f ? 0.f : 1.f);
+  if (!__syncthreads_or(top != 0.f)) {
+    store(-1);
+    return;
+  }
+#pragma unroll 1
+  for (int slot = 0; slot < rpw; ++slot) {
+    __syncthreads();                                                  // the stages are free
+    open_ring();
+    walk(std::true_type{}, slot);
+    store(slot);
   }
 }
 

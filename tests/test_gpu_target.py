@@ -231,6 +231,42 @@ def test_grouped_head_attention_at_the_edges_of_its_tiles(heads, kvh, rows, wind
             assert ((packet[r].view(heads, vd) - have).abs() <= 2.0 ** -4 * top + 1e-2 * top).all(), (mode, r)
 
 
+@pytest.mark.parametrize("heads,kvh,rows,window,pos0", [(8, 8, 70, 33, 0), (64, 8, 13, 40, 90), (24, 8, 9, 128, 300), (16, 1, 6, 5, 2)])
+def test_window_attention_keeps_unseen_values_out(heads, kvh, rows, window, pos0):
+    """An infinity in the last value row and a NaN in the one that only the first row still sees: the rows between are, bit for bit,
+    what they are with finite values, the two rows that see them are not finite there."""
+    from naivert_b200.ops import kernels as K
+    K.lib()
+    g = torch.Generator(device="cuda").manual_seed(rows + window)
+    hd, vd, cap = 192, 128, pos0 + rows
+    q = torch.randn(rows, heads, hd, device="cuda", generator=g).bfloat16()
+    kc = torch.randn(cap, kvh, hd, device="cuda", generator=g).bfloat16()
+    vc = torch.randn(cap, kvh, vd, device="cuda", generator=g).bfloat16()
+    p = torch.tensor([pos0], dtype=torch.int32, device="cuda")
+    first = max(0, pos0 - window + 1)
+    outs = []
+    for bad in (False, True):
+        if bad:
+            vc[cap - 1, :, 3] = float("inf")
+            if pos0 >= window - 1:
+                vc[first, :, 70] = float("nan")
+        o = torch.zeros(rows, heads * vd, device="cuda", dtype=torch.bfloat16)
+        o8, osc = torch.zeros(rows, heads * vd, device="cuda", dtype=torch.uint8), torch.zeros(rows, heads, device="cuda")
+        a = K.AttnArgs()
+        a.q, a.k_cache, a.v_cache, a.pos0 = q.data_ptr(), kc.data_ptr(), vc.data_ptr(), p.data_ptr()
+        a.rows, a.heads, a.kv_heads, a.head_dim, a.v_dim, a.scale, a.mode, a.window = rows, heads, kvh, hd, vd, hd ** -0.5, 0, window
+        a.o_bf16, a.o8, a.o_scale = o.data_ptr(), o8.data_ptr(), osc.data_ptr()
+        K.attn_group(a, pdl=False)
+        torch.cuda.synchronize()
+        outs.append((o, o8, osc))
+    between = slice(1 if pos0 >= window - 1 else 0, rows - 1)
+    for want, got in zip(*outs):
+        assert torch.equal(got[between], want[between])
+    o = outs[1][0].view(rows, heads, vd)
+    assert torch.isinf(o[-1, :, 3]).all() and (pos0 < window - 1 or torch.isnan(o[0, :, 70]).all())
+    assert torch.isfinite(o[-1, :, 4:64]).all() and torch.isfinite(o[0, :, :64]).all()
+
+
 def test_tcgen05_index_sweep_matches_cuda_core_form():
     from naivert_b200.ops import kernels as K
     spec, rt, _ = _build(layers=1, capacity=2048)
