@@ -150,12 +150,33 @@ __global__ void __launch_bounds__(kRowWarps * 32) latent_attn_rows_kernel(const 
 #pragma unroll
       for (int c = 0; c < NC; ++c) o[i][c] *= corr;
     }
-    const int used = min(kRowTile, end - j0);
     int at[NC];                                                  // channels beyond the head's read (and drop) its first one
 #pragma unroll
     for (int c = 0; c < NC; ++c) at[c] = lane + 32 * c < a.vdim ? lane + 32 * c : 0;
+    // a row takes the values it sees and no others (zero times an infinity is not zero): first those before both rows' common
+    // range [both, until), then that range, then those behind it
+    int from[kRowsWarp], to[kRowsWarp], both = 0, until = kRowTile;
+#pragma unroll
+    for (int i = 0; i < kRowsWarp; ++i) {
+      from[i] = max(0, low[i] - j0);
+      to[i] = max(from[i], min(kRowTile, n[i] - j0));
+      if (row0 + warp * kRowsWarp + i < a.rows) {                // (a row beyond the chunk goes along: nothing of it is stored)
+        both = max(both, from[i]);
+        until = min(until, to[i]);
+      }
+    }
+    until = max(both, until);
+    auto alone = [&](int i, int t0, int t1) {
+      for (int t = t0; t < t1; ++t) {
+        const float pt = __shfl_sync(0xffffffffu, p[i], t);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) o[i][c] = fmaf(pt, sv[t * vs + at[c]], o[i][c]);
+      }
+    };
+#pragma unroll
+    for (int i = 0; i < kRowsWarp; ++i) alone(i, from[i], min(to[i], both));
 #pragma unroll 8
-    for (int t = 0; t < used; ++t) {
+    for (int t = both; t < until; ++t) {
       float pt[kRowsWarp];
 #pragma unroll
       for (int i = 0; i < kRowsWarp; ++i) pt[i] = __shfl_sync(0xffffffffu, p[i], t);
@@ -166,6 +187,8 @@ __global__ void __launch_bounds__(kRowWarps * 32) latent_attn_rows_kernel(const 
         for (int i = 0; i < kRowsWarp; ++i) o[i][c] = fmaf(pt[i], v, o[i][c]);
       }
     }
+#pragma unroll
+    for (int i = 0; i < kRowsWarp; ++i) alone(i, max(from[i], until), to[i]);
     __syncthreads();                                             // everybody is done with this tile
     if (stages == 2) stage ^= 1;
   }

@@ -337,6 +337,41 @@ def test_plain_chunk_attention_against_torch(rows, heads, group, dim, vdim, pos0
     assert float((out.double() - want).abs().max() / want.abs().max()) < (5e-6 if f32 else 2.0 ** -8)
 
 
+@pytest.mark.parametrize("f32", [1, 0])
+@pytest.mark.parametrize("rows,heads,group,dim,vdim,pos0,window", [
+    (8, 2, 1, 48, 40, 0, 0), (9, 4, 2, 33, 70, 27, 0), (11, 2, 1, 60, 64, 40, 16), (3, 1, 1, 512, 510, 61, 48), (40, 2, 1, 24, 130, 5, 20)])
+def test_plain_chunk_attention_keeps_unseen_values_out(rows, heads, group, dim, vdim, pos0, window, f32):
+    """An infinity in the last value row and, with masks by chunk, a NaN in the last one before the last row's own chunk: rows that do not
+    see them are, bit for bit, what they are with finite values."""
+    from naivert_b200.ops import stack_kernels as S
+    S.lib()
+    g = torch.Generator(device="cuda").manual_seed(rows + dim)
+    t, n, kv = torch.float32 if f32 else torch.bfloat16, pos0 + rows, heads // group
+    q, k, v = (torch.randn(*s, generator=g, device="cuda").to(t) for s in ((rows, heads, dim), (n, kv, dim), (n, kv, vdim)))
+    pos = torch.tensor([pos0], dtype=torch.int32, device="cuda")
+    start = (n - 1) // window * window if window else 0
+    outs = []
+    for bad in (False, True):
+        if bad:
+            v[n - 1, :, 2] = float("inf")
+            if start:
+                v[start - 1, :, 5] = float("nan")
+        out = torch.zeros(rows, heads, vdim, dtype=t, device="cuda")
+        a = S.LatentAttnArgs()
+        a.q, a.k, a.v, a.out, a.f32 = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), f32
+        a.rows, a.heads, a.dim, a.vdim, a.scale, a.pos0, a.group, a.window = rows, heads, dim, vdim, dim ** -0.5, pos.data_ptr(), group, window
+        a.kv0, a.kv_rows, a.first, a.last = 0, n, 1, 1
+        S.latent_attn_rows(a)
+        torch.cuda.synchronize()
+        outs.append(out)
+    at = pos0 + torch.arange(rows, device="cuda")
+    clean = at < n - 1
+    if start:
+        clean &= (at // window * window >= start) | (at < start - 1)
+    assert clean.any() and torch.equal(outs[1][clean], outs[0][clean])
+    assert not torch.isfinite(outs[1][-1, :, 2]).any() and torch.isfinite(outs[1][-1, :, 3:]).all()
+
+
 @pytest.mark.parametrize("rows", [1, 64, 65, 129, 187, 192, 193, 256])
 def test_few_rows_are_one_tile(rows):
     """Products of many features: tiles of 64 to 256 rows, one and (two products of 192 rows) a single accumulator in flight."""
