@@ -26,6 +26,7 @@ SMS = 148
 # tile sizes of the chunk products by epilogue (the others: 64 and 256)
 TILE_ROWS = {S.EPI_STORE: (64, 128, 192, 256), S.EPI_RELU2: (64, 128, 192, 256), S.EPI_BIAS: (64, 128, 192, 256), S.EPI_CLAMPED_GLU: (64, 128, 192),
              S.EPI_SILU_GLU: (64, 128)}
+FUNCTION_EPI = (S.EPI_TANH, S.EPI_DECAY_SOFT, S.EPI_DECAY_EXP)
 # Pairs (token, choice) per expert that a span is filled up to, and its most rows.  Below, an expert's product is bound by the read of its
 # weights (12.9 GB a layer at 256 experts of 4096 x 2048), which a span does once: with three such layers, 8192 rows in chunks of 2048 take
 # 30.1 ms, 47.0 ms when every chunk went through the experts by itself (their products: 28.3 -> 11.0 ms).  A span's rows cost 2 GB there.
@@ -127,13 +128,16 @@ class StackPrefill:
 
     @staticmethod
     def tile_rows(epi: int, tiles: int, rows: int) -> int:
-        """Token rows per tile of a product with ``tiles`` feature tiles.  Few rows are one tile where the feature tiles occupy about
+        """Token rows per tile of a product with ``tiles`` feature tiles.  Few rows are one tile where the feature tiles occupy more than
         half of the SMs: every weight is then fetched by one CTA only, and what is in flight - which bounds a product that streams
         its weights - is all different: 152,576 features of 4096 x 1 row 419 -> 212 us, 10,240 x 187 rows 49 -> 38 us, and 16,384 x 187
-        rows of two products 90 -> 87 us against the widest tile that fills the SMs, which larger products take."""
+        rows of two products 90 -> 87 us against the widest tile that fills the SMs, which larger products take.  With fewer feature
+        tiles two rows of tiles are still one wave (8,192 features of 4096: 100 rows in tiles of 64 / 128 21.1 / 22.5 us, of two products
+        34.6 / 40.0; feature-major stores of 512, 100 / 200 rows in tiles of 64 / 256 6.6 / 7.9 and 8.5 / 9.2).  Tanh and the decays are
+        bound by their special functions, a thread's share of which grows with the tile (12,288 features of 128, 100 rows: 12.5 / 16.1)."""
         sizes = TILE_ROWS.get(epi, (64, 256))
         whole = next((t for t in sizes if t >= rows), None)
-        if whole is not None and tiles >= 64:
+        if whole is not None and 2 * tiles > SMS and (whole == 64 or epi not in FUNCTION_EPI):
             return whole
         return next((t for t in reversed(sizes) if t != 192 and tiles * -(-rows // t) >= SMS - 20), 64)
 

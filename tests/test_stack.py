@@ -173,6 +173,27 @@ def test_plain_model_is_causal():
     assert torch.isfinite(full).all() and full.std() > 1e-3
 
 
+# --------------------------------------------------------------------------- tiles of prompt chunks
+def test_token_rows_per_tile():
+    """One tile for few rows only where it was the faster one; everywhere else the widest tile that fills the SMs."""
+    from naivert_b200.ops import stack_kernels as S
+    from naivert_b200.prefill.stack import StackPrefill
+    rule = StackPrefill.tile_rows
+    functions = (S.EPI_TANH, S.EPI_DECAY_SOFT, S.EPI_DECAY_EXP)
+    for epi in (S.EPI_STORE, S.EPI_BIAS, S.EPI_RELU2, S.EPI_CLAMPED_GLU, S.EPI_TRANSPOSE) + functions:
+        for rows in (1, 64):
+            assert [rule(epi, tiles, rows) for tiles in (1, 64, 75, 128, 1192)] == [64] * 5
+    for epi in (S.EPI_TRANSPOSE,) + functions:                   # no sizes between: 64 feature tiles keep tiles of 64
+        assert [rule(epi, 64, rows) for rows in (65, 128, 129, 256)] == [64] * 4
+        assert [rule(epi, 96, rows) for rows in (65, 256)] == ([256] * 2 if epi == S.EPI_TRANSPOSE else [64] * 2)
+        assert [rule(epi, 128, rows) for rows in (65, 256)] == [256] * 2
+    for epi in (S.EPI_STORE, S.EPI_BIAS, S.EPI_RELU2):
+        assert [rule(epi, 64, rows) for rows in (65, 128, 129, 187, 256)] == [64, 64, 128, 128, 128]
+        assert [rule(epi, 80, rows) for rows in (65, 128, 129, 187, 256)] == [128, 128, 192, 192, 256]
+    assert [rule(S.EPI_CLAMPED_GLU, 64, rows) for rows in (100, 187)] == [64, 128]
+    assert [rule(S.EPI_CLAMPED_GLU, 128, rows) for rows in (100, 187, 256)] == [128, 192, 128]
+
+
 # --------------------------------------------------------------------------- trace replay
 class FakeEngine:
     def __init__(self):
