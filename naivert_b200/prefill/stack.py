@@ -299,7 +299,8 @@ class StackPrefill:
 
     # ------------------------------------------------------------------ public API (that of ``NativePrefill``)
     def extend(self, tokens: torch.Tensor, pos0: int, want: Sequence[int] = (), trace: Optional[list] = None) -> torch.Tensor:
-        """Feed ``tokens`` (host or device) at positions pos0 .. in spans of chunks; logits [len(want), vocab] of the rows in ``want``."""
+        """Feed ``tokens`` (host or device) at positions pos0 .. in spans of chunks; logits [len(want), vocab] of the rows in ``want``.
+        ``trace`` collects, chunk by chunk, the stream after every layer run."""
         n = int(tokens.numel())
         if not 0 <= pos0 <= pos0 + n <= self.t.capacity:
             raise ValueError(f"rows [{pos0}, {pos0 + n}) outside the cache capacity {self.t.capacity}")
@@ -310,7 +311,10 @@ class StackPrefill:
         for c0 in range(0, n, self.span):
             R = min(self.span, n - c0)
             self.tokens[:R].copy_(tokens[c0:c0 + R].to(torch.int32), non_blocking=True)
-            got = self._chunk(pos0 + c0, R, [w - c0 for w in order if c0 <= w < c0 + R], trace)
+            seen: Optional[list] = None if trace is None else []
+            got = self._chunk(pos0 + c0, R, [w - c0 for w in order if c0 <= w < c0 + R], seen)
+            for i in range(0, R if seen else 0, self.C):
+                trace.extend(x[i:i + self.C] for x in seen)
             if got is not None:
                 out.append(got)
         return torch.cat(out) if out else torch.empty(0, self.spec.vocab, dtype=torch.float32, device=self.dev)

@@ -158,6 +158,16 @@ def test_stream_after_every_layer_run():
         eng.close()
 
 
+def test_stream_comes_chunk_by_chunk_from_spans():
+    cfg = CASES["mixed"]
+    eng, got = engine(cfg, weights(cfg, 3)), []
+    try:
+        eng.prefill.extend(torch.tensor(tokens(cfg, 212)), 0, (), got)
+        assert [x.shape[0] for x in got] == [96] * 14 + [20] * 7
+    finally:
+        eng.close()
+
+
 # --------------------------------------------------------------------------- keys far away and at borders
 def needle_model(width=64):
     """One attention layer in which token 58 looks up token 59: that one key carries nearly the whole weight wherever it
