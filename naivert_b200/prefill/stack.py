@@ -47,38 +47,15 @@ class StackPrefill:
         moe = [f for f in ffs if f.kind == "moe"]
         self.h_ld = pad(s.hidden, 8)
         filled = min([-(-SPAN_PAIRS * f.routing.expert_count // f.routing.top_k) for f in moe], default=0)
-        self.span = max(C, min(SPAN_ROWS, filled, runtime.capacity) // C * C)
-        P = self.span
-
-        def z(n: int, t=f32) -> torch.Tensor:
-            return torch.zeros(max(8, n), dtype=t, device=dev)
-
-        def most(it) -> int:
-            return max(list(it), default=0)
-
-        self.tokens = torch.zeros(P, dtype=i32, device=dev)
-        # per span: position of each chunk, stream, input and output rows of the sublayers
-        self.rows_of = {"pos": torch.zeros(P // C, dtype=i32, device=dev), "x": torch.zeros(P, s.hidden, dtype=f32, device=dev),
-                        "h": torch.zeros(P, self.h_ld, dtype=self.act, device=dev), "y": torch.zeros(P, s.hidden, dtype=f32, device=dev),
-                        "y2": torch.zeros(P, s.hidden, dtype=f32, device=dev) if any(d["kind"] == "parallel" for d in L) else None}
-        self._window()
+        self.span_limit = max(C, min(SPAN_ROWS, filled, runtime.capacity) // C * C)
+        self._size_span(C)
         # buffers of the mixers, one per role, shared by the layers (sizes differ from layer to layer)
         sizes: Dict[tuple, int] = {}
         for d in L:
             for name, (n, t) in MIXERS[d["kind"]].scratch(self, d["spec"].mixer, d).items():
                 sizes[name, t] = max(n, sizes.get((name, t), 0))
-        self.buf = {name: z(n, t) for (name, t), n in sizes.items()}
-        self.ff = z(C * most(pad(f.ff, 8) for f in ffs if f.kind != "moe"), self.act)
-        if moe:
-            E, T = most(f.routing.expert_count for f in moe), most(f.routing.top_k for f in moe)
-            self.scores, self.ids, self.probs = z(P * E), z(P * T, i32), z(P * T)
-            self.slot_of, self.n_items, self.seg_rows = z(P * T, i32), z(1, i32), z(E, i32)
-            self.max_items = -(-P * T // 64) + E
-            self.item_z, self.item_row = z(self.max_items, i32), z(self.max_items, i32)
-            self.cap = most(self._segment_rows(P, f.routing) for f in moe)
-            self.sorted = z(self.cap * self.h_ld, self.act)
-            self.ea = z(self.cap * most(pad(f.ff, 8) for f in moe), self.act)
-            self.ey = z(self.cap * s.hidden)
+        self.buf = {name: self._zeros(n, t) for (name, t), n in sizes.items()}
+        self.ff = self._zeros(C * max([pad(f.ff, 8) for f in ffs if f.kind != "moe"], default=0), self.act)
         self.head_rows = 256
         self.hw = torch.zeros(self.head_rows, self.h_ld, dtype=self.act, device=dev)
         self.tensor_cores = not self.f32              # attention of chunk rows on tcgen05 (else the plain kernel)
@@ -86,6 +63,45 @@ class StackPrefill:
         self.phases: dict = {}
         self.profile = False                          # per-stage CUDA-event timing (adds an event pair per stage)
         self._timed: Dict[str, list] = {}
+
+    def _zeros(self, n: int, t=torch.float32) -> torch.Tensor:
+        return torch.zeros(max(8, n), dtype=t, device=self.dev)
+
+    def _size_span(self, P: int) -> None:
+        """Buffers for spans of ``P`` rows (whole chunks); an allocation that fails leaves the present ones."""
+        s, C, L, z, f32, i32 = self.spec, self.C, self.t.layers, self._zeros, torch.float32, torch.int32
+        moe = [d["spec"].mlp for d in L if d["spec"].mlp is not None and d["spec"].mlp.kind == "moe"]
+
+        def rows(width: int, t=f32) -> torch.Tensor:
+            return torch.zeros(P, width, dtype=t, device=self.dev)
+
+        # position of each chunk, stream, input and output rows of the sublayers
+        rows_of = {"pos": torch.zeros(P // C, dtype=i32, device=self.dev), "x": rows(s.hidden), "h": rows(self.h_ld, self.act), "y": rows(s.hidden),
+                   "y2": rows(s.hidden) if any(d["kind"] == "parallel" for d in L) else None}
+        new = {"tokens": torch.zeros(P, dtype=i32, device=self.dev)}
+        if moe:
+            E, T = max(f.routing.expert_count for f in moe), max(f.routing.top_k for f in moe)
+            items, cap = -(-P * T // 64) + E, max(self._segment_rows(P, f.routing) for f in moe)
+            new.update(scores=z(P * E), ids=z(P * T, i32), probs=z(P * T), slot_of=z(P * T, i32), n_items=z(1, i32), seg_rows=z(E, i32),
+                       max_items=items, item_z=z(items, i32), item_row=z(items, i32), cap=cap, sorted=z(cap * self.h_ld, self.act),
+                       ea=z(cap * max(pad(f.ff, 8) for f in moe), self.act), ey=z(cap * s.hidden))
+        self.rows_of, self.span = rows_of, P
+        for name, v in new.items():
+            setattr(self, name, v)
+        self._window()
+
+    def _fit_span(self, n: int) -> None:
+        """Spans for ``n`` rows as far as the limit and the memory go.  What a span needs beyond a chunk is taken when a prompt first asks
+        for it: an engine that sees short prompts only never holds it, and without the memory chunks go on one by one."""
+        P = min(self.span_limit, -(-n // self.C) * self.C)
+        if P > self.span:
+            torch.cuda.synchronize(self.dev)              # earlier calls may still use the buffers that go, on any stream
+        while P > self.span:
+            try:
+                self._size_span(P)
+            except torch.OutOfMemoryError:
+                P -= self.C
+                self.span_limit = P
 
     @contextmanager
     def stage(self, name: str):
@@ -308,6 +324,7 @@ class StackPrefill:
         order = [w for w in want]
         if order != sorted(order):
             raise ValueError("wanted rows must ascend")
+        self._fit_span(n)
         for c0 in range(0, n, self.span):
             R = min(self.span, n - c0)
             self.tokens[:R].copy_(tokens[c0:c0 + R].to(torch.int32), non_blocking=True)
@@ -337,10 +354,12 @@ class StackPrefill:
         return a.elapsed_time(b)
 
     def warm_chunks(self, sizes=None) -> None:
-        """Run chunk sizes once at position 0 (module loading, kernel attributes); the next request overwrites the rows."""
-        for r in sorted(set(sizes or [1, self.C])):
+        """Run row counts once at position 0 (module loading, kernel attributes, scratch); the next request overwrites the rows.  The
+        default ends with the longest span: its products of the routed experts are others than a chunk's."""
+        for r in sorted(set(sizes or [1, self.C, self.span_limit])):
+            self._fit_span(min(r, self.t.capacity))
             self.tokens.zero_()
-            self._chunk(0, min(r, self.C, self.t.capacity))
+            self._chunk(0, min(r, self.span, self.t.capacity))
         torch.cuda.current_stream().synchronize()
         self.check()
 

@@ -168,6 +168,29 @@ def test_stream_comes_chunk_by_chunk_from_spans():
         eng.close()
 
 
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+def test_spans_give_what_chunks_one_by_one_give(dtype):
+    """A routed prompt across the border of two spans, the last chunk a short one: logits on both sides of the border, the stream after
+    every layer run chunk by chunk, and the scratch, which grows at the first long prompt only.  Sums do not depend on the span."""
+    cfg = CASES["mixed"]
+    eng = engine(cfg, weights(cfg, 3), dtype, capacity=512, chunk=96)
+    pf, toks, want = eng.prefill, torch.tensor(tokens(cfg, 500)), [0, 95, 96, 478, 479, 480, 499]
+    try:
+        assert pf.span == 96 and pf.span_limit == 480
+        pf.extend(toks[:96], 0)
+        assert pf.span == 96 and pf.x.shape[0] == 96
+        got = []
+        for limit in (96, 480):
+            pf.span_limit, trace = limit, []
+            logits = pf.extend(toks, 0, want, trace)
+            assert pf.span == limit and [x.shape[0] for x in trace] == [96] * 35 + [20] * 7
+            got.append((logits, trace))
+        assert torch.equal(got[0][0], got[1][0]) and all(torch.equal(a, b) for a, b in zip(got[0][1], got[1][1]))
+        pf.warm_chunks()
+    finally:
+        eng.close()
+
+
 # --------------------------------------------------------------------------- keys far away and at borders
 def needle_model(width=64):
     """One attention layer in which token 58 looks up token 59: that one key carries nearly the whole weight wherever it

@@ -173,7 +173,7 @@ def test_plain_model_is_causal():
     assert torch.isfinite(full).all() and full.std() > 1e-3
 
 
-# --------------------------------------------------------------------------- tiles of prompt chunks
+# --------------------------------------------------------------------------- tiles and spans of prompt chunks
 def test_token_rows_per_tile():
     """One tile for few rows only where it was the faster one; everywhere else the widest tile that fills the SMs."""
     from naivert_b200.ops import stack_kernels as S
@@ -192,6 +192,34 @@ def test_token_rows_per_tile():
         assert [rule(epi, 80, rows) for rows in (65, 128, 129, 187, 256)] == [128, 128, 192, 192, 256]
     assert [rule(S.EPI_CLAMPED_GLU, 64, rows) for rows in (100, 187)] == [64, 128]
     assert [rule(S.EPI_CLAMPED_GLU, 128, rows) for rows in (100, 187, 256)] == [128, 192, 128]
+
+
+def test_spans_grow_with_the_prompt_as_far_as_memory_goes(monkeypatch):
+    from naivert_b200.prefill.stack import StackPrefill
+    sized = []
+
+    class Fake(StackPrefill):
+        def __init__(self, room):
+            self.C, self.span, self.span_limit, self.dev, self.room = 4, 4, 16, "cuda", room
+
+        def _size_span(self, P):
+            sized.append(P)
+            if P > self.room:
+                raise torch.OutOfMemoryError("no room")
+            self.span = P
+
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda *a: None)
+    pf = Fake(100)
+    for n, span in ((1, 4), (4, 4), (5, 8), (3, 8), (1000, 16)):
+        pf._fit_span(n)
+        assert pf.span == span
+    assert sized == [8, 16]
+    sized.clear()
+    pf = Fake(8)
+    for n, span in ((3, 4), (13, 8), (1000, 8)):                # what does not fit is tried once
+        pf._fit_span(n)
+        assert pf.span == span
+    assert sized == [16, 12, 8]
 
 
 # --------------------------------------------------------------------------- trace replay
