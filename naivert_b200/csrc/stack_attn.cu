@@ -321,7 +321,8 @@ __global__ void __launch_bounds__(kDecThreads, DIM <= 128 ? 2 : 1) group_decode_
     const int c = lane & (lanes - 1), rows = 32 / lanes;
     if (c >= width / 8) return;
     const long long row_step = (long long)p.kv_heads * width;
-#pragma unroll 8
+    // rolled: a launch inside a step fetches its instructions anew, and at short contexts it is little more than that (1.5 us less)
+#pragma unroll 1
     for (int t = lane / lanes; t < kWalkKeys; t += rows) {
       const bool in = j0 + t < j_hi && j0 + t != n - 1;                  // the token's own row is not in the cache yet
       cp16(dst + t * pitch + c * 8, in ? src + (long long)(start + j0 + t) * row_step + c * 8 : src, in);
@@ -456,7 +457,8 @@ __global__ void __launch_bounds__(kDecThreads, DIM <= 128 ? 2 : 1) group_decode_
       }
     }
     __syncthreads();                                                     // the rings are free
-    if (walks) {
+    const int fed = min(ws.warps, (j_hi - j_lo + kWalkKeys - 1) / kWalkKeys);      // warps that had a tile: short contexts have few to merge
+    if (warp < fed) {
       float* d = part + (warp * kWalkM + fr) * part_row + fc;
 #pragma unroll
       for (int t = 0; t < DIM / 8; ++t)
@@ -472,9 +474,9 @@ __global__ void __launch_bounds__(kDecThreads, DIM <= 128 ? 2 : 1) group_decode_
       float mx = -FLT_MAX, sum = 0.f;
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
-      for (int w = 0; w < ws.warps; ++w) mx = fmaxf(mx, sm[(w + 1) * kWalkM + h]);
+      for (int w = 0; w < fed; ++w) mx = fmaxf(mx, sm[(w + 1) * kWalkM + h]);
 #pragma unroll 4
-      for (int w = 0; w < ws.warps; ++w) {
+      for (int w = 0; w < fed; ++w) {
         const float f = exp2_approx(sm[(w + 1) * kWalkM + h] - mx);
         const float4 x = *reinterpret_cast<const float4*>(part + (w * kWalkM + h) * part_row + c);
         sum = fmaf(f, sl[(w + 1) * kWalkM + h], sum);
