@@ -129,8 +129,16 @@ def ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
 
-def _stream() -> int:
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+def stream_getter(binding):
+    """Handle of the current stream in one call where torch's binding offers it (``torch.cuda.current_stream`` builds an object through
+    five, 8 us of a launch from the host), else through the public function."""
+    raw, device = getattr(binding, "_cuda_getCurrentRawStream", None), getattr(binding, "_cuda_getDevice", None)
+    if raw is None or device is None:
+        return lambda: torch.cuda.current_stream().cuda_stream
+    return lambda: raw(device())
+
+
+_stream = stream_getter(torch._C)
 
 
 LAUNCHES = {"count": 0}          # kernels launched through this module (sampler chain counts as 9)

@@ -67,8 +67,11 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_handle = K._stream
+
+
 def _stream() -> VP:
-    return VP(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return VP(_handle())
 
 
 def weight_map(w: torch.Tensor, k: int) -> K.TensorMap:

@@ -394,3 +394,12 @@ def test_stamp_reports_from_synthetic_buffers():
         samp[2 * ph], samp[2 * ph + 1] = t0 + 10_000 * ph + 3000, t0 + 10_000 * ph + 8000
     out = report_sampler_stamps(samp)
     assert len(out) == 8 and "maxima" in out[1] and "3.00 /     8.00" in out[1] and "63.00 /    68.00" in out[7]
+
+
+def test_stream_handle_does_not_depend_on_private_names(monkeypatch):
+    from types import SimpleNamespace
+    from naivert_b200.ops import kernels as K
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: SimpleNamespace(cuda_stream=77))
+    assert K.stream_getter(SimpleNamespace())() == 77
+    assert K.stream_getter(SimpleNamespace(_cuda_getCurrentRawStream=lambda d: d))() == 77
+    assert K.stream_getter(SimpleNamespace(_cuda_getCurrentRawStream=lambda d: 10 + d, _cuda_getDevice=lambda: 3))() == 13
