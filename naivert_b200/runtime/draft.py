@@ -96,11 +96,11 @@ class DraftRuntime:
         V = spec.vocab_shard(self.tp)
         self.dlogits = torch.zeros(PAD_ROWS, V, dtype=f32, device=dev)
         self.zq = torch.zeros(8, V, dtype=f32, device=dev)
-        self.best = torch.zeros(8, dtype=torch.int64, device=dev)
-        self.markov_sync = torch.zeros(2, dtype=torch.int64, device=dev)
+        # words that the proposals' launches leave as they found them, or further on: best candidates, arrivals and generation, ticket
+        self.markov_words = torch.zeros(11, dtype=torch.int64, device=dev)
+        self.best, self.markov_sync, self.ticket = self.markov_words[:8], self.markov_words[8:10], self.markov_words[10:].view(i32)
         import os
         self.markov_chain = target.fused and os.environ.get("NAIVERT_MARKOV_CHAIN", "1") == "1"
-        self.ticket = torch.zeros(1, dtype=i32, device=dev)
         self.seed_buf, self.params_buf = seed_buf, params_buf
         # per-tile sums of squares of h (fc output) and of the block residual xd for the fused RMSNorms
         self.ssq_h = torch.zeros(Hd // 128, PAD_ROWS, dtype=f32, device=dev)
@@ -279,6 +279,11 @@ class DraftRuntime:
         self.markov_chain = False
         for step in range(d.block_size):
             K.markov_step(self.args_markov, step, pdl=pdl)
+
+    def forget_proposals(self) -> None:
+        """A launch whose bounded wait gave up leaves candidates behind and its arrivals off a multiple of the grid: the next one would be
+        released too early and could draw a stale candidate.  On the stream of the rounds, wherever a recorded fault is cleared."""
+        self.markov_words.zero_()
 
     def kv_bytes(self) -> int:
         return sum(L[k].numel() * 2 for L in self.layers for k in ("k", "v"))

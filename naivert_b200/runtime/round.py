@@ -213,7 +213,7 @@ class DecodeRound:
         ctrl[CTRL_MAX_TOKENS], ctrl[CTRL_CAPACITY], ctrl[CTRL_CURSOR], ctrl[CTRL_PROMPT_CTX] = max_tokens, self.capacity, start_pos, n - 1
         self.t.ctrl.copy_(ctrl)
         self.counts.zero_()
-        self.fab.status.zero_()
+        self._clear_faults()
         steps = -(-(n - 1 - start_pos) // self.t.rows)
         if steps:
             if use_graphs:
@@ -249,6 +249,12 @@ class DecodeRound:
         self.host_launches = 0
         self.ring.consumed.value = 0
 
+    def _clear_faults(self) -> None:
+        self.fab.status.zero_()
+        if self.draft is not None:
+            with torch.cuda.stream(self.stream):
+                self.draft.forget_proposals()
+
     def _capture_prefill(self):
         saved = self.t.ctrl.clone()
         g = self._capture(self.prefill_phases)
@@ -275,7 +281,7 @@ class DecodeRound:
         self.block_ids.copy_(saved_ids)
         if saved_feats is not None:
             self.t.feats.copy_(saved_feats)              # round 0 re-ingests the last replay chunk's features
-        self.fab.status.zero_()
+        self._clear_faults()
         torch.cuda.synchronize()
 
     def _capture_native(self):

@@ -72,6 +72,22 @@ def test_forced_acceptance_counts_and_determinism():
     assert all(0 <= t < spec.vocab for t in a.tokens)
 
 
+def test_request_after_a_proposal_launch_that_gave_up():
+    """What such a launch leaves (arrivals off a multiple of the grid, a candidate nobody cleared, a ticket) does not reach the next request:
+    proposals, all of them accepted here, are those of an untouched engine."""
+    from naivert_b200.models.spec import SamplingParams
+    spec, eng = _engine()
+    prompt, sp = torch.arange(3, 40), SamplingParams(temperature=0.4, seed=5, forced_accept_p=1.0)
+    want = eng.generate(prompt, 40, sp).tokens
+    d = eng.round.draft
+    d.markov_sync[0] += 5
+    d.best[2] = -4                                               # token 3 with the highest score
+    d.ticket[0] = 1
+    torch.cuda.synchronize()
+    assert eng.generate(prompt, 40, sp).tokens == want
+    eng.fabric.check()
+
+
 def test_speculative_equals_target_greedy():
     """With a one-token nucleus the committed sequence must equal plain greedy decoding of the
     target (every position rejected -> one verified token per round), whatever the draft proposes."""
