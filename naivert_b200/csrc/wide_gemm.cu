@@ -217,7 +217,9 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
     const int nt_count = p.n_total / kTileN;
     bool ok = true;
     int v = 0, t = 0;                                // pairs of K blocks and tiles so far
-    for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
+    constexpr int kBars = FP8 ? (EPI == kEpiSiluQuant ? 4 : 2) : 0;       // barriers of a tile
+    int w = blockIdx.x, owed = 0;                    // owed: of tile w when this warp's wait gave up there
+    for (; w < total; w += gridDim.x) {
       NRT_WIDE_DECODE(w, n_tile, item)
       if (item >= na) continue;
       const int z = p.active_ids[item];
@@ -268,7 +270,7 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
           }
         };
         ok = ask(0);
-        if (!ok) break;
+        if (!ok) { owed = kBars; break; }
         // activation scales of the item's 64 rows, transposed to [K block][row]; read coherently after the first
         // accumulator is ready (in the expert-parallel path peers wrote them shortly before).  The first barrier
         // keeps a fast warp from overwriting the table while a slow one still reads the previous tile's scales.
@@ -313,7 +315,7 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
             }
           }
         }
-        if (!ok) break;
+        if (!ok) { owed = kBars - 2; break; }
         v += (kb_total + 1) / 2;
 #pragma unroll
         for (int r = 0; r < kWCols / 2; ++r) {
@@ -378,6 +380,17 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
             st_tagged(dst, rtag, pack_bf16x2(acc0[r], other));
           }
         }
+      }
+    }
+    // A warp whose wait gave up (its limit, or a fault recorded elsewhere on the device meanwhile) still takes the barriers of the tiles it
+    // leaves: others may have seen the same accumulator in time, and would wait for it for good.
+    if (FP8 && !ok) {
+      for (;;) {
+        for (int i = 0; i < owed; ++i) asm volatile("bar.sync 1, 512;" ::: "memory");
+        if ((w += gridDim.x) >= total) break;
+        NRT_WIDE_DECODE(w, n_tile, item)
+        (void)n_tile;
+        owed = item < na ? kBars : 0;
       }
     }
   }

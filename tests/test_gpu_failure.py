@@ -61,6 +61,49 @@ def test_mailbox_wait_times_out_with_status_and_context_survives():
     assert (out.float() - ref).abs().max().item() <= 0.02 * ref.abs().max().item()
 
 
+@pytest.mark.parametrize("dual", [False, True])
+def test_chunk_gemm_launched_after_a_recorded_fault_returns(dual):
+    """Launches that were queued behind a kernel that gave up find its word in the status: some of their waits give up at once, some have what
+    they wait for.  Every launch ends, and with the word cleared the next one is right."""
+    from naivert_b200.ops import kernels as K
+    from naivert_b200.ops.quant import dequant_act, quantize_act_pow2, quantize_fp8_block, w8a8_linear_ref
+    K.lib()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    n, k, rows = 2048, 1152, 1024                                      # two tiles for some CTAs
+    ws = [quantize_fp8_block(torch.randn(n, k, device="cuda", generator=g) * 0.05) for _ in range(2)]
+    x = torch.randn(rows, k, device="cuda", generator=g).bfloat16().float()
+    xq, xs = quantize_act_pow2(x)
+    x8, xs = xq.view(torch.uint8).contiguous(), xs.float().contiguous()
+    off = torch.arange(rows // 64, dtype=torch.int32, device="cuda") * 64
+    ids, cnt = torch.zeros(rows // 64, dtype=torch.int32, device="cuda"), torch.tensor([rows // 64], dtype=torch.int32, device="cuda")
+    out = torch.zeros(rows, n, dtype=torch.bfloat16, device="cuda")
+    y8, ys = torch.zeros(rows, n, dtype=torch.uint8, device="cuda"), torch.zeros(rows, n // 128, device="cuda")
+    status = torch.tensor([0x501, 0, 0, 0], dtype=torch.int32, device="cuda")
+    maps = [K.weight_tmap(w.view(torch.uint8)) for w, _ in ws]
+    a = K.GemmArgs()
+    a.n_total, a.k_total, a.rows, a.out_scale = n, k, 64, 1.0
+    a.n_active, a.active_ids, a.max_slots, a.row_offsets = cnt.data_ptr(), ids.data_ptr(), rows // 64, off.data_ptr()
+    a.w_scale0, a.w_scale1, a.a_scale = ws[0][1].data_ptr(), ws[1][1].data_ptr(), xs.data_ptr()
+    a.out_q, a.out_qscale, a.out_bf16, a.ld_out, a.status = y8.data_ptr(), ys.data_ptr(), out.data_ptr(), n, status.data_ptr()
+    variant = K.gemm_variant(True, dual, K.EPI_SILU_QUANT if dual else K.EPI_STORE_BF16, K.GROUP_ITEM)
+
+    def launch():
+        K.wide_gemm(variant, maps[0], maps[1] if dual else None, K.act_tmap(x8, 64), a, n // 128, rows // 64)
+
+    for _ in range(30):
+        launch()
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0x501
+    status.zero_()
+    launch()
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0
+    gate, up = (w8a8_linear_ref(x, w, sc) for w, sc in ws)
+    want = torch.nn.functional.silu(gate) * up if dual else gate
+    got = dequant_act(y8.view(torch.float8_e4m3fn), ys) if dual else out.float()
+    assert (got - want).abs().max().item() <= (0.07 if dual else 0.01) * want.abs().max().item()
+
+
 def test_step_outputs_stay_inside_their_buffers():
     """Canary-fenced copies of the step's scratch and output buffers: a verify step must not touch the guard bytes
     around any of them."""
