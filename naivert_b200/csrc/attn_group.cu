@@ -8,7 +8,7 @@
 //       Bound by the gather, 1.3 MB per CTA at 2048 keys: 2048 rows x 4 KV heads in 1.51 ms, 7.1 TB/s out of the L2.
 //   sliding window   one CTA per (KV head, 4 warps x 16 / heads rows): neighbouring rows share all but one key of their
 //       window, so the rows' keys are staged once, 32 at a time, and every warp masks what its rows do not see.  Window 128,
-//       2048 rows x 64 heads: 114 us.
+//       2048 rows x 64 heads: 116 us, 2.5 of them for the look at what came out (attn_window_kernel's end).
 // A 16,001-token document of two sparse and four window layers spends 27.8 ms in them; 61.2 ms when every row gathered its keys for
 // itself into tiles that eight warps shared between four barriers.
 // Against fp64 (bf16 outputs, windows / lists of 2048 / prefixes): 1.82e-3 / 1.81e-3 / 1.79e-3; before 1.84e-3 / 1.91e-3 / 1.88e-3.
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(kWinWarps * 32, 2) attn_window_kernel(const At
       const int k0 = key0 + t * kWinKeys;
       if (k0 > w_high || k0 + kWinKeys <= w_low || r_lo >= a.rows) continue;
       const uint32_t sk = base + (t % kWinStages) * kWinStage;
-      w.tile<kWinKeys, ONE>(sk, sk + kWinKeys * kKRow, lane, a.scale, [&](int hi, int i) { return on[hi] && k0 + i >= low[hi] && k0 + i <= high[hi]; },
+      w.tile<kWinKeys, ONE>(sk, sk + kWinKeys * kKRow, lane, a.scale, [&](int hi, int i) { return (!ONE || on[hi]) && k0 + i >= low[hi] && k0 + i <= high[hi]; },
                             [&](int i) { return k0 + i >= w_low && k0 + i <= w_high; });
     }
     cp_async_wait<0>();
@@ -434,12 +434,12 @@ __global__ void __launch_bounds__(kWinWarps * 32, 2) attn_window_kernel(const At
   walk(std::false_type{}, 0);
   // A probability of zero does not hide an infinity or NaN of a value row that only other rows of the CTA see; what it
   // leaves in an output stays non-finite to the end.  Then every token row is walked again by itself, unseen values zeroed.
-  float top = 0.f;
+  float bad = 0.f;                                                    // zero times a finite value is zero
 #pragma unroll
   for (int t = 0; t < kVd / 8; ++t)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) top = fmaxf(top, fabsf(w.o[t][j] - w.o[t][j]) == 0.f ? 0.f : 1.f);
-  if (!__syncthreads_or(top != 0.f)) {
+    for (int j = 0; j < 4; ++j) bad = fmaf(w.o[t][j], 0.f, bad);
+  if (!__syncthreads_or(bad != 0.f)) {
     store(-1);
     return;
   }
