@@ -389,12 +389,7 @@ __global__ void __launch_bounds__(256, 2) attn_decode_kernel(const AttnArgs a) {
 
 template <int HD>
 int launch_decode(const AttnArgs& a, int splits, cudaStream_t stream, int pdl) {
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem<HD>));
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (const int rc = allow_shared(attn_decode_kernel<HD>, (int)sizeof(Smem<HD>))) return rc;
   return launch_pdl(attn_decode_kernel<HD>, dim3(a.kv_heads, a.rows, splits), dim3(256), sizeof(Smem<HD>), stream, pdl != 0, a);
 }
 

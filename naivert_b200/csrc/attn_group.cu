@@ -464,13 +464,7 @@ extern "C" int nrt_attn_group(const void* args, void* stream, int pdl) {
   if (a.head_dim != kHd || a.v_dim != kVd || a.kv_heads < 1 || a.heads % a.kv_heads || a.heads / a.kv_heads > kM) return -3;
   if (a.mode != 0 && a.mode != 1) return -3;
   if (a.rows > 65535) return -3;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kListSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_window_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWinSmem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (const int rc = a.mode == 1 ? allow_shared(attn_list_kernel, kListSmem) : allow_shared(attn_window_kernel, kWinSmem)) return rc;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (a.mode == 1) return launch_pdl(attn_list_kernel, dim3(a.kv_heads, a.rows), dim3(kListWarps * 32), kListSmem, s, pdl != 0, a);
   const int rows = kWinWarps * (kM / (a.heads / a.kv_heads));

@@ -409,16 +409,16 @@ extern "C" int nrt_markov_chain(const void* args, int steps, void* sync, void* s
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, markov_chain_kernel, 256, 0) != cudaSuccess) return -3;
-    if (cudaFuncSetAttribute(markov_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wide_smem) != cudaSuccess) return -3;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wide_per_sm, markov_wide_kernel, kWideWarps * 32, wide_smem) != cudaSuccess)
-      return -3;
+    if (allow_shared(markov_wide_kernel, wide_smem) ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wide_per_sm, markov_wide_kernel, kWideWarps * 32, wide_smem) != cudaSuccess)
+      wide_per_sm = 0;                            // the other forms do not need it
     wide = wide_per_sm * sms;
     resident = per_sm * sms;
   }
   unsigned long long* w = reinterpret_cast<unsigned long long*>(sync);
   // the in-grid hand-over needs every CTA resident: shards beyond what the register form holds at once take the wide one
   if (grid > resident) {
-    if (a.rank_dim != 256 || wide < 1) return -9;
+    if (a.rank_dim != 256 || wide < 1 || allow_shared(markov_wide_kernel, wide_smem)) return -9;
     const int iters = (a.vlocal + wide * kWideWarps * 4 - 1) / (wide * kWideWarps * 4);
     if (iters > 8 * kWideBatches) return -9;      // beyond 227,328 tokens: one launch per step
     const int ctas = (a.vlocal + kWideWarps * 4 * iters - 1) / (kWideWarps * 4 * iters);

@@ -14,12 +14,7 @@ int launch_variant(const CUtensorMap& a0, const CUtensorMap& a1, const CUtensorM
   using Cfg = GemmCfg<FP8, DUAL, BSRC>;
   auto* kern = skinny_gemm_kernel<FP8, DUAL, EPI, GROUP, BSRC>;
   constexpr int kMaxSmem = 227 * 1024;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (const int rc = allow_shared(kern, kMaxSmem)) return rc;
   if ((EPI == kEpiAllReduce || (GROUP != kGroupItem && gy > 1)) && args.rows > kArRows) return -5;
   const bool clustered = GROUP != kGroupItem && gy > 1;
   if (clustered && gy > kMaxSplit) return -4;

@@ -165,12 +165,7 @@ extern "C" int nrt_index_sweep(const void* tmK, const void* tmQ, const void* arg
   const int ncol = (a.rows > 16 ? 16 : a.rows) * a.heads;
   if (a.heads % 16 || ncol > 256 || ncol % 16) return -3;
   constexpr int smem = kSweepStages * kATileBytes + 256 * 128 + 2048 + 1024;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(index_sweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (const int rc = allow_shared(index_sweep_kernel, smem)) return rc;
   return launch_pdl(index_sweep_kernel, dim3(blocks, groups), dim3(kSweepThreads), smem, reinterpret_cast<cudaStream_t>(stream),
                     pdl != 0, k, q, a);
 }

@@ -692,24 +692,14 @@ __global__ void __launch_bounds__(256, 1) latent_decode_tc_kernel(const LatentDe
 
 template <int MT>
 int launch_decode_tc(const LatentDecodeArgs& a, cudaStream_t stream, bool pdl) {
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(latent_decode_tc_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (const int rc = allow_shared(latent_decode_tc_kernel<MT>, 227 * 1024)) return rc;
   return launch_pdl(latent_decode_tc_kernel<MT>, dim3((a.heads + MT * 16 - 1) / (MT * 16), a.splits), dim3(256), dec_smem(a.rank, MT), stream, pdl, a);
 }
 
 template <int NC>
 int launch_rows(const LatentAttnArgs& a, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    // (the largest of the sizes on both sides of the change from two stages to one)
-    const cudaError_t e = cudaFuncSetAttribute(latent_attn_rows_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 24 * 1024 * 4 + 8 * rows_ld(512) * 4);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  // (the largest of the sizes on both sides of the change from two stages to one)
+  if (const int rc = allow_shared(latent_attn_rows_kernel<NC>, 2 * 24 * 1024 * 4 + 8 * rows_ld(512) * 4)) return rc;
   const int per = kRowWarps * kRowsWarp;
   return launch_pdl(latent_attn_rows_kernel<NC>, dim3((a.rows + per - 1) / per, a.heads), dim3(kRowWarps * 32), rows_smem(a.dim, a.vdim), stream, false, a);
 }
@@ -738,12 +728,7 @@ extern "C" int nrt_latent_attn_tc(const void* tmQ, const void* tmK, const void* 
   memcpy(&a, args, sizeof(a));
   if (a.rows < 1 || a.group < 1 || a.heads % a.group || a.window < 0 || a.f32 || a.dim > 256 || a.vdim > 256 || a.dim % 8 || a.vdim % 8 || !(a.scale > 0.f) || ((!a.first || !a.last) && !a.state)) return -3;
   const int smem = tc_smem(a.dim, a.vdim);
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(latent_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (const int rc = allow_shared(latent_attn_tc_kernel, 227 * 1024)) return rc;
   return launch_pdl(latent_attn_tc_kernel, dim3((a.rows + kQRows - 1) / kQRows, a.heads), dim3(kTcThreads), smem,
                     reinterpret_cast<cudaStream_t>(stream), false, q, k, v, a);
 }

@@ -9,6 +9,8 @@
 #include <mutex>
 #include <unordered_set>
 
+#include "per_device.hpp"
+
 namespace nrt {
 
 // Every kernel asks for the same (maximum) shared-memory carve-out: kernels that follow one
@@ -20,6 +22,15 @@ inline void prefer_max_shared(const void* kernel) {
   std::lock_guard<std::mutex> lock(mu);
   if (done.insert(kernel).second)
     cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+}
+
+// Dynamic shared memory beyond 48 KB has to be asked for.
+template <typename... KArgs>
+int allow_shared(void (*kernel)(KArgs...), int bytes) {
+  static OncePerDevice once;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return once(reinterpret_cast<const void*>(kernel), dev, [&]() { return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
 }
 
 template <typename... KArgs, typename... Args>

@@ -542,6 +542,7 @@ extern "C" int nrt_moe_layer(const void* tmGate, const void* tmUp, const void* t
   if (r.rows * (r.hidden / 128) > 16 * kMoeCtas || r.hidden / 128 > 64) return -3;
   if (!a.sync || !a.slot_flags || !a.part || !a.part_flags || !a.y8 || !a.ys || !a.ar.status) return -3;
   constexpr int smem = kMoeStages * kMoeStageBytes + 1024 + (int)sizeof(MoeSmem);
+  if (const int rc = r.w != nullptr ? allow_shared(moe_layer_kernel<true>, smem) : allow_shared(moe_layer_kernel<false>, smem)) return rc;
   static int resident = -1;
   if (resident < 0) {
     int dev = 0, sms = 0;
@@ -549,11 +550,9 @@ extern "C" int nrt_moe_layer(const void* tmGate, const void* tmUp, const void* t
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int worst = 1 << 30;
     for (int route = 0; route < 2; ++route) {
-      const void* k = route ? (const void*)moe_layer_kernel<true> : (const void*)moe_layer_kernel<false>;
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      if (e != cudaSuccess) return (int)e;
+      if (const int rc = route ? allow_shared(moe_layer_kernel<true>, smem) : allow_shared(moe_layer_kernel<false>, smem)) return rc;
       int per_sm = 0;
-      e = route ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, moe_layer_kernel<true>, kMoeThreads, smem)
+      const cudaError_t e = route ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, moe_layer_kernel<true>, kMoeThreads, smem)
                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, moe_layer_kernel<false>, kMoeThreads, smem);
       if (e != cudaSuccess) return (int)e;
       worst = per_sm * sms < worst ? per_sm * sms : worst;

@@ -506,12 +506,7 @@ __global__ void __launch_bounds__(kDecThreads, DIM <= 128 ? 2 : 1) group_decode_
 
 template <int DIM>
 int launch_decode_tc(const GroupDecodeArgs& a, cudaStream_t stream, bool pdl) {
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(group_decode_tc_kernel<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWalkSmem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (const int rc = allow_shared(group_decode_tc_kernel<DIM>, kWalkSmem)) return rc;
   // eight warps with the most stages that fit, four where the rows are too wide for two stages of eight (or the merge for their rings)
   WalkShape w = {8, 4};
   const int dp = a.p.dp, vp = a.p.vp;
@@ -528,12 +523,7 @@ int launch_decode_tc(const GroupDecodeArgs& a, cudaStream_t stream, bool pdl) {
 template <bool F32, int VC>
 int launch_decode(const GroupDecodeArgs& a, cudaStream_t stream, bool pdl) {
   const int smem = 4 * group_smem_floats(a.p.dp, a.p.vp);
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(group_decode_kernel<F32, VC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (const int rc = allow_shared(group_decode_kernel<F32, VC>, 64 * 1024)) return rc;
   const int group = a.p.heads / a.p.kv_heads;
   return launch_cluster(group_decode_kernel<F32, VC>, dim3(a.splits, a.p.kv_heads, (group + kHB - 1) / kHB), dim3(kDecThreads), dim3(a.splits, 1, 1), smem, stream,
                         pdl, a);

@@ -255,12 +255,7 @@ int launch(const CUtensorMap& w, const CUtensorMap& w2, const CUtensorMap& x, co
   constexpr bool DUAL = EPI == kSEpiClampedGlu || EPI == kSEpiSiluGlu;
   using C = Cfg<NTOK, DUAL>;
   auto* kern = stack_gemm_kernel<NTOK, EPI>;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (const int rc = allow_shared(kern, C::kSmem)) return rc;
   const int n_tiles = (a.n + kFeat - 1) / kFeat;
   const int row_tiles = (a.rows + NTOK - 1) / NTOK;
   const int items = a.n_items ? a.max_items : a.zcount * row_tiles;
@@ -410,12 +405,7 @@ template <int T, int EPI>
 int launch_f32_tile(const StackGemmArgs& a, cudaStream_t stream) {
   constexpr bool DUAL = EPI == kSEpiClampedGlu || EPI == kSEpiSiluGlu;
   constexpr int smem = kFStages * (int)sizeof(F32Stage<T, DUAL>);
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(stack_gemm_f32_kernel<T, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (const int rc = allow_shared(stack_gemm_f32_kernel<T, EPI>, smem)) return rc;
   const int row_tiles = (a.rows + T - 1) / T;
   const long long items = a.n_items ? (long long)a.max_items * ((a.item_rows + T - 1) / T) : (long long)a.zcount * row_tiles;
   if (items < 1 || items > 65535) return -3;

@@ -416,12 +416,7 @@ extern "C" int nrt_stack_rows(const void* args, void* stream) {
   if (a.rows < 1 || a.width < 1 || (a.y && !a.post_w) || (a.y2 && (!a.y || a.slot_of || !a.join_w || !a.join_w2))) return -3;
   const size_t smem = (size_t)a.width * 8;
   if (smem > 200 * 1024) return -7;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(stack_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (const int rc = allow_shared(stack_rows_kernel, 200 * 1024)) return rc;
   return launch_pdl(stack_rows_kernel, dim3(a.rows), dim3(256), smem, S(stream), false, a);
 }
 

@@ -903,18 +903,9 @@ __global__ void __launch_bounds__(kStepT, 1) state_step_kernel(const StateStepAr
 
 constexpr int kMaxSmem = 220 * 1024;
 
-template <class K>
-int allow_smem(K kern, bool& done) {
-  if (done) return 0;
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-  done = e == cudaSuccess;
-  return (int)e;
-}
-
 template <int KIND, int L, int NV>
 int launch_chunk(const StateChunkArgs& a, cudaStream_t stream) {
-  static bool configured = false;
-  if (const int rc = allow_smem(state_chunk_kernel<KIND, L, NV, false>, configured)) return rc;
+  if (const int rc = allow_shared(state_chunk_kernel<KIND, L, NV, false>, kMaxSmem)) return rc;
   constexpr int PER_WARP = 32 / L * kQuad;
   const int C = a.vdim + extra_columns<KIND>();
   int warps = 8;                               // as few as it takes to give most SMs a CTA
@@ -933,8 +924,7 @@ int launch_chunk(const StateChunkArgs& a, cudaStream_t stream) {
   if (smem > kMaxSmem) return -7;
   if constexpr (KIND != kStateDelta) {
     if (pieces > 1) {
-      static bool sums_configured = false;
-      if (const int rc = allow_smem(state_chunk_kernel<KIND, L, NV, true>, sums_configured)) return rc;
+      if (const int rc = allow_shared(state_chunk_kernel<KIND, L, NV, true>, kMaxSmem)) return rc;
       const int rc = launch_pdl(state_chunk_kernel<KIND, L, NV, true>, dim3(grid.x, grid.y, pieces - 1), dim3(warps * 32), smem, stream, false, a, per);
       if (rc) return rc;
     }
@@ -958,8 +948,7 @@ int chunk_by_dim(const StateChunkArgs& a, cudaStream_t stream) {
 }
 template <int KIND, int NV>
 int launch_state_step(const StateStepArgs& a, cudaStream_t stream, bool pdl) {
-  static bool configured = false;
-  if (const int rc = allow_smem(state_step_kernel<KIND, NV>, configured)) return rc;
+  if (const int rc = allow_shared(state_step_kernel<KIND, NV>, kMaxSmem)) return rc;
   int ctas = 1;                                // per head: a cluster, while that fits the SMs and leaves 16 columns each
   while (ctas < 8 && a.heads * ctas * 2 <= 148 && a.vdim >= 32 * ctas) ctas *= 2;
   const int per = (a.vdim + ctas - 1) / ctas;

@@ -576,12 +576,7 @@ int launch_step(const StepArgs& a, const RouterArgs& r, int groups, int keep, cu
   constexpr bool PER_GROUP = PRO == kProLoad || PRO == kProMerge || PRO == kProMix;
   constexpr int CUT = DUAL ? kSlot / 32 : kSlot / 16;
   auto* kern = stack_step_kernel<PRO, EPI, ROUTE>;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxStepSmem - (ROUTE ? 8192 : 0));
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (const int rc = allow_shared(kern, kMaxStepSmem - (ROUTE ? 8192 : 0))) return rc;
   const int n_last = a.n_last ? a.n_last : a.n;
   const long long R = (long long)(a.groups - 1) * a.n + n_last;
   if (R > 0x7fffffffLL) return -3;

@@ -949,11 +949,7 @@ extern "C" int nrt_attn_rows(const void* args, int splits, void* stream, int pdl
   AttnArgs a;
   memcpy(&a, args, sizeof(a));
   const size_t smem = (size_t)kAttnChunk * ((a.head_dim + kAttnKPad) + a.v_dim) * 2;
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(attn_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
-    configured = true;
-  }
+  if (const int rc = allow_shared(attn_rows_kernel, 128 * 1024)) return rc;
   if (a.head_dim % 8 || a.v_dim % 8 || a.head_dim > 256 || a.v_dim > 128 || smem > 128 * 1024) return -3;
   if (splits > 1 && (!a.part || !a.tickets)) return -3;
   return launch_pdl(attn_rows_kernel, dim3(a.heads, a.rows, splits < 1 ? 1 : splits), dim3(128), smem, S(stream), pdl != 0, a);
@@ -963,11 +959,7 @@ extern "C" int nrt_index_logits_simple(const void* args, int blocks, void* strea
   IndexArgs a;
   memcpy(&a, args, sizeof(a));
   const size_t smem = (size_t)a.rows * a.heads * a.dim * sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(index_logits_simple_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-    configured = true;
-  }
+  if (const int rc = allow_shared(index_logits_simple_kernel, 160 * 1024)) return rc;
   return launch_pdl(index_logits_simple_kernel, dim3(blocks), dim3(256), smem, S(stream), pdl != 0, a);
 }
 extern "C" int nrt_topk_rows(const float* logits, int ld, const int* pos0, int rows, int top_k, int* sel, void* stream,

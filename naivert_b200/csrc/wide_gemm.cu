@@ -407,12 +407,7 @@ int launch_wide(const CUtensorMap& a0, const CUtensorMap& a1, const CUtensorMap&
                 int order, cudaStream_t stream, int pdl) {
   using Cfg = WideCfg<FP8, DUAL>;
   auto* kern = wide_gemm_kernel<FP8, DUAL, EPI>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  if (const int rc = allow_shared(kern, Cfg::kSmemBytes)) return rc;
   if (FP8 && args.k_total / 128 > Cfg::kMaxKBlocks) return -6;        // scale table size
   if (n_tiles < 1 || items < 1 || (long long)n_tiles * items > 0x7fffffffLL) return -3;
   static int sms = 0;

@@ -1,6 +1,7 @@
 """Guarded tensors, layering (import direction), build manifest."""
 import ast
 import os
+import subprocess
 
 import pytest
 import torch
@@ -394,6 +395,41 @@ def test_stamp_reports_from_synthetic_buffers():
         samp[2 * ph], samp[2 * ph + 1] = t0 + 10_000 * ph + 3000, t0 + 10_000 * ph + 8000
     out = report_sampler_stamps(samp)
     assert len(out) == 8 and "maxima" in out[1] and "3.00 /     8.00" in out[1] and "63.00 /    68.00" in out[7]
+
+
+def test_kernel_limits_are_told_once_per_device(tmp_path):
+    """The registry behind the kernels' shared-memory limits: every device of a process is told, a refusal is not remembered, and
+    several threads tell it once; no launcher keeps a flag of its own."""
+    csrc = os.path.join(ROOT, "naivert_b200", "csrc")
+    for name in os.listdir(csrc):
+        if name != "launch.hpp":
+            with open(os.path.join(csrc, name)) as f:
+                assert "cudaFuncAttributeMaxDynamicSharedMemorySize" not in f.read(), name
+    main = tmp_path / "main.cpp"
+    main.write_text('''
+#include "per_device.hpp"
+#include <atomic>
+#include <cstdio>
+#include <thread>
+#include <vector>
+int main() {
+  nrt::OncePerDevice once;
+  int a = 0, b = 0;
+  std::atomic<int> told{0};
+  auto ok = [&]() { ++told; return 0; };
+  int rc = once(&a, 0, [&]() { ++told; return 7; });
+  if (rc != 7) return 1;
+  if (once(&a, 0, ok) || once(&a, 0, ok) || told != 2) return 2;
+  if (once(&a, 1, ok) || told != 3) return 3;
+  if (once(&b, 1, ok) || told != 4) return 4;
+  std::vector<std::thread> ts;
+  for (int i = 0; i < 8; ++i) ts.emplace_back([&]() { for (int d = 0; d < 50; ++d) once(&b, 2 + d, ok); });
+  for (auto& t : ts) t.join();
+  return told == 54 ? 0 : 5;
+}
+''')
+    subprocess.run(["g++", "-std=c++17", "-pthread", "-I", csrc, str(main), "-o", str(tmp_path / "main")], check=True)
+    assert subprocess.run([str(tmp_path / "main")]).returncode == 0
 
 
 def test_stream_handle_does_not_depend_on_private_names(monkeypatch):
