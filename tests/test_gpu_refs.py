@@ -227,3 +227,52 @@ def test_markov_chain_equals_its_steps(vlocal):
         got.append((zq, block))
     for zq, block in got[1:]:
         assert torch.equal(zq, got[0][0]) and torch.equal(block, got[0][1])
+
+
+@pytest.mark.parametrize("vlocal", [1500, 37888, 37889, 76288])
+def test_markov_chain_with_the_other_ranks_candidates(vlocal):
+    """Two ranks: the words of rank 1 lie in rank 0's mailbox before the launch (no kernel waits for another), so that steps 0 and 2 go to
+    this rank and 1 and 3 to the other one.  Both one-launch forms against single steps: logits, proposals and the words pushed out."""
+    K = _K()
+    g = torch.Generator(device="cuda").manual_seed(vlocal)
+    vocab, steps, epoch_no, slabs, words = 2 * vlocal, 4, 9, 4, 4096
+    w1 = (torch.randn(vocab, 256, device="cuda", generator=g) * 0.3).bfloat16()
+    w2 = (torch.randn(vlocal, 256, device="cuda", generator=g) * 0.3).bfloat16()
+    logits = torch.randn(16, vlocal, device="cuda", generator=g) * 2
+    params = torch.tensor([1, 0.95, 1, 0, 0, -1, 1.25, 0], dtype=torch.float32, device="cuda")
+    seed, ctrl = torch.tensor([99], dtype=torch.int64, device="cuda"), torch.full((16,), 3, dtype=torch.int32, device="cuda")
+    sync = torch.zeros(2, dtype=torch.int64, device="cuda")
+    box = torch.zeros(2, slabs * 2 * words * 2, 2, dtype=torch.int32)          # rank -> (slab, sender, word, half) -> (payload, tag)
+    theirs = []
+    for step in range(steps):
+        score, token = (1e6 if step % 2 else -1e6), vlocal + 7 * step + 1
+        bits = int(torch.tensor(score).view(torch.int32)) & 0xffffffff
+        order = (~bits & 0xffffffff) if bits >> 31 else bits | 0x80000000
+        for half, payload in enumerate((~token & 0xffffffff, order)):
+            at = (((16 + step) % slabs * 2 + 1) * words + 0) * 2 + half
+            box[0, at] = torch.tensor([payload - (payload >> 31 << 32), epoch_no * 64 + 16 + step + 1], dtype=torch.int32)
+        theirs.append(token)
+    got = []
+    for chain in (False, True, True):
+        zq, block = torch.zeros(8, vlocal, device="cuda"), torch.tensor([5] + [0] * 7, dtype=torch.int32, device="cuda")
+        best, ticket = torch.zeros(8, dtype=torch.int64, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        st, epoch = torch.zeros(4, dtype=torch.int32, device="cuda"), torch.full((1,), epoch_no, dtype=torch.int32, device="cuda")
+        mail = box.cuda()
+        m = K.MarkovArgs()
+        m.logits, m.ld, m.w1, m.w2, m.rank_dim = logits.data_ptr(), vlocal, w1.data_ptr(), w2.data_ptr(), 256
+        m.vlocal, m.vbase, m.vocab = vlocal, 0, vocab
+        m.block_ids, m.zq, m.params, m.seed, m.ctrl = block.data_ptr(), zq.data_ptr(), params.data_ptr(), seed.data_ptr(), ctrl.data_ptr()
+        m.best, m.ticket = best.data_ptr(), ticket.data_ptr()
+        m.x.box[0], m.x.box[1] = mail[0].data_ptr(), mail[1].data_ptr()
+        m.x.epoch, m.x.status, m.x.tp, m.x.rank, m.x.timeout_ns = epoch.data_ptr(), st.data_ptr(), 2, 0, 10 ** 9
+        if chain:
+            assert K.markov_chain(m, steps, sync, pdl=False) == 0
+        else:
+            for i in range(steps):
+                K.markov_step(m, i, pdl=False)
+        torch.cuda.synchronize()
+        assert int(st[0]) == 0 and not best.any()
+        assert block[2] == theirs[1] and block[4] == theirs[3] and 0 <= block[1] < vlocal and 0 <= block[3] < vlocal
+        got.append((zq, block, mail[1]))
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], other))
