@@ -62,16 +62,20 @@ def chunk_work(eng, pos0: int, R: int) -> Dict[str, List[float]]:
         d = r["layer"]
         m, f = d["spec"].mixer, d["spec"].mlp
         w.add("rows", 0, R * W * (4 + 4 + 4 + es))
-        CHUNK_MIXERS[d["kind"]].work(w, m, d, pos0, R)
+        parts = [(c0, min(eng.prefill.C, R - c0)) for c0 in range(0, R, eng.prefill.C)]     # of a span: experts alone take its chunks together
+        for c0, n in parts:
+            CHUNK_MIXERS[d["kind"]].work(w, m, d, pos0 + c0, n)
         if f is None:
             continue
         w.add("rows", 0, R * W * (4 + 4 + 4 + es))
         if f.kind == "relu2":
-            w.gemm("ff_up", f.ff, W, R, es)
-            w.gemm("ff_down", W, f.ff, R, 4)
+            for _, n in parts:
+                w.gemm("ff_up", f.ff, W, n, es)
+                w.gemm("ff_down", W, f.ff, n, 4)
         elif f.kind == "dense":
-            w.gemm("dense_gate_up", f.ff, W, R, es, mats=2)
-            w.gemm("dense_down", W, f.ff, R, 4)
+            for _, n in parts:
+                w.gemm("dense_gate_up", f.ff, W, n, es, mats=2)
+                w.gemm("dense_down", W, f.ff, n, 4)
         else:
             rt = f.routing
             P = R * rt.top_k
@@ -224,7 +228,7 @@ def run(model: str, prompt_len: int, steps: int, warmup: int, chunk: int, kernel
     try:
         g = torch.Generator().manual_seed(0)
         prompt = torch.randint(0, spec.vocab, (prompt_len,), generator=g, dtype=torch.int32).pin_memory()
-        eng.prefill.warm_chunks([chunk])
+        eng.prefill.warm_chunks([chunk, prompt_len])
         eng.prefill.run(prompt, 0, prompt_len - 1)
         torch.cuda.synchronize()
         pre = []
@@ -267,6 +271,9 @@ def run(model: str, prompt_len: int, steps: int, warmup: int, chunk: int, kernel
             n0 = min(prompt_len // 2, prompt_len - 1 - chunk) if prompt_len > chunk else 0
             eng.prefill.run(prompt, 0, n0) if n0 else None
             out["chunk_kernels"] = {"pos0": n0, "rows": chunk, "table": chunk_table(eng, prompt, n0, min(chunk, prompt_len - n0))}
+            span = min(eng.prefill.span_limit, prompt_len)
+            if span > chunk:                              # chunks that go through the routed experts together, as the prompt above
+                out["span_kernels"] = {"pos0": 0, "rows": span, "table": chunk_table(eng, prompt, 0, span)}
             eng.prefill.run(prompt, 0, prompt_len - 1)
             out["step_kernels"] = {"pos": prompt_len - 1, "table": step_table(eng, prompt_len - 1)}
         eng.fabric.check()
