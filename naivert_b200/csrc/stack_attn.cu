@@ -272,7 +272,9 @@ __global__ void __launch_bounds__(kDecThreads) group_decode_kernel(const GroupDe
 // 140 KB in flight that one SM's share of the memory's rate needs.  The warps' results are merged once, then the cluster's.  The first
 // tiles are requested before the wait for the predecessor (older rows do not depend on it; the token's own row is put into its tile by
 // hand).  tcgen05 is not used: the kernel streams the cache once, and most of its M = 128 rows would idle.
-// 12,290 keys, 8 key heads of 4 x 128: 40 us inside a step; 62 us with tiles of 64 keys that all warps worked on between four barriers.
+// 12,290 keys, 8 key heads of 4 x 128: 44 us inside a step from launch to end (the wait for the predecessor included), 59 us with tiles of 64
+// keys that all warps worked on between four barriers; alone 39.7 and 53.9 us.  Groups of more than 16 heads take a CTA per 16, each of
+// which reads the split's rows (the second from L2): 32 heads of one key head 41.5 us alone, 83.9 us as one tile of 32 rows in that form.
 constexpr int kTcHead = 256, kWalkKeys = 16, kWalkM = 16, kWalkSmem = 225 * 1024;
 __host__ __device__ inline int tc_pitch(int n) { return (n + 15) / 16 * 16 + 8; }              // bf16 elements; rows fall into distinct banks
 struct WalkShape { int warps, stages; };               // walking warps of a CTA, ring stages of each
@@ -281,8 +283,8 @@ __host__ __device__ inline int walk_smem(int dp, int vp, WalkShape w) {
   return walk_ring(dp, vp, w) + 2 * kWalkM * tc_pitch(dp) + 4 * (2 * kWalkM * (w.warps + 1) + 8 * kTcHead + kTcHead) + 2 * (dp + vp);
 }
 
-// DIM: most columns of keys and values (registers of the outputs).  Up to 128 the kernel keeps to half of an SM's registers, so that it starts
-// while its predecessor still runs.
+// DIM: most columns of keys and values (registers of the outputs).  Up to 128 the kernel keeps to half of an SM's registers: its rings (224 KB of
+// shared memory at 128 x 128) leave room for a state step's few KB beside them, but not for the launch of a product.
 template <int DIM>
 __global__ void __launch_bounds__(kDecThreads, DIM <= 128 ? 2 : 1) group_decode_tc_kernel(const GroupDecodeArgs a, const WalkShape ws) {
   extern __shared__ __align__(16) uint8_t raw[];
