@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kDecThreads) group_decode_kernel(const GroupDe
 // hand).  tcgen05 is not used: the kernel streams the cache once, and most of its M = 128 rows would idle.
 // 12,290 keys, 8 key heads of 4 x 128: 44 us inside a step from launch to end (the wait for the predecessor included), 59 us with tiles of 64
 // keys that all warps worked on between four barriers; alone 39.7 and 53.9 us.  Groups of more than 16 heads take a CTA per 16, each of
-// which reads the split's rows (the second from L2): 32 heads of one key head 41.5 us alone, 83.9 us as one tile of 32 rows in that form.
+// which reads the split's rows (the second from L2): 32 heads of one key head 41.6 us alone, 83.9 us as one tile of 32 rows in that form.
 constexpr int kTcHead = 256, kWalkKeys = 16, kWalkM = 16, kWalkSmem = 225 * 1024;
 __host__ __device__ inline int tc_pitch(int n) { return (n + 15) / 16 * 16 + 8; }              // bf16 elements; rows fall into distinct banks
 struct WalkShape { int warps, stages; };               // walking warps of a CTA, ring stages of each
@@ -323,8 +323,9 @@ __global__ void __launch_bounds__(kDecThreads, DIM <= 128 ? 2 : 1) group_decode_
     const int c = lane & (lanes - 1), rows = 32 / lanes;
     if (c >= width / 8) return;
     const long long row_step = (long long)p.kv_heads * width;
-    // rolled: a launch inside a step fetches its instructions anew, and at short contexts it is little more than that (1.5 us less)
-#pragma unroll 1
+    // Rolled where a pass of the lanes is two rows or more: a launch inside a step fetches its instructions anew, and at short contexts it is
+    // little more than that (1.5 us less).  Wider rows take sixteen passes, which have to overlap (2 x 32 heads of 256, 12,289 keys: 84 / 96 us).
+#pragma unroll (DIM <= 128 ? 1 : 8)
     for (int t = lane / lanes; t < kWalkKeys; t += rows) {
       const bool in = j0 + t < j_hi && j0 + t != n - 1;                  // the token's own row is not in the cache yet
       cp16(dst + t * pitch + c * 8, in ? src + (long long)(start + j0 + t) * row_step + c * 8 : src, in);
