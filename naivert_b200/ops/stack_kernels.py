@@ -48,6 +48,14 @@ ENTRIES = {"nrt_stack_gemm": ("StackGemmArgs", "nrt_stack_gemm_args_size"), "nrt
            "nrt_short_conv": ("ShortConvArgs", "nrt_short_conv_args_size"), "nrt_token_mix": ("TokenMixArgs", "nrt_token_mix_args_size"),
            "nrt_head_gate": ("HeadGateArgs", "nrt_head_gate_args_size")}
 
+# what the entry points take, so that addresses and handles go in as plain integers (wrapping each costs as much as the call)
+_I = C.c_int
+_TYPES = {**{n: [VP, VP] for n in ("nrt_stack_rows", "nrt_latent_prep", "nrt_latent_attn_rows", "nrt_stack_conv", "nrt_stack_scan", "nrt_moe_gather",
+                                   "nrt_group_prep", "nrt_transpose", "nrt_short_conv", "nrt_token_mix", "nrt_head_gate")},
+          **{n: [VP, VP, _I] for n in ("nrt_latent_decode", "nrt_group_decode", "nrt_state_step", "nrt_ep_count")},
+          "nrt_stack_gemm": [_I, _I, VP, VP, VP, VP, _I, VP], "nrt_stack_gemm_f32": [_I, VP, VP], "nrt_state_chunk": [_I, VP, VP],
+          "nrt_latent_attn_tc": [VP, VP, VP, VP, VP], "nrt_stack_route": [VP, _I, _I, VP], "nrt_stack_step": [_I, _I, VP, VP, _I, _I, VP, _I]}
+
 _lib = None
 
 
@@ -63,15 +71,13 @@ def lib() -> C.CDLL:
                 raise RuntimeError(f"{struct}: library has {getattr(L, size)()} bytes, bindings {C.sizeof(_G[struct])}")
         if L.nrt_ep_args_size() != C.sizeof(K.EpArgs):
             raise RuntimeError("EpArgs layout drift")
+        for entry, types in _TYPES.items():
+            getattr(L, entry).argtypes = types
         _lib = L
     return _lib
 
 
-_handle = K._stream
-
-
-def _stream() -> VP:
-    return VP(_handle())
+_stream = K._stream
 
 
 def weight_map(w: torch.Tensor, k: int) -> K.TensorMap:

@@ -11,8 +11,9 @@ the step continues from.  Where the chunks are too short to fill the routed expe
 """
 from __future__ import annotations
 
-from contextlib import contextmanager
-from typing import Dict, List, Optional, Sequence, Tuple
+from contextlib import contextmanager, nullcontext
+from functools import lru_cache
+from typing import Callable, Dict, List, Optional, Sequence, Tuple
 
 import torch
 
@@ -33,6 +34,9 @@ FUNCTION_EPI = (S.EPI_TANH, S.EPI_DECAY_SOFT, S.EPI_DECAY_EXP)
 SPAN_PAIRS, SPAN_ROWS = 256, 8192
 
 
+_UNTIMED = nullcontext()
+
+
 class StackPrefill:
     quantum = 1
 
@@ -46,6 +50,10 @@ class StackPrefill:
         ffs = [d["spec"].mlp for d in L if d["spec"].mlp is not None]
         moe = [f for f in ffs if f.kind == "moe"]
         self.h_ld = pad(s.hidden, 8)
+        # Argument blocks by launch: a prompt of a small model is 77 launches of a few microseconds, and filling some twenty fields anew for
+        # each took longer.  What changes from prompt to prompt - rows, positions, segments - is set every time.  (Buffers that are taken
+        # anew clear it.)
+        self._kept: Dict[tuple, object] = {}
         filled = min([-(-SPAN_PAIRS * f.routing.expert_count // f.routing.top_k) for f in moe], default=0)
         self.span_limit = max(C, min(SPAN_ROWS, filled, runtime.capacity) // C * C)
         self._size_span(C)
@@ -86,6 +94,7 @@ class StackPrefill:
                        max_items=items, item_z=z(items, i32), item_row=z(items, i32), cap=cap, sorted=z(cap * self.h_ld, self.act),
                        ea=z(cap * max(pad(f.ff, 8) for f in moe), self.act), ey=z(cap * s.hidden))
         self.rows_of, self.span = rows_of, P
+        self._kept.clear()
         for name, v in new.items():
             setattr(self, name, v)
         self._window()
@@ -103,11 +112,18 @@ class StackPrefill:
                 P -= self.C
                 self.span_limit = P
 
-    @contextmanager
+    def kept(self, key: tuple, build: Callable[[], object]):
+        """The argument block that ``build`` made for ``key`` (its launch, layer run and whatever else its fixed fields hang on)."""
+        a = self._kept.get(key)
+        if a is None:
+            a = self._kept[key] = build()
+        return a
+
     def stage(self, name: str):
-        if not self.profile:
-            yield
-            return
+        return self._stage(name) if self.profile else _UNTIMED
+
+    @contextmanager
+    def _stage(self, name: str):
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         a.record()
         yield
@@ -143,6 +159,7 @@ class StackPrefill:
         return self.maps[key]
 
     @staticmethod
+    @lru_cache(maxsize=4096)
     def tile_rows(epi: int, tiles: int, rows: int) -> int:
         """Token rows per tile of a product with ``tiles`` feature tiles.  Few rows are one tile where the feature tiles occupy more than
         half of the SMs: every weight is then fetched by one CTA only, and what is in flight - which bounds a product that streams
@@ -165,21 +182,31 @@ class StackPrefill:
 
     def gemm(self, epi: int, w: Packed, x: torch.Tensor, x_ld: int, rows: int, out: torch.Tensor, out_ld: int, *, w2: Optional[Packed] = None,
               z: int = 1, x_z: int = 0, out_z: int = 0, x_off: int = 0, x_rows: Optional[int] = None, items: Optional[tuple] = None,
-              bias: Optional[torch.Tensor] = None, rate: Optional[torch.Tensor] = None, act_cols: int = 0, scale: float = 1.0, limit: float = 0.0, alpha: float = 0.0) -> None:
-        """out[row, z, :] = epilogue(W_z x[row, z, :]) for every token row; ``items`` = (segment rows, most segments)."""
-        a = S.StackGemmArgs()
-        a.n, a.k, a.rows, a.zcount = w.n, w.k, rows, z
-        a.out, a.out_ld, a.out_zstride, a.out_f32 = out.data_ptr(), out_ld, out_z, int(out.dtype == torch.float32)
-        a.bias = None if bias is None else bias.data_ptr()
-        a.rate = None if rate is None else rate.data_ptr()
-        a.act_cols, a.scale, a.limit, a.alpha, a.status = act_cols, scale, limit, alpha, self.t.fab.status.data_ptr()
+              bias: Optional[torch.Tensor] = None, rate: Optional[torch.Tensor] = None, act_cols: int = 0, scale: float = 1.0, limit: float = 0.0, alpha: float = 0.0,
+             keep: bool = False) -> None:
+        """out[row, z, :] = epilogue(W_z x[row, z, :]) for every token row; ``items`` = (segment rows, most segments).  ``keep``: weights
+        and buffers are the engine's own, which stay, and so does the argument block (a weight and an epilogue have one caller)."""
+        def build():
+            a = S.StackGemmArgs()
+            a.n, a.k, a.zcount = w.n, w.k, z
+            a.out, a.out_ld, a.out_zstride, a.out_f32 = out.data_ptr(), out_ld, out_z, int(out.dtype == torch.float32)
+            a.bias = None if bias is None else bias.data_ptr()
+            a.rate = None if rate is None else rate.data_ptr()
+            a.act_cols, a.scale, a.limit, a.alpha, a.status = act_cols, scale, limit, alpha, self.t.fab.status.data_ptr()
+            if items is not None:
+                a.n_items, a.item_z, a.item_row = self.n_items.data_ptr(), self.item_z.data_ptr(), self.item_row.data_ptr()
+            if self.f32:
+                a.act, a.act_ld, a.act_zstride = x.data_ptr() + 4 * x_off, x_ld, x_z
+                a.w, a.w2 = w.w.data_ptr(), None if w2 is None else w2.w.data_ptr()
+                a.w_ld, a.w_zstride = w.ld, w.n * w.ld
+            return a, w, {}                              # (the weight's name in the key stays its own)
+
+        key = ("gemm", epi, id(w), x.data_ptr(), x_off, out.data_ptr(), out_ld, items is None)
+        a, _, maps = self.kept(key, build) if keep else build()
+        a.rows = rows
         if items is not None:
-            a.n_items, a.item_z, a.item_row = self.n_items.data_ptr(), self.item_z.data_ptr(), self.item_row.data_ptr()
             a.item_rows, a.max_items = items
         if self.f32:
-            a.act, a.act_ld, a.act_zstride = x.data_ptr() + 4 * x_off, x_ld, x_z
-            a.w, a.w2 = w.w.data_ptr(), None if w2 is None else w2.w.data_ptr()
-            a.w_ld, a.w_zstride = w.ld, w.n * w.ld
             S.gemm_f32(epi, a)
             return
         dual = w2 is not None
@@ -188,17 +215,27 @@ class StackPrefill:
         else:
             ntok = self.tile_rows(epi, -(-w.n // 128) * z, rows)
         live = x_rows if x_rows is not None else x.numel() // x_ld
-        xm = self._xmap(x, w.k, z, x_z, live, x_ld, ntok, x_off)
-        wbytes = w.nbytes * (2 if dual else 1)
-        S.gemm(epi, ntok, self._wmap(w), self._wmap(w2) if dual else None, xm, a, items is None and wbytes > (96 << 20))
+        made = maps.get((ntok, live))
+        if made is None:
+            made = maps[ntok, live] = (self._wmap(w), self._wmap(w2) if dual else None, self._xmap(x, w.k, z, x_z, live, x_ld, ntok, x_off),
+                                       items is None and w.nbytes * (2 if dual else 1) > (96 << 20))
+        S.gemm(epi, ntok, *made[:3], a, made[3])
+
+    def product(self, *args, **more) -> None:
+        """``gemm`` of the engine's own weights and buffers."""
+        self.gemm(*args, keep=True, **more)
 
     # ------------------------------------------------------------------ one span
     def _window(self, chunk: Optional[int] = None) -> None:
-        """``pos``, ``x``, ``h``, ``y`` and ``y2`` become those of one chunk of the span, or of the whole of it."""
-        for name, t in self.rows_of.items():
-            if chunk is not None and t is not None:
-                t = t[chunk:chunk + 1] if name == "pos" else t[chunk * self.C:(chunk + 1) * self.C]
-            setattr(self, name, t)
+        """``pos``, ``x``, ``h``, ``y`` and ``y2`` become those of one chunk of the span, or of the whole of it (``at``: which, -1 all)."""
+        self.at = -1 if chunk is None else chunk
+
+        def build():
+            if chunk is None:
+                return self.rows_of
+            return {name: None if t is None else t[chunk:chunk + 1] if name == "pos" else t[chunk * self.C:(chunk + 1) * self.C] for name, t in self.rows_of.items()}
+
+        self.__dict__.update(self.kept(("window", chunk), build))
 
     def _chunks(self, R: int, pos0: int):
         """(rows, first position) of the chunks of a span of R rows, each with its own rows in place."""
@@ -210,20 +247,30 @@ class StackPrefill:
     def _rows(self, R: int, *, embed: bool = False, y: Optional[torch.Tensor] = None, post=None, y2: Optional[torch.Tensor] = None, join=None,
               moe=None, add=None, pre=None, copy: bool = False) -> None:
         """Stream update; then the input rows ``h`` of the next sublayer: normed by ``pre``, or the stream itself (``copy``)."""
-        s, a = self.spec, S.StackRowArgs()
-        if embed:
-            a.tokens, a.table, a.vocab, a.embed_scale = self.tokens.data_ptr(), self.t.embed.data_ptr(), s.vocab, s.embed_scale
-        if y is not None:
-            a.y, a.y_ld, a.post_w = y.data_ptr(), s.hidden, post.data_ptr()
-            if join is not None:
-                a.y2, a.join_w, a.join_w2 = y2.data_ptr(), join[0].data_ptr(), join[1].data_ptr()
-            if moe is not None:
-                a.slot_of, a.probs, a.top_k = self.slot_of.data_ptr(), self.probs.data_ptr(), moe.top_k
-        a.add = None if add is None else add.data_ptr()
-        a.x, a.width, a.rows, a.eps = self.x.data_ptr(), s.hidden, R, s.norm_eps
-        a.pre_w = None if pre is None else pre.data_ptr()
-        a.norm, a.copy_h = S.NORM[s.norm], int(copy)
-        a.h, a.h_f32, a.h_ld = self.h.data_ptr(), int(self.f32), self.h_ld
+        s = self.spec
+
+        def build():
+            a = S.StackRowArgs()
+            if embed:
+                a.tokens, a.table, a.vocab, a.embed_scale = self.tokens.data_ptr(), self.t.embed.data_ptr(), s.vocab, s.embed_scale
+            if y is not None:
+                a.y, a.y_ld, a.post_w = y.data_ptr(), s.hidden, post.data_ptr()
+                if join is not None:
+                    a.y2, a.join_w, a.join_w2 = y2.data_ptr(), join[0].data_ptr(), join[1].data_ptr()
+                if moe is not None:
+                    a.slot_of, a.probs, a.top_k = self.slot_of.data_ptr(), self.probs.data_ptr(), moe.top_k
+            a.add = None if add is None else add.data_ptr()
+            a.x, a.width, a.eps = self.x.data_ptr(), s.hidden, s.norm_eps
+            a.pre_w = None if pre is None else pre.data_ptr()
+            a.norm, a.copy_h = S.NORM[s.norm], int(copy)
+            a.h, a.h_f32, a.h_ld = self.h.data_ptr(), int(self.f32), self.h_ld
+            return a
+
+        # (norms and vectors belong to the layers, whose addresses stay)
+        key = ("rows", embed, y is not None and y.data_ptr(), post is not None and post.data_ptr(), join is not None, moe is not None,
+               add is not None and add.data_ptr(), pre is not None and pre.data_ptr(), copy)
+        a = self.kept(key, build)
+        a.rows = R
         with self.stage("rows"):
             S.rows(a)
 
@@ -234,47 +281,54 @@ class StackPrefill:
         if f.kind == "relu2":
             for n, _ in self._chunks(R, 0):
                 with self.stage("ff_up"):
-                    self.gemm(S.EPI_RELU2, d["up"], self.h, self.h_ld, n, self.ff, fp)
+                    self.product(S.EPI_RELU2, d["up"], self.h, self.h_ld, n, self.ff, fp)
                 with self.stage("ff_down"):
-                    self.gemm(S.EPI_STORE, d["down"], self.ff, fp, n, self.y, W)
+                    self.product(S.EPI_STORE, d["down"], self.ff, fp, n, self.y, W)
             return self.y
         if f.kind == "dense":
             for n, _ in self._chunks(R, 0):
                 with self.stage("dense_gate_up"):
-                    self.gemm(S.EPI_CLAMPED_GLU, d["gate"], self.h, self.h_ld, n, self.ff, fp, w2=d["up"], limit=f.limit, alpha=f.alpha)
+                    self.product(S.EPI_CLAMPED_GLU, d["gate"], self.h, self.h_ld, n, self.ff, fp, w2=d["up"], limit=f.limit, alpha=f.alpha)
                 with self.stage("dense_down"):
-                    self.gemm(S.EPI_STORE, d["down"], self.ff, fp, n, self.y, W)
+                    self.product(S.EPI_STORE, d["down"], self.ff, fp, n, self.y, W)
             return self.y
         rt = f.routing
         with self.stage("router"):
-            self.gemm(S.EPI_STORE, d["router"], self.h, self.h_ld, R, self.scores, rt.expert_count)
-        q = K.RouterArgs()
-        q.bias, q.hidden, q.experts, q.rows, q.top_k = d["correction"].data_ptr(), W, rt.expert_count, R, rt.top_k
-        q.sigmoid, q.normalize, q.route_scale = 1, int(rt.normalize_top_k), rt.route_scale
-        q.scores, q.topk_ids, q.topk_p = self.scores.data_ptr(), self.ids.data_ptr(), self.probs.data_ptr()
-        with self.stage("choice"):
-            S.route(q, rt.group_count, rt.limited_group_count)
+            self.product(S.EPI_STORE, d["router"], self.h, self.h_ld, R, self.scores, rt.expert_count)
         ir = self._item_rows(R, rt, self.f32)
         items = self._items(R, rt, ir)
-        e = K.EpArgs()
-        e.topk_ids, e.topk_p, e.tokens, e.top_k = self.ids.data_ptr(), self.probs.data_ptr(), R, rt.top_k
-        e.experts = e.experts_local = rt.expert_count
-        e.slot_of, e.n_items, e.item_expert, e.item_row = (self.slot_of.data_ptr(), self.n_items.data_ptr(), self.item_z.data_ptr(),
-                                                           self.item_row.data_ptr())
-        e.seg_rows, e.max_items, e.item_rows, e.x_args = self.seg_rows.data_ptr(), items, ir, self.t.fab.xchg_args()
+
+        def build():
+            q = K.RouterArgs()
+            q.bias, q.hidden, q.experts, q.top_k = d["correction"].data_ptr(), W, rt.expert_count, rt.top_k
+            q.sigmoid, q.normalize, q.route_scale = 1, int(rt.normalize_top_k), rt.route_scale
+            q.scores, q.topk_ids, q.topk_p = self.scores.data_ptr(), self.ids.data_ptr(), self.probs.data_ptr()
+            e = K.EpArgs()
+            e.topk_ids, e.topk_p, e.top_k = self.ids.data_ptr(), self.probs.data_ptr(), rt.top_k
+            e.experts = e.experts_local = rt.expert_count
+            e.slot_of, e.n_items, e.item_expert, e.item_row = (self.slot_of.data_ptr(), self.n_items.data_ptr(), self.item_z.data_ptr(),
+                                                               self.item_row.data_ptr())
+            e.seg_rows, e.x_args = self.seg_rows.data_ptr(), self.t.fab.xchg_args()
+            g = S.MoeGatherArgs()
+            eb = self.h.element_size()
+            g.h, g.h_ld, g.sorted, g.slot_of = self.h.data_ptr(), self.h_ld * eb, self.sorted.data_ptr(), self.slot_of.data_ptr()
+            g.top_k, g.row_bytes, g.cap = rt.top_k, self.h_ld * eb, self.cap
+            return q, e, g
+
+        q, e, g = self.kept(("experts", d["correction"].data_ptr()), build)
+        q.rows = e.tokens = g.rows = R
+        e.max_items, e.item_rows = items, ir
+        with self.stage("choice"):
+            S.route(q, rt.group_count, rt.limited_group_count)
         with self.stage("expert_count"):
             S.moe_count(e)
-        g = S.MoeGatherArgs()
-        eb = self.h.element_size()
-        g.h, g.h_ld, g.sorted, g.slot_of = self.h.data_ptr(), self.h_ld * eb, self.sorted.data_ptr(), self.slot_of.data_ptr()
-        g.rows, g.top_k, g.row_bytes, g.cap = R, rt.top_k, self.h_ld * eb, self.cap
         with self.stage("expert_gather"):
             S.moe_gather(g)
         seg = dict(items=(ir, items))
         with self.stage("expert_gate_up"):
-            self.gemm(S.EPI_SILU_GLU, d["gate"], self.sorted, self.h_ld, ir, self.ea, fp, w2=d["up"], x_rows=self.cap, **seg)
+            self.product(S.EPI_SILU_GLU, d["gate"], self.sorted, self.h_ld, ir, self.ea, fp, w2=d["up"], x_rows=self.cap, **seg)
         with self.stage("expert_down"):
-            self.gemm(S.EPI_STORE, d["down"], self.ea, fp, ir, self.ey, W, x_rows=self.cap, **seg)
+            self.product(S.EPI_STORE, d["down"], self.ea, fp, ir, self.ey, W, x_rows=self.cap, **seg)
         return self.ey
 
     def _chunk(self, pos0: int, R: int, want: Sequence[int] = (), trace: Optional[list] = None) -> Optional[torch.Tensor]:
@@ -305,12 +359,15 @@ class StackPrefill:
         if not len(want):
             return None
         self._rows(R, pre=t.g_final, **wait)
-        idx = torch.as_tensor(list(want), dtype=torch.long, device=self.dev)
-        out = torch.empty(len(idx), s.vocab, dtype=torch.float32, device=self.dev)
-        for i in range(0, len(idx), self.head_rows):
-            n = min(self.head_rows, len(idx) - i)
-            self.hw[:n].copy_(self.h.index_select(0, idx[i:i + n]))
-            self.gemm(S.EPI_STORE, t.head, self.hw, self.h_ld, n, out[i:i + n], s.vocab, scale=s.logit_scale)
+        out = torch.empty(len(want), s.vocab, dtype=torch.float32, device=self.dev)
+        straight = want[-1] - want[0] + 1 == len(want) == len(set(want))         # (ascending: rows that follow one another)
+        idx = None if straight else torch.as_tensor(list(want), dtype=torch.long, device=self.dev)
+        for i in range(0, len(want), self.head_rows):
+            n = min(self.head_rows, len(want) - i)
+            rows = self.h[want[0] + i:want[0] + i + n] if idx is None else self.h.index_select(0, idx[i:i + n])
+            if not self.f32:                             # (one tensor map for all prompts)
+                rows = self.hw[:n].copy_(rows)
+            self.gemm(S.EPI_STORE, t.head, rows if self.f32 else self.hw, self.h_ld, n, out[i:i + n], s.vocab, scale=s.logit_scale)
         return out
 
     # ------------------------------------------------------------------ public API (that of ``NativePrefill``)
@@ -334,7 +391,7 @@ class StackPrefill:
                 trace.extend(x[i:i + self.C] for x in seen)
             if got is not None:
                 out.append(got)
-        return torch.cat(out) if out else torch.empty(0, self.spec.vocab, dtype=torch.float32, device=self.dev)
+        return out[0] if len(out) == 1 else torch.cat(out) if out else torch.empty(0, self.spec.vocab, dtype=torch.float32, device=self.dev)
 
     def run(self, prompt: torch.Tensor, start: int = 0, end: Optional[int] = None) -> int:
         n = int(prompt.numel())
@@ -368,3 +425,4 @@ class StackPrefill:
 
     def close(self) -> None:
         self.maps.clear()
+        self._kept.clear()

@@ -54,45 +54,51 @@ class LatentAttention:
         n_in, qp = d["in"].n, pad(m.q_rank, 8)
         proj, cq, q, kx, vx, o = (pf.buf[n] for n in ("proj", "cq", "q", "kx", "vx", "o"))
         with pf.stage("attn_in"):
-            pf.gemm(S.EPI_STORE, d["in"], pf.h, pf.h_ld, R, proj, n_in)
-        p = S.LatentPrepArgs()
-        p.proj, p.ld, p.rows, p.q_rank, p.kv_rank = proj.data_ptr(), n_in, R, m.q_rank, m.kv_rank
-        p.q_w, p.kv_w, p.eps = d["dq_norm"].data_ptr(), d["dkv_norm"].data_ptr(), pf.spec.norm_eps
+            pf.product(S.EPI_STORE, d["in"], pf.h, pf.h_ld, R, proj, n_in)
         cache = r["cache"]
-        p.cq, p.cq_ld, p.cache, p.cache_ld = cq.data_ptr(), qp, cache.data_ptr(), cache.shape[1]
-        p.f32, p.pos0, p.capacity = int(pf.f32), pf.pos.data_ptr(), t.capacity
+        hq, hv = m.heads * dp, m.heads * vp
+
+        def build():
+            p = S.LatentPrepArgs()
+            p.proj, p.ld, p.q_rank, p.kv_rank = proj.data_ptr(), n_in, m.q_rank, m.kv_rank
+            p.q_w, p.kv_w, p.eps = d["dq_norm"].data_ptr(), d["dkv_norm"].data_ptr(), pf.spec.norm_eps
+            p.cq, p.cq_ld, p.cache, p.cache_ld = cq.data_ptr(), qp, cache.data_ptr(), cache.shape[1]
+            p.f32, p.pos0, p.capacity = int(pf.f32), pf.pos.data_ptr(), t.capacity
+            a = S.LatentAttnArgs()
+            a.q, a.k, a.v, a.out, a.f32 = q.data_ptr(), kx.data_ptr(), vx.data_ptr(), o.data_ptr(), int(pf.f32)
+            a.gate, a.gate_ld = proj.data_ptr() + 4 * (m.q_rank + m.kv_rank), n_in
+            a.heads, a.dim, a.vdim, a.scale, a.pos0, a.group = m.heads, dp, vp, m.scale, pf.pos.data_ptr(), 1
+            a.state = pf.buf["carry"].data_ptr() if "carry" in pf.buf else None
+            a.status = t.fab.status.data_ptr()
+            return p, a
+
+        p, a = pf.kept(("latent", r["run"].run, pf.at), build)
+        p.rows = a.rows = R
         with pf.stage("latent_prep"):
             S.latent_prep(p)
-        hq, hv = m.heads * dp, m.heads * vp
         with pf.stage("queries"):
-            pf.gemm(S.EPI_STORE, d["uq"], cq, qp, R, q, hq)
-        a = S.LatentAttnArgs()
-        a.q, a.k, a.v, a.out, a.f32 = q.data_ptr(), kx.data_ptr(), vx.data_ptr(), o.data_ptr(), int(pf.f32)
-        a.gate, a.gate_ld = proj.data_ptr() + 4 * (m.q_rank + m.kv_rank), n_in
-        a.rows, a.heads, a.dim, a.vdim, a.scale, a.pos0, a.group = R, m.heads, dp, vp, m.scale, pf.pos.data_ptr(), 1
-        a.state = pf.buf["carry"].data_ptr() if "carry" in pf.buf else None
-        a.status = t.fab.status.data_ptr()
+            pf.product(S.EPI_STORE, d["uq"], cq, qp, R, q, hq)
         total = pos0 + R
         for kv0 in range(0, total, pf.kv_block):
             n = min(pf.kv_block, total - kv0)
             off = kv0 * cache.shape[1]
             kw = dict(x_off=off, x_rows=t.capacity - kv0)
             with pf.stage("expand_k"):
-                pf.gemm(S.EPI_STORE, d["uk"], cache, cache.shape[1], n, kx, hq, **kw)
+                pf.product(S.EPI_STORE, d["uk"], cache, cache.shape[1], n, kx, hq, **kw)
             a.kv0, a.kv_rows, a.first, a.last = kv0, n, int(kv0 == 0), int(kv0 + n == total)
             if pf.tensor_cores and max(dp, vp) <= 256:
                 a.v_ld = pf.kv_block                 # values feature-major: the K-major operand of P V
                 with pf.stage("expand_v"):
-                    pf.gemm(S.EPI_TRANSPOSE, d["uv"], cache, cache.shape[1], n, vx, pf.kv_block, **kw)
+                    pf.product(S.EPI_TRANSPOSE, d["uv"], cache, cache.shape[1], n, vx, pf.kv_block, **kw)
                 with pf.stage("attention"):
                     S.latent_attn_tc(*LatentAttention.maps(pf, m.heads, dp, vp), a)
             else:
                 a.v_ld = hv
-                pf.gemm(S.EPI_STORE, d["uv"], cache, cache.shape[1], n, vx, hv, **kw)
+                pf.product(S.EPI_STORE, d["uv"], cache, cache.shape[1], n, vx, hv, **kw)
                 with pf.stage("attention_plain"):
                     S.latent_attn_rows(a)
         with pf.stage("attn_out"):
-            pf.gemm(S.EPI_STORE, d["o"], o, hv, R, pf.y, pf.spec.hidden)
+            pf.product(S.EPI_STORE, d["o"], o, hv, R, pf.y, pf.spec.hidden)
 
     @staticmethod
     def work(w, m, d, pos0: int, R: int) -> None:
@@ -121,23 +127,28 @@ class GatedRecurrence:
         bp, wp = pad(m.block, 8), pad(m.width, 8)
         xy, u, gates, agg, o = (pf.buf[n] for n in ("xy", "u", "gates", "agg", "o"))
         with pf.stage("rec_in"):
-            pf.gemm(S.EPI_BIAS, d["in"], pf.h, pf.h_ld, R, xy, 2 * m.width, bias=d["in_b"], act_cols=m.width)
-        a = S.RecurrenceArgs()
-        a.xy, a.xy_ld, a.conv, a.conv_b, a.taps = xy.data_ptr(), 2 * m.width, d["conv"].data_ptr(), d["conv_b"].data_ptr(), m.taps
-        a.history, a.hist_rows, a.u = r["history"].data_ptr(), m.hist_rows, u.data_ptr()
-        a.gates, a.softplus_lam, a.decay = gates.data_ptr(), d["sp"].data_ptr(), m.decay
-        a.state, a.tags, a.agg = r["state"].data_ptr(), r["tags"].data_ptr(), agg.data_ptr()
-        a.out, a.out_ld, a.f32, a.rows = o.data_ptr(), wp, int(pf.f32), R
-        a.width, a.blocks, a.block, a.block_pad = m.width, m.blocks, m.block, bp
-        a.pos0, a.status = pf.pos.data_ptr(), pf.t.fab.status.data_ptr()
+            pf.product(S.EPI_BIAS, d["in"], pf.h, pf.h_ld, R, xy, 2 * m.width, bias=d["in_b"], act_cols=m.width)
+        def build():
+            a = S.RecurrenceArgs()
+            a.xy, a.xy_ld, a.conv, a.conv_b, a.taps = xy.data_ptr(), 2 * m.width, d["conv"].data_ptr(), d["conv_b"].data_ptr(), m.taps
+            a.history, a.hist_rows, a.u = r["history"].data_ptr(), m.hist_rows, u.data_ptr()
+            a.gates, a.softplus_lam, a.decay = gates.data_ptr(), d["sp"].data_ptr(), m.decay
+            a.state, a.tags, a.agg = r["state"].data_ptr(), r["tags"].data_ptr(), agg.data_ptr()
+            a.out, a.out_ld, a.f32 = o.data_ptr(), wp, int(pf.f32)
+            a.width, a.blocks, a.block, a.block_pad = m.width, m.blocks, m.block, bp
+            a.pos0, a.status = pf.pos.data_ptr(), pf.t.fab.status.data_ptr()
+            return a
+
+        a = pf.kept(("rglru", r["run"].run, pf.at), build)
+        a.rows = R
         with pf.stage("conv"):
             S.conv(a)
         with pf.stage("rec_gates"):
-            pf.gemm(S.EPI_BIAS, d["gates"], u, m.blocks * bp, R, gates, 2 * m.width, z=m.blocks, x_z=bp, out_z=2 * m.block, bias=d["gates_b"])
+            pf.product(S.EPI_BIAS, d["gates"], u, m.blocks * bp, R, gates, 2 * m.width, z=m.blocks, x_z=bp, out_z=2 * m.block, bias=d["gates_b"])
         with pf.stage("scan"):
             S.scan(a)
         with pf.stage("rec_out"):
-            pf.gemm(S.EPI_STORE, d["o"], o, wp, R, pf.y, pf.spec.hidden)
+            pf.product(S.EPI_STORE, d["o"], o, wp, R, pf.y, pf.spec.hidden)
 
     @staticmethod
     def work(w, m, d, pos0: int, R: int) -> None:
@@ -203,7 +214,7 @@ class DeltaState:
         qk, hd, hv, ld, low_ld = m.kv_heads * m.dim, m.heads * m.dim, m.heads * m.vdim, pad(d["in"].n, 4), DeltaState.low_ld(m)
         proj, sq, sk, sv, low, decay, sgate, so, o = (pf.buf[n] for n in ("proj", "sq", "sk", "sv", "low", "decay", "sgate", "so", "o"))
         with pf.stage("delta_in"):
-            pf.gemm(S.EPI_STORE, d["in"], pf.h, pf.h_ld, R, proj, ld)
+            pf.product(S.EPI_STORE, d["in"], pf.h, pf.h_ld, R, proj, ld)
         c = S.ShortConvArgs()
         c.proj, c.ld, c.rows, c.heads, c.kv_heads, c.dim, c.vdim, c.taps = proj.data_ptr(), ld, R, m.heads, m.kv_heads, m.dim, m.vdim, m.taps
         c.conv, c.history, c.hist_rows, c.q_scale = d["conv"].data_ptr(), r["history"].data_ptr(), m.hist_rows, m.dim ** -0.5
@@ -213,9 +224,9 @@ class DeltaState:
         with pf.stage("short_conv"):
             S.short_conv(c)
         with pf.stage("delta_decay"):
-            pf.gemm(S.EPI_DECAY_SOFT, d["a2"], low, low_ld, R, decay, hd, bias=d["dt_bias"], rate=d["rate"])
+            pf.product(S.EPI_DECAY_SOFT, d["a2"], low, low_ld, R, decay, hd, bias=d["dt_bias"], rate=d["rate"])
         with pf.stage("delta_gate"):
-            pf.gemm(S.EPI_STORE, d["g2"], low, low_ld, R, sgate, hv, x_off=pad(m.decay_rank, 8))
+            pf.product(S.EPI_STORE, d["g2"], low, low_ld, R, sgate, hv, x_off=pad(m.decay_rank, 8))
         a = state_args(pf, r, m, R, so)
         a.q, a.k, a.v, a.g, a.q_ld, a.k_ld, a.v_ld, a.g_ld = sq.data_ptr(), sk.data_ptr(), sv.data_ptr(), decay.data_ptr(), qk, qk, hv, hd
         a.beta, a.beta_ld = proj.data_ptr() + 4 * d["beta_at"], ld
@@ -225,7 +236,7 @@ class DeltaState:
             S.state_chunk(S.STATE_DELTA, a)
         o_ld = head_gate(pf, m, R, so, sgate.data_ptr(), hv, S.GATE_SIGMOID, d["norm"], False, o)
         with pf.stage("delta_out"):
-            pf.gemm(S.EPI_STORE, d["o"], o, o_ld, R, pf.y, pf.spec.hidden)
+            pf.product(S.EPI_STORE, d["o"], o, o_ld, R, pf.y, pf.spec.hidden)
 
     @staticmethod
     def work(w, m, d, pos0: int, R: int) -> None:
@@ -251,6 +262,8 @@ class BonusState:
         m, part = d["spec"].mixer, d["part"]
         n, zs = m.heads * m.dim, pad(part, 4)
         mixes, proj, low, decay, so, o = (pf.buf[x] for x in ("mixes", "proj", "low", "decay", "so", "o"))
+        if "in_mixes" not in d:
+            d["in_mixes"], d["in_low"] = d["in"].rows(0, part, 4), d["in"].rows(4 * part, m.decay_rank)
         t = S.TokenMixArgs()
         t.x, t.rows, t.width, t.mixes, t.mu = pf.x.data_ptr(), R, W, 5, d["mu"].data_ptr()
         t.out, t.out_ld, t.f32 = mixes.data_ptr(), hl, int(pf.f32)
@@ -259,12 +272,12 @@ class BonusState:
         with pf.stage("token_mix"):
             S.token_mix(t)
         with pf.stage("wkv_in"):
-            pf.gemm(S.EPI_STORE, d["in"].rows(0, part, 4), mixes, 5 * hl, R, proj, 4 * zs, z=4, x_z=hl, out_z=zs)
+            pf.product(S.EPI_STORE, d["in_mixes"], mixes, 5 * hl, R, proj, 4 * zs, z=4, x_z=hl, out_z=zs)
         lp = pad(m.decay_rank, 8)
         with pf.stage("wkv_low"):
-            pf.gemm(S.EPI_TANH, d["in"].rows(4 * part, m.decay_rank), mixes, 5 * hl, R, low, lp, x_off=4 * hl)
+            pf.product(S.EPI_TANH, d["in_low"], mixes, 5 * hl, R, low, lp, x_off=4 * hl)
         with pf.stage("wkv_decay"):
-            pf.gemm(S.EPI_DECAY_EXP, d["w2"], low, lp, R, decay, n, bias=d["w0"])
+            pf.product(S.EPI_DECAY_EXP, d["w2"], low, lp, R, decay, n, bias=d["w0"])
         a = state_args(pf, r, m, R, so)
         at = proj.data_ptr()
         a.q, a.k, a.v, a.g, a.q_ld, a.k_ld, a.v_ld, a.g_ld = at, at + 4 * zs, at + 8 * zs, decay.data_ptr(), 4 * zs, 4 * zs, 4 * zs, n
@@ -273,7 +286,7 @@ class BonusState:
             S.state_chunk(S.STATE_BONUS, a)
         o_ld = head_gate(pf, m, R, so, at + 12 * zs, 4 * zs, S.GATE_SILU, d["norm"], True, o)
         with pf.stage("wkv_out"):
-            pf.gemm(S.EPI_STORE, d["o"], o, o_ld, R, pf.y, W)
+            pf.product(S.EPI_STORE, d["o"], o, o_ld, R, pf.y, W)
 
     @staticmethod
     def work(w, m, d, pos0: int, R: int) -> None:
@@ -338,7 +351,7 @@ class Parallel:
             with pf.stage("attention_plain"):
                 S.latent_attn_rows(a)
         with pf.stage("attn_out"):
-            pf.gemm(S.EPI_STORE, d["o"], o, m.heads * vp, R, pf.y, pf.spec.hidden)
+            pf.product(S.EPI_STORE, d["o"], o, m.heads * vp, R, pf.y, pf.spec.hidden)
 
     @staticmethod
     def run(pf, r: dict, R: int, pos0: int) -> None:
@@ -346,7 +359,7 @@ class Parallel:
         s, ld = d["spec"].mixer.right, pad(d["in"].n, 4)
         proj, so, den, o = (pf.buf[n] for n in ("proj", "so", "den", "o"))
         with pf.stage("parallel_in"):
-            pf.gemm(S.EPI_BIAS, d["in"], pf.h, pf.h_ld, R, proj, ld, bias=d["in_b"])
+            pf.product(S.EPI_BIAS, d["in"], pf.h, pf.h_ld, R, proj, ld, bias=d["in_b"])
         Parallel.attention(pf, r, R, pos0, proj, ld)
 
         def at(name: str) -> int:
@@ -360,7 +373,7 @@ class Parallel:
             S.state_chunk(S.STATE_NORMALIZED, a)
         o_ld = head_gate(pf, s, R, so, at("g"), ld, S.GATE_SIGMOID, d["norm"], True, o, den)
         with pf.stage("mlstm_out"):
-            pf.gemm(S.EPI_STORE, d["o2"], o, o_ld, R, pf.y2, pf.spec.hidden)
+            pf.product(S.EPI_STORE, d["o2"], o, o_ld, R, pf.y2, pf.spec.hidden)
 
     @staticmethod
     def work(w, m, d, pos0: int, R: int) -> None:

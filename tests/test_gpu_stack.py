@@ -480,6 +480,28 @@ def test_products_against_torch(rows):
         eng.close()
 
 
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+def test_wanted_rows_and_repeated_prompts(dtype):
+    """Rows that follow one another are read where they lie, others gathered: the same logits.  Argument blocks that stay from an earlier
+    prompt of another length, or from before a longer span's buffers, leave nothing behind."""
+    cfg = CASES["mixed"]
+    w = weights(cfg, 3)
+    toks = tokens(cfg, 200, 5)
+    eng = engine(cfg, w, dtype, chunk=64)
+    fresh = engine(cfg, w, dtype, chunk=64)
+    try:
+        eng.extend(toks[:7], [6])
+        eng.reset()
+        every = eng.extend(toks, range(200))
+        assert torch.equal(every, fresh.extend(toks, range(200)))
+        for want in ([5], [199], [1, 3, 4], [3, 3, 5], [0, 63, 64, 199], list(range(60, 70))):
+            eng.reset()
+            assert torch.equal(eng.extend(toks, want), every[want])
+    finally:
+        eng.close()
+        fresh.close()
+
+
 @pytest.mark.parametrize("experts,top,count,keep", [(24, 3, 4, 2), (256, 8, 8, 4), (30, 5, 10, 4), (9, 2, 1, 1), (32, 1, 32, 1)])
 def test_group_limited_choice(experts, top, count, keep):
     """Choices and weights of the routing kernel, with negative choice scores and exact ties."""
