@@ -697,11 +697,11 @@ int launch_decode_tc(const LatentDecodeArgs& a, cudaStream_t stream, bool pdl) {
 }
 
 template <int NC>
-int launch_rows(const LatentAttnArgs& a, cudaStream_t stream) {
+int launch_rows(const LatentAttnArgs& a, cudaStream_t stream, bool pdl) {
   // (the largest of the sizes on both sides of the change from two stages to one)
   if (const int rc = allow_shared(latent_attn_rows_kernel<NC>, 2 * 24 * 1024 * 4 + 8 * rows_ld(512) * 4)) return rc;
   const int per = kRowWarps * kRowsWarp;
-  return launch_pdl(latent_attn_rows_kernel<NC>, dim3((a.rows + per - 1) / per, a.heads), dim3(kRowWarps * 32), rows_smem(a.dim, a.vdim), stream, false, a);
+  return launch_pdl(latent_attn_rows_kernel<NC>, dim3((a.rows + per - 1) / per, a.heads), dim3(kRowWarps * 32), rows_smem(a.dim, a.vdim), stream, pdl, a);
 }
 
 }  // namespace
@@ -709,12 +709,13 @@ int launch_rows(const LatentAttnArgs& a, cudaStream_t stream) {
 extern "C" int nrt_latent_attn_args_size() { return (int)sizeof(LatentAttnArgs); }
 extern "C" int nrt_latent_decode_args_size() { return (int)sizeof(LatentDecodeArgs); }
 
-extern "C" int nrt_latent_attn_rows(const void* args, void* stream) {
+extern "C" int nrt_latent_attn_rows(const void* args, void* stream, int pdl) {
   LatentAttnArgs a;
   memcpy(&a, args, sizeof(a));
   if (a.rows < 1 || a.group < 1 || a.heads % a.group || a.window < 0 || a.dim > 512 || a.vdim > 512 || ((!a.first || !a.last) && !a.state)) return -3;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  return a.vdim <= 64 ? launch_rows<2>(a, s) : a.vdim <= 128 ? launch_rows<4>(a, s) : a.vdim <= 256 ? launch_rows<8>(a, s) : launch_rows<16>(a, s);
+  const bool p = pdl != 0;
+  return a.vdim <= 64 ? launch_rows<2>(a, s, p) : a.vdim <= 128 ? launch_rows<4>(a, s, p) : a.vdim <= 256 ? launch_rows<8>(a, s, p) : launch_rows<16>(a, s, p);
 }
 
 // bf16; a.dim and a.vdim multiples of 8 up to 256.  tmQ / tmK: (dim, heads, rows) boxes of 64 x 1 x 128 / 64; tmV: feature-major
@@ -729,6 +730,7 @@ extern "C" int nrt_latent_attn_tc(const void* tmQ, const void* tmK, const void* 
   if (a.rows < 1 || a.group < 1 || a.heads % a.group || a.window < 0 || a.f32 || a.dim > 256 || a.vdim > 256 || a.dim % 8 || a.vdim % 8 || !(a.scale > 0.f) || ((!a.first || !a.last) && !a.state)) return -3;
   const int smem = tc_smem(a.dim, a.vdim);
   if (const int rc = allow_shared(latent_attn_tc_kernel, 227 * 1024)) return rc;
+  // (not under the end of another launch: CTAs that then share an SM take twice as long, and other SMs stay empty)
   return launch_pdl(latent_attn_tc_kernel, dim3((a.rows + kQRows - 1) / kQRows, a.heads), dim3(kTcThreads), smem,
                     reinterpret_cast<cudaStream_t>(stream), false, q, k, v, a);
 }

@@ -546,18 +546,18 @@ extern "C" int nrt_group_prep_args_size() { return (int)sizeof(GroupPrepArgs); }
 extern "C" int nrt_transpose_args_size() { return (int)sizeof(TransposeArgs); }
 extern "C" int nrt_group_decode_args_size() { return (int)sizeof(GroupDecodeArgs); }
 
-extern "C" int nrt_group_prep(const void* args, void* stream) {
+extern "C" int nrt_group_prep(const void* args, void* stream, int pdl) {
   GroupPrepArgs p;
   memcpy(&p, args, sizeof(p));
   if (!prep_ok(p) || !p.q) return -3;
-  return launch_pdl(group_prep_kernel, dim3(p.rows), dim3(256), 0, S(stream), false, p);
+  return launch_pdl(group_prep_kernel, dim3(p.rows), dim3(256), 0, S(stream), pdl != 0, p);
 }
 
-extern "C" int nrt_transpose(const void* args, void* stream) {
+extern "C" int nrt_transpose(const void* args, void* stream, int pdl) {
   TransposeArgs a;
   memcpy(&a, args, sizeof(a));
   if (a.rows < 1 || a.cols < 1 || a.cols % 2 || a.dst_ld % 2 || a.dst_ld < a.rows) return -3;
-  return launch_pdl(transpose_kernel, dim3((a.rows + 63) / 64, (a.cols + 63) / 64), dim3(256), 0, S(stream), false, a);
+  return launch_pdl(transpose_kernel, dim3((a.rows + 63) / 64, (a.cols + 63) / 64), dim3(256), 0, S(stream), pdl != 0, a);
 }
 
 extern "C" int nrt_group_decode(const void* args, void* stream, int pdl) {

@@ -100,14 +100,26 @@ stack_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tail->tmem;
-  griddep_wait();
-  griddep_launch();
-
-  const int na = p.n_items ? min(min(*p.n_items, p.max_items), items) : items;
   const int total = n_tiles * items;
 #define NRT_TILE(w, tile, item)                                    \
   const int tile = items_fastest ? (w) / items : (w) % n_tiles;    \
   const int item = items_fastest ? (w) % items : (w) / n_tiles;
+
+  // The weights of a CTA's first tile are on their way while the launch in front ends.
+  int ahead = 0;                                           // stages whose weights have been asked for
+  if (warp == 0 && elect_one() && !p.n_items && blockIdx.x < total) {
+    NRT_TILE((int)blockIdx.x, tile, item)
+    const Item it = item_of(p, item, row_tiles, NTOK, items);
+    for (; ahead < C::kStages && ahead < kb_total; ++ahead) {
+      uint8_t* s = smem + ahead * C::kStage;
+      mbar_expect_tx(&tail->full[ahead], C::kStage);
+      tma_load_3d(s, &tmW, &tail->full[ahead], ahead * kKStep, tile * kFeat, it.z);
+      if (DUAL) tma_load_3d(s + kATile, &tmW2, &tail->full[ahead], ahead * kKStep, tile * kFeat, it.z);
+    }
+  }
+  griddep_wait();
+  griddep_launch();
+  const int na = p.n_items ? min(min(*p.n_items, p.max_items), items) : items;
 
   if (warp == 0) {
     if (elect_one()) {
@@ -121,9 +133,11 @@ stack_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           const int st = u % C::kStages;
           if (u >= C::kStages && !mbar_wait(&tail->empty[st], ((u / C::kStages) & 1) ^ 1, p.status, kSiteStageEmpty | st)) { ok = false; break; }
           uint8_t* s = smem + st * C::kStage;
-          mbar_expect_tx(&tail->full[st], C::kStage);
-          tma_load_3d(s, &tmW, &tail->full[st], kb * kKStep, tile * kFeat, it.z);
-          if (DUAL) tma_load_3d(s + kATile, &tmW2, &tail->full[st], kb * kKStep, tile * kFeat, it.z);
+          if (u >= ahead) {
+            mbar_expect_tx(&tail->full[st], C::kStage);
+            tma_load_3d(s, &tmW, &tail->full[st], kb * kKStep, tile * kFeat, it.z);
+            if (DUAL) tma_load_3d(s + kATile, &tmW2, &tail->full[st], kb * kKStep, tile * kFeat, it.z);
+          }
           tma_load_3d(s + (DUAL ? 2 : 1) * kATile, &tmX, &tail->full[st], kb * kKStep, p.n_items ? 0 : it.z, it.row0);
         }
       }
@@ -251,7 +265,7 @@ int sm_count() {
 
 template <int NTOK, int EPI>
 int launch(const CUtensorMap& w, const CUtensorMap& w2, const CUtensorMap& x, const StackGemmArgs& a, int items_fastest,
-           cudaStream_t stream) {
+           cudaStream_t stream, bool pdl) {
   constexpr bool DUAL = EPI == kSEpiClampedGlu || EPI == kSEpiSiluGlu;
   using C = Cfg<NTOK, DUAL>;
   auto* kern = stack_gemm_kernel<NTOK, EPI>;
@@ -261,7 +275,7 @@ int launch(const CUtensorMap& w, const CUtensorMap& w2, const CUtensorMap& x, co
   const int items = a.n_items ? a.max_items : a.zcount * row_tiles;
   if (items < 1 || n_tiles < 1 || (long long)items * n_tiles > 0x7fffffffLL) return -3;
   const int total = items * n_tiles, sms = sm_count();
-  return launch_pdl(kern, dim3(total < sms ? total : sms), dim3(kThreads), C::kSmem, stream, false, w, w2, x, a, n_tiles, items,
+  return launch_pdl(kern, dim3(total < sms ? total : sms), dim3(kThreads), C::kSmem, stream, pdl, w, w2, x, a, n_tiles, items,
                     row_tiles, items_fastest);
 }
 
@@ -402,22 +416,22 @@ __global__ void __launch_bounds__(T * 4) stack_gemm_f32_kernel(const StackGemmAr
 }
 
 template <int T, int EPI>
-int launch_f32_tile(const StackGemmArgs& a, cudaStream_t stream) {
+int launch_f32_tile(const StackGemmArgs& a, cudaStream_t stream, bool pdl) {
   constexpr bool DUAL = EPI == kSEpiClampedGlu || EPI == kSEpiSiluGlu;
   constexpr int smem = kFStages * (int)sizeof(F32Stage<T, DUAL>);
   if (const int rc = allow_shared(stack_gemm_f32_kernel<T, EPI>, smem)) return rc;
   const int row_tiles = (a.rows + T - 1) / T;
   const long long items = a.n_items ? (long long)a.max_items * ((a.item_rows + T - 1) / T) : (long long)a.zcount * row_tiles;
   if (items < 1 || items > 65535) return -3;
-  return launch_pdl(stack_gemm_f32_kernel<T, EPI>, dim3((a.n + T - 1) / T, (unsigned)items), dim3(T * 4), smem, stream, false, a, row_tiles);
+  return launch_pdl(stack_gemm_f32_kernel<T, EPI>, dim3((a.n + T - 1) / T, (unsigned)items), dim3(T * 4), smem, stream, pdl, a, row_tiles);
 }
 
 // Tiles of 32 until tiles of 64 fill the SMs twice: below that the longest CTA is the time of the launch.
 template <int EPI>
-int launch_f32(const StackGemmArgs& a, cudaStream_t stream) {
+int launch_f32(const StackGemmArgs& a, cudaStream_t stream, bool pdl) {
   const long long rows = a.n_items ? (long long)a.max_items * a.item_rows : (long long)a.zcount * a.rows;
   const long long big = ((a.n + 63) / 64) * ((rows + 63) / 64);
-  return big >= 2 * sm_count() || (rows + 31) / 32 > 32767 ? launch_f32_tile<64, EPI>(a, stream) : launch_f32_tile<32, EPI>(a, stream);
+  return big >= 2 * sm_count() || (rows + 31) / 32 > 32767 ? launch_f32_tile<64, EPI>(a, stream, pdl) : launch_f32_tile<32, EPI>(a, stream, pdl);
 }
 
 }  // namespace
@@ -426,7 +440,7 @@ extern "C" int nrt_stack_gemm_args_size() { return (int)sizeof(StackGemmArgs); }
 
 // ntok: token rows per tile (64 to 256; two-product epilogues up to 192); the token map's box has that many rows.
 extern "C" int nrt_stack_gemm(int epi, int ntok, const void* tmW, const void* tmW2, const void* tmX, const void* args,
-                              int items_fastest, void* stream) {
+                              int items_fastest, void* stream, int pdl) {
   CUtensorMap w, w2, x;
   memcpy(&w, tmW, sizeof(w));
   memcpy(&w2, tmW2 ? tmW2 : tmW, sizeof(w2));
@@ -438,7 +452,7 @@ extern "C" int nrt_stack_gemm(int epi, int ntok, const void* tmW, const void* tm
   if (epi == kSEpiTranspose && (a.out_f32 || a.out_ld % 8 || a.out_zstride % 8)) return -3;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
 #define NRT_CASE(N, E) \
-  if (ntok == N && epi == E) return launch<N, E>(w, w2, x, a, items_fastest, s);
+  if (ntok == N && epi == E) return launch<N, E>(w, w2, x, a, items_fastest, s, pdl != 0);
   NRT_CASE(64, kSEpiStore) NRT_CASE(128, kSEpiStore) NRT_CASE(192, kSEpiStore) NRT_CASE(256, kSEpiStore)
   NRT_CASE(64, kSEpiBias) NRT_CASE(128, kSEpiBias) NRT_CASE(192, kSEpiBias) NRT_CASE(256, kSEpiBias)
   NRT_CASE(64, kSEpiTranspose) NRT_CASE(256, kSEpiTranspose)
@@ -452,20 +466,20 @@ extern "C" int nrt_stack_gemm(int epi, int ntok, const void* tmW, const void* tm
   return -2;
 }
 
-extern "C" int nrt_stack_gemm_f32(int epi, const void* args, void* stream) {
+extern "C" int nrt_stack_gemm_f32(int epi, const void* args, void* stream, int pdl) {
   StackGemmArgs a;
   memcpy(&a, args, sizeof(a));
   if (a.n < 1 || a.k < 1 || a.rows < 1) return -3;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   switch (epi) {
-    case kSEpiStore: return launch_f32<kSEpiStore>(a, s);
-    case kSEpiBias: return launch_f32<kSEpiBias>(a, s);
-    case kSEpiClampedGlu: return launch_f32<kSEpiClampedGlu>(a, s);
-    case kSEpiSiluGlu: return launch_f32<kSEpiSiluGlu>(a, s);
-    case kSEpiRelu2: return launch_f32<kSEpiRelu2>(a, s);
-    case kSEpiTanh: return launch_f32<kSEpiTanh>(a, s);
-    case kSEpiDecaySoft: return launch_f32<kSEpiDecaySoft>(a, s);
-    case kSEpiDecayExp: return launch_f32<kSEpiDecayExp>(a, s);
+    case kSEpiStore: return launch_f32<kSEpiStore>(a, s, pdl != 0);
+    case kSEpiBias: return launch_f32<kSEpiBias>(a, s, pdl != 0);
+    case kSEpiClampedGlu: return launch_f32<kSEpiClampedGlu>(a, s, pdl != 0);
+    case kSEpiSiluGlu: return launch_f32<kSEpiSiluGlu>(a, s, pdl != 0);
+    case kSEpiRelu2: return launch_f32<kSEpiRelu2>(a, s, pdl != 0);
+    case kSEpiTanh: return launch_f32<kSEpiTanh>(a, s, pdl != 0);
+    case kSEpiDecaySoft: return launch_f32<kSEpiDecaySoft>(a, s, pdl != 0);
+    case kSEpiDecayExp: return launch_f32<kSEpiDecayExp>(a, s, pdl != 0);
   }
   return -2;
 }

@@ -410,52 +410,52 @@ extern "C" int nrt_recurrence_args_size() { return (int)sizeof(RecurrenceArgs); 
 extern "C" int nrt_moe_gather_args_size() { return (int)sizeof(MoeGatherArgs); }
 extern "C" int nrt_stack_scan_tokens() { return kScanTokens; }
 
-extern "C" int nrt_stack_rows(const void* args, void* stream) {
+extern "C" int nrt_stack_rows(const void* args, void* stream, int pdl) {
   StackRowArgs a;
   memcpy(&a, args, sizeof(a));
   if (a.rows < 1 || a.width < 1 || (a.y && !a.post_w) || (a.y2 && (!a.y || a.slot_of || !a.join_w || !a.join_w2))) return -3;
   const size_t smem = (size_t)a.width * 8;
   if (smem > 200 * 1024) return -7;
   if (const int rc = allow_shared(stack_rows_kernel, 200 * 1024)) return rc;
-  return launch_pdl(stack_rows_kernel, dim3(a.rows), dim3(256), smem, S(stream), false, a);
+  return launch_pdl(stack_rows_kernel, dim3(a.rows), dim3(256), smem, S(stream), pdl != 0, a);
 }
 
-extern "C" int nrt_latent_prep(const void* args, void* stream) {
+extern "C" int nrt_latent_prep(const void* args, void* stream, int pdl) {
   LatentPrepArgs a;
   memcpy(&a, args, sizeof(a));
   if (a.rows < 1 || a.q_rank < 1 || a.kv_rank < 1) return -3;
-  return launch_pdl(latent_prep_kernel, dim3(a.rows, 2), dim3(256), 0, S(stream), false, a);
+  return launch_pdl(latent_prep_kernel, dim3(a.rows, 2), dim3(256), 0, S(stream), pdl != 0, a);
 }
 
-extern "C" int nrt_stack_conv(const void* args, void* stream) {
+extern "C" int nrt_stack_conv(const void* args, void* stream, int pdl) {
   RecurrenceArgs a;
   memcpy(&a, args, sizeof(a));
   if (a.rows < 1 || a.taps < 1 || a.hist_rows < 2 * (a.taps - 1) || a.hist_rows < 1 || a.width != a.blocks * a.block) return -3;
-  return launch_pdl(stack_conv_kernel, dim3((a.rows + kConvRows - 1) / kConvRows, (a.width + 127) / 128), dim3(128), 0, S(stream), false, a);
+  return launch_pdl(stack_conv_kernel, dim3((a.rows + kConvRows - 1) / kConvRows, (a.width + 127) / 128), dim3(128), 0, S(stream), pdl != 0, a);
 }
 
 // The recurrence over the chunk's rows: pieces, then the scan with the state hand-over.
-extern "C" int nrt_stack_scan(const void* args, void* stream) {
+extern "C" int nrt_stack_scan(const void* args, void* stream, int pdl) {
   RecurrenceArgs a;
   memcpy(&a, args, sizeof(a));
   if (a.rows < 1 || a.width != a.blocks * a.block) return -3;
   const int pieces = (a.rows + kScanTokens - 1) / kScanTokens;
   const dim3 grid(pieces, (a.width + 127) / 128);
   int rc = 0;
-  if ((rc = launch_pdl(stack_scan_pieces_kernel, grid, dim3(128), 0, S(stream), false, a))) return rc;
-  return launch_pdl(stack_scan_kernel, grid, dim3(128), 0, S(stream), false, a);
+  if ((rc = launch_pdl(stack_scan_pieces_kernel, grid, dim3(128), 0, S(stream), pdl != 0, a))) return rc;
+  return launch_pdl(stack_scan_kernel, grid, dim3(128), 0, S(stream), pdl != 0, a);
 }
 
-extern "C" int nrt_stack_route(const void* args, int groups, int keep, void* stream) {
+extern "C" int nrt_stack_route(const void* args, int groups, int keep, void* stream, int pdl) {
   RouterArgs a;
   memcpy(&a, args, sizeof(a));
   if (a.rows < 1 || a.experts > 256 || a.top_k > 32 || groups < 1 || groups > 32 || a.experts % groups || !a.scores || a.probs) return -3;
-  return launch_pdl(stack_route_kernel, dim3((a.rows + kRouterRows - 1) / kRouterRows), dim3(256), 0, S(stream), false, a, groups, keep);
+  return launch_pdl(stack_route_kernel, dim3((a.rows + kRouterRows - 1) / kRouterRows), dim3(256), 0, S(stream), pdl != 0, a, groups, keep);
 }
 
-extern "C" int nrt_moe_gather(const void* args, void* stream) {
+extern "C" int nrt_moe_gather(const void* args, void* stream, int pdl) {
   MoeGatherArgs a;
   memcpy(&a, args, sizeof(a));
   if (a.rows < 1 || a.row_bytes % 16 || a.h_ld % 16) return -3;
-  return launch_pdl(moe_gather_kernel, dim3(a.rows, a.top_k), dim3(128), 0, S(stream), false, a);
+  return launch_pdl(moe_gather_kernel, dim3(a.rows, a.top_k), dim3(128), 0, S(stream), pdl != 0, a);
 }

@@ -904,7 +904,7 @@ __global__ void __launch_bounds__(kStepT, 1) state_step_kernel(const StateStepAr
 constexpr int kMaxSmem = 220 * 1024;
 
 template <int KIND, int L, int NV>
-int launch_chunk(const StateChunkArgs& a, cudaStream_t stream) {
+int launch_chunk(const StateChunkArgs& a, cudaStream_t stream, bool pdl) {
   if (const int rc = allow_shared(state_chunk_kernel<KIND, L, NV, false>, kMaxSmem)) return rc;
   constexpr int PER_WARP = 32 / L * kQuad;
   const int C = a.vdim + extra_columns<KIND>();
@@ -915,10 +915,10 @@ int launch_chunk(const StateChunkArgs& a, cudaStream_t stream) {
   const int per = (blocks + pieces - 1) / pieces;
   pieces = (blocks + per - 1) / per;
   if (KIND == kStateNormalized) {
-    if (const int rc = launch_pdl(gate_scan_kernel, dim3(a.heads), dim3(kScanT), 0, stream, false, a)) return rc;
+    if (const int rc = launch_pdl(gate_scan_kernel, dim3(a.heads), dim3(kScanT), 0, stream, pdl, a)) return rc;
   }
   constexpr int NC = NV * 4 * L / 32 < 2 ? 1 : 2;                        // wider slices cost occupancy
-  if (const int rc = launch_pdl(state_blocks_kernel<KIND, NC>, dim3(blocks, (a.heads + 3) / 4), dim3(128), 0, stream, false, a)) return rc;
+  if (const int rc = launch_pdl(state_blocks_kernel<KIND, NC>, dim3(blocks, (a.heads + 3) / 4), dim3(128), 0, stream, pdl, a)) return rc;
   const dim3 grid((C + cols - 1) / cols, a.heads, pieces);
   const int smem = 4 * (kStages * (state_record(KIND, a.dim) + kStateBlock * cols) + warps * (32 / L) * 2 * kStateBlock * kQuad);
   if (smem > kMaxSmem) return -7;
@@ -929,22 +929,23 @@ int launch_chunk(const StateChunkArgs& a, cudaStream_t stream) {
       if (rc) return rc;
     }
   }
+  // (not under the end of another launch: CTAs that then share an SM take twice as long, and other SMs stay empty)
   return launch_pdl(state_chunk_kernel<KIND, L, NV, false>, grid, dim3(warps * 32), smem, stream, false, a, per);
 }
 // L * NV * 4 = state_row(dim).  Fewer lanes per column mean fewer reductions but also fewer warps: the delta rule, which has no pieces
 // to spread, takes more lanes.
 template <int KIND>
-int chunk_by_dim(const StateChunkArgs& a, cudaStream_t stream) {
-  if (a.dim <= 32) return launch_chunk<KIND, 8, 1>(a, stream);
+int chunk_by_dim(const StateChunkArgs& a, cudaStream_t stream, bool pdl) {
+  if (a.dim <= 32) return launch_chunk<KIND, 8, 1>(a, stream, pdl);
   if constexpr (KIND == kStateDelta) {
-    if (a.dim <= 64) return launch_chunk<KIND, 16, 1>(a, stream);
-    if (a.dim <= 128) return launch_chunk<KIND, 16, 2>(a, stream);
+    if (a.dim <= 64) return launch_chunk<KIND, 16, 1>(a, stream, pdl);
+    if (a.dim <= 128) return launch_chunk<KIND, 16, 2>(a, stream, pdl);
   } else {
-    if (a.dim <= 64) return launch_chunk<KIND, 8, 2>(a, stream);
-    if (a.dim <= 128) return launch_chunk<KIND, 8, 4>(a, stream);
+    if (a.dim <= 64) return launch_chunk<KIND, 8, 2>(a, stream, pdl);
+    if (a.dim <= 128) return launch_chunk<KIND, 8, 4>(a, stream, pdl);
   }
-  if (a.dim <= 256) return launch_chunk<KIND, 16, 4>(a, stream);
-  return launch_chunk<KIND, 32, 4>(a, stream);
+  if (a.dim <= 256) return launch_chunk<KIND, 16, 4>(a, stream, pdl);
+  return launch_chunk<KIND, 32, 4>(a, stream, pdl);
 }
 template <int KIND, int NV>
 int launch_state_step(const StateStepArgs& a, cudaStream_t stream, bool pdl) {
@@ -984,15 +985,15 @@ extern "C" long long nrt_state_sum_floats(int kind, int heads, int dim, int vdim
 }
 extern "C" int nrt_state_step_args_size() { return (int)sizeof(StateStepArgs); }
 
-extern "C" int nrt_state_chunk(int kind, const void* args, void* stream) {
+extern "C" int nrt_state_chunk(int kind, const void* args, void* stream, int pdl) {
   StateChunkArgs a;
   memcpy(&a, args, sizeof(a));
   if (a.rows < 1 || !sizes_ok(a.heads, a.kv_heads, a.dim, a.vdim) || a.state_stride % 4 || !a.blocks || (kind != kStateDelta && !a.sums)) return -3;
   if (a.history && (a.hist_rows < 1 || a.hist_rows < 2 * (a.taps - 1))) return -3;
   if ((kind != kStateNormalized && !a.g) || (kind == kStateNormalized && (!a.gi || !a.gf || !a.den || !a.keep)) || (kind == kStateDelta && !a.beta) || (kind == kStateBonus && !a.u)) return -3;
-  if (kind == kStateDelta) return chunk_by_dim<kStateDelta>(a, S(stream));
-  if (kind == kStateBonus) return chunk_by_dim<kStateBonus>(a, S(stream));
-  if (kind == kStateNormalized) return chunk_by_dim<kStateNormalized>(a, S(stream));
+  if (kind == kStateDelta) return chunk_by_dim<kStateDelta>(a, S(stream), pdl != 0);
+  if (kind == kStateBonus) return chunk_by_dim<kStateBonus>(a, S(stream), pdl != 0);
+  if (kind == kStateNormalized) return chunk_by_dim<kStateNormalized>(a, S(stream), pdl != 0);
   return -2;
 }
 
@@ -1009,29 +1010,29 @@ extern "C" int nrt_state_step(const void* args, void* stream, int pdl) {
   return -2;
 }
 
-extern "C" int nrt_short_conv(const void* args, void* stream) {
+extern "C" int nrt_short_conv(const void* args, void* stream, int pdl) {
   ShortConvArgs a;
   memcpy(&a, args, sizeof(a));
   if (a.rows < 1 || a.taps < 1 || !sizes_ok(a.heads, a.kv_heads, a.dim, a.vdim) || a.vdim > 512 || a.hist_rows < 1 || a.hist_rows < 2 * (a.taps - 1)) return -3;
   const dim3 grid((a.rows + kConvStrip - 1) / kConvStrip, (2 * a.kv_heads + a.heads + 1 + 3) / 4);
   const int w = a.dim > a.vdim ? a.dim : a.vdim;
-  if (w <= 32) return launch_pdl(short_conv_kernel<1>, grid, dim3(128), 0, S(stream), false, a);
-  if (w <= 64) return launch_pdl(short_conv_kernel<2>, grid, dim3(128), 0, S(stream), false, a);
-  if (w <= 128) return launch_pdl(short_conv_kernel<4>, grid, dim3(128), 0, S(stream), false, a);
-  if (w <= 256) return launch_pdl(short_conv_kernel<8>, grid, dim3(128), 0, S(stream), false, a);
-  return launch_pdl(short_conv_kernel<16>, grid, dim3(128), 0, S(stream), false, a);
+  if (w <= 32) return launch_pdl(short_conv_kernel<1>, grid, dim3(128), 0, S(stream), pdl != 0, a);
+  if (w <= 64) return launch_pdl(short_conv_kernel<2>, grid, dim3(128), 0, S(stream), pdl != 0, a);
+  if (w <= 128) return launch_pdl(short_conv_kernel<4>, grid, dim3(128), 0, S(stream), pdl != 0, a);
+  if (w <= 256) return launch_pdl(short_conv_kernel<8>, grid, dim3(128), 0, S(stream), pdl != 0, a);
+  return launch_pdl(short_conv_kernel<16>, grid, dim3(128), 0, S(stream), pdl != 0, a);
 }
 
-extern "C" int nrt_token_mix(const void* args, void* stream) {
+extern "C" int nrt_token_mix(const void* args, void* stream, int pdl) {
   TokenMixArgs a;
   memcpy(&a, args, sizeof(a));
   if (a.rows < 1 || a.width < 1 || a.mixes < 1) return -3;
-  return launch_pdl(token_mix_kernel, dim3(a.rows), dim3(256), 0, S(stream), false, a);
+  return launch_pdl(token_mix_kernel, dim3(a.rows), dim3(256), 0, S(stream), pdl != 0, a);
 }
 
-extern "C" int nrt_head_gate(const void* args, void* stream) {
+extern "C" int nrt_head_gate(const void* args, void* stream, int pdl) {
   HeadGateArgs a;
   memcpy(&a, args, sizeof(a));
   if (a.rows < 1 || a.heads < 1 || a.vdim < 1 || !a.gate || !a.norm) return -3;
-  return launch_pdl(head_gate_kernel, dim3(a.rows, (a.heads + 7) / 8), dim3(256), 0, S(stream), false, a);
+  return launch_pdl(head_gate_kernel, dim3(a.rows, (a.heads + 7) / 8), dim3(256), 0, S(stream), pdl != 0, a);
 }

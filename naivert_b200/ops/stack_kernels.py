@@ -50,11 +50,11 @@ ENTRIES = {"nrt_stack_gemm": ("StackGemmArgs", "nrt_stack_gemm_args_size"), "nrt
 
 # what the entry points take, so that addresses and handles go in as plain integers (wrapping each costs as much as the call)
 _I = C.c_int
-_TYPES = {**{n: [VP, VP] for n in ("nrt_stack_rows", "nrt_latent_prep", "nrt_latent_attn_rows", "nrt_stack_conv", "nrt_stack_scan", "nrt_moe_gather",
+_TYPES = {**{n: [VP, VP, _I] for n in ("nrt_stack_rows", "nrt_latent_prep", "nrt_latent_attn_rows", "nrt_stack_conv", "nrt_stack_scan", "nrt_moe_gather",
                                    "nrt_group_prep", "nrt_transpose", "nrt_short_conv", "nrt_token_mix", "nrt_head_gate")},
           **{n: [VP, VP, _I] for n in ("nrt_latent_decode", "nrt_group_decode", "nrt_state_step", "nrt_ep_count")},
-          "nrt_stack_gemm": [_I, _I, VP, VP, VP, VP, _I, VP], "nrt_stack_gemm_f32": [_I, VP, VP], "nrt_state_chunk": [_I, VP, VP],
-          "nrt_latent_attn_tc": [VP, VP, VP, VP, VP], "nrt_stack_route": [VP, _I, _I, VP], "nrt_stack_step": [_I, _I, VP, VP, _I, _I, VP, _I]}
+          "nrt_stack_gemm": [_I, _I, VP, VP, VP, VP, _I, VP, _I], "nrt_stack_gemm_f32": [_I, VP, VP, _I], "nrt_state_chunk": [_I, VP, VP, _I],
+          "nrt_latent_attn_tc": [VP, VP, VP, VP, VP], "nrt_stack_route": [VP, _I, _I, VP, _I], "nrt_stack_step": [_I, _I, VP, VP, _I, _I, VP, _I]}
 
 _lib = None
 
@@ -97,25 +97,26 @@ def value_map(v: torch.Tensor, keys: int, features: int, box: int) -> K.TensorMa
     return K.TensorMap(v, (keys, features), (keys * 2,), (64, box), 1, library=lib())
 
 
-def gemm(epi: int, ntok: int, w: K.TensorMap, w2: Optional[K.TensorMap], x: K.TensorMap, args: StackGemmArgs, items_fastest: bool) -> None:
+def gemm(epi: int, ntok: int, w: K.TensorMap, w2: Optional[K.TensorMap], x: K.TensorMap, args: StackGemmArgs, items_fastest: bool,
+         pdl: bool = False) -> None:
     K.check(lib().nrt_stack_gemm(epi, ntok, C.byref(w.buf), C.byref(w2.buf) if w2 is not None else None, C.byref(x.buf),
-                                 C.byref(args), int(items_fastest), _stream()), "stack gemm")
+                                 C.byref(args), int(items_fastest), _stream(), int(pdl)), "stack gemm")
 
 
-def gemm_f32(epi: int, args: StackGemmArgs) -> None:
-    K.check(lib().nrt_stack_gemm_f32(epi, C.byref(args), _stream()), "stack gemm (float)")
+def gemm_f32(epi: int, args: StackGemmArgs, pdl: bool = False) -> None:
+    K.check(lib().nrt_stack_gemm_f32(epi, C.byref(args), _stream(), int(pdl)), "stack gemm (float)")
 
 
-def rows(args: StackRowArgs) -> None:
-    K.check(lib().nrt_stack_rows(C.byref(args), _stream()), "stack rows")
+def rows(args: StackRowArgs, pdl: bool = False) -> None:
+    K.check(lib().nrt_stack_rows(C.byref(args), _stream(), int(pdl)), "stack rows")
 
 
-def latent_prep(args: LatentPrepArgs) -> None:
-    K.check(lib().nrt_latent_prep(C.byref(args), _stream()), "latent prep")
+def latent_prep(args: LatentPrepArgs, pdl: bool = False) -> None:
+    K.check(lib().nrt_latent_prep(C.byref(args), _stream(), int(pdl)), "latent prep")
 
 
-def latent_attn_rows(args: LatentAttnArgs) -> None:
-    K.check(lib().nrt_latent_attn_rows(C.byref(args), _stream()), "latent attention (rows)")
+def latent_attn_rows(args: LatentAttnArgs, pdl: bool = False) -> None:
+    K.check(lib().nrt_latent_attn_rows(C.byref(args), _stream(), int(pdl)), "latent attention (rows)")
 
 
 def latent_attn_tc(q: K.TensorMap, k: K.TensorMap, v: K.TensorMap, args: LatentAttnArgs) -> None:
@@ -126,40 +127,40 @@ def latent_decode(args: LatentDecodeArgs, pdl: bool) -> None:
     K.check(lib().nrt_latent_decode(C.byref(args), _stream(), int(pdl)), "latent attention (step)")
 
 
-def conv(args: RecurrenceArgs) -> None:
-    K.check(lib().nrt_stack_conv(C.byref(args), _stream()), "short convolution")
+def conv(args: RecurrenceArgs, pdl: bool = False) -> None:
+    K.check(lib().nrt_stack_conv(C.byref(args), _stream(), int(pdl)), "short convolution")
 
 
-def scan(args: RecurrenceArgs) -> None:
-    K.check(lib().nrt_stack_scan(C.byref(args), _stream()), "recurrence scan")
+def scan(args: RecurrenceArgs, pdl: bool = False) -> None:
+    K.check(lib().nrt_stack_scan(C.byref(args), _stream(), int(pdl)), "recurrence scan")
 
 
 def scan_tokens() -> int:
     return lib().nrt_stack_scan_tokens()
 
 
-def group_prep(args: GroupPrepArgs) -> None:
-    K.check(lib().nrt_group_prep(C.byref(args), _stream()), "grouped attention prep")
+def group_prep(args: GroupPrepArgs, pdl: bool = False) -> None:
+    K.check(lib().nrt_group_prep(C.byref(args), _stream(), int(pdl)), "grouped attention prep")
 
 
-def transpose(args: TransposeArgs) -> None:
-    K.check(lib().nrt_transpose(C.byref(args), _stream()), "transpose")
+def transpose(args: TransposeArgs, pdl: bool = False) -> None:
+    K.check(lib().nrt_transpose(C.byref(args), _stream(), int(pdl)), "transpose")
 
 
 def group_decode(args: GroupDecodeArgs, pdl: bool) -> None:
     K.check(lib().nrt_group_decode(C.byref(args), _stream(), int(pdl)), "grouped attention (step)")
 
 
-def short_conv(args: ShortConvArgs) -> None:
-    K.check(lib().nrt_short_conv(C.byref(args), _stream()), "short convolution with SiLU")
+def short_conv(args: ShortConvArgs, pdl: bool = False) -> None:
+    K.check(lib().nrt_short_conv(C.byref(args), _stream(), int(pdl)), "short convolution with SiLU")
 
 
-def token_mix(args: TokenMixArgs) -> None:
-    K.check(lib().nrt_token_mix(C.byref(args), _stream()), "token mixes")
+def token_mix(args: TokenMixArgs, pdl: bool = False) -> None:
+    K.check(lib().nrt_token_mix(C.byref(args), _stream(), int(pdl)), "token mixes")
 
 
-def state_chunk(kind: int, args: StateChunkArgs) -> None:
-    K.check(lib().nrt_state_chunk(kind, C.byref(args), _stream()), "matrix-state recurrence (chunk)")
+def state_chunk(kind: int, args: StateChunkArgs, pdl: bool = False) -> None:
+    K.check(lib().nrt_state_chunk(kind, C.byref(args), _stream(), int(pdl)), "matrix-state recurrence (chunk)")
 
 
 STATE_BLOCK = 8                                       # tokens per block record of the chunk recurrence
@@ -181,20 +182,20 @@ def state_step(args: StateStepArgs, pdl: bool) -> None:
     K.check(lib().nrt_state_step(C.byref(args), _stream(), int(pdl)), "matrix-state recurrence (step)")
 
 
-def head_gate(args: HeadGateArgs) -> None:
-    K.check(lib().nrt_head_gate(C.byref(args), _stream()), "read-out norm and gate")
+def head_gate(args: HeadGateArgs, pdl: bool = False) -> None:
+    K.check(lib().nrt_head_gate(C.byref(args), _stream(), int(pdl)), "read-out norm and gate")
 
 
-def route(args: K.RouterArgs, groups: int, keep: int) -> None:
-    K.check(lib().nrt_stack_route(C.byref(args), groups, keep, _stream()), "expert choice")
+def route(args: K.RouterArgs, groups: int, keep: int, pdl: bool = False) -> None:
+    K.check(lib().nrt_stack_route(C.byref(args), groups, keep, _stream(), int(pdl)), "expert choice")
 
 
-def moe_count(args: K.EpArgs) -> None:
-    K.check(lib().nrt_ep_count(C.byref(args), _stream(), 0), "expert counts")
+def moe_count(args: K.EpArgs, pdl: bool = False) -> None:
+    K.check(lib().nrt_ep_count(C.byref(args), _stream(), int(pdl)), "expert counts")
 
 
-def moe_gather(args: MoeGatherArgs) -> None:
-    K.check(lib().nrt_moe_gather(C.byref(args), _stream()), "expert gather")
+def moe_gather(args: MoeGatherArgs, pdl: bool = False) -> None:
+    K.check(lib().nrt_moe_gather(C.byref(args), _stream(), int(pdl)), "expert gather")
 
 
 def step(pro: int, epi: int, args: StepArgs, router: Optional[K.RouterArgs], groups: int, keep: int, pdl: bool) -> None:

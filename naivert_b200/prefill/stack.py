@@ -65,6 +65,7 @@ class StackPrefill:
         self.buf = {name: self._zeros(n, t) for (name, t), n in sizes.items()}
         self.ff = self._zeros(C * max([pad(f.ff, 8) for f in ffs if f.kind != "moe"], default=0), self.act)
         self.head_rows = 256
+        self.pdl = False
         self.hw = torch.zeros(self.head_rows, self.h_ld, dtype=self.act, device=dev)
         self.tensor_cores = not self.f32              # attention of chunk rows on tcgen05 (else the plain kernel)
         self.maps: Dict[tuple, object] = {}
@@ -207,7 +208,7 @@ class StackPrefill:
         if items is not None:
             a.item_rows, a.max_items = items
         if self.f32:
-            S.gemm_f32(epi, a)
+            S.gemm_f32(epi, a, self.pdl)
             return
         dual = w2 is not None
         if items is not None:
@@ -219,7 +220,15 @@ class StackPrefill:
         if made is None:
             made = maps[ntok, live] = (self._wmap(w), self._wmap(w2) if dual else None, self._xmap(x, w.k, z, x_z, live, x_ld, ntok, x_off),
                                        items is None and w.nbytes * (2 if dual else 1) > (96 << 20))
-        S.gemm(epi, ntok, *made[:3], a, made[3])
+        S.gemm(epi, ntok, *made[:3], a, made[3], self.pdl)
+
+    def early(self, rows: int) -> bool:
+        """Whether the launches of ``rows`` rows begin under the end of the one in front.  That takes 2 us off a launch: 32 / 187 / 800 rows of
+        the bench models 1.06 / 1.03 / 1.01 times as fast, of the small models 1.03 / 1.05 / 1.15, of their 32-bit form 1.19 / 1.16 / 0.95
+        (2048 of the routed bench model: 0.97).  Long launches lose by it: CTAs that start while others of the last launch hold their SMs
+        stand closer than one to an SM, and two kernels whose grids are about an SM each never begin early for that (attention on the tensor
+        cores, matrix-state recurrence: with them 400 / 1200 rows of the matrix-state model were 0.95 / 0.89)."""
+        return self.t.pdl and (rows <= 512 if self.f32 else rows * self.spec.hidden <= 1 << 22)
 
     def product(self, *args, **more) -> None:
         """``gemm`` of the engine's own weights and buffers."""
@@ -272,7 +281,7 @@ class StackPrefill:
         a = self.kept(key, build)
         a.rows = R
         with self.stage("rows"):
-            S.rows(a)
+            S.rows(a, self.pdl)
 
     def _feed_forward(self, d: dict, R: int) -> torch.Tensor:
         """Returns the buffer that holds the result rows (sorted by expert for routed layers)."""
@@ -319,11 +328,11 @@ class StackPrefill:
         q.rows = e.tokens = g.rows = R
         e.max_items, e.item_rows = items, ir
         with self.stage("choice"):
-            S.route(q, rt.group_count, rt.limited_group_count)
+            S.route(q, rt.group_count, rt.limited_group_count, self.pdl)
         with self.stage("expert_count"):
-            S.moe_count(e)
+            S.moe_count(e, self.pdl)
         with self.stage("expert_gather"):
-            S.moe_gather(g)
+            S.moe_gather(g, self.pdl)
         seg = dict(items=(ir, items))
         with self.stage("expert_gate_up"):
             self.product(S.EPI_SILU_GLU, d["gate"], self.sorted, self.h_ld, ir, self.ea, fp, w2=d["up"], x_rows=self.cap, **seg)
@@ -335,6 +344,7 @@ class StackPrefill:
         """Rows [0, R) of ``tokens`` at positions pos0 ..: fills caches and states; logits of the rows in ``want``.
         ``trace`` collects the stream after every layer run."""
         t, s = self.t, self.spec
+        self.pdl = self.early(R)
         self._window()
         for i in range(-(-R // self.C)):
             self.pos[i:i + 1].fill_(pos0 + i * self.C)

@@ -75,7 +75,7 @@ class LatentAttention:
         p, a = pf.kept(("latent", r["run"].run, pf.at), build)
         p.rows = a.rows = R
         with pf.stage("latent_prep"):
-            S.latent_prep(p)
+            S.latent_prep(p, pf.pdl)
         with pf.stage("queries"):
             pf.product(S.EPI_STORE, d["uq"], cq, qp, R, q, hq)
         total = pos0 + R
@@ -96,7 +96,7 @@ class LatentAttention:
                 a.v_ld = hv
                 pf.product(S.EPI_STORE, d["uv"], cache, cache.shape[1], n, vx, hv, **kw)
                 with pf.stage("attention_plain"):
-                    S.latent_attn_rows(a)
+                    S.latent_attn_rows(a, pf.pdl)
         with pf.stage("attn_out"):
             pf.product(S.EPI_STORE, d["o"], o, hv, R, pf.y, pf.spec.hidden)
 
@@ -142,11 +142,11 @@ class GatedRecurrence:
         a = pf.kept(("rglru", r["run"].run, pf.at), build)
         a.rows = R
         with pf.stage("conv"):
-            S.conv(a)
+            S.conv(a, pf.pdl)
         with pf.stage("rec_gates"):
             pf.product(S.EPI_BIAS, d["gates"], u, m.blocks * bp, R, gates, 2 * m.width, z=m.blocks, x_z=bp, out_z=2 * m.block, bias=d["gates_b"])
         with pf.stage("scan"):
-            S.scan(a)
+            S.scan(a, pf.pdl)
         with pf.stage("rec_out"):
             pf.product(S.EPI_STORE, d["o"], o, wp, R, pf.y, pf.spec.hidden)
 
@@ -183,7 +183,7 @@ def head_gate(pf, m, R: int, o: torch.Tensor, gate: int, gate_ld: int, kind: int
     a.den = None if den is None else den.data_ptr()
     a.out, a.out_ld, a.f32, a.rows, a.heads, a.vdim, a.eps = out.data_ptr(), pad(hv, 8), int(pf.f32), R, m.heads, m.vdim, pf.spec.norm_eps
     with pf.stage("head_gate"):
-        S.head_gate(a)
+        S.head_gate(a, pf.pdl)
     return a.out_ld
 
 
@@ -222,7 +222,7 @@ class DeltaState:
         c.low_off, c.low_cols, c.low2_off, c.low2_cols, c.low2_at = d["a1_at"], m.decay_rank, d["g1_at"], m.gate_rank, pad(m.decay_rank, 8)
         c.f32, c.pos0 = int(pf.f32), pf.pos.data_ptr()
         with pf.stage("short_conv"):
-            S.short_conv(c)
+            S.short_conv(c, pf.pdl)
         with pf.stage("delta_decay"):
             pf.product(S.EPI_DECAY_SOFT, d["a2"], low, low_ld, R, decay, hd, bias=d["dt_bias"], rate=d["rate"])
         with pf.stage("delta_gate"):
@@ -233,7 +233,7 @@ class DeltaState:
         a.hist_src, a.hist_ld, a.hist_cols, a.taps = proj.data_ptr(), ld, m.conv_columns, m.taps
         a.hist_rows, a.history = m.hist_rows, r["history"].data_ptr()
         with pf.stage("delta_state"):
-            S.state_chunk(S.STATE_DELTA, a)
+            S.state_chunk(S.STATE_DELTA, a, pf.pdl)
         o_ld = head_gate(pf, m, R, so, sgate.data_ptr(), hv, S.GATE_SIGMOID, d["norm"], False, o)
         with pf.stage("delta_out"):
             pf.product(S.EPI_STORE, d["o"], o, o_ld, R, pf.y, pf.spec.hidden)
@@ -270,7 +270,7 @@ class BonusState:
         t.shift, t.state_stride, t.tags = r["state"].data_ptr() + 4 * m.shift_at, r["state"].shape[1], r["tags"].data_ptr()
         t.pos0, t.status = pf.pos.data_ptr(), pf.t.fab.status.data_ptr()
         with pf.stage("token_mix"):
-            S.token_mix(t)
+            S.token_mix(t, pf.pdl)
         with pf.stage("wkv_in"):
             pf.product(S.EPI_STORE, d["in_mixes"], mixes, 5 * hl, R, proj, 4 * zs, z=4, x_z=hl, out_z=zs)
         lp = pad(m.decay_rank, 8)
@@ -283,7 +283,7 @@ class BonusState:
         a.q, a.k, a.v, a.g, a.q_ld, a.k_ld, a.v_ld, a.g_ld = at, at + 4 * zs, at + 8 * zs, decay.data_ptr(), 4 * zs, 4 * zs, 4 * zs, n
         a.u = d["u"].data_ptr()
         with pf.stage("wkv_state"):
-            S.state_chunk(S.STATE_BONUS, a)
+            S.state_chunk(S.STATE_BONUS, a, pf.pdl)
         o_ld = head_gate(pf, m, R, so, at + 12 * zs, 4 * zs, S.GATE_SILU, d["norm"], True, o)
         with pf.stage("wkv_out"):
             pf.product(S.EPI_STORE, d["o"], o, o_ld, R, pf.y, W)
@@ -332,7 +332,7 @@ class Parallel:
         p = StepParallel.prep_args(t, r, proj, ld, R, pf.pos)
         p.q = q.data_ptr()
         with pf.stage("group_prep"):
-            S.group_prep(p)
+            S.group_prep(p, pf.pdl)
         start = pos0 // m.window * m.window if m.window else 0           # keys before it belong to other mask chunks
         n, es = pos0 + R - start, q.element_size()
         a = S.LatentAttnArgs()
@@ -344,12 +344,12 @@ class Parallel:
             x = S.TransposeArgs()
             x.src, x.dst, x.dst_ld, x.rows, x.cols = a.v, vx.data_ptr(), Parallel.keys(pf, m), n, m.kv_heads * vp
             with pf.stage("values_t"):
-                S.transpose(x)
+                S.transpose(x, pf.pdl)
             with pf.stage("attention"):
                 S.latent_attn_tc(*Parallel.maps(pf, r), a)
         else:
             with pf.stage("attention_plain"):
-                S.latent_attn_rows(a)
+                S.latent_attn_rows(a, pf.pdl)
         with pf.stage("attn_out"):
             pf.product(S.EPI_STORE, d["o"], o, m.heads * vp, R, pf.y, pf.spec.hidden)
 
@@ -370,7 +370,7 @@ class Parallel:
         a.gi, a.gf, a.gate_ld, a.cap, a.den = at("i"), at("f"), ld, s.cap, den.data_ptr()
         a.keep = pf.buf["keep"].data_ptr()
         with pf.stage("mlstm_state"):
-            S.state_chunk(S.STATE_NORMALIZED, a)
+            S.state_chunk(S.STATE_NORMALIZED, a, pf.pdl)
         o_ld = head_gate(pf, s, R, so, at("g"), ld, S.GATE_SIGMOID, d["norm"], True, o, den)
         with pf.stage("mlstm_out"):
             pf.product(S.EPI_STORE, d["o2"], o, o_ld, R, pf.y2, pf.spec.hidden)

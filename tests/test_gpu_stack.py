@@ -483,12 +483,13 @@ def test_products_against_torch(rows):
 @pytest.mark.parametrize("dtype", ["fp32", "bf16"])
 def test_wanted_rows_and_repeated_prompts(dtype):
     """Rows that follow one another are read where they lie, others gathered: the same logits.  Argument blocks that stay from an earlier
-    prompt of another length, or from before a longer span's buffers, leave nothing behind."""
+    prompt of another length, or from before a longer span's buffers, leave nothing behind, and neither do launches that begin early."""
     cfg = CASES["mixed"]
     w = weights(cfg, 3)
     toks = tokens(cfg, 200, 5)
     eng = engine(cfg, w, dtype, chunk=64)
     fresh = engine(cfg, w, dtype, chunk=64)
+    fresh.target.pdl = False
     try:
         eng.extend(toks[:7], [6])
         eng.reset()
