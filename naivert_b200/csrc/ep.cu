@@ -59,6 +59,17 @@ struct EpArgs {
 };
 
 // ----------------------------------------------------------------------------- counts + layout
+constexpr int kBatch = 8;                  // pairs of a lane that are loaded at once
+// sum over the lower lanes of a warp
+__device__ __forceinline__ int lanes_before(int v, int lane) {
+  int s = v;
+#pragma unroll
+  for (int o = 1; o < 32; o *= 2) {
+    const int t = __shfl_up_sync(0xffffffffu, s, o);
+    if (lane >= o) s += t;
+  }
+  return s - v;
+}
 __global__ void __launch_bounds__(1024) ep_count_kernel(const EpArgs a) {
   __shared__ unsigned int hist[kEpMaxExperts + 1];
   __shared__ uint64_t xv[kXchgMaxWords];          // [tp][experts]
@@ -68,24 +79,76 @@ __global__ void __launch_bounds__(1024) ep_count_kernel(const EpArgs a) {
   const int tp = a.x_args.tp, rank = a.x_args.rank;
   const int n = a.tokens * a.top_k;
   const int ir = a.item_rows > 0 ? a.item_rows : 16;
-  for (int i = threadIdx.x; i < a.experts; i += 1024) hist[i] = 0u;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // Up to 256 experts every warp owns one contiguous range of the pairs.  Pass 1 counts the range's pairs per expert (warp-private row of
+  // 16-bit counters, in the unused upper half of the exchange buffer: 32 x 256 x 2 bytes), a prefix over the warps turns the counts into
+  // each range's offset inside the expert's segment, pass 2 walks the range in index order and hands out rows.  Same stable order as ranking
+  // the pairs one by one (lower index first).  A pass is a chain of loads and exchanges over 32 pairs at a time, so eight loads are made at
+  // once, nothing else reads the pairs, and lanes find their like by votes: 65,536 pairs of 256 experts 80 us (295 us with a load at a
+  // time, a match over the warp and a histogram in front), 16,384 pairs 27 us (95 us).
+  const bool ranges = a.experts <= 256 && tp * a.experts <= kXchgMaxWords / 2;
+  unsigned short (*wc)[256] = reinterpret_cast<unsigned short (*)[256]>(xv + kXchgMaxWords / 2);
+  const int per = (n + 31) / 32, lo = warp * per, hi = min(n, lo + per);
+  auto walk = [&](auto&& each) {                             // each(pair, its expert or -1, lanes with the same)
+    for (int i0 = lo; i0 < hi; i0 += 32 * kBatch) {
+      int e[kBatch];
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        const int i = i0 + b * 32 + lane;
+        e[b] = i < hi ? a.topk_ids[i] : -1;
+      }
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        if (i0 + b * 32 >= hi) break;
+        // lanes with the same expert: nine votes (a match over the warp takes a turn per different value)
+        unsigned peers = __ballot_sync(0xffffffffu, e[b] >= 0);
+#pragma unroll
+        for (int bit = 0; bit < 8; ++bit) {
+          const unsigned with = __ballot_sync(0xffffffffu, (e[b] >> bit) & 1);
+          peers &= (e[b] >> bit) & 1 ? with : ~with;
+        }
+        each(i0 + b * 32 + lane, e[b], peers);
+        __syncwarp();
+      }
+    }
+  };
   for (int i = threadIdx.x; i < tp * a.experts; i += 1024) xv[i] = 0ull;
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += 1024) atomicAdd(&hist[a.topk_ids[i]], 1u);
-  __syncthreads();
-  for (int e = threadIdx.x; e < a.experts; e += 1024) xv[rank * a.experts + e] = hist[e];
+  if (ranges) {
+    for (int i = threadIdx.x; i < 32 * 256; i += 1024) (&wc[0][0])[i] = 0;
+    __syncthreads();
+    walk([&](int, int e, unsigned peers) {
+      if (e >= 0 && (peers & ((1u << lane) - 1u)) == 0u) wc[warp][e] += (unsigned short)__popc(peers);
+    });
+    __syncthreads();
+    if ((int)threadIdx.x < a.experts) {
+      unsigned run = 0;
+#pragma unroll 8
+      for (int w = 0; w < 32; ++w) { const unsigned t = wc[w][threadIdx.x]; wc[w][threadIdx.x] = (unsigned short)run; run += t; }
+      xv[rank * a.experts + threadIdx.x] = run;
+    }
+  } else {
+    for (int i = threadIdx.x; i < a.experts; i += 1024) hist[i] = 0u;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += 1024) atomicAdd(&hist[a.topk_ids[i]], 1u);
+    __syncthreads();
+    for (int e = threadIdx.x; e < a.experts; e += 1024) xv[rank * a.experts + e] = hist[e];
+  }
   __syncthreads();
   xchg_reduce_u64<kXSum>(xv, tp * a.experts, a.x_args, 32 + (a.call & 15));
-  // padded segment bases on every destination rank (all ranks compute the same table)
-  if (threadIdx.x < tp) {
-    const int d = threadIdx.x;
-    int base = 0;
-    for (int el = 0; el < a.experts_local; ++el) {
-      const int e = d * a.experts_local + el;
+  // padded segment bases on every destination rank (all ranks compute the same table): a warp per rank, a lane per run of its experts
+  if (warp < tp) {
+    const int run = (a.experts_local + 31) / 32, first = lane * run, last = min(a.experts_local, first + run);
+    auto padded = [&](int el) {
       int rows = 0;
-      for (int s = 0; s < tp; ++s) rows += (int)xv[s * a.experts + e];
-      seg_base[e] = base;
-      base += (rows + ir - 1) / ir * ir;
+      for (int s = 0; s < tp; ++s) rows += (int)xv[s * a.experts + warp * a.experts_local + el];
+      return (rows + ir - 1) / ir * ir;
+    };
+    int sum = 0;
+    for (int el = first; el < last; ++el) sum += padded(el);
+    int base = lanes_before(sum, lane);
+    for (int el = first; el < last; ++el) {
+      seg_base[warp * a.experts_local + el] = base;
+      base += padded(el);
     }
   }
   __syncthreads();
@@ -98,44 +161,13 @@ __global__ void __launch_bounds__(1024) ep_count_kernel(const EpArgs a) {
     hist[e] = (unsigned)pos;
   }
   __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (a.experts <= 256 && tp * a.experts <= kXchgMaxWords / 2) {
-    // Every warp owns one contiguous range of the pairs.  Pass 1 counts the range's pairs per expert (warp-private
-    // row of 16-bit counters), a prefix over the warps turns the counts into each range's offset inside the expert's
-    // segment, pass 2 walks the range in index order and hands out rows.  Same stable order as ranking the pairs one
-    // by one (lower index first), with three block barriers instead of two thousand.
-    // (the counters live in the unused upper half of the exchange buffer: 32 x 256 x 2 bytes)
-    unsigned short (*wc)[256] = reinterpret_cast<unsigned short (*)[256]>(xv + kXchgMaxWords / 2);
-    for (int i = threadIdx.x; i < 32 * 256; i += 1024) (&wc[0][0])[i] = 0;
-    __syncthreads();
-    const int per = (n + 31) / 32;
-    const int lo = warp * per, hi = min(n, lo + per);
-    for (int i0 = lo; i0 < hi; i0 += 32) {
-      const int i = i0 + lane;
-      const int e = i < hi ? a.topk_ids[i] : -1;
-      const unsigned peers = __match_any_sync(0xffffffffu, e);
-      if (e >= 0 && (peers & ((1u << lane) - 1u)) == 0u) wc[warp][e] += (unsigned short)__popc(peers);
-      __syncwarp();
-    }
-    __syncthreads();
-    if ((int)threadIdx.x < a.experts) {
-      unsigned run = 0;
-      for (int w = 0; w < 32; ++w) { const unsigned t = wc[w][threadIdx.x]; wc[w][threadIdx.x] = (unsigned short)run; run += t; }
-    }
-    __syncthreads();
-    for (int i0 = lo; i0 < hi; i0 += 32) {
-      const int i = i0 + lane;
-      const int e = i < hi ? a.topk_ids[i] : -1;
-      const unsigned peers = __match_any_sync(0xffffffffu, e);
+  if (ranges) {
+    walk([&](int i, int e, unsigned peers) {
       const int below = __popc(peers & ((1u << lane) - 1u));
-      if (e >= 0) {
-        unsigned base = 0;
-        if (below == 0) { base = hist[e] + wc[warp][e]; wc[warp][e] += (unsigned short)__popc(peers); }
-        base = __shfl_sync(peers, base, __ffs(peers) - 1);
-        a.slot_of[i] = (int)base + below;
-      }
+      if (e >= 0) a.slot_of[i] = (int)(hist[e] + wc[warp][e]) + below;
       __syncwarp();
-    }
+      if (e >= 0 && below == 0) wc[warp][e] += (unsigned short)__popc(peers);
+    });
     __syncthreads();
   } else
   for (int c0 = 0; c0 < n; c0 += 1024) {
@@ -170,9 +202,14 @@ __global__ void __launch_bounds__(1024) ep_count_kernel(const EpArgs a) {
     if (el < a.experts_local) first_item[el + 1] = my_items;
     if (el == 0) first_item[0] = 0;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int i = 0; i < a.experts_local; ++i) first_item[i + 1] += first_item[i];
-      *a.n_items = first_item[a.experts_local] < a.max_items ? first_item[a.experts_local] : a.max_items;
+    if (warp == 0) {
+      const int run = (a.experts_local + 31) / 32, first = lane * run, last = min(a.experts_local, first + run);
+      int sum = 0;
+      for (int i = first; i < last; ++i) sum += first_item[i + 1];
+      int before = lanes_before(sum, lane);
+      for (int i = first; i < last; ++i) first_item[i + 1] = before += first_item[i + 1];
+      __syncwarp();
+      if (lane == 0) *a.n_items = min(first_item[a.experts_local], a.max_items);
     }
     __syncthreads();
     if (el < a.experts_local) {
@@ -295,11 +332,34 @@ __global__ void __launch_bounds__(256) ep_combine_kernel(const EpCombineArgs a) 
   const uint32_t tag = (*a.epoch) * 1024u + (uint32_t)a.call + 1u;
   const int words = a.hidden / 2;
   const uint64_t deadline = globaltimer() + a.timeout_ns;
-  for (int w = threadIdx.x; w < words; w += 256) {
+  // Two words (each complete in itself) per load; those that have not arrived are waited for in turn.  2048 rows of 8 choices x 4096: 79 us,
+  // 100 us word by word, 112 us with the words of eight choices at once.
+  const int pairs = words & 1 ? 0 : words / 2;
+  for (int w = threadIdx.x; w < pairs; w += 256) {
+    const uint2 r = reinterpret_cast<const uint2*>(a.resid + (size_t)t * a.hidden)[w];
+    float s[4] = {bf16_lo(r.x), bf16_hi(r.x), bf16_lo(r.y), bf16_hi(r.y)};
+    bool ok = true;
+#pragma unroll 4
+    for (int k = 0; k < a.top_k && ok; ++k) {                 // fixed k order
+      const uint64_t* src = a.slots + ((size_t)(t * a.top_k + k)) * words + 2 * w;
+      uint64_t x, y;
+      asm volatile("ld.relaxed.sys.global.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(src) : "memory");
+      uint32_t u = (uint32_t)x, v = (uint32_t)y;
+      if ((uint32_t)(x >> 32) != tag) ok = wait_tagged(src, tag, u, deadline, a.status, kSiteMailbox | 0x80 | (uint32_t)k);
+      if ((uint32_t)(y >> 32) != tag && ok) ok = wait_tagged(src + 1, tag, v, deadline, a.status, kSiteMailbox | 0x80 | (uint32_t)k);
+      const float p = a.topk_p[t * a.top_k + k];
+      s[0] += p * bf16_lo(u);
+      s[1] += p * bf16_hi(u);
+      s[2] += p * bf16_lo(v);
+      s[3] += p * bf16_hi(v);
+    }
+    reinterpret_cast<uint2*>(a.out + (size_t)t * a.hidden)[w] = make_uint2(pack_bf16x2(s[0], s[1]), pack_bf16x2(s[2], s[3]));
+  }
+  for (int w = 2 * pairs + threadIdx.x; w < words; w += 256) {
     const float2 r = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(a.resid + (size_t)t * a.hidden)[w]);
     float lo = r.x, hi = r.y;
     bool ok = true;
-    for (int k = 0; k < a.top_k && ok; ++k) {                 // fixed k order
+    for (int k = 0; k < a.top_k && ok; ++k) {
       uint32_t v;
       ok = wait_tagged(a.slots + ((size_t)(t * a.top_k + k)) * words + w, tag, v, deadline, a.status, kSiteMailbox | 0x80 | (uint32_t)k);
       const float p = a.topk_p[t * a.top_k + k];

@@ -234,6 +234,8 @@ __global__ void __launch_bounds__(256) attn_post_kernel(const AttnPostArgs a) {
   // q heads and k heads: [optional head RMS norm] -> bf16 -> RoPE on adjacent pairs -> bf16
   const int qk_heads = a.heads + a.kv_heads;
   const int part = blockIdx.y, parts = gridDim.y;          // heads are spread over grid.y CTAs per row
+  constexpr int kPairs = 3;                                // per lane: heads up to 192 wide in one go
+  const bool pairs_lie = (reinterpret_cast<uintptr_t>(a.qkv) & 7) == 0 && ((a.ld | a.col_q | a.col_k | a.head_dim) & 1) == 0;
   for (int h = part * 8 + warp; h < qk_heads; h += 8 * parts) {
     const bool is_q = h < a.heads;
     const float* hs = is_q ? src + a.col_q + h * a.head_dim : src + a.col_k + (h - a.heads) * a.head_dim;
@@ -247,14 +249,27 @@ __global__ void __launch_bounds__(256) attn_post_kernel(const AttnPostArgs a) {
       ss = warp_sum(ss);
       rs = rsqrtf(ss / (float)a.head_dim + a.norm_eps);
     }
-    for (int i = lane; i < a.head_dim / 2; i += 32) {
-      float x0 = round_bf16(hs[2 * i]), x1 = round_bf16(hs[2 * i + 1]);
-      if (nw) {
-        x0 = round_bf16(x0 * rs * __bfloat162float(nw[2 * i]));
-        x1 = round_bf16(x1 * rs * __bfloat162float(nw[2 * i + 1]));
+    // (a head's values are asked for at once, pairs as one load where they lie so: 2048 rows of 72 heads x 192 44 us, 58 us value by value)
+    for (int i0 = lane; i0 < a.head_dim / 2; i0 += 32 * kPairs) {
+      float2 x[kPairs];
+#pragma unroll
+      for (int t = 0; t < kPairs; ++t) {
+        const int i = i0 + 32 * t;
+        x[t] = make_float2(0.f, 0.f);
+        if (i < a.head_dim / 2) x[t] = pairs_lie ? reinterpret_cast<const float2*>(hs)[i] : make_float2(hs[2 * i], hs[2 * i + 1]);
       }
-      if (2 * i < a.rope_dim) rope_pair(x0, x1, rt[i]);
-      reinterpret_cast<__nv_bfloat162*>(dst)[i] = __floats2bfloat162_rn(x0, x1);
+#pragma unroll
+      for (int t = 0; t < kPairs; ++t) {
+        const int i = i0 + 32 * t;
+        if (i >= a.head_dim / 2) continue;
+        float x0 = round_bf16(x[t].x), x1 = round_bf16(x[t].y);
+        if (nw) {
+          x0 = round_bf16(x0 * rs * __bfloat162float(nw[2 * i]));
+          x1 = round_bf16(x1 * rs * __bfloat162float(nw[2 * i + 1]));
+        }
+        if (2 * i < a.rope_dim) rope_pair(x0, x1, rt[i]);
+        reinterpret_cast<__nv_bfloat162*>(dst)[i] = __floats2bfloat162_rn(x0, x1);
+      }
     }
   }
   // v heads

@@ -503,6 +503,38 @@ def test_wanted_rows_and_repeated_prompts(dtype):
         fresh.close()
 
 
+@pytest.mark.parametrize("rows,top,experts,segment", [(1, 1, 3, 64), (5, 2, 7, 16), (32, 1, 256, 16), (301, 3, 24, 64), (333, 4, 300, 16), (1000, 8, 8, 128),
+                                                      (8192, 8, 256, 128)])
+def test_expert_lists(rows, top, experts, segment):
+    """Rows, segments and work list of the sorted choices against the host's restatement: few and many pairs, one expert for all, lists
+    beyond what the warps' counters hold."""
+    from naivert_b200.ops import kernels as K
+    from naivert_b200.ops import stack_kernels as S
+    from naivert_b200.parallel.fabric import Fabric
+    from naivert_b200.prefill.ep_moe import ep_layout_reference
+    g = torch.Generator().manual_seed(rows)
+    ids = torch.stack([torch.randperm(experts, generator=g)[:top] for _ in range(rows)]).int()
+    fab = Fabric(0, 1, 128, device=torch.device("cuda", 0))
+    try:
+        n, items = rows * top, rows * top // segment + min(rows * top, experts)
+        sizes = {"slot_of": n, "n_items": 1, "item_expert": items, "item_row": items, "seg_rows": experts}
+        out = {k: torch.full((m,), -7, dtype=torch.int32, device="cuda") for k, m in sizes.items()}
+        on_device = ids.cuda()
+        a = K.EpArgs()
+        a.topk_ids, a.tokens, a.top_k, a.experts, a.experts_local = on_device.data_ptr(), rows, top, experts, experts
+        for k, t in out.items():
+            setattr(a, k, t.data_ptr())
+        a.max_items, a.item_rows, a.x_args = items, segment, fab.xchg_args()
+        S.moe_count(a)
+        torch.cuda.synchronize()
+        want = ep_layout_reference([ids], experts, segment)
+        assert torch.equal(out["slot_of"].cpu().view(rows, top), want["slot"][0].int()) and out["seg_rows"].tolist() == want["seg_rows"][0]
+        used = int(out["n_items"])
+        assert list(zip(out["item_expert"].tolist(), out["item_row"].tolist()))[:used] == [tuple(i) for i in want["items"][0]]
+    finally:
+        fab.close()
+
+
 @pytest.mark.parametrize("experts,top,count,keep", [(24, 3, 4, 2), (256, 8, 8, 4), (30, 5, 10, 4), (9, 2, 1, 1), (32, 1, 32, 1)])
 def test_group_limited_choice(experts, top, count, keep):
     """Choices and weights of the routing kernel, with negative choice scores and exact ties."""
