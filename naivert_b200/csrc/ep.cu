@@ -56,6 +56,7 @@ struct EpArgs {
   int call;                      // tag call index of this layer's dispatch
   int item_rows;                 // rows per grouped-GEMM work item and segment padding (16 or 64; 0 = 16)
   XchgArgs x_args;
+  int* item_live;                // [max_items] rows of the item that carry a token (null: not wanted)
 };
 
 // ----------------------------------------------------------------------------- counts + layout
@@ -216,7 +217,11 @@ __global__ void __launch_bounds__(1024) ep_count_kernel(const EpArgs a) {
       const int e = rank * a.experts_local + el;
       for (int k = 0; k < my_items; ++k) {
         const int idx = first_item[el] + k;
-        if (idx < a.max_items) { a.item_expert[idx] = el; a.item_row[idx] = seg_base[e] + k * ir; }
+        if (idx < a.max_items) {
+          a.item_expert[idx] = el;
+          a.item_row[idx] = seg_base[e] + k * ir;
+          if (a.item_live) a.item_live[idx] = min(ir, my_rows - k * ir);
+        }
       }
     }
   }

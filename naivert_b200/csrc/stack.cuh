@@ -35,6 +35,7 @@ struct StackGemmArgs {
   const int* n_items;           // item form (routed experts): number of row segments, else null
   const int* item_z;            // weight group of a segment
   const int* item_row;          // its first row
+  const int* item_live;         // rows of it that count (null: all); the others' results are unspecified
   int max_items;
   int item_rows;                // rows of a segment
   void* out;

@@ -40,7 +40,7 @@ struct Tail {
   uint32_t tmem;
 };
 
-struct Item { int z, row0; bool live; };
+struct Item { int z, row0, rows; bool live; };              // rows: that count
 
 __device__ __forceinline__ Item item_of(const StackGemmArgs& p, int item, int row_tiles, int ntok, int na) {
   Item it;
@@ -48,10 +48,12 @@ __device__ __forceinline__ Item item_of(const StackGemmArgs& p, int item, int ro
     it.live = item < na;
     it.z = it.live ? p.item_z[item] : 0;
     it.row0 = it.live ? p.item_row[item] : 0;
+    it.rows = it.live && p.item_live ? p.item_live[item] : ntok;
   } else {
     it.live = true;
     it.z = item / row_tiles;
     it.row0 = (item % row_tiles) * ntok;
+    it.rows = min(ntok, p.rows - it.row0);
   }
   return it;
 }
@@ -144,13 +146,16 @@ stack_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = umma_idesc(1u, kFeat, NTOK);
       bool ok = true;
       int u = 0, t = 0;
       for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
         NRT_TILE(w, tile, item)
         (void)tile;
-        if (!item_of(p, item, row_tiles, NTOK, na).live) continue;
+        const Item it = item_of(p, item, row_tiles, NTOK, na);
+        if (!it.live) continue;
+        // A tile with few rows is as many columns as it has rows: the rest of a 256-expert layer's second and third segments (8192 rows:
+        // 640 segments of 128 for 65,536 pairs) took a fifth of its products.
+        const uint32_t idesc = umma_idesc(1u, kFeat, (min(it.rows, NTOK) + 15) / 16 * 16);
         const int buf = t % C::kBufs;
         if (t >= C::kBufs && !mbar_wait(&tail->acc_empty[buf], ((t / C::kBufs) & 1) ^ 1, p.status, kSiteAccEmpty | buf)) { ok = false; break; }
         tc_fence_after();
@@ -193,9 +198,10 @@ stack_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       const float rate = (EPI == kSEpiDecaySoft && live) ? p.rate[n] : 0.f;
       const long long zoff = p.n_items ? 0 : it.z * p.out_zstride;
       const uint32_t acc = tmem + (uint32_t(quad * 32) << 16) + buf * C::kAccCols + half * kHalf;
-      const int row_end = p.n_items ? 0x7fffffff : p.rows;
+      const int row_end = it.row0 + it.rows, cols = min(kHalf, it.rows - half * kHalf);      // this half's rows
+      if (cols <= 0) mbar_arrive(&tail->acc_empty[buf]);
 #pragma unroll 1
-      for (int c = 0; c < kHalf; c += 32) {
+      for (int c = 0; c < cols; c += 32) {
         uint32_t v0[32], v1[DUAL ? 32 : 1];
         __syncwarp();                               // the loads below are warp-collective
         tmem_ld16_nowait(acc + c, v0);
@@ -205,7 +211,7 @@ stack_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           tmem_ld16_nowait(acc + NTOK + c + 16, v1 + (DUAL ? 16 : 0));
         }
         tmem_ld_wait();
-        if (c + 32 == kHalf) {                      // last read of this accumulator: hand it back
+        if (c + 32 >= cols) {                       // last read of this accumulator: hand it back
           tc_fence_before();
           mbar_arrive(&tail->acc_empty[buf]);
         }
@@ -314,8 +320,9 @@ __global__ void __launch_bounds__(T * 4) stack_gemm_f32_kernel(const StackGemmAr
     it.live = item < min(*p.n_items, p.max_items);
     if (!it.live) return;
     it.z = p.item_z[item];
-    row_lim = p.item_row[item] + p.item_rows;
+    row_lim = p.item_row[item] + (p.item_live ? p.item_live[item] : p.item_rows);
     it.row0 = p.item_row[item] + part * T;
+    if (it.row0 >= row_lim) return;
   } else {
     it = item_of(p, blockIdx.y, row_tiles, T, 0);
     row_lim = p.rows;

@@ -503,7 +503,7 @@ class EpArgs(C.Structure):
                 ("hidden", I32), ("slot_of", VP), ("n_items", VP), ("item_expert", VP), ("item_row", VP), ("seg_rows", VP),
                 ("max_items", I32), ("cap_rows", I32), ("x", VP), ("gamma", VP), ("eps", F32),
                 ("recv8", VP * K_MAX_PEERS), ("recvs", VP * K_MAX_PEERS), ("meta", VP * K_MAX_PEERS), ("flags", VP * K_MAX_PEERS),
-                ("ticket", VP), ("call", I32), ("item_rows", I32), ("x_args", XchgArgs)]
+                ("ticket", VP), ("call", I32), ("item_rows", I32), ("x_args", XchgArgs), ("item_live", VP)]
 
 
 class EpCombineArgs(C.Structure):

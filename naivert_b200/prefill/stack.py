@@ -92,7 +92,7 @@ class StackPrefill:
             E, T = max(f.routing.expert_count for f in moe), max(f.routing.top_k for f in moe)
             items, cap = -(-P * T // 64) + E, max(self._segment_rows(P, f.routing) for f in moe)
             new.update(scores=z(P * E), ids=z(P * T, i32), probs=z(P * T), slot_of=z(P * T, i32), n_items=z(1, i32), seg_rows=z(E, i32),
-                       max_items=items, item_z=z(items, i32), item_row=z(items, i32), cap=cap, sorted=z(cap * self.h_ld, self.act),
+                       max_items=items, item_z=z(items, i32), item_row=z(items, i32), item_live=z(items, i32), cap=cap, sorted=z(cap * self.h_ld, self.act),
                        ea=z(cap * max(pad(f.ff, 8) for f in moe), self.act), ey=z(cap * s.hidden))
         self.rows_of, self.span = rows_of, P
         self._kept.clear()
@@ -195,7 +195,8 @@ class StackPrefill:
             a.rate = None if rate is None else rate.data_ptr()
             a.act_cols, a.scale, a.limit, a.alpha, a.status = act_cols, scale, limit, alpha, self.t.fab.status.data_ptr()
             if items is not None:
-                a.n_items, a.item_z, a.item_row = self.n_items.data_ptr(), self.item_z.data_ptr(), self.item_row.data_ptr()
+                a.n_items, a.item_z, a.item_row, a.item_live = (self.n_items.data_ptr(), self.item_z.data_ptr(), self.item_row.data_ptr(),
+                                                                self.item_live.data_ptr())
             if self.f32:
                 a.act, a.act_ld, a.act_zstride = x.data_ptr() + 4 * x_off, x_ld, x_z
                 a.w, a.w2 = w.w.data_ptr(), None if w2 is None else w2.w.data_ptr()
@@ -317,7 +318,7 @@ class StackPrefill:
             e.experts = e.experts_local = rt.expert_count
             e.slot_of, e.n_items, e.item_expert, e.item_row = (self.slot_of.data_ptr(), self.n_items.data_ptr(), self.item_z.data_ptr(),
                                                                self.item_row.data_ptr())
-            e.seg_rows, e.x_args = self.seg_rows.data_ptr(), self.t.fab.xchg_args()
+            e.seg_rows, e.item_live, e.x_args = self.seg_rows.data_ptr(), self.item_live.data_ptr(), self.t.fab.xchg_args()
             g = S.MoeGatherArgs()
             eb = self.h.element_size()
             g.h, g.h_ld, g.sorted, g.slot_of = self.h.data_ptr(), self.h_ld * eb, self.sorted.data_ptr(), self.slot_of.data_ptr()

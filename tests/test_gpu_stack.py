@@ -517,7 +517,7 @@ def test_expert_lists(rows, top, experts, segment):
     fab = Fabric(0, 1, 128, device=torch.device("cuda", 0))
     try:
         n, items = rows * top, rows * top // segment + min(rows * top, experts)
-        sizes = {"slot_of": n, "n_items": 1, "item_expert": items, "item_row": items, "seg_rows": experts}
+        sizes = {"slot_of": n, "n_items": 1, "item_expert": items, "item_row": items, "item_live": items, "seg_rows": experts}
         out = {k: torch.full((m,), -7, dtype=torch.int32, device="cuda") for k, m in sizes.items()}
         on_device = ids.cuda()
         a = K.EpArgs()
@@ -531,6 +531,8 @@ def test_expert_lists(rows, top, experts, segment):
         assert torch.equal(out["slot_of"].cpu().view(rows, top), want["slot"][0].int()) and out["seg_rows"].tolist() == want["seg_rows"][0]
         used = int(out["n_items"])
         assert list(zip(out["item_expert"].tolist(), out["item_row"].tolist()))[:used] == [tuple(i) for i in want["items"][0]]
+        left = [min(segment, c - r) for c in want["seg_rows"][0] for r in range(0, c, segment)]
+        assert out["item_live"].tolist()[:used] == left
     finally:
         fab.close()
 
