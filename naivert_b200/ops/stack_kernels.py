@@ -77,6 +77,21 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_products = None
+
+
+def products() -> C.CDLL:
+    """The main library, for chunk products of bf16 projections (``csrc/stack_gemm.cu`` is compiled into both)."""
+    global _products
+    if _products is None:
+        L = K.lib()
+        if L.nrt_stack_gemm_args_size() != C.sizeof(StackGemmArgs):
+            raise RuntimeError("StackGemmArgs layout drift")
+        L.nrt_stack_gemm.argtypes = _TYPES["nrt_stack_gemm"]
+        _products = L
+    return _products
+
+
 _stream = K._stream
 
 
@@ -98,8 +113,8 @@ def value_map(v: torch.Tensor, keys: int, features: int, box: int) -> K.TensorMa
 
 
 def gemm(epi: int, ntok: int, w: K.TensorMap, w2: Optional[K.TensorMap], x: K.TensorMap, args: StackGemmArgs, items_fastest: bool,
-         pdl: bool = False) -> None:
-    K.check(lib().nrt_stack_gemm(epi, ntok, C.byref(w.buf), C.byref(w2.buf) if w2 is not None else None, C.byref(x.buf),
+         pdl: bool = False, library: Optional[C.CDLL] = None) -> None:
+    K.check((library or lib()).nrt_stack_gemm(epi, ntok, C.byref(w.buf), C.byref(w2.buf) if w2 is not None else None, C.byref(x.buf),
                                  C.byref(args), int(items_fastest), _stream(), int(pdl)), "stack gemm")
 
 

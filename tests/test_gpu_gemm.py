@@ -223,6 +223,37 @@ def test_chunk_gemm_bf16_matches_torch(order):
     assert (out - ref).abs().max().item() <= 2e-3 * ref.abs().max().item()
 
 
+@pytest.mark.parametrize("n,k", [(640, 1024), (9600, 192), (18944, 64)])
+@pytest.mark.parametrize("rows", [1, 63, 64, 65, 187, 320])
+def test_chunk_projection(rows, n, k):
+    """bf16 projections of a chunk (rows of a wider buffer, fp32 and bf16 stores) at the edges of 64- and 256-row tiles; rows past the
+    chunk's are left alone.  Products are exact in fp32: a sum of k of them is off by at most k half steps of 2^-24, doubled for the
+    tensor unit's truncation."""
+    from types import SimpleNamespace
+    from naivert_b200.prefill.native import NativePrefill
+    K = _setup()
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    w = (torch.randn(n, k, device="cuda", generator=g) * 0.05).bfloat16()
+    x = torch.randn(384, k + 64, device="cuda", generator=g).bfloat16()[:, 64:]
+    st, wm = _status(), K.weight_tmap(w)
+    owner = SimpleNamespace(wide=True, _bf16={})
+    ref, size = x[:rows].double() @ w.double().T, x[:rows].double().abs() @ w.double().abs().T
+    for dtype in (torch.float32, torch.bfloat16):
+        out = torch.full((384, n), 7.0, device="cuda", dtype=dtype)
+        a = K.GemmArgs()
+        a.n_total, a.k_total, a.out_scale, a.ld_out, a.status = n, k, 1.0, n, st.data_ptr()
+        setattr(a, "out_f32" if dtype == torch.float32 else "out_bf16", out.data_ptr())
+        owner._bf16 = {}
+        torch.cuda.synchronize()
+        with torch.cuda.stream(torch.cuda.Stream()):
+            NativePrefill._bf16_gemm(owner, 0, wm, x, a, n // 128, rows, 0, False)
+        torch.cuda.synchronize()
+        assert int(st[0]) == 0
+        bound = 2 * k * 2.0 ** -24 * size + (0 if dtype == torch.float32 else 2.0 ** -8 * ref.abs())
+        assert bool(((out[:rows].double() - ref).abs() <= bound).all())
+        assert bool((out[rows:] == 7).all())
+
+
 def test_chunk_gemm_fp8_gate_up_matches_torch():
     """e4m3 block-scaled gate/up with SiLU and e4m3 re-quantisation on the chunk engine vs the torch recipe."""
     K = _setup()
