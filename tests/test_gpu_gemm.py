@@ -322,3 +322,9 @@ def test_chunk_gemm_fp8_pairs_of_k_blocks(k, n, rows):
         else:
             slack = k * 2.0 ** -24 * dequant_act(xq, xs).abs().max() * k ** 0.5
             assert ((out.float() - gate).abs() <= 2.0 ** -8 * gate.abs() + slack).all()
+
+
+@pytest.mark.parametrize("k", [15360, 15488, 16384])
+def test_chunk_gemm_fp8_longest_rows(k):
+    """The table of scales takes the room of a stage from two products of more than 15,360 channels."""
+    test_chunk_gemm_fp8_pairs_of_k_blocks(k, 128, 64)
