@@ -154,7 +154,8 @@ stack_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         const Item it = item_of(p, item, row_tiles, NTOK, na);
         if (!it.live) continue;
         // A tile with few rows is as many columns as it has rows: the rest of a 256-expert layer's second and third segments (8192 rows:
-        // 640 segments of 128 for 65,536 pairs) took a fifth of its products.
+        // 640 segments of 128 for 65,536 pairs) took a fifth of its products (three layers of 4096 x 2048: gate and up 7.66 -> 7.16 ms,
+        // down 4.56 -> 4.34).
         const uint32_t idesc = umma_idesc(1u, kFeat, (min(it.rows, NTOK) + 15) / 16 * 16);
         const int buf = t % C::kBufs;
         if (t >= C::kBufs && !mbar_wait(&tail->acc_empty[buf], ((t / C::kBufs) & 1) ^ 1, p.status, kSiteAccEmpty | buf)) { ok = false; break; }

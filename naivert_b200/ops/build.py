@@ -1,7 +1,8 @@
 """Native build: the CUDA translation units are compiled for sm_100a with nvcc into in-tree shared
 libraries and loaded through ctypes.  ``main`` holds the speculative-decoding target, the sampler and the
 fabric; ``stack`` holds the layer-stack kernels (``csrc/stack*``, ``csrc/latent_attn.cu``), so a process that
-only runs such a model on a fresh checkout compiles only those.
+only runs such a model on a fresh checkout compiles only those.  The expert lists and the chunk products, which prompts
+of both kinds of model use, are in both.
 
 A manifest (source digest + flags) is written beside the library; ``load_library`` rebuilds
 when the digest changes and nvcc is present, and otherwise loads the library that travelled

@@ -7,6 +7,9 @@ kernels and caches as the decode/verify step, launched over row groups:
     indexer keys -> [tcgen05 indexer sweep per row group -> exact top-k per row] -> row attention ->
     o_proj partials -> tensor-parallel reduction -> MoE -> draft feature ingest at the tap layers
 
+On one GPU consecutive chunks of a prompt form a span (up to ``SPAN_ROWS`` rows): a layer's attention and routing take them in turn,
+its experts together.
+
 Parallel layout (``tp`` ranks, one process per GPU):
 
 * attention is tensor parallel (heads split, KV caches of this rank's heads), the partial o_proj
@@ -43,6 +46,7 @@ from .ep_moe import EPMoE, EPWeights
 from .stack import StackPrefill
 
 ROWS = K.K_TOK
+SPAN_ROWS = 8192          # rows whose experts run together: 256 experts of top 8 see 256 rows each
 
 
 @dataclass
@@ -91,13 +95,9 @@ class NativePrefill:
         # multiple of 64 rows; otherwise the step engine's 16-column tiles in item mode
         self.wide = os.environ.get("NAIVERT_PREFILL_WIDE", "1") == "1" and chunk % K.WIDE_TOK == 0
         self.step = K.WIDE_TOK if self.wide else ROWS
-        self._gemm = self._wide_gemm if self.wide else K.gemm
         s, dev = spec, self.dev
         H = s.hidden
         bf, f32, i32, u8 = torch.bfloat16, torch.float32, torch.int32, torch.uint8
-        self.pos = torch.zeros(4, dtype=i32, device=dev)                 # [0] = position of the chunk's row 0
-        self.tokens = torch.zeros(C, dtype=i32, device=dev)
-        self.x = torch.zeros(C, H, dtype=bf, device=dev)
         self.xn = torch.zeros(C, H, dtype=bf, device=dev)
         self.x8 = torch.zeros(C, H, dtype=u8, device=dev)
         self.xs = torch.ones(C, H // 128, dtype=f32, device=dev)
@@ -109,12 +109,10 @@ class NativePrefill:
         self.o8 = torch.zeros(C, t.o8.shape[1], dtype=u8, device=dev)
         self.os = torch.ones(C, t.os.shape[1], dtype=f32, device=dev)
         self.map_o8 = K.act_tmap(self.o8, self.step)
-        self.rope = {k: torch.zeros(C, v.shape[1], 2, dtype=f32, device=dev) for k, v in t.rope.items()}
-        self.idx_rope = torch.zeros(C, t.idx_rope.shape[1], 2, dtype=f32, device=dev)
         self.items = C // self.step
         self.row_offsets = (torch.arange(self.items, dtype=i32, device=dev) * self.step).contiguous()
         self.zero_ids = torch.zeros(self.items, dtype=i32, device=dev)
-        self.n_items = torch.zeros(1, dtype=i32, device=dev)
+        self.n_items = torch.arange(self.items + 1, dtype=i32, device=dev)         # work items of a launch, by address
         ix = s.indexer
         if FULL_DSA in s.layer_kinds:
             self.iq8 = torch.zeros(C * ix.head_count, ix.head_dim, dtype=u8, device=dev)
@@ -136,8 +134,6 @@ class NativePrefill:
         self.T = C // self.tp if self.ep else C                            # rows a rank routes
         self.scores = torch.zeros(self.T, rt.expert_count, dtype=f32, device=dev)
         self.tickets = torch.zeros(-(-self.T // ROWS), dtype=i32, device=dev)
-        self.topk_ids = torch.zeros(self.T, rt.top_k, dtype=i32, device=dev)
-        self.topk_p = torch.zeros(self.T, rt.top_k, dtype=f32, device=dev)
         self.xl = torch.zeros(self.T, H, dtype=bf, device=dev)             # this rank's rows between scatter and gather
         self.rs = torch.zeros(self.T, H, dtype=bf, device=dev)
         self.zeros = torch.zeros(self.T, H, dtype=bf, device=dev) if (self.tp > 1 and not self.ep) else None
@@ -145,9 +141,11 @@ class NativePrefill:
         self.moe_fab = t.fab if (self.ep or self.tp == 1) else LocalFabric(dev)
         self.moe: Optional[EPMoE] = None
         self.moe_w: List[Optional[EPWeights]] = []
+        # Rows of several chunks go through a layer's experts together on one GPU: its weights are read once for all of them, and fewer
+        # segments of 64 are padding.  16,001 tokens at 2048 rows a chunk, spans of one / four chunks: gate and up 42.3 -> 31.3 ms, down 24.4 -> 19.5 ms.
+        self.span_limit = max(C, SPAN_ROWS // C * C) if has_moe and self.tp == 1 else C
+        self._size_span(C)
         if has_moe:
-            inter = rt.intermediate if self.ep else s.expert_inter_local(self.tp)
-            self.moe = EPMoE(self.moe_fab, H, inter, rt.expert_count, rt.top_k, self.T, eps=s.norm_eps, item_rows=self.step)
             for L, d in enumerate(t.layers):
                 if "gate" not in d:
                     self.moe_w.append(None)
@@ -158,14 +156,10 @@ class NativePrefill:
                     self.moe_w.append(EPWeights(*({"w": d[n].w, "s": d[n].s} for n in ("gate", "up", "down"))))
         # ---- draft feature ingest
         if draft is not None:
-            taps = len(s.draft.target_layer_ids)
             Hd = s.draft.hidden
-            self.feats = torch.zeros(C, max(1, taps) * H, dtype=bf, device=dev)
-            self.taps = self.feats[:, self.rank * draft.kf:(self.rank + 1) * draft.kf]
             self.dh = torch.zeros(C, Hd, dtype=bf, device=dev)
             self.dxn = torch.zeros(C, Hd, dtype=bf, device=dev)
             self.draw = torch.zeros(C, draft.wkv.shape[0], dtype=f32, device=dev)
-            self.drope = torch.zeros(C, s.draft.head_dim // 2, 2, dtype=f32, device=dev)
         self.phases: dict = {}
         # grouped-head attention kernel; NAIVERT_PREFILL_GROUP_ATTN=0 keeps the per-head row kernel of the step
         # path (bitwise-comparable with replay)
@@ -174,11 +168,51 @@ class NativePrefill:
         self._timed: Dict[str, list] = {}
         self._build_args()
 
-    @staticmethod
-    def _wide_gemm(variant, a0, a1, b, args, n_tiles, items, pdl=False):
+    def _size_span(self, P: int) -> None:
+        """Buffers of a span of ``P`` rows (whole chunks); an allocation that fails leaves the present ones."""
+        s, t, C, dev, rt = self.spec, self.t, self.C, self.dev, self.spec.routing
+        bf, f32, i32, H, T = torch.bfloat16, torch.float32, torch.int32, self.spec.hidden, P // self.tp if self.ep else P
+        new = {
+            "pos": torch.zeros(P // C, 4, dtype=i32, device=dev),           # [c][0] = position of chunk c's row 0
+            "_steps": torch.arange(P // C, dtype=i32, device=dev)[:, None].expand(-1, 4) * C,
+            "tokens": torch.zeros(P, dtype=i32, device=dev), "x": torch.zeros(P, H, dtype=bf, device=dev),
+            "rope": {k: torch.zeros(P, v.shape[1], 2, dtype=f32, device=dev) for k, v in t.rope.items()},
+            "idx_rope": torch.zeros(P, t.idx_rope.shape[1], 2, dtype=f32, device=dev),
+            "topk_ids": torch.zeros(T, rt.top_k, dtype=i32, device=dev), "topk_p": torch.zeros(T, rt.top_k, dtype=f32, device=dev)}
+        if any("gate" in d for d in t.layers):
+            inter = rt.intermediate if self.ep else s.expert_inter_local(self.tp)
+            new["moe"] = EPMoE(self.moe_fab, H, inter, rt.expert_count, rt.top_k, T, eps=s.norm_eps, item_rows=self.step)
+        if self.draft is not None:
+            kf = self.draft.kf
+            new["feats"] = torch.zeros(P, max(1, len(s.draft.target_layer_ids)) * H, dtype=bf, device=dev)
+            new["taps"] = new["feats"][:, self.rank * kf:(self.rank + 1) * kf]
+            new["drope"] = torch.zeros(P, s.draft.head_dim // 2, 2, dtype=f32, device=dev)
+        for name, v in new.items():
+            setattr(self, name, v)
+        self.span = P
+        self._bf16.clear()
+
+    def _fit_span(self, n: int) -> None:
+        """Spans for ``n`` rows as far as the limit and the memory go: what a span needs beyond a chunk is taken when a prompt first asks
+        for it, and without the memory chunks go on one by one."""
+        P = min(self.span_limit, -(-n // self.C) * self.C)
+        if P > self.span:
+            torch.cuda.synchronize(self.dev)              # earlier calls may still use the buffers that go, on any stream
+        while P > self.span:
+            try:
+                self._size_span(P)
+            except torch.OutOfMemoryError:
+                P -= self.C
+                self.span_limit = P
+
+    def _gemm(self, variant, a0, a1, b, args, n_tiles, items, pdl=False):
         """Plain projections share one weight matrix over all items.  A matrix that fits the L2 (126 MB) stays
         resident while feature tiles vary fastest (tokens stream once); a larger one is walked item-fastest so
         that each weight tile is fetched from HBM once and the (smaller) token operand stays resident instead."""
+        args.n_active = self.n_items[items].data_ptr()
+        if not self.wide:
+            K.gemm(variant, a0, a1, b, args, n_tiles, items, pdl=pdl)
+            return
         wbytes = a0.tensor.numel() * a0.tensor.element_size() * (2 if a1 is not None else 1)
         K.wide_gemm(variant, a0, a1, b, args, n_tiles, items, pdl=pdl, items_fastest=wbytes > (96 << 20))
 
@@ -195,7 +229,7 @@ class NativePrefill:
         if not self.wide:
             if ROWS not in maps:
                 maps[ROWS] = K.act_tmap(x, ROWS)
-            K.gemm(variant, weight, None, maps[ROWS], args, n_tiles, items, pdl=pdl)
+            self._gemm(variant, weight, None, maps[ROWS], args, n_tiles, items, pdl=pdl)
             return
         a.rows = R
         ntok = StackPrefill.tile_rows(S.EPI_STORE, n_tiles, R)
@@ -208,7 +242,7 @@ class NativePrefill:
     def _item_args(self, n, k) -> K.GemmArgs:
         g = K.GemmArgs()
         g.n_total, g.k_total, g.rows, g.a_group, g.out_scale = n, k, self.step, 0, 1.0
-        g.n_active, g.active_ids, g.max_slots = self.n_items.data_ptr(), self.zero_ids.data_ptr(), self.items
+        g.active_ids, g.max_slots = self.zero_ids.data_ptr(), self.items
         g.row_offsets = self.row_offsets.data_ptr()
         g.status = self.t.fab.status.data_ptr()
         return g
@@ -216,7 +250,6 @@ class NativePrefill:
     def _build_args(self):
         s, t = self.spec, self.t
         H, ix = s.hidden, s.indexer
-        pos0 = self.pos.data_ptr()
         self.L: List[dict] = []
         for L, d in enumerate(t.layers):
             a, nh, nkv, cols = d["a"], d["nh"], d["nkv"], d["cols"]
@@ -225,21 +258,21 @@ class NativePrefill:
             g.out_f32, g.ld_out = self.qkv.data_ptr(), self.qkv.shape[1]
             e["qkv"] = g
             p = K.AttnPostArgs.from_buffer_copy(d["args_post"])
-            p.qkv, p.ld, p.pos0, p.rope, p.q_out = self.qkv.data_ptr(), self.qkv.shape[1], pos0, self.rope[d["kind"]].data_ptr(), self.q.data_ptr()
+            p.qkv, p.ld, p.q_out = self.qkv.data_ptr(), self.qkv.shape[1], self.q.data_ptr()
             if d["kind"] == FULL_DSA:
-                p.idx_rope_tab, p.iq8, p.ihw = self.idx_rope.data_ptr(), self.iq8.data_ptr(), self.ihw.data_ptr()
+                p.iq8, p.ihw = self.iq8.data_ptr(), self.ihw.data_ptr()
                 # the step runtime keeps the query quantisation scale in a 16-row side buffer; a chunk has more rows,
                 # so here the scale is folded into the head weights (the kernel's form without that buffer)
                 p.iq_scale = None
                 e["sweep_maps"] = K.sweep_maps(d["ik"], self.iq8)
                 sw = K.SweepArgs()
-                sw.ihw, sw.iks, sw.pos0 = self.ihw.data_ptr(), d["iks"].data_ptr(), pos0
+                sw.ihw, sw.iks = self.ihw.data_ptr(), d["iks"].data_ptr()
                 sw.heads, sw.top_k = ix.head_count, ix.top_k
                 sw.logits, sw.ld, sw.status = self.idx_logits.data_ptr(), self.idx_logits.shape[1], t.fab.status.data_ptr()
                 e["sweep"] = sw
             e["post"] = p
             q = K.AttnArgs.from_buffer_copy(d["args_attn"])
-            q.q, q.pos0, q.o8, q.o_scale, q.part, q.tickets = self.q.data_ptr(), pos0, self.o8.data_ptr(), self.os.data_ptr(), None, None
+            q.q, q.o8, q.o_scale, q.part, q.tickets = self.q.data_ptr(), self.o8.data_ptr(), self.os.data_ptr(), None, None
             if d["kind"] == FULL_DSA:
                 q.sel = self.sel.data_ptr()
             e["attn"] = q
@@ -268,7 +301,7 @@ class NativePrefill:
                 r.hidden, r.experts, r.top_k = H, rt.expert_count, rt.top_k
                 r.sigmoid, r.normalize, r.route_scale = int(rt.score_func == "sigmoid"), int(rt.normalize_top_k), rt.route_scale
                 r.scores, r.ticket = self.scores.data_ptr(), self.tickets.data_ptr()
-                r.topk_ids, r.topk_p, r.max_slots = self.topk_ids.data_ptr(), self.topk_p.data_ptr(), 0
+                r.max_slots = 0
                 e["router"] = r
             self.L.append(e)
         if self.draft is not None:
@@ -282,7 +315,7 @@ class NativePrefill:
             self.args_ingest = []
             for Ld in dr.layers:
                 p = K.AttnPostArgs.from_buffer_copy(Ld["args_ingest_post"])
-                p.qkv, p.ld, p.pos0, p.rope = self.draw.data_ptr(), self.draw.shape[1], pos0, self.drope.data_ptr()
+                p.qkv, p.ld = self.draw.data_ptr(), self.draw.shape[1]
                 self.args_ingest.append(p)
 
     @contextmanager
@@ -308,121 +341,140 @@ class NativePrefill:
         if self.tp > 1:
             dist.all_reduce(buf, group=self.group)
 
-    # ------------------------------------------------------------------ one chunk
+    # ------------------------------------------------------------------ chunks
     def _chunk(self, pos0: int, R: int) -> None:
+        self._span(pos0, [R])
+
+    def _span(self, start: int, sizes: List[int]) -> None:
+        """Consecutive chunks of ``sizes`` rows (all but the last of ``chunk``) from position ``start`` on, layer by layer: attention and
+        routing chunk by chunk, the experts for all of them."""
         s, t, tp = self.spec, self.t, self.tp
-        H, pdl = s.hidden, False
-        items = -(-R // self.step)
-        self.pos.fill_(pos0)
-        if getattr(self, "shard_index", False) and R % (ROWS * tp) == 0:
-            self.pos[1:2].fill_(pos0 + self.rank * (R // tp))
-        self.n_items.fill_(items)
-        x, xn, part = self.x, self.xn, self.part
-        K.embed_rows(self.tokens, t.embed, x, R, pdl=pdl)
+        pdl, n = False, sum(sizes)
+        rows = [(c, c * self.C, R) for c, R in enumerate(sizes)]          # chunk, its first row, its rows
+        torch.add(self._steps[:len(sizes)], start, out=self.pos[:len(sizes)])
+        if getattr(self, "shard_index", False) and n % (ROWS * tp) == 0:   # ranks: spans of one chunk
+            self.pos[0, 1:2].fill_(start + self.rank * (n // tp))
+        x = self.x
+        K.embed_rows(self.tokens, t.embed, x, n, pdl=pdl)
         for kind, tab in self.rope.items():
             a = s.attention[kind]
-            K.rope_table(self.pos, R, a.rope_dim, a.rope_theta, tab, pdl=pdl)
+            K.rope_table(self.pos, n, a.rope_dim, a.rope_theta, tab, pdl=pdl)
         if FULL_DSA in self.rope:
-            K.rope_table(self.pos, R, s.indexer.rope_dim, s.attention[FULL_DSA].rope_theta, self.idx_rope, pdl=pdl)
-        T = R // tp if self.ep else R
-        xl = x[self.rank * T:(self.rank + 1) * T] if self.ep else x[:R]
+            K.rope_table(self.pos, n, s.indexer.rope_dim, s.attention[FULL_DSA].rope_theta, self.idx_rope, pdl=pdl)
+        T = n // tp if self.ep else n
+        src = self.xl if self.ep else x
+        xl = x[self.rank * T:(self.rank + 1) * T] if self.ep else x[:n]
         for L, (d, e) in enumerate(zip(t.layers, self.L)):
-            # ---- attention (tensor parallel)
-            with self._stage("norm"):
-                K.prep_norm(x, d["g_in"], R, s.norm_eps, xn=xn, pdl=pdl)
-            with self._stage("qkv_gemm"):
-                self._bf16_gemm(self.V_BF16_F32, d["map_qkv"], self.xn, e["qkv"], d["wqkv"].shape[0] // 128, R, items, pdl)
-            e["post"].rows = R
-            with self._stage("attn_post"):
-                K.attn_post(e["post"], pdl=pdl)
-            if d["kind"] == FULL_DSA and pos0 + R > s.indexer.top_k:
-                sw = e["sweep"]
-                sw.rows = R
-                shard = self.shard_index and R % (ROWS * tp) == 0
-                Rl = R // tp if shard else R                         # rows this rank selects for
-                row0 = self.rank * Rl if shard else 0
-                sw.group0, sw.ngroups = row0 // ROWS, Rl // ROWS
-                tiles = -(-(pos0 + R) // 128)
-                with self._stage("index_sweep"):
-                    K.index_sweep(*e["sweep_maps"], sw, max(1, min(tiles, 592 // (Rl // ROWS))), pdl=pdl)
-                with self._stage("topk"):
-                    logits, pos_l = self.idx_logits[row0:row0 + Rl], self.pos[1:]          # pos[1] = pos0 + row0
-                    sel = self.sel_local if shard else self.sel
-                    if t.topk_grid:
-                        K.topk_rows_grid(logits, pos_l, Rl, s.indexer.top_k, sel, self.topk_state, 16, pdl=pdl)
-                    else:
-                        K.topk_rows(logits, pos_l, Rl, s.indexer.top_k, sel, pdl=pdl)
-                    if shard:
-                        dist.all_gather_into_tensor(self.sel[:R], self.sel_local[:Rl], group=self.group)
-            e["attn"].rows = R
-            with self._stage("attn_dsa" if d["kind"] == FULL_DSA else "attn_swa"):
-                if e["group_attn"]:
-                    K.attn_group(e["attn"], pdl=pdl)
-                else:
-                    K.attn_rows(e["attn"], 1, pdl=pdl)
-            with self._stage("o_gemm"):
-                self._gemm(self.V_FP8_BF16, d["wo"].map, None, self.map_o8, e["o"], H // 128, items, pdl=pdl)
-            moe = "dense" not in d
-            with self._stage("tp_reduce"):
-                if self.ep and moe:
-                    # sequence parallel from here to the end of the layer: this rank keeps rows [rank*T, (rank+1)*T)
-                    dist.reduce_scatter_tensor(self.rs[:T], part[:R], group=self.group)
-                    torch.add(xl, self.rs[:T], out=self.xl[:T])
-                else:
-                    self._all_reduce(part[:R])
-                    torch.add(x[:R], part[:R], out=x[:R])
-            # ---- MLP
-            if not moe:
-                dn = d["dense"]
-                with self._stage("dense_mlp"):
-                    K.prep_norm(x, d["g_post"], R, s.norm_eps, x8=self.x8, xs=self.xs, pdl=pdl)
-                    self._gemm(self.V_FP8_GU, dn["gate"].map, dn["up"].map, self.map_x8, e["gu"], dn["gate"].n // 128, items, pdl=pdl)
-                    self._gemm(self.V_FP8_BF16, dn["down"].map, None, self.map_yd8, e["down"], H // 128, items, pdl=pdl)
-                with self._stage("tp_reduce"):
-                    self._all_reduce(part[:R])
-                    torch.add(x[:R], part[:R], out=x[:R])
-            else:
-                src = self.xl if self.ep else x
-                with self._stage("router"):
-                    K.prep_norm(src, d["g_post"], T, s.norm_eps, xn=xn, pdl=pdl)
-                    # scores of all chunk rows as one fp32 matrix product (library GEMM, no TF32: the same products as
-                    # the step's FMA loop, summed in another order), selection by the router kernel per 16 rows
-                    tf32 = torch.backends.cuda.matmul.allow_tf32
-                    torch.backends.cuda.matmul.allow_tf32 = False
-                    torch.mm(xn[:T].float(), d["router_wt"], out=self.scores[:T])
-                    torch.backends.cuda.matmul.allow_tf32 = tf32
-                    e["router"].rows = T
-                    K.router(e["router"], pdl=pdl)
+            for c, row0, R in rows:
+                self._layer_rows(L, d, e, c, row0, start + row0, R, xl)
+            if "dense" not in d:
                 self.moe.stage = self._stage if self.profile else None
                 with self._stage("moe"):
                     if self.ep or tp == 1:
                         self.moe.run(src, d["g_post"], self.topk_ids, self.topk_p, src, src, weights=self.moe_w[L], tokens=T)
                     else:
-                        self.moe.run(src, d["g_post"], self.topk_ids, self.topk_p, self.zeros, part, weights=self.moe_w[L], tokens=T)
+                        self.moe.run(src, d["g_post"], self.topk_ids, self.topk_p, self.zeros, self.part, weights=self.moe_w[L], tokens=T)
                 with self._stage("tp_reduce"):
                     if self.ep:
-                        dist.all_gather_into_tensor(x[:R], src[:T], group=self.group)
+                        dist.all_gather_into_tensor(x[:n], src[:T], group=self.group)
                     elif tp > 1:
-                        self._all_reduce(part[:R])
-                        torch.add(x[:R], part[:R], out=x[:R])
+                        self._all_reduce(self.part[:n])
+                        torch.add(x[:n], self.part[:n], out=x[:n])
             tap = t.tap_of_layer.get(L)
             if tap is not None and self.draft is not None:
-                self.feats[:R, tap * H:(tap + 1) * H].copy_(x[:R])
+                H = s.hidden
+                self.feats[:n, tap * H:(tap + 1) * H].copy_(x[:n])
         if self.draft is not None:
             with self._stage("draft_ingest"):
-                self._ingest(R, items)
+                K.rope_table(self.pos, n, s.draft.head_dim, s.draft.rope_theta, self.drope, pdl=pdl)
+                for c, row0, R in rows:
+                    self._ingest(c, row0, R)
 
-    def _ingest(self, R: int, items: int) -> None:
-        """Draft context for the chunk's rows: fc over this rank's feature taps (reduced over the ranks),
+    def _layer_rows(self, L: int, d: dict, e: dict, c: int, row0: int, pos0: int, R: int, xl: torch.Tensor) -> None:
+        """One layer for the R rows of chunk ``c`` (rows ``row0`` on of the span) up to the choice of their experts, or through the dense MLP."""
+        s, t, tp = self.spec, self.t, self.tp
+        H, pdl, items = s.hidden, False, -(-R // self.step)
+        x, xn, part, pos = self.x[row0:row0 + R], self.xn, self.part, self.pos[c]
+        # ---- attention (tensor parallel)
+        with self._stage("norm"):
+            K.prep_norm(x, d["g_in"], R, s.norm_eps, xn=xn, pdl=pdl)
+        with self._stage("qkv_gemm"):
+            self._bf16_gemm(self.V_BF16_F32, d["map_qkv"], self.xn, e["qkv"], d["wqkv"].shape[0] // 128, R, items, pdl)
+        p, q = e["post"], e["attn"]
+        p.rows, p.pos0, p.rope = R, pos.data_ptr(), self.rope[d["kind"]][row0].data_ptr()
+        if d["kind"] == FULL_DSA:
+            p.idx_rope_tab = self.idx_rope[row0].data_ptr()
+        with self._stage("attn_post"):
+            K.attn_post(p, pdl=pdl)
+        if d["kind"] == FULL_DSA and pos0 + R > s.indexer.top_k:
+            sw = e["sweep"]
+            sw.rows, sw.pos0 = R, pos.data_ptr()
+            shard = self.shard_index and R % (ROWS * tp) == 0
+            Rl = R // tp if shard else R                         # rows this rank selects for
+            first = self.rank * Rl if shard else 0
+            sw.group0, sw.ngroups = first // ROWS, Rl // ROWS
+            tiles = -(-(pos0 + R) // 128)
+            with self._stage("index_sweep"):
+                K.index_sweep(*e["sweep_maps"], sw, max(1, min(tiles, 592 // (Rl // ROWS))), pdl=pdl)
+            with self._stage("topk"):
+                logits, pos_l = self.idx_logits[first:first + Rl], pos[1:]             # pos[1] = pos0 + first
+                sel = self.sel_local if shard else self.sel
+                if t.topk_grid:
+                    K.topk_rows_grid(logits, pos_l, Rl, s.indexer.top_k, sel, self.topk_state, 16, pdl=pdl)
+                else:
+                    K.topk_rows(logits, pos_l, Rl, s.indexer.top_k, sel, pdl=pdl)
+                if shard:
+                    dist.all_gather_into_tensor(self.sel[:R], self.sel_local[:Rl], group=self.group)
+        q.rows, q.pos0 = R, pos.data_ptr()
+        with self._stage("attn_dsa" if d["kind"] == FULL_DSA else "attn_swa"):
+            if e["group_attn"]:
+                K.attn_group(q, pdl=pdl)
+            else:
+                K.attn_rows(q, 1, pdl=pdl)
+        with self._stage("o_gemm"):
+            self._gemm(self.V_FP8_BF16, d["wo"].map, None, self.map_o8, e["o"], H // 128, items, pdl=pdl)
+        moe = "dense" not in d
+        T = R // tp if self.ep else R
+        with self._stage("tp_reduce"):
+            if self.ep and moe:
+                # sequence parallel from here to the end of the layer: this rank keeps rows [rank*T, (rank+1)*T)
+                dist.reduce_scatter_tensor(self.rs[:T], part[:R], group=self.group)
+                torch.add(xl, self.rs[:T], out=self.xl[:T])
+            else:
+                self._all_reduce(part[:R])
+                torch.add(x, part[:R], out=x)
+        if not moe:
+            dn = d["dense"]
+            with self._stage("dense_mlp"):
+                K.prep_norm(x, d["g_post"], R, s.norm_eps, x8=self.x8, xs=self.xs, pdl=pdl)
+                self._gemm(self.V_FP8_GU, dn["gate"].map, dn["up"].map, self.map_x8, e["gu"], dn["gate"].n // 128, items, pdl=pdl)
+                self._gemm(self.V_FP8_BF16, dn["down"].map, None, self.map_yd8, e["down"], H // 128, items, pdl=pdl)
+            with self._stage("tp_reduce"):
+                self._all_reduce(part[:R])
+                torch.add(x, part[:R], out=x)
+            return
+        with self._stage("router"):
+            K.prep_norm(self.xl if self.ep else x, d["g_post"], T, s.norm_eps, xn=xn, pdl=pdl)
+            # scores of all chunk rows as one fp32 matrix product (library GEMM, no TF32: the same products as
+            # the step's FMA loop, summed in another order), selection by the router kernel per 16 rows
+            tf32 = torch.backends.cuda.matmul.allow_tf32
+            torch.backends.cuda.matmul.allow_tf32 = False
+            torch.mm(xn[:T].float(), d["router_wt"], out=self.scores[:T])
+            torch.backends.cuda.matmul.allow_tf32 = tf32
+            r = e["router"]
+            r.rows, r.topk_ids, r.topk_p = T, self.topk_ids[row0].data_ptr(), self.topk_p[row0].data_ptr()
+            K.router(r, pdl=pdl)
+
+    def _ingest(self, c: int, row0: int, R: int) -> None:
+        """Draft context for a chunk's rows: fc over this rank's feature taps (reduced over the ranks),
         RMSNorm, every draft layer's k/v projection in one GEMM, k-norm + RoPE + append."""
-        dr, dd, pdl = self.draft, self.spec.draft, False
-        K.rope_table(self.pos, R, dd.head_dim, dd.rope_theta, self.drope, pdl=pdl)
-        self._bf16_gemm(self.V_BF16_BF16, dr.map_fc, self.taps, self.args_fc, dd.hidden // 128, R, items, pdl)
+        dr, dd, pdl, items = self.draft, self.spec.draft, False, -(-R // self.step)
+        self._bf16_gemm(self.V_BF16_BF16, dr.map_fc, self.taps[row0:row0 + self.C], self.args_fc, dd.hidden // 128, R, items, pdl)
         self._all_reduce(self.dh[:R])
         K.prep_norm(self.dh, dr.hidden_norm, R, dd.norm_eps, xn=self.dxn, pdl=pdl)
         self._bf16_gemm(self.V_BF16_F32, dr.map_kv, self.dxn, self.args_kv, dr.wkv.shape[0] // 128, R, items, pdl)
         for p in self.args_ingest:
-            p.rows = R
+            p.rows, p.pos0, p.rope = R, self.pos[c].data_ptr(), self.drope[row0].data_ptr()
             K.attn_post(p, pdl=pdl)
 
     # ------------------------------------------------------------------ public API
@@ -438,10 +490,13 @@ class NativePrefill:
         ev0.record()
         p = start
         chunks = plan_chunks(start, end, self.C, self.quantum)
-        for c in chunks:
-            self.tokens[:c.rows].copy_(prompt[c.pos0:c.pos0 + c.rows].to(torch.int32), non_blocking=True)
-            self._chunk(c.pos0, c.rows)
-            p = c.pos0 + c.rows
+        self._fit_span(sum(c.rows for c in chunks))
+        each = self.span // self.C
+        for i in range(0, len(chunks), each):
+            sizes = [c.rows for c in chunks[i:i + each]]
+            first, p = chunks[i].pos0, chunks[i].pos0 + sum(sizes)
+            self.tokens[:p - first].copy_(prompt[first:p].to(torch.int32), non_blocking=True)
+            self._span(first, sizes)
         ev1.record()
         self.phases = {"chunks": len(chunks), "rows": p - start, "events": (ev0, ev1)}
         return p

@@ -203,3 +203,31 @@ def test_round_graph_carries_programmatic_edges():
     assert plain["programmatic_edges"] == 0 and plain["kernel_nodes"] == prog["kernel_nodes"]
     # every kernel but the first and the relaunch node (an ordinary launch) hangs on a programmatic edge
     assert prog["programmatic_edges"] >= prog["kernel_nodes"] - 2, prog
+
+
+@pytest.mark.parametrize("chunk,most,n", [(64, 8, 699), (128, 2, 700), (48, 3, 300), (256, 4, 256), (256, 4, 272)])
+def test_prompt_spans_equal_single_chunks(chunk, most, n):
+    """Chunks that share a layer's experts leave the bits in the target's and the draft's caches that they leave one by one, in several
+    spans with a short last one too."""
+    from naivert_b200.models.naive_n0p5 import small_w8a8_spec
+    from naivert_b200.runtime.engine import Engine
+    spec = small_w8a8_spec(4)
+    eng = Engine.build(spec, capacity=1024, seed=0, prefill_chunk=chunk)
+    pf, caches = eng.prefill, []
+    for d in list(eng.target.layers) + list(eng.round.draft.layers):
+        caches += [d[k] for k in ("k", "v", "ik", "iks") if k in d]
+    prompt = torch.randint(0, spec.vocab - 16, (n,), generator=torch.Generator().manual_seed(n))
+
+    def run(limit):
+        for c in caches:
+            c.zero_()
+        pf.span_limit = limit * chunk
+        assert pf.run(prompt) == n // 16 * 16
+        torch.cuda.synchronize()
+        pf.check()
+        assert pf.span == min(limit * chunk, -(-(n // 16 * 16) // chunk) * chunk)
+        return [c.clone() for c in caches]
+
+    single, spans = run(1), run(most)
+    assert any(c.any() for c in single)
+    assert all(torch.equal(a, b) for a, b in zip(single, spans))
