@@ -50,7 +50,7 @@ class StackPrefill:
         ffs = [d["spec"].mlp for d in L if d["spec"].mlp is not None]
         moe = [f for f in ffs if f.kind == "moe"]
         self.h_ld = pad(s.hidden, 8)
-        # Argument blocks by launch: a prompt of a small model is 77 launches of a few microseconds, and filling some twenty fields anew for
+        # Argument blocks by launch: a prompt of a small model is some 70 launches of a few microseconds, and filling some twenty fields anew for
         # each took longer.  What changes from prompt to prompt - rows, positions, segments - is set every time.  (Buffers that are taken
         # anew clear it.)
         self._kept: Dict[tuple, object] = {}
