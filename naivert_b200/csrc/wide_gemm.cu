@@ -210,10 +210,11 @@ wide_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_constant
       }
     }
   } else {
-    // e4m3: every K block is promoted - commit, load from TMEM, scale, add - and these hand-overs and the two threads that drive the
-    // ring are what bounds a block, not the tensor cores (29 % busy) or the copies.  Per K block: o_proj (K 8192, 2048 rows, weights in
-    // L2) 382 ns, 500 ns with one accumulator per hand-over and eight warps that finished one block before they asked for the next; gate
-    // and up of 256 experts of ~64 rows 767 ns (4.2 TB/s of weights), 1079 ns.
+    // e4m3: every K block is promoted - commit, load from TMEM, scale, add.  Per K block: o_proj (K 8192, 2048 rows, weights in L2)
+    // 382 ns with accumulators in pairs, 500 ns with one accumulator per hand-over and eight warps that finished one block before they
+    // asked for the next; gate and up of 256 experts of ~64 rows 767 ns (4.2 TB/s of weights), 1079 ns.  What bounds a block now is
+    // several things that overlap: without additions, TMEM loads and products its copies alone take 0.7 of it (o_proj) to 0.9 (experts,
+    // which stream from HBM), without the products 0.83, without the additions 0.88; the tensor cores are busy 29 %.
     const int quad = warp & 3;                       // TMEM lane quadrant this warp may read
     const int c0 = ((warp - 2) >> 2) * kWCols;       // first of its token columns
     const int row = quad * 32 + lane;                // feature within the tile
