@@ -371,8 +371,9 @@ class StackPrefill:
             return None
         self._rows(R, pre=t.g_final, **wait)
         out = torch.empty(len(want), s.vocab, dtype=torch.float32, device=self.dev)
-        straight = want[-1] - want[0] + 1 == len(want) == len(set(want))         # (ascending: rows that follow one another)
-        idx = None if straight else torch.as_tensor(list(want), dtype=torch.long, device=self.dev)
+        want = list(want)
+        straight = want == list(range(want[0], want[0] + len(want)))             # rows that follow one another
+        idx = None if straight else torch.as_tensor(want, dtype=torch.long, device=self.dev)
         for i in range(0, len(want), self.head_rows):
             n = min(self.head_rows, len(want) - i)
             rows = self.h[want[0] + i:want[0] + i + n] if idx is None else self.h.index_select(0, idx[i:i + n])
@@ -397,7 +398,7 @@ class StackPrefill:
             R = min(self.span, n - c0)
             self.tokens[:R].copy_(tokens[c0:c0 + R].to(torch.int32), non_blocking=True)
             seen: Optional[list] = None if trace is None else []
-            got = self._chunk(pos0 + c0, R, [w - c0 for w in order if c0 <= w < c0 + R], seen)
+            got = self._chunk(pos0 + c0, R, [int(w) - c0 for w in order if c0 <= w < c0 + R], seen)
             for i in range(0, R if seen else 0, self.C):
                 trace.extend(x[i:i + self.C] for x in seen)
             if got is not None:

@@ -5,6 +5,7 @@ import json
 import math
 import os
 import struct
+from types import SimpleNamespace
 
 import pytest
 import torch
@@ -192,6 +193,28 @@ def test_token_rows_per_tile():
         assert [rule(epi, 80, rows) for rows in (65, 128, 129, 187, 256)] == [128, 128, 192, 192, 256]
     assert [rule(S.EPI_CLAMPED_GLU, 64, rows) for rows in (100, 187)] == [64, 128]
     assert [rule(S.EPI_CLAMPED_GLU, 128, rows) for rows in (100, 187, 256)] == [128, 192, 128]
+
+
+@pytest.mark.parametrize("want", [[3, 3, 5], torch.tensor([3, 3, 5]), (torch.tensor(3), 3, 5), torch.tensor([0, 4, 4, 4, 9, 11]), torch.tensor([[2], [2], [4]])])
+def test_wanted_rows_of_any_kind_are_plain_numbers(want):
+    """Rows equal as numbers count as repeated whatever holds them: elements of a tensor hash by identity."""
+    from naivert_b200.prefill.stack import StackPrefill
+    seen = []
+
+    class Fake(StackPrefill):
+        def __init__(self):
+            self.t, self.C, self.span, self.tokens = SimpleNamespace(capacity=64), 8, 8, torch.zeros(8, dtype=torch.int32)
+
+        def _fit_span(self, n):
+            pass
+
+        def _chunk(self, pos0, R, want, trace):
+            seen.append(want)
+            return torch.tensor([float(pos0 + w) for w in want]).view(-1, 1) if want else None
+
+    got = Fake().extend(torch.zeros(12, dtype=torch.int32), 0, want)
+    assert got.flatten().tolist() == [float(w) for w in want]
+    assert all(type(w) is int for rows in seen for w in rows)
 
 
 def test_spans_grow_with_the_prompt_as_far_as_memory_goes(monkeypatch):
