@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256) group_prep_kernel(const GroupPrepArgs p) 
       __syncwarp();
     } else {
       const int h = u - p.heads - p.kv_heads;
-      for (int c = lane; c < p.vdim; c += 32) store_act(p.v_cache, ((long long)pos * p.kv_heads + h) * p.vp + c, __ldg(row + p.v_off + h * p.vdim + c), p.f32);
+      for (int c = lane; c < p.vdim; c += 32) store_act(p.v_cache, ((long long)pos * p.kv_heads + h) * p.vp + c, row[p.v_off + h * p.vdim + c], p.f32);
     }
   }
 }
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(256) transpose_kernel(const TransposeArgs a) {
   for (int i = 0; i < 64; i += 8) {
     const int r = r0 + ty + i;
     uint32_t v = 0u;
-    if (r < a.rows && c0 + tx < a.cols) v = __ldg(reinterpret_cast<const uint32_t*>(a.src + (long long)r * a.cols + c0 + tx));
+    if (r < a.rows && c0 + tx < a.cols) v = *reinterpret_cast<const uint32_t*>(a.src + (long long)r * a.cols + c0 + tx);
     *reinterpret_cast<uint32_t*>(&tile[ty + i][tx]) = v;
   }
   __syncthreads();

@@ -205,9 +205,9 @@ __global__ void __launch_bounds__(128, 3) state_blocks_kernel(const StateChunkAr
       for (int i = 0; i < NC; ++i) {
         const int d = min(d0 + lane + 32 * i, a.dim - 1);
         const long long r = min(r0 + t, a.rows - 1);
-        q[t][i] = __ldg(a.q + r * a.q_ld + hk * a.dim + d);
-        k[t][i] = __ldg(a.k + r * a.k_ld + hk * a.dim + d);
-        g[t][i] = KIND == kStateNormalized ? keep[t] : __ldg(a.g + r * a.g_ld + h * a.dim + d);
+        q[t][i] = a.q[r * a.q_ld + hk * a.dim + d];
+        k[t][i] = a.k[r * a.k_ld + hk * a.dim + d];
+        g[t][i] = KIND == kStateNormalized ? keep[t] : a.g[r * a.g_ld + h * a.dim + d];
       }
 #pragma unroll
     for (int t = 0; t < B; ++t)
@@ -519,8 +519,8 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const ShortConvArgs a) 
   if (seg == total && a.low) {
     for (int r = r0; r < r1; ++r) {
       const float* p = a.proj + r * a.ld;
-      for (int c = lane; c < a.low_cols; c += 32) store_act(a.low, r * a.low_ld + c, __ldg(p + a.low_off + c), a.f32);
-      for (int c = lane; c < a.low2_cols; c += 32) store_act(a.low, r * a.low_ld + a.low2_at + c, __ldg(p + a.low2_off + c), a.f32);
+      for (int c = lane; c < a.low_cols; c += 32) store_act(a.low, r * a.low_ld + c, p[a.low_off + c], a.f32);
+      for (int c = lane; c < a.low2_cols; c += 32) store_act(a.low, r * a.low_ld + a.low2_at + c, p[a.low2_off + c], a.f32);
     }
   }
   if (seg >= total) return;
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const ShortConvArgs a) 
   const long long out_ld = (long long)(is_v ? a.heads * a.vdim : G * a.dim);
   const __nv_bfloat16* kern = a.conv + (long long)col * a.taps;
   auto input = [&](int rr, int c) {            // row rr of the projection, or what earlier chunks left
-    if (rr >= 0) return __ldg(a.proj + rr * a.ld + col + c);
+    if (rr >= 0) return a.proj[rr * a.ld + col + c];
     return pos0 + rr >= 0 ? a.history[(long long)((pos0 + rr) % a.hist_rows) * columns + col + c] : 0.f;
   };
   auto finish = [&](int r, float (&y)[NC]) {
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(128) short_conv_kernel(const ShortConvArgs a) 
 #pragma unroll
       for (int q = 0; q < BATCH; ++q)
 #pragma unroll
-        for (int i = 0; i < NC; ++i) in[q][i] = rb + q < r1 && lane + 32 * i < w ? __ldg(a.proj + (rb + q) * a.ld + col + lane + 32 * i) : 0.f;
+        for (int i = 0; i < NC; ++i) in[q][i] = rb + q < r1 && lane + 32 * i < w ? a.proj[(rb + q) * a.ld + col + lane + 32 * i] : 0.f;
 #pragma unroll
       for (int q = 0; q < BATCH; ++q) {
         if (rb + q >= r1) break;
@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(256) token_mix_kernel(const TokenMixArgs a) {
   const long long o0 = (long long)r * a.mixes * a.out_ld;
   if (((a.width | (int)a.out_ld | (int)a.state_stride) & 3) == 0 && (reinterpret_cast<uintptr_t>(a.shift) & 15) == 0) {
     for (int c = threadIdx.x * 4; c < a.width; c += 1024) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(x + c));
+      const float4 v = *reinterpret_cast<const float4*>(x + c);
       const float4 b = before ? *reinterpret_cast<const float4*>(before + c) : make_float4(0.f, 0.f, 0.f, 0.f);
       const float4 d = make_float4(b.x - v.x, b.y - v.y, b.z - v.z, b.w - v.w);
 #pragma unroll 5
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(256) token_mix_kernel(const TokenMixArgs a) {
     return;
   }
   for (int c = threadIdx.x; c < a.width; c += 256) {
-    const float v = __ldg(x + c), d = (before ? before[c] : 0.f) - v;
+    const float v = x[c], d = (before ? before[c] : 0.f) - v;
     for (int s = 0; s < a.mixes; ++s) store_act(a.out, o0 + s * a.out_ld + c, fmaf(d, bf(a.mu + (long long)s * a.width + c), v), a.f32);
     if (keep) keep[c] = v;
   }
@@ -660,8 +660,8 @@ __global__ void __launch_bounds__(256) head_gate_kernel(const HeadGateArgs a) {
       const int c = (lane + 32 * i) * 4;
       keep[i] = z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (c < a.vdim) {
-        keep[i] = __ldg(reinterpret_cast<const float4*>(o + c));
-        z[i] = __ldg(reinterpret_cast<const float4*>(g + c));
+        keep[i] = *reinterpret_cast<const float4*>(o + c);
+        z[i] = *reinterpret_cast<const float4*>(g + c);
       }
     }
     auto sq = [&](const float4& v) { return v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w; };
@@ -671,20 +671,20 @@ __global__ void __launch_bounds__(256) head_gate_kernel(const HeadGateArgs a) {
     };
 #pragma unroll
     for (int i = 0; i < KEEP; ++i) ss += sq(keep[i]);
-    for (int c = (lane + 32 * KEEP) * 4; c < a.vdim; c += 128) ss += sq(__ldg(reinterpret_cast<const float4*>(o + c)));
+    for (int c = (lane + 32 * KEEP) * 4; c < a.vdim; c += 128) ss += sq(*reinterpret_cast<const float4*>(o + c));
     const float rs = inv / sqrtf(lane_sum(ss) * inv * inv / (float)a.vdim + a.eps);
 #pragma unroll
     for (int i = 0; i < KEEP; ++i)
       if ((lane + 32 * i) * 4 < a.vdim) put((lane + 32 * i) * 4, keep[i], z[i], rs);
-    for (int c = (lane + 32 * KEEP) * 4; c < a.vdim; c += 128) put(c, __ldg(reinterpret_cast<const float4*>(o + c)), __ldg(reinterpret_cast<const float4*>(g + c)), rs);
+    for (int c = (lane + 32 * KEEP) * 4; c < a.vdim; c += 128) put(c, *reinterpret_cast<const float4*>(o + c), *reinterpret_cast<const float4*>(g + c), rs);
     return;
   }
   for (int c = lane; c < a.vdim; c += 32) {
-    const float v = __ldg(o + c) * inv;
+    const float v = o[c] * inv;
     ss = fmaf(v, v, ss);
   }
   const float rs = inv / sqrtf(lane_sum(ss) / (float)a.vdim + a.eps);
-  for (int c = lane; c < a.vdim; c += 32) store_act(a.out, at + c, __ldg(o + c) * rs * bf(w + c) * gated(__ldg(g + c)), a.f32);
+  for (int c = lane; c < a.vdim; c += 32) store_act(a.out, at + c, o[c] * rs * bf(w + c) * gated(g[c]), a.f32);
 }
 
 // ------------------------------------------------------------------------------------ one token

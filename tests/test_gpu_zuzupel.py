@@ -178,6 +178,23 @@ def test_long_chunks(name, dtype):
         eng.close()
 
 
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+@pytest.mark.parametrize("name", ["mixed", "delta_very_wide", "wkv_odd", "parallel_beyond_tensor_cores"])
+def test_launches_that_begin_early_leave_the_same_bits(name, dtype):
+    """Every launch of a prompt under the end of the one in front, against launches that start as a whole: prompts and turns."""
+    cfg = CASES[name]
+    w = weights(cfg, 4)
+    toks = tokens(cfg, 1188, 6)
+    early, plain = (engine(cfg, w, dtype, capacity=1300, chunk=1024) for _ in range(2))
+    early.prefill.early, plain.prefill.early = (lambda rows: True), (lambda rows: False)
+    try:
+        for sizes in ([1, 187], [1000, 188], [187, 1, 1000]):
+            assert torch.equal(feed(early, toks[:sum(sizes)], sizes), feed(plain, toks[:sum(sizes)], sizes))
+    finally:
+        early.close()
+        plain.close()
+
+
 def test_stream_after_every_layer_run():
     cfg = CASES["mixed"]
     w = weights(cfg, 3)
