@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kListWarps * 32, 2) attn_list_kernel(const Att
 
   auto ids_of = [&](int t) {                                        // lane i < 16: key i of the tile (-1: none)
     const int j = t * kListKeys + lane;
-    return lane < kListKeys && t < tiles && j < count ? (sel ? __ldg(sel + j) : j) : -1;
+    return lane < kListKeys && t < tiles && j < count ? (sel ? sel[j] : j) : -1;
   };
   // eight lanes copy one key, 128 bytes at a time
   auto request = [&](int stage, int ids) {

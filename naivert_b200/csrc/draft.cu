@@ -19,7 +19,7 @@ using namespace nrt;
 namespace {
 
 // x[0] = embed[anchor], x[1..rows) = mask embedding, x[rows..16) = 0
-__global__ void draft_block_input_kernel(const int* __restrict__ block_ids, const __nv_bfloat16* __restrict__ embed,
+__global__ void draft_block_input_kernel(const int* block_ids, const __nv_bfloat16* __restrict__ embed,
                                          const __nv_bfloat16* __restrict__ mask, __nv_bfloat16* __restrict__ x, int hidden,
                                          int rows, int vocab) {
   griddep_wait();

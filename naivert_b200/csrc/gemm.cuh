@@ -439,8 +439,8 @@ __device__ __forceinline__ PostCtx qkv_post_prepare(const AttnPostArgs& a_in, in
   }
   if (c.rope) {
     const float4* t = reinterpret_cast<const float4*>(c.tab + (c.d >> 1));      // two pairs = 16 bytes, 16-byte aligned
-    if (quad < rows) c.cs0 = __ldg(t + (size_t)quad * (c.half >> 1));
-    if (quad + 4 < rows) c.cs1 = __ldg(t + (size_t)(quad + 4) * (c.half >> 1));
+    if (quad < rows) c.cs0 = t[(size_t)quad * (c.half >> 1)];
+    if (quad + 4 < rows) c.cs1 = t[(size_t)(quad + 4) * (c.half >> 1)];
   }
   return c;
 }
@@ -464,7 +464,7 @@ __device__ __forceinline__ void qkv_post_epilogue(const AttnPostArgs& a_in, cons
     float x[4] = {v4.x, v4.y, v4.z, v4.w};
     const int pos = c.p0 + r;
     float4 cs = make_float4(1.f, 0.f, 1.f, 0.f);
-    if (c.rope) cs = it == 0 ? c.cs0 : (it == 1 ? c.cs1 : __ldg(reinterpret_cast<const float4*>(c.tab + (c.d >> 1)) + (size_t)r * (c.half >> 1)));
+    if (c.rope) cs = it == 0 ? c.cs0 : (it == 1 ? c.cs1 : reinterpret_cast<const float4*>(c.tab + (c.d >> 1))[(size_t)r * (c.half >> 1)]);
     if (c.kind == kPostIq || c.kind == kPostIk) {
       // whole tile = one indexer head / the indexer key (uniform over the warp)
       if (c.kind == kPostIk) {
@@ -748,7 +748,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_consta
     int lo = 0, hi = 0;
     for (int i0 = 0; i0 < na; i0 += 32) {
       const int i = i0 + lane;
-      const int id = i < na ? __ldg(p.active_ids + i) : 0x7fffffff;
+      const int id = i < na ? p.active_ids[i] : 0x7fffffff;
       lo += __popc(__ballot_sync(0xffffffffu, id < id_lo));
       hi += __popc(__ballot_sync(0xffffffffu, id < id_hi));
     }
@@ -900,7 +900,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmA0, const __grid_consta
             for (int r = 0; r < kTok; ++r) sc[r] = r < p.rows ? bscale[r * kb_count + kb] : 0.f;
           } else if (!gathered) {
 #pragma unroll
-            for (int r = 0; r < kTok; ++r) sc[r] = __ldg(as + r * kb_total + kb);
+            for (int r = 0; r < kTok; ++r) sc[r] = as[r * kb_total + kb];
           }
           const float w0 = __ldg(ws0 + kb);
           const float w1 = DUAL ? __ldg(ws1 + kb) : 0.f;

@@ -724,7 +724,7 @@ __global__ void tail_commit_kernel(const TailArgs a) {
 
 // Prompt replay cursor: loads the next `rows` prompt tokens into the step's token buffer, points
 // the step (ctrl[0]) and the draft ingest (ctrl[2]) at their position and advances ctrl[10].
-__global__ void prefill_cursor_kernel(const int* __restrict__ prompt, int n_prompt, int rows, int* ctrl, int* tokens) {
+__global__ void prefill_cursor_kernel(const int* prompt, int n_prompt, int rows, int* ctrl, int* tokens) {
   griddep_wait();
   griddep_launch();
   const int cur = ctrl[NRT_CTRL_CURSOR];

@@ -62,7 +62,7 @@ __device__ __forceinline__ float from_e4m3(uint8_t b) {
 }
 
 // ----------------------------------------------------------------------------- embedding gather
-__global__ void embed_rows_kernel(const int* __restrict__ tokens, const __nv_bfloat16* __restrict__ table,
+__global__ void embed_rows_kernel(const int* tokens, const __nv_bfloat16* __restrict__ table,
                                   __nv_bfloat16* __restrict__ x, int hidden, int rows, int vocab) {
   griddep_wait();
   griddep_launch();
@@ -78,7 +78,7 @@ __global__ void embed_rows_kernel(const int* __restrict__ tokens, const __nv_bfl
 
 // ----------------------------------------------------------------------------- RoPE tables for this step
 // table[r][i] = (cos, sin)(pos_r * theta^(-2i/dim)), evaluated in fp64 and rounded to fp32.
-__global__ void rope_table_kernel(const int* __restrict__ pos0, int rows, int dim, double theta, float2* __restrict__ out) {
+__global__ void rope_table_kernel(const int* pos0, int rows, int dim, double theta, float2* __restrict__ out) {
   griddep_wait();
   griddep_launch();
   const int r = blockIdx.x, i = threadIdx.x;
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(128) step_prologue_kernel(const PrologueArgs a
 // xn = bf16(x * rsqrt(mean(x^2) + eps) * g); optional packet: e4m3(xn / s) with one power-of-two
 // scale s per 128 channels.
 __global__ void __launch_bounds__(256)
-prep_norm_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma, int hidden, int rows,
+prep_norm_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ gamma, int hidden, int rows,
                  float eps, __nv_bfloat16* __restrict__ xn, uint8_t* __restrict__ x8, float* __restrict__ xs) {
   __shared__ float red[8];
   griddep_wait();
@@ -567,7 +567,7 @@ __device__ __forceinline__ uint32_t order_key(float f) {
 // covers a contiguous span), so the final sweep can emit winners in ascending index order from one block-wide
 // prefix sum.  Each radix pass builds a 256-bin shared histogram; warp 0 locates the threshold bin with a
 // shuffle scan (lane l owns bins 255 - 8l .. 248 - 8l).
-__global__ void __launch_bounds__(1024) topk_rows_kernel(const float* __restrict__ logits, int ld, const int* pos0,
+__global__ void __launch_bounds__(1024) topk_rows_kernel(const float* logits, int ld, const int* pos0,
                                                          int rows, int top_k, int* __restrict__ sel) {
   __shared__ uint32_t hist[256];
   __shared__ uint32_t s_prefix, s_need;
@@ -748,7 +748,7 @@ struct TopkGridState {          // per row
   unsigned int seg_gt[64], seg_eq[64];
 };
 
-__global__ void __launch_bounds__(1024) topk_grid_hist_kernel(const float* __restrict__ logits, int ld, const int* pos0,
+__global__ void __launch_bounds__(1024) topk_grid_hist_kernel(const float* logits, int ld, const int* pos0,
                                                                int rows, int top_k, TopkGridState* st, int pass) {
   __shared__ unsigned int sh[256];
   __shared__ bool s_last;
@@ -797,7 +797,7 @@ __global__ void __launch_bounds__(1024) topk_grid_hist_kernel(const float* __res
   if (threadIdx.x < 256) S.hist[threadIdx.x] = 0u;
 }
 
-__global__ void __launch_bounds__(1024) topk_grid_count_kernel(const float* __restrict__ logits, int ld, const int* pos0,
+__global__ void __launch_bounds__(1024) topk_grid_count_kernel(const float* logits, int ld, const int* pos0,
                                                                 int rows, int top_k, TopkGridState* st) {
   __shared__ unsigned int s_gt, s_eq;
   griddep_wait();
@@ -824,7 +824,7 @@ __global__ void __launch_bounds__(1024) topk_grid_count_kernel(const float* __re
   if (threadIdx.x == 0) { S.seg_gt[blockIdx.x] = s_gt; S.seg_eq[blockIdx.x] = s_eq; }
 }
 
-__global__ void __launch_bounds__(1024) topk_grid_write_kernel(const float* __restrict__ logits, int ld, const int* pos0,
+__global__ void __launch_bounds__(1024) topk_grid_write_kernel(const float* logits, int ld, const int* pos0,
                                                                 int rows, int top_k, TopkGridState* st, int* __restrict__ sel) {
   __shared__ uint32_t wsum_gt[32], wsum_eq[32];
   __shared__ uint32_t base_out, base_eq;
