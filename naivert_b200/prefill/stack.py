@@ -54,6 +54,7 @@ class StackPrefill:
         # each took longer.  What changes from prompt to prompt - rows, positions, segments - is set every time.  (Buffers that are taken
         # anew clear it.)
         self._kept: Dict[tuple, object] = {}
+        self.maps: Dict[tuple, object] = {}
         filled = min([-(-SPAN_PAIRS * f.routing.expert_count // f.routing.top_k) for f in moe], default=0)
         self.span_limit = max(C, min(SPAN_ROWS, filled, runtime.capacity) // C * C)
         self._size_span(C)
@@ -68,7 +69,6 @@ class StackPrefill:
         self.pdl = False
         self.hw = torch.zeros(self.head_rows, self.h_ld, dtype=self.act, device=dev)
         self.tensor_cores = not self.f32              # attention of chunk rows on tcgen05 (else the plain kernel)
-        self.maps: Dict[tuple, object] = {}
         self.phases: dict = {}
         self.profile = False                          # per-stage CUDA-event timing (adds an event pair per stage)
         self._timed: Dict[str, list] = {}
@@ -96,6 +96,8 @@ class StackPrefill:
                        ea=z(cap * max(pad(f.ff, 8) for f in moe), self.act), ey=z(cap * s.hidden))
         self.rows_of, self.span = rows_of, P
         self._kept.clear()
+        for key in [k for k in self.maps if k[0] == "x"]:      # maps hold the tensors they describe, and these go
+            del self.maps[key]
         for name, v in new.items():
             setattr(self, name, v)
         self._window()

@@ -217,6 +217,27 @@ def test_wanted_rows_of_any_kind_are_plain_numbers(want):
     assert all(type(w) is int for rows in seen for w in rows)
 
 
+def test_buffers_of_a_shorter_span_are_given_back(monkeypatch):
+    """Tensor maps of token rows hold their tensors: those of buffers that a longer span replaces go with them, weights' stay."""
+    import weakref
+    from naivert_b200.ops import stack_kernels as S
+    from naivert_b200.prefill.stack import StackPrefill
+    spec = tumatar.small_spec()
+    monkeypatch.setattr(S, "token_map", lambda t, *shape: SimpleNamespace(tensor=t))
+    pf = object.__new__(StackPrefill)
+    pf.__dict__.update(spec=spec, C=8, dev="cpu", act=torch.bfloat16, h_ld=spec.hidden, _kept={}, maps={("w", 1): "weight"},
+                       t=SimpleNamespace(layers=[{"spec": layer, "kind": layer.mixer.kind} for layer in spec.layers]))
+    pf._size_span(8)
+    old = []
+    for chunks in (2, 3):
+        for t in (pf.h, pf.sorted, pf.ea):
+            pf._xmap(t, 8, 1, 0, 8, 8, 64, 0)
+        old += [weakref.ref(t) for t in (pf.h, pf.sorted, pf.ea, pf.ey, pf.x)]
+        del t
+        pf._size_span(8 * chunks)
+        assert all(r() is None for r in old) and list(pf.maps) == [("w", 1)]
+
+
 def test_spans_grow_with_the_prompt_as_far_as_memory_goes(monkeypatch):
     from naivert_b200.prefill.stack import StackPrefill
     sized = []
