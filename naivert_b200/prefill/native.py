@@ -508,12 +508,14 @@ class NativePrefill:
         return ev0.elapsed_time(ev1)
 
     def warm_chunks(self, sizes=None) -> None:
-        """Run every chunk size once on scratch positions so that module loading, kernel attributes and NCCL
-        channels are paid before the first request.  The rows it writes into the caches start at position 0 and
+        """Run row counts once on scratch positions so that module loading, kernel attributes, NCCL channels and span buffers are paid
+        before the first request.  The default ends with the longest span.  The rows it writes into the caches start at position 0 and
         are overwritten by the next request."""
-        for r in sorted(set(sizes or [self.quantum, self.C])):
+        for r in sorted(set(sizes or [self.quantum, self.C, self.span_limit])):
+            rows = [r] if r <= self.C else [c.rows for c in plan_chunks(0, min(r, self.t.capacity), self.C, self.quantum)]
+            self._fit_span(sum(rows))
             self.tokens.zero_()
-            self._chunk(0, r)
+            self._span(0, rows[:self.span // self.C])
         torch.cuda.current_stream().synchronize()
         self.check()
 

@@ -71,6 +71,39 @@ def test_prefill_chunk_plan():
         plan_chunks(0, 100, 250, 16)
 
 
+@pytest.mark.parametrize("capacity,room,sizes,ran", [(1000, 512, None, [[16], [64], [64] * 4]), (200, 512, None, [[16], [64], [64, 64, 64]]),
+                                                     (1000, 128, None, [[16], [64], [64, 64]]), (1000, 512, [16, 64], [[16], [64]]),
+                                                     (1000, 512, [150], [[64, 64, 16]])])
+def test_native_prefill_warms_its_longest_span(monkeypatch, capacity, room, sizes, ran):
+    """Unless told otherwise, warming takes the buffers of the longest span that capacity and memory allow, so that no request does."""
+    from types import SimpleNamespace
+    from naivert_b200.prefill.native import NativePrefill
+    seen = []
+
+    class Fake(NativePrefill):
+        def __init__(self):
+            self.C, self.quantum, self.span, self.span_limit, self.dev = 64, 16, 64, 256, "cuda"
+            self.t, self.tokens = SimpleNamespace(capacity=capacity), torch.ones(8)
+
+        def _size_span(self, P):
+            if P > room:
+                raise torch.OutOfMemoryError("no room")
+            self.span = P
+
+        def _span(self, start, rows):
+            assert start == 0 and sum(rows) <= self.span
+            seen.append(rows)
+
+        def check(self):
+            pass
+
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda *a: None)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: SimpleNamespace(synchronize=lambda: None))
+    Fake().warm_chunks(sizes)
+    assert seen == ran
+
+
+
 def test_contract_header_matches_python():
     from naivert_b200.runtime import contract as C
     h = C.parse_header()
