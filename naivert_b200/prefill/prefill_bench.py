@@ -55,7 +55,7 @@ def main() -> int:
     prompt = torch.randint(0, spec.vocab - 16, (a.tokens + 1,), generator=g, dtype=torch.int32).pin_memory()
     stream = eng.round.stream
     with torch.cuda.stream(stream):
-        pf.warm_chunks([pf.quantum, a.chunk])
+        pf.warm_chunks([pf.quantum, a.chunk, max(a.chunk, a.tokens)])
         pos = pf.run(prompt, 0, a.tokens)
         ms = pf.executor_ms()
         pf.check()

@@ -413,6 +413,7 @@ class StackPrefill:
         if not 0 <= start <= end <= n or end > self.t.capacity:
             raise ValueError(f"prefill range [{start}, {end}) outside the prompt / cache capacity")
         ev = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        self._fit_span(end - start)
         ev[0].record()
         self.extend(prompt[start:end], start)
         ev[1].record()

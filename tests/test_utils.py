@@ -104,6 +104,35 @@ def test_native_prefill_warms_its_longest_span(monkeypatch, capacity, room, size
 
 
 
+@pytest.mark.parametrize("kind", ["native", "stack"])
+def test_prefill_time_starts_behind_the_span_buffers(monkeypatch, kind):
+    """What a longer span allocates once is not part of a prompt's device time."""
+    from types import SimpleNamespace
+    from naivert_b200.prefill.native import NativePrefill
+    from naivert_b200.prefill.stack import StackPrefill
+    order = []
+
+    class Fake(NativePrefill if kind == "native" else StackPrefill):
+        def __init__(self):
+            self.C, self.quantum, self.span, self.span_limit, self.dev = 64, 16, 64, 256, "cpu"
+            self.spec, self.t, self.tokens = SimpleNamespace(vocab=3), SimpleNamespace(capacity=512), torch.ones(256, dtype=torch.int32)
+
+        def _size_span(self, P):
+            order.append("size")
+            self.span = P
+
+        def _span(self, start, rows):
+            order.append("rows")
+
+        def _chunk(self, *a):
+            order.append("rows")
+
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda *a: None)
+    monkeypatch.setattr(torch.cuda, "Event", lambda **kw: SimpleNamespace(record=lambda: order.append("event")))
+    assert Fake().run(torch.zeros(192, dtype=torch.int32)) == 192
+    assert order == ["size", "event", "rows", "event"]
+
+
 def test_contract_header_matches_python():
     from naivert_b200.runtime import contract as C
     h = C.parse_header()
