@@ -26,7 +26,7 @@ ARCH = "sm100a"
 class KernelVariant:
     variant_id: str
     entry: str                              # extern "C" launcher
-    args_struct: Optional[str] = None       # ctypes class in ops.kernels (None: scalar arguments only)
+    args_struct: Optional[str] = None       # ctypes class in ops.kernels or ops.stack_kernels (None: scalar arguments only)
     size_symbol: Optional[str] = None       # extern "C" int f(): sizeof the struct as compiled
     abi_version: int = 1
     args_bytes: Optional[int] = None        # filled from the ctypes mirror (expected) or the library (actual)
@@ -52,6 +52,7 @@ def _v(op: str, entry: str, struct: Optional[str] = None, size: Optional[str] = 
 _TABLE: List[KernelVariant] = [
     _v("skinny_gemm.fused_epilogues", "nrt_gemm_launch", "GemmArgs", "nrt_gemm_args_size", abi=4, max_rows=16),
     _v("chunk_gemm.persistent", "nrt_wide_gemm_launch", "GemmArgs", "nrt_gemm_args_size", abi=4),
+    _v("chunk_gemm.row_tiles", "nrt_stack_gemm", "StackGemmArgs", "nrt_stack_gemm_args_size"),
     _v("attn_post.rope_kv_append", "nrt_attn_post", "AttnPostArgs", "nrt_attn_post_args_size", abi=2),
     _v("attn_decode.tensor_core", "nrt_attn_decode", "AttnArgs", "nrt_attn_decode_args_size", abi=3),
     _v("attn_rows.scalar", "nrt_attn_rows", "AttnArgs", "nrt_attn_args_size", abi=3),
@@ -70,8 +71,8 @@ _TABLE: List[KernelVariant] = [
     _v("markov.step", "nrt_markov_step", "MarkovArgs", "nrt_markov_args_size"),
     _v("markov.chain", "nrt_markov_chain", "MarkovArgs", "nrt_markov_args_size"),
     _v("ag_push.peer_store", "nrt_ag_push", "AgPushArgs", "nrt_ag_push_args_size"),
-    _v("ep.count", "nrt_ep_count", "EpArgs", "nrt_ep_args_size"),
-    _v("ep.dispatch", "nrt_ep_dispatch", "EpArgs", "nrt_ep_args_size"),
+    _v("ep.count", "nrt_ep_count", "EpArgs", "nrt_ep_args_size", abi=2),
+    _v("ep.dispatch", "nrt_ep_dispatch", "EpArgs", "nrt_ep_args_size", abi=2),
     _v("ep.combine", "nrt_ep_combine", "EpCombineArgs", "nrt_ep_combine_args_size"),
     _v("graph.relaunch", "nrt_relaunch"),
     _v("draft.block_input", "nrt_draft_block_input"),
@@ -82,8 +83,8 @@ _TABLE: List[KernelVariant] = [
 def _expected(v: KernelVariant) -> KernelVariant:
     if v.args_struct is None:
         return v
-    from . import kernels as K
-    return replace(v, args_bytes=C.sizeof(getattr(K, v.args_struct)))
+    from . import kernels as K, stack_kernels as S
+    return replace(v, args_bytes=C.sizeof(getattr(K, v.args_struct, None) or getattr(S, v.args_struct)))
 
 
 def variants() -> Dict[str, KernelVariant]:
@@ -102,8 +103,9 @@ def by_entry(entry: str) -> KernelVariant:
 STEP_VARIANTS = ("nrt_gemm_launch", "nrt_attn_decode", "nrt_index_sweep", "nrt_topk_rows", "nrt_moe_layer", "nrt_router",
                  "nrt_step_prologue", "nrt_sampler_persistent", "nrt_sampler_run", "nrt_tail_commit", "nrt_markov_chain",
                  "nrt_markov_step", "nrt_draft_block_input", "nrt_argmax_rows")
-PREFILL_VARIANTS = ("nrt_wide_gemm_launch", "nrt_attn_post", "nrt_attn_group", "nrt_index_sweep", "nrt_topk_rows_grid",
-                    "nrt_router", "nrt_ep_count", "nrt_ep_dispatch", "nrt_ep_combine", "nrt_ag_push")
+PREFILL_VARIANTS = ("nrt_wide_gemm_launch", "nrt_stack_gemm", "nrt_gemm_launch", "nrt_attn_post", "nrt_attn_group", "nrt_attn_rows",
+                    "nrt_index_sweep", "nrt_topk_rows_grid", "nrt_topk_rows", "nrt_router", "nrt_ep_count", "nrt_ep_dispatch",
+                    "nrt_ep_combine", "nrt_ag_push")
 
 
 def library_variant(lib, expected: KernelVariant) -> KernelVariant:

@@ -103,8 +103,9 @@ MODES: Dict[str, DecodeMode] = {m.mode_id: m for m in (
     # layer-stack models: their own step kernels (ops.stack_kernels checks that library), the shared sampler and tail
     DecodeMode("stack_round", 1, False, ("nrt_sampler_persistent", "nrt_sampler_run", "nrt_tail_commit"), buffer_table(1, False, True)),
     DecodeMode("prefill_native", 0, True,
-               ("nrt_wide_gemm_launch", "nrt_attn_post", "nrt_attn_group", "nrt_index_sweep", "nrt_topk_rows_grid", "nrt_router",
-                "nrt_ep_count", "nrt_ep_dispatch", "nrt_ep_combine", "nrt_ag_push"), buffer_table(0, True, False)),
+               ("nrt_wide_gemm_launch", "nrt_stack_gemm", "nrt_gemm_launch", "nrt_attn_post", "nrt_attn_group", "nrt_attn_rows",
+                "nrt_index_sweep", "nrt_topk_rows_grid", "nrt_topk_rows", "nrt_router", "nrt_ep_count", "nrt_ep_dispatch",
+                "nrt_ep_combine", "nrt_ag_push"), buffer_table(0, True, False)),
 )}
 
 

@@ -340,6 +340,26 @@ def test_kernel_variants_fail_closed():
     assert len(V.require_entries(lib, V.STEP_VARIANTS + V.PREFILL_VARIANTS)) == len(V.STEP_VARIANTS + V.PREFILL_VARIANTS)
 
 
+def test_native_prefill_launches_only_checked_entries():
+    """Every launcher with an argument struct that the native prefill's modules reach through the bindings is among those that the
+    engine requires from the library before a request."""
+    import inspect
+    import re
+    from naivert_b200.ops import kernels as K, stack_kernels as S, variants as V
+    from naivert_b200.prefill import ep_moe, native
+    from naivert_b200.runtime.modes import MODES
+    bindings, launched = {"K": K, "S": S}, set()
+    for module in (native, ep_moe):
+        for n in ast.walk(ast.parse(inspect.getsource(module))):
+            if isinstance(n, ast.Attribute) and isinstance(n.value, ast.Name) and n.value.id in bindings:
+                f = getattr(bindings[n.value.id], n.attr)
+                if inspect.isfunction(f) and "args" in inspect.signature(f).parameters:
+                    launched |= {e for e in re.findall(r"\.(nrt_\w+)\(", inspect.getsource(f)) if not e.endswith("_args_size")}
+    launched |= {"nrt_topk_rows", "nrt_topk_rows_grid"}          # (scalar arguments, recorded with the indexer's struct)
+    assert {"nrt_stack_gemm", "nrt_wide_gemm_launch", "nrt_ep_count"} <= launched <= set(V.PREFILL_VARIANTS)
+    assert set(MODES["prefill_native"].entries) == set(V.PREFILL_VARIANTS)
+
+
 def test_decode_modes_and_call_plans():
     import re
     from naivert_b200.models.registry import resolve_model
