@@ -337,9 +337,11 @@ __global__ void __launch_bounds__(256) ep_combine_kernel(const EpCombineArgs a) 
   const uint32_t tag = (*a.epoch) * 1024u + (uint32_t)a.call + 1u;
   const int words = a.hidden / 2;
   const uint64_t deadline = globaltimer() + a.timeout_ns;
-  // Two words (each complete in itself) per load; those that have not arrived are waited for in turn.  2048 rows of 8 choices x 4096: 79 us,
-  // 100 us word by word, 112 us with the words of eight choices at once.
-  const int pairs = words & 1 ? 0 : words / 2;
+  // Two words (each complete in itself) per load where rows lie so; those that have not arrived are waited for in turn.  2048 rows of 8
+  // choices x 4096: 79 us, 100 us word by word, 112 us with the words of eight choices at once.
+  const bool pairs_lie = (words & 1) == 0 && (reinterpret_cast<uintptr_t>(a.slots) & 15) == 0 &&
+                         ((reinterpret_cast<uintptr_t>(a.resid) | reinterpret_cast<uintptr_t>(a.out)) & 7) == 0;
+  const int pairs = pairs_lie ? words / 2 : 0;
   for (int w = threadIdx.x; w < pairs; w += 256) {
     const uint2 r = reinterpret_cast<const uint2*>(a.resid + (size_t)t * a.hidden)[w];
     float s[4] = {bf16_lo(r.x), bf16_hi(r.x), bf16_lo(r.y), bf16_hi(r.y)};

@@ -537,6 +537,36 @@ def test_expert_lists(rows, top, experts, segment):
         fab.close()
 
 
+@pytest.mark.parametrize("hidden", [256, 258, 260, 1024])
+def test_combine_of_rows_at_any_address(hidden):
+    """Rows that come back from their experts, added to residual rows: pairs of words where they lie so, else (an odd number of words, rows that
+    begin between two pairs) word by word, with the same bits; one rounding to bf16 from the same sum in 64 bits."""
+    from naivert_b200.ops import kernels as K
+    rows, top, epoch, call = 5, 3, 7, 901
+    g = torch.Generator().manual_seed(hidden)
+    y = torch.randn(rows, top, hidden, generator=g).bfloat16()
+    p, resid = torch.rand(rows, top, generator=g), torch.randn(rows, hidden, generator=g).bfloat16()
+    words = y.view(torch.int32).long() & 0xffffffff | (epoch * 1024 + call + 1) << 32
+    want = resid.double() + (p[:, :, None].double() * y.double()).sum(1)
+    size = resid.double().abs() + (p[:, :, None] * y).double().abs().sum(1)
+    got = []
+    for first, before in ((0, 0), (0, 2), (2, 0), (2, 2), (1, 0)):           # slots (8 bytes), bf16 values in front of the rows
+        slots = torch.zeros(words.numel() + first, dtype=torch.int64, device="cuda")
+        slots[first:].copy_(words.flatten())
+        x, out = (torch.zeros(rows * hidden + before, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        x[before:].copy_(resid.flatten())
+        dp, de, st = p.cuda(), torch.tensor([epoch], dtype=torch.int32, device="cuda"), torch.zeros(64, dtype=torch.int32, device="cuda")
+        c = K.EpCombineArgs()
+        c.slots, c.topk_p, c.resid, c.out = slots[first:].data_ptr(), dp.data_ptr(), x[before:].data_ptr(), out[before:].data_ptr()
+        c.epoch, c.status, c.tokens, c.top_k, c.hidden, c.call, c.timeout_ns = de.data_ptr(), st.data_ptr(), rows, top, hidden, call, 10 ** 9
+        K.ep_combine(c, pdl=False)
+        torch.cuda.synchronize()
+        assert int(st.abs().max()) == 0
+        got.append(out[before:].view(rows, hidden).cpu())
+    assert all(torch.equal(got[0], o) for o in got[1:])
+    assert bool(((got[0].double() - want).abs() <= 2.0 ** -8 * want.abs() + top * 2.0 ** -23 * size).all())
+
+
 @pytest.mark.parametrize("experts,top,count,keep", [(24, 3, 4, 2), (256, 8, 8, 4), (30, 5, 10, 4), (9, 2, 1, 1), (32, 1, 32, 1)])
 def test_group_limited_choice(experts, top, count, keep):
     """Choices and weights of the routing kernel, with negative choice scores and exact ties."""
