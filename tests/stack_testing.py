@@ -1,4 +1,6 @@
 """Helpers of the layer-stack tests: tokens, portions, row-wise errors against a plain implementation."""
+import ctypes
+
 import torch
 
 TOL = {"fp32": 2e-4, "bf16": 4e-2}
@@ -24,3 +26,33 @@ def feed(eng, toks, sizes):
         out.append(eng.extend(toks[at:at + n], list(range(n))))
         at, i = at + n, i + 1
     return torch.cat(out)
+
+
+SET_EVERY_TIME = {"StackGemmArgs": ("rows", "item_rows", "max_items"), "EpArgs": ("tokens", "max_items", "item_rows"),
+                  "LatentAttnArgs": ("rows", "kv0", "kv_rows", "first", "last", "v_ld")}
+
+
+def watch_kept_blocks(pf):
+    """From now on every argument block that a prompt takes from the kept ones is compared with one built anew, but for what is set every
+    time; returns the counts of blocks made and compared."""
+    met, keep = {"made": 0, "checked": 0}, pf.kept
+
+    def parts(a):
+        if isinstance(a, dict):
+            return [(k, None if t is None else (t.data_ptr(), t.shape, t.dtype)) for k, t in a.items()]
+        out = []
+        for s in a if isinstance(a, tuple) else (a,):
+            if isinstance(s, ctypes.Structure):
+                raw, free = bytes(s), SET_EVERY_TIME.get(type(s).__name__, ("rows",))
+                out += [(f[0], raw[getattr(type(s), f[0]).offset:][:getattr(type(s), f[0]).size]) for f in s._fields_ if f[0] not in free]
+        return out
+
+    def kept(key, build):
+        met["made"] += key not in pf._kept
+        a, fresh = keep(key, build), build()
+        met["checked"] += 1
+        assert parts(a) == parts(fresh) and parts(a), key
+        return a
+
+    pf.kept = kept
+    return met

@@ -231,3 +231,24 @@ def test_prompt_spans_equal_single_chunks(chunk, most, n):
     single, spans = run(1), run(most)
     assert any(c.any() for c in single)
     assert all(torch.equal(a, b) for a, b in zip(single, spans))
+
+
+def test_warming_takes_what_later_prompts_need():
+    """After the default warming no prompt allocates span buffers, and what warming left in the caches is overwritten."""
+    from naivert_b200.models.naive_n0p5 import small_w8a8_spec
+    from naivert_b200.runtime.engine import Engine
+    spec = small_w8a8_spec(4)
+    prompt = torch.randint(0, spec.vocab - 16, (701,), generator=torch.Generator().manual_seed(9))
+    caches = []
+    for warm in (False, True):
+        eng = Engine.build(spec, capacity=1024, seed=0, prefill_chunk=64)
+        if warm:
+            eng.prefill.warm_chunks()
+            assert eng.prefill.span == 1024
+        held = torch.cuda.memory_allocated()
+        assert eng.prefill.run(prompt) == 688
+        torch.cuda.synchronize()
+        eng.prefill.check()
+        assert (torch.cuda.memory_allocated() == held) == warm
+        caches.append([d[k][:688].clone() for d in eng.target.layers for k in ("k", "v") if d["k"].shape[0] == 1024])
+    assert caches[0] and all(torch.equal(a, b) for a, b in zip(*caches))

@@ -17,7 +17,7 @@ import pytest
 import torch
 
 import tumatar_oracle as oracle
-from stack_testing import TOL, error, feed, tokens
+from stack_testing import TOL, error, feed, tokens, watch_kept_blocks
 
 pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -481,6 +481,22 @@ def test_products_against_torch(rows):
 
 
 @pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+def test_argument_blocks_that_stay_equal_fresh_ones(dtype):
+    """Whatever hangs on a kept block's launch is in its key: prompts of several lengths, spans and chunks meet no block of another caller."""
+    cfg = CASES["mixed"]
+    toks = tokens(cfg, 400, 8)
+    eng = engine(cfg, weights(cfg, 3), dtype, chunk=64, kv_block=128)
+    try:
+        met = watch_kept_blocks(eng.prefill)
+        for n in (1, 40, 64, 400, 65, 400):
+            eng.reset()
+            eng.extend(toks[:n], [0, n - 1])
+        assert met["checked"] > met["made"] > 40
+    finally:
+        eng.close()
+
+
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
 def test_wanted_rows_and_repeated_prompts(dtype):
     """Rows that follow one another are read where they lie, others gathered: the same logits.  Argument blocks that stay from an earlier
     prompt of another length, or from before a longer span's buffers, leave nothing behind, and neither do launches that begin early."""
@@ -503,17 +519,13 @@ def test_wanted_rows_and_repeated_prompts(dtype):
         fresh.close()
 
 
-@pytest.mark.parametrize("rows,top,experts,segment", [(1, 1, 3, 64), (5, 2, 7, 16), (32, 1, 256, 16), (301, 3, 24, 64), (333, 4, 300, 16), (1000, 8, 8, 128),
-                                                      (8192, 8, 256, 128)])
-def test_expert_lists(rows, top, experts, segment):
-    """Rows, segments and work list of the sorted choices against the host's restatement: few and many pairs, one expert for all, lists
-    beyond what the warps' counters hold."""
+def check_expert_lists(ids, experts, segment, pdl=False):
+    """Rows, segments and work list that the device makes of the choices (one rank's) against the host's restatement."""
     from naivert_b200.ops import kernels as K
     from naivert_b200.ops import stack_kernels as S
     from naivert_b200.parallel.fabric import Fabric
     from naivert_b200.prefill.ep_moe import ep_layout_reference
-    g = torch.Generator().manual_seed(rows)
-    ids = torch.stack([torch.randperm(experts, generator=g)[:top] for _ in range(rows)]).int()
+    rows, top = ids.shape
     fab = Fabric(0, 1, 128, device=torch.device("cuda", 0))
     try:
         n, items = rows * top, rows * top // segment + min(rows * top, experts)
@@ -525,7 +537,7 @@ def test_expert_lists(rows, top, experts, segment):
         for k, t in out.items():
             setattr(a, k, t.data_ptr())
         a.max_items, a.item_rows, a.x_args = items, segment, fab.xchg_args()
-        S.moe_count(a)
+        S.moe_count(a, pdl)
         torch.cuda.synchronize()
         want = ep_layout_reference([ids], experts, segment)
         assert torch.equal(out["slot_of"].cpu().view(rows, top), want["slot"][0].int()) and out["seg_rows"].tolist() == want["seg_rows"][0]
@@ -535,6 +547,27 @@ def test_expert_lists(rows, top, experts, segment):
         assert out["item_live"].tolist()[:used] == left
     finally:
         fab.close()
+
+
+@pytest.mark.parametrize("rows,top,experts,segment", [(1, 1, 3, 64), (5, 2, 7, 16), (32, 1, 256, 16), (301, 3, 24, 64), (333, 4, 300, 16), (1000, 8, 8, 128),
+                                                      (8192, 8, 256, 128)])
+def test_expert_lists(rows, top, experts, segment):
+    """Few and many pairs, every expert for every token, lists beyond what the warps' counters hold."""
+    g = torch.Generator().manual_seed(rows)
+    check_expert_lists(torch.stack([torch.randperm(experts, generator=g)[:top] for _ in range(rows)]).int(), experts, segment)
+
+
+@pytest.mark.parametrize("pdl", [False, True])
+@pytest.mark.parametrize("rows,experts,segment,chosen,share", [(8192, 256, 128, [255], 1), (8192, 256, 128, [255, 0, 17, 18, 19, 128, 64, 254], 1), (8191, 256, 64, [0, 3], 1),
+                                                               (2048, 256, 64, [254, 255], 0.9), (700, 300, 16, [299], 0.97), (33, 64, 16, [63, 1], 1)])
+def test_expert_lists_of_skewed_choices(rows, experts, segment, chosen, share, pdl):
+    """The same experts for all tokens, or for most of them, beside experts that nobody chose: whole warps that vote alike, counters up to the
+    number of tokens, the last expert, empty segments."""
+    g = torch.Generator().manual_seed(rows)
+    ids = torch.tensor(chosen, dtype=torch.int32).repeat(rows, 1)
+    rare = torch.rand(rows, generator=g) >= share
+    ids[rare, 0] = torch.randint(20, 60, (int(rare.sum()),), generator=g, dtype=torch.int32)
+    check_expert_lists(ids, experts, segment, pdl)
 
 
 @pytest.mark.parametrize("hidden", [256, 258, 260, 1024])

@@ -15,7 +15,7 @@ import pytest
 import torch
 
 import zuzupel_oracle as oracle
-from stack_testing import TOL, error, feed, tokens
+from stack_testing import TOL, error, feed, tokens, watch_kept_blocks
 
 pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -193,6 +193,22 @@ def test_launches_that_begin_early_leave_the_same_bits(name, dtype):
     finally:
         early.close()
         plain.close()
+
+
+@pytest.mark.parametrize("name,dtype", [("mixed", "fp32"), ("mixed", "bf16"), ("shared", "bf16"), ("shared_ahead", "fp32")])
+def test_argument_blocks_that_stay_equal_fresh_ones(name, dtype):
+    """Layers that share weights included."""
+    cfg = CASES[name]
+    toks = tokens(cfg, 300, 8)
+    eng = engine(cfg, weights(cfg, 3), dtype, chunk=64)
+    try:
+        met = watch_kept_blocks(eng.prefill)
+        for n in (1, 40, 300, 65):
+            eng.reset()
+            eng.extend(toks[:n], [0, n - 1])
+        assert met["checked"] > met["made"] >= 15
+    finally:
+        eng.close()
 
 
 def test_stream_after_every_layer_run():
