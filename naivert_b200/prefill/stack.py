@@ -11,6 +11,7 @@ the step continues from.  Where the chunks are too short to fill the routed expe
 """
 from __future__ import annotations
 
+from bisect import bisect_left
 from contextlib import contextmanager, nullcontext
 from functools import lru_cache
 from typing import Callable, Dict, List, Optional, Sequence, Tuple
@@ -373,7 +374,6 @@ class StackPrefill:
             return None
         self._rows(R, pre=t.g_final, **wait)
         out = torch.empty(len(want), s.vocab, dtype=torch.float32, device=self.dev)
-        want = list(want)
         straight = want == list(range(want[0], want[0] + len(want)))             # rows that follow one another
         idx = None if straight else torch.as_tensor(want, dtype=torch.long, device=self.dev)
         for i in range(0, len(want), self.head_rows):
@@ -392,7 +392,7 @@ class StackPrefill:
         if not 0 <= pos0 <= pos0 + n <= self.t.capacity:
             raise ValueError(f"rows [{pos0}, {pos0 + n}) outside the cache capacity {self.t.capacity}")
         out: List[torch.Tensor] = []
-        order = [w for w in want]
+        order = list(want)
         if order != sorted(order):
             raise ValueError("wanted rows must ascend")
         self._fit_span(n)
@@ -400,7 +400,8 @@ class StackPrefill:
             R = min(self.span, n - c0)
             self.tokens[:R].copy_(tokens[c0:c0 + R].to(torch.int32), non_blocking=True)
             seen: Optional[list] = None if trace is None else []
-            got = self._chunk(pos0 + c0, R, [int(w) - c0 for w in order if c0 <= w < c0 + R], seen)
+            rows = map(int, order[bisect_left(order, c0):bisect_left(order, c0 + R)])
+            got = self._chunk(pos0 + c0, R, [w - c0 for w in rows] if c0 else list(rows), seen)
             for i in range(0, R if seen else 0, self.C):
                 trace.extend(x[i:i + self.C] for x in seen)
             if got is not None:
