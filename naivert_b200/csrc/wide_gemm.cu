@@ -1,18 +1,19 @@
 // Chunk GEMM for prefill: the same swapped-operand tcgen05 engine as gemm.cuh with 64 token columns per tile.
 //
 // The 16-column engine re-reads every 16 KiB weight tile from L2 once per 16 tokens, which bounds a
-// prefill chunk by L2 -> SM bandwidth (~18 KiB per 0.5 MFLOP).  Here one CTA owns 128 output features x
-// 64 token rows of one work item (grid.y = item; an item is 64 consecutive rows of the token operand that
-// share one weight group: a row group of a prefill chunk, or a padded expert segment of the expert-parallel
-// receive buffer), so a weight tile feeds four times the math.
+// prefill chunk by L2 -> SM bandwidth (~18 KiB per 0.5 MFLOP).  Here a tile is 128 output features x
+// 64 token rows of one work item (64 consecutive rows of the token operand that share one weight group: a row
+// group of a prefill chunk, or a padded expert segment of the expert-parallel receive buffer), so a weight
+// tile feeds four times the math; one CTA per SM walks the tiles.
 //   warp 0     : TMA producer (weights 128 x 128 B, tokens 64 x 128 B, 128-byte swizzle, no multicast)
 //   warp 1     : TMEM allocator + UMMA issuer (M = 128, N = 64; kind::f8f6f4 or kind::f16)
 //   warps 2..17: epilogue; thread = output feature x a quarter (16) of the token columns: four warps per TMEM lane
 //                quadrant, so that a thread has the registers to fetch the next accumulator while it adds the last one
 // Block-scaled e4m3: one fresh TMEM accumulator per 128-wide K block (a ring of pairs), scaled by weight-block x
 // activation-block scale and promoted in fp32 registers in ascending K order (the same arithmetic as the
-// 16-column engine, so both produce identical values).  Activation scales of the item are staged in shared
-// memory once (after the first accumulator is ready, i.e. after the producer has seen the rows arrive).
+// 16-column engine, so both produce identical values).  Scales of the item's rows times those of the weights are
+// put into shared memory once per tile (after the first accumulator is ready, i.e. after the producer has seen
+// the rows arrive).
 // Epilogues: fp32 / bf16 store, SiLU(gate) * up with e4m3 re-quantisation, and the expert-parallel return
 // (tagged bf16 pairs into the token owner's combine slots in peer memory).
 //
@@ -447,6 +448,7 @@ extern "C" int nrt_wide_gemm_launch(int variant, const void* tmA0, const void* t
     NRT_WCASE(1, 1, kEpiSiluQuant)
     NRT_WCASE(1, 0, kEpiReturn)
     NRT_WCASE(1, 0, kEpiStoreBF16)
+    // bf16 stores: for callers of this entry (64-row items with a row offset each); prompts multiply bf16 rows in stack_gemm.cu
     NRT_WCASE(0, 0, kEpiStoreF32)
     NRT_WCASE(0, 0, kEpiStoreBF16)
     default:

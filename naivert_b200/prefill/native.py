@@ -3,7 +3,7 @@
 A chunk of ``R`` rows (a multiple of 16, up to ``chunk``) is processed layer by layer with the same
 kernels and caches as the decode/verify step, launched over row groups:
 
-    RMSNorm -> q/k/v(/indexer) projection (tcgen05, grid.y = 16-row groups) -> RoPE / KV append /
+    RMSNorm -> q/k/v(/indexer) projection (tcgen05, tiles of up to 256 rows) -> RoPE / KV append /
     indexer keys -> [tcgen05 indexer sweep per row group -> exact top-k per row] -> row attention ->
     o_proj partials -> tensor-parallel reduction -> MoE -> draft feature ingest at the tap layers
 
